@@ -502,7 +502,7 @@ Deck1DArgs deck1d_args(const CellArgs &ca) {
     Deck1DArgs a{};
     a.nx = ca.nx; a.nc = ca.nc; a.K = ca.K;
     a.bc[0] = ca.bc[0]; a.bc[1] = ca.bc[1];
-    a.dx = ca.dx; a.sa = ca.sa; a.fleck = ca.fleck; a.ss = ca.ss; a.scales = ca.scales;
+    a.tab = ca.tab; a.scales = ca.scales;
     a.dep_acc = ca.dep_acc; a.rad_acc = ca.rad_acc; a.lost_acc = ca.lost_acc;
     a.c = ca.c; a.ds = ca.ds;
     a.seg_cap = ca.seg_cap;
@@ -735,6 +735,15 @@ int imc_create(const ImcDeck *d, ImcHandle **out) {
     if ((rc = upload<long long>(h, &ca.slot_n, nullptr, h->nslots))) return bail(rc);
     if ((rc = upload<long long>(h, &ca.slot_off, nullptr, h->nslots))) return bail(rc);
     if ((rc = upload<double>(h, &ca.slot_q, nullptr, h->nslots))) return bail(rc);
+    ca.prec = h->prec;
+    {
+        // 32-byte rows in 1D, 16-byte rows in 2D (imc_transport.cuh)
+        char *tp;
+        if ((rc = upload<char>(h, &tp, nullptr, (size_t)(d->geometry == IMC_GEOM_1D ? 32 : 16) * nc))) return bail(rc);
+        ca.tab = tp;
+        if (d->geometry == IMC_GEOM_2D && h->prec == IMC_FP64)
+            if ((rc = upload<double>(h, &ca.tab_rs, nullptr, nc))) return bail(rc);
+    }
     ca.nblk_slot = (h->nslots + kCellThreads - 1) / kCellThreads;
     ca.nblk_cell = (nc + kCellThreads - 1) / kCellThreads;
     if ((rc = upload<double>(h, &ca.part_src, nullptr, (size_t)ca.nblk_slot * 12))) return bail(rc);
@@ -751,7 +760,7 @@ int imc_create(const ImcDeck *d, ImcHandle **out) {
     ca.seed = d->seed;
     double dxmin = *std::min_element(d->dx, d->dx + h->nx);
     double dymin = d->geometry == IMC_GEOM_2D ? *std::min_element(d->dy, d->dy + h->ny) : 1.0;
-    ca.vol_min = dxmin * dymin;
+    ca.vol_min = h->prec == IMC_FP64 ? 1.0 : dxmin * dymin;  // least divisor of a deposit (FP64: energies)
     ca.scale_min = *std::min_element(d->energyscales, d->energyscales + K);
     ca.t_end = d->t_end; ca.dtmax = d->dtmax; ca.kfac = d->k;
     // particle buffers
@@ -839,6 +848,7 @@ int imc_sourcing(ImcHandle *h) {
 int imc_transport(ImcHandle *h) {
     if (!h) return IMC_ERR_INVALID_ARG;
     if (h->stage != Stage::Sourced) launch_prepare_transport(h->ca, h->d_sc, h->stream);
+    launch_table(h->ca, h->stream);
     if (h->timing) CK(h, cudaEventRecord(h->ev[0], h->stream));
     run_transport(h, pair(h), h->stream);
     CKL(h);

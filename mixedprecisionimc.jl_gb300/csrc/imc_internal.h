@@ -94,6 +94,11 @@ struct CellArgs {
     unsigned long long seed;
     double vol_min, scale_min;
     double t_end, dtmax, kfac;
+    // the transport's per-cell table (imc_transport.cuh: Tab1 rows, or Tab2
+    // rows and, FP64 in 2D, 1/seff), written by k_update
+    int prec;
+    void *tab;
+    double *tab_rs;
     // learned thick-cell surrogate: tensor-core image of the network
     // (imc_surrogate.cuh), or null for analog transport everywhere
     const uint4 *surr_image;
@@ -122,6 +127,9 @@ struct DevStats {
 
 // launchers (imc_kernels.cu / imc_transport.cu); all asynchronous on `st`
 void launch_update(const CellArgs &ca, Scalars *sc, cudaStream_t st);
+// the transport's per-cell table from the cell fields as they are now (the
+// stage-by-stage entry point: they may have been set since the update)
+void launch_table(const CellArgs &ca, cudaStream_t st);
 void launch_source(const CellArgs &ca, Scalars *sc, int prec, PBufPair bufs, int grid, cudaStream_t st);
 struct TransportShape {
     bool smem_tally;  // block-private tallies in shared memory
@@ -191,8 +199,7 @@ const void *transport_kernel_ptr(const CellArgs &ca, int prec);
 // single deck's kernel parameters, they cost no registers in the history loop.
 struct Deck1DArgs {
     int nx, nc, K, bc[2];
-    const double *dx;
-    double *sa, *fleck, *ss;
+    const void *tab;
     const double *scales;
     long long *dep_acc, *rad_acc, *lost_acc;
     double c, ds;

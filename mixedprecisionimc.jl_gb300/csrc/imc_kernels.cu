@@ -19,6 +19,7 @@
 #include "imc_device.cuh"
 #include "imc_internal.h"
 #include "imc_state.cuh"
+#include "imc_transport.cuh"
 
 namespace imc {
 
@@ -75,15 +76,30 @@ __global__ void __launch_bounds__(kCellThreads) k_update(CellArgs ca, Scalars *s
     double sa = ca.sa_val[i] * (psa == 0.0 ? 1.0 : pow(Tc, psa));
     if (ca.marshak) sa = ca.sa_val[i] / Tc / Tc / Tc;
     ca.sa[i] = sa;
-    ca.ss[i] = ca.ss_val[i] * (pss == 0.0 ? 1.0 : pow(Tc, pss));
+    const double ss = ca.ss_val[i] * (pss == 0.0 ? 1.0 : pow(Tc, pss));
+    ca.ss[i] = ss;
     double v[6] = {ca.ds, ca.alpha, beta, c, dt, sa};
     int j;
     double prod = sorter_n<0, 6>(v, one, 1, &j);
-    ca.fleck[i] = 1.0 / (1.0 + prod);
+    const double f = 1.0 / (1.0 + prod);
+    ca.fleck[i] = f;
+    if (ca.prec == 0) store_tab<double>(ca, i, sa, f, ss);
+    else store_tab<float>(ca, i, sa, f, ss);
+}
+
+__global__ void __launch_bounds__(kCellThreads) k_table(CellArgs ca) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= ca.nc) return;
+    if (ca.prec == 0) store_tab<double>(ca, i, ca.sa[i], ca.fleck[i], ca.ss[i]);
+    else store_tab<float>(ca, i, ca.sa[i], ca.fleck[i], ca.ss[i]);
 }
 
 void launch_update(const CellArgs &ca, Scalars *sc, cudaStream_t st) {
     k_update<<<ca.nblk_cell, kCellThreads, 0, st>>>(ca, sc);
+}
+
+void launch_table(const CellArgs &ca, cudaStream_t st) {
+    k_table<<<ca.nblk_cell, kCellThreads, 0, st>>>(ca);
 }
 
 // ---------------------------------------------------------------- sourcing
@@ -785,7 +801,9 @@ __device__ __forceinline__ void finalize_cell(const CellArgs &ca, Scalars *sc, i
             const size_t idx = (size_t)k * nc + i;
             const int se = scale_exp(ca.scales[k]);
             long long *d = ca.dep_acc + 3 * idx;
-            ca.energydep[idx] = fix_value(d, b_dep + se);
+            // FP64 histories deposit energies, FP32 ones densities
+            const double dep = fix_value(d, b_dep + se);
+            ca.energydep[idx] = ca.prec == 0 ? dep / vol : dep;
             d[0] = d[1] = d[2] = 0;
             long long *g = ca.rad_acc + 3 * idx;
             r += fix_value(g, b_rad + se) / (vol * ca.scales[k]);

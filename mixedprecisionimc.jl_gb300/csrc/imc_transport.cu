@@ -55,8 +55,9 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
     Tab1<T> *tab = reinterpret_cast<Tab1<T> *>(smem_raw);
     const int N = ca.nx;
     const T ds = (T)ca.ds, c = (T)ca.c;
-    const bool ds_one = ds == (T)1;
+    const bool ds_one = ds == (T)1, c_one = c == (T)1;
     const T rdsc = (T)1 / (ds * c);
+    const T rds = sizeof(T) == 8 ? (T)1 / ds : (T)0, rc = sizeof(T) == 8 ? (T)1 / c : (T)0;
     long long *dep_acc = ca.dep_acc, *rad_acc = ca.rad_acc;
     if (SMT) {
         dep_acc = tally_smem(smem_raw, table_bytes(ca, sizeof(T)));
@@ -66,7 +67,7 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
     static_assert(TM != kTallySharedDep || MODE == kModePlain, "deposition-only tallies: plain pass only");
     const T endsteptime = (T)sc->dt;
     float *gate = reinterpret_cast<float *>(smem_raw + analog1d_smem(ca, sizeof(T), RAD_SMT, false));
-    for (int i = threadIdx.x; i < N; i += blockDim.x) tab[i] = make_tab1<T>(ca.sa[i], ca.fleck[i], ca.ss[i], ca.dx[i], ds);
+    load_tab(tab, ca.tab, N);
     __shared__ int s_sexp[16];
     load_scale_exps(ca, s_sexp);
     if constexpr (kPause) fill_gate<T>(ca, gate, ds, c, endsteptime);
@@ -110,7 +111,7 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
         acc_cell = cell;
         prv_cell = -1;
         seg = 0;
-        rmu = (T)1 / mu;  // FP32: the face distance as a product (reset at each new direction)
+        rmu = (T)1 / mu;  // the face distance as a product (reset at each new direction)
     };
     // one entry of the list (or of the resume queue): false if it holds no history
     auto load = [&](long long e, int &cs_now, T &lt, T &lx, T &lmu, T &lE, T &lE0, long long &li, int &lcs) -> bool {
@@ -169,29 +170,67 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
             end = 1;
         } else {
             const Tab1<T> ce = tab[cell];
-            T dist_b;
-            if constexpr (sizeof(T) == 4) dist_b = mu > (T)0 ? (ce.dxs - x) * rmu : m_abs(x * rmu);
-            else dist_b = mu > (T)0 ? (ce.dxs - x) / mu : m_abs(x / mu);
+            T dist_b, dist_cen, dist;
+            bool at_b, at_col, at_cen, odd = false;  // odd (FP64): a distance below +0 or not a number
             const T dist_col = M::flight(rs, ce);
-            const T dist_cen = c * (endsteptime - t) * ds;
-            const T dist = jmin(jmin(dist_b, dist_col), dist_cen);
-            if (dist != dist) {
+            if constexpr (sizeof(T) == 4) {
+                dist_b = mu > (T)0 ? (ce.dxs - x) * rmu : m_abs(x * rmu);
+                dist_cen = c * (endsteptime - t) * ds;
+                dist = jmin(jmin(dist_b, dist_col), dist_cen);
+                at_b = dist == dist_b;
+                at_col = dist == dist_col;
+                at_cen = dist == dist_cen;
+            } else {
+                const bool fwd = pos64(mu);
+                dist_b = m64::div_r(fwd ? ce.dxs - x : x, mu, rmu);
+                if (!fwd) dist_b = m_abs(dist_b);
+                dist_cen = endsteptime - t;
+                if (!c_one) dist_cen = c * dist_cen;
+                if (!ds_one) dist_cen = dist_cen * ds;
+                odd = !(plain64(dist_b) && plain64(dist_col) && plain64(dist_cen));
+                if (!odd) {
+                    dist = min64(min64(dist_b, dist_col), dist_cen);
+                    at_b = m64::bits(dist) == m64::bits(dist_b);
+                    at_col = m64::bits(dist) == m64::bits(dist_col);
+                    at_cen = m64::bits(dist) == m64::bits(dist_cen);
+                } else {
+                    dist_b = mu > (T)0 ? (ce.dxs - x) / mu : m_abs(x / mu);
+                    dist = jmin(jmin(dist_b, dist_col), dist_cen);
+                    at_b = dist == dist_b;
+                    at_col = dist == dist_col;
+                    at_cen = dist == dist_cen;
+                }
+            }
+            if (odd ? dist != dist : sizeof(T) == 4 && dist != dist) {
                 flags |= 1u;
                 end = 1;
             } else {
-                T dep;
-                const T newenergy = M::attenuate(E, ce, dist, &dep);
+                T dep, newenergy;
+                bool dead;
+                if constexpr (sizeof(T) == 4) {
+                    newenergy = M::attenuate(E, ce, dist, &dep);
+                    dead = newenergy <= minenergy;
+                } else {
+                    newenergy = M::attenuate(E, ce.saf, dist, odd, &dep);
+                    dead = le64(newenergy, minenergy);
+                }
                 enter_cell();
-                if (newenergy <= minenergy) {
+                if (dead) {
                     nadd(acc_s, acc_c, M::all_in(E, ce));
                     end = 1;
                 } else {
                     nadd(acc_s, acc_c, dep);
-                    x += mu * dist;
-                    if constexpr (sizeof(T) == 4) t += dist * rdsc;
-                    else t += (ds_one ? dist : dist / ds) / c;
+                    if constexpr (sizeof(T) == 4) {
+                        x += mu * dist;
+                        t += dist * rdsc;
+                    } else {
+                        x = fma(mu, dist, x);
+                        T dt_seg = ds_one ? dist : m64::div_r(dist, ds, rds);
+                        if (!c_one) dt_seg = m64::div_r(dt_seg, c, rc);
+                        t += dt_seg;
+                    }
                     E = newenergy;
-                    if (dist == dist_b) {
+                    if (at_b) {
                         if (mu > (T)0) {
                             if (cell == N - 1) {
                                 if (reflect_r) {
@@ -220,17 +259,17 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
                             }
                         }
                     }
-                    if (!end && dist == dist_col) {
+                    if (!end && at_col) {
                         // mu = 1 - 2*rand, redrawn while zero (src/imc_transport.jl:178-181);
                         // a zero needs rand == 0.5 exactly, so 64 redraws never run out
                         mu = (T)0;
-                        for (int r = 0; r < 64 && mu == (T)0; ++r) mu = (T)1 - (T)2 * Rand<T>::u(rs);
+                        for (int r = 0; r < 64 && mu == (T)0; ++r) mu = Rand<T>::cosine(rs);
                         if (mu == (T)0) mu = (T)1;
                         rmu = (T)1 / mu;
                     }
                     // census: t = 0 and the state written back by finish()
                     // (src/imc_transport.jl:185-193)
-                    if (!end && dist == dist_cen) end = 2;
+                    if (!end && at_cen) end = 2;
                 }
             }
         }
@@ -457,25 +496,16 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
     Face<T> *fx = reinterpret_cast<Face<T> *>(tab + nc);
     Face<T> *fy = fx + NX;
     const T ds = (T)ca.ds, c = (T)ca.c;
-    const bool ds_one = ds == (T)1;
+    const bool ds_one = ds == (T)1, c_one = c == (T)1;
     const T rdsc = (T)1 / (ds * c);
+    const T rds = sizeof(T) == 8 ? (T)1 / ds : (T)0, rc = sizeof(T) == 8 ? (T)1 / c : (T)0;
     long long *dep_acc = ca.dep_acc, *rad_acc = ca.rad_acc;
     if (SMT) {
         dep_acc = tally_smem(smem_raw, table_bytes(ca, sizeof(T)));
         if (RAD_SMT) rad_acc = dep_acc + 3 * (size_t)ca.K * ca.nc;
         for (int i = threadIdx.x; i < (RAD_SMT ? 6 : 3) * ca.K * ca.nc; i += blockDim.x) dep_acc[i] = 0;
     }
-    for (int i = threadIdx.x; i < nc; i += blockDim.x) {
-        T sa = (T)ca.sa[i], f = (T)ca.fleck[i], ss = (T)ca.ss[i];
-        Tab2<T> e;
-        e.saf = sa * f;
-        e.seff = sa * ((T)1 - f) + ss;
-        if constexpr (sizeof(T) == 4) {
-            e.rseff = 1.0f / e.seff;
-            e.rarea = 1.0f / ((float)ca.dx[i % NX] * (float)ca.dy[i / NX]);
-        }
-        tab[i] = e;
-    }
+    load_tab(tab, ca.tab, nc);
     for (int i = threadIdx.x; i < NX; i += blockDim.x) { fx[i].wT = (T)ca.dx[i]; fx[i].ws = fx[i].wT * ds; }
     for (int i = threadIdx.x; i < NY; i += blockDim.x) { fy[i].wT = (T)ca.dy[i]; fy[i].ws = fy[i].wT * ds; }
     __shared__ int s_sexp[16];
@@ -496,6 +526,7 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
     int cs = 0, xi = 0, yi = 0, k = 0, acc_cell = 0;
     T t = (T)0, xp = (T)0, yp = (T)0, vx = (T)0, vy = (T)0, E = (T)0, E0 = (T)0, minenergy = (T)0;
     T acc_s = (T)0, acc_c = (T)0;
+    T rvx = (T)0, rvy = (T)0;  // FP64: 1/vx, 1/vy
     long long seg = 0;
     Stream rs;
     auto start = [&]() {
@@ -509,6 +540,10 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
         acc_c = (T)0;
         acc_cell = cell0;
         seg = 0;
+        if constexpr (sizeof(T) == 8) {
+            rvx = 1.0 / vx;
+            rvy = 1.0 / vy;
+        }
     };
     auto load = [&](long long e, int &lcs, T &lt, T &lx, T &ly, T &lvx, T &lvy, T &lE, T &lE0) -> bool {
         if (!pb.alive[e]) return false;
@@ -534,60 +569,90 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
     // the warp runs converged once per history.
     auto segment = [&]() -> int {
         if (++seg > cap) { flags |= (1u << 2); return 1; }
-        const T dist_bx = vx > (T)0 ? m_abs((fx[xi].ws - xp) / vx) : m_abs(xp / vx);
-        const T dist_by = vy > (T)0 ? m_abs((fy[yi].ws - yp) / vy) : m_abs(yp / vy);
-        T dist_b;
-        if (dist_bx != dist_bx) dist_b = dist_by;
-        else if (dist_by != dist_by) dist_b = dist_bx;
-        else dist_b = jmin(dist_bx, dist_by);
         const int cell = xi + yi * NX;
         const Tab2<T> ce = tab[cell];
-        T dist_col, Edens, newenergy, dep;
+        T dist_bx, dist_by, dist_col, dist_cen, dist, Edens, newenergy, dep;
+        bool at_b, at_col, at_cen, dead;
+        // the distances by the reference's expressions and order
+        auto general = [&]() {
+            dist_bx = vx > (T)0 ? m_abs((fx[xi].ws - xp) / vx) : m_abs(xp / vx);
+            dist_by = vy > (T)0 ? m_abs((fy[yi].ws - yp) / vy) : m_abs(yp / vy);
+            T dist_b;
+            if (dist_bx != dist_bx) dist_b = dist_by;
+            else if (dist_by != dist_by) dist_b = dist_bx;
+            else dist_b = jmin(dist_bx, dist_by);
+            dist = jmin(jmin(dist_b, dist_col), dist_cen);
+            at_b = dist == dist_bx || dist == dist_by;
+            at_col = dist == dist_col;
+            at_cen = dist == dist_cen;
+        };
         if constexpr (sizeof(T) == 4) {
             // FP32: the 1D kernels' formulation (SegMath<float>)
             const float v = (float)((rs.next() >> 8) | 1u) * 0x1p-24f;
             dist_col = -__logf(v) * ce.rseff;
-        } else {
-            dist_col = Rand<T>::exp1(rs) / ce.seff;
-        }
-        const T dist_cen = c * (dtT - t) * ds;
-        const T dist = jmin(jmin(dist_b, dist_col), dist_cen);
-        if (dist != dist) { flags |= 1u; return 1; }
-        if constexpr (sizeof(T) == 4) {
+            dist_cen = c * (dtT - t) * ds;
+            general();
+            if (dist != dist) { flags |= 1u; return 1; }
             const float em1 = expm1_seg(-ce.saf * dist);
             newenergy = E + E * em1;
             Edens = E * ce.rarea;
             dep = -Edens * em1;
+            dead = newenergy <= minenergy;
         } else {
-            newenergy = E * m_exp(-ce.saf * dist);
-            Edens = (E / fx[xi].wT) / fy[yi].wT;
-            dep = -Edens * m_expm1(-ce.saf * dist);
+            // FP64: SegMath<double>'s formulation; the deposits are energies
+            dist_col = SegMath<double>::flight(rs, ce.seff, ca.tab_rs[cell]);
+            dist_cen = dtT - t;
+            if (!c_one) dist_cen = c * dist_cen;
+            if (!ds_one) dist_cen = dist_cen * ds;
+            dist_bx = m_abs(m64::div_r(pos64(vx) ? fx[xi].ws - xp : xp, vx, rvx));
+            dist_by = m_abs(m64::div_r(pos64(vy) ? fy[yi].ws - yp : yp, vy, rvy));
+            const bool odd = !(plain64(dist_bx) && plain64(dist_by) && plain64(dist_col) && plain64(dist_cen));
+            if (!odd) {
+                dist = min64(min64(dist_bx, dist_by), min64(dist_col, dist_cen));
+                const uint64_t b = m64::bits(dist);
+                at_b = b == m64::bits(dist_bx) || b == m64::bits(dist_by);
+                at_col = b == m64::bits(dist_col);
+                at_cen = b == m64::bits(dist_cen);
+            } else {
+                general();
+                if (dist != dist) { flags |= 1u; return 1; }
+            }
+            Edens = E;
+            newenergy = SegMath<double>::attenuate(E, ce.saf, dist, odd, &dep);
+            dead = le64(newenergy, minenergy);
         }
         if (cell != acc_cell) {
             flush_pair<T, SMT>(dep_acc, k * nc + acc_cell, acc_s, acc_c, b_dep + s_sexp[k], flags);
             acc_s = (T)0; acc_c = (T)0; acc_cell = cell;
         }
-        if (newenergy <= minenergy) {
+        if (dead) {
             nadd(acc_s, acc_c, Edens);
             return 1;
         }
         nadd(acc_s, acc_c, dep);
-        xp += dist * vx;
-        yp += dist * vy;
-        if constexpr (sizeof(T) == 4) t += dist * rdsc;
-        else t += (ds_one ? dist : dist / ds) / c;
+        if constexpr (sizeof(T) == 4) {
+            xp += dist * vx;
+            yp += dist * vy;
+            t += dist * rdsc;
+        } else {
+            xp = fma(dist, vx, xp);
+            yp = fma(dist, vy, yp);
+            T dt_seg = ds_one ? dist : m64::div_r(dist, ds, rds);
+            if (!c_one) dt_seg = m64::div_r(dt_seg, c, rc);
+            t += dt_seg;
+        }
         E = newenergy;
-        if (dist == dist_bx || dist == dist_by) {
+        if (at_b) {
             if (dist_bx < dist_by) {
                 if (vx > (T)0) {
                     if (xi == NX - 1) {
-                        if (refl_r) { vx = -vx; return 0; }
+                        if (refl_r) { vx = -vx; rvx = -rvx; return 0; }
                         return 4;
                     }
                     xi += 1; xp = (T)0;
                 } else {
                     if (xi == 0) {
-                        if (refl_l) { vx = -vx; return 0; }
+                        if (refl_l) { vx = -vx; rvx = -rvx; return 0; }
                         return 4;
                     }
                     xi -= 1; xp = fx[xi].ws;
@@ -595,13 +660,13 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
             } else {
                 if (vy > (T)0) {
                     if (yi == NY - 1) {
-                        if (refl_t) { vy = -vy; return 0; }
+                        if (refl_t) { vy = -vy; rvy = -rvy; return 0; }
                         return 4;
                     }
                     yi += 1; yp = (T)0;
                 } else {
                     if (yi == 0) {
-                        if (refl_b) { vy = -vy; return 0; }
+                        if (refl_b) { vy = -vy; rvy = -rvy; return 0; }
                         return 4;
                     }
                     yi -= 1; yp = fy[yi].ws;
@@ -609,7 +674,7 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
             }
             return 0;
         }
-        if (dist == dist_col) {
+        if (at_col) {
             // isotropic re-emission: angle 2*pi*rand in Float64, rounded to T
             // (binary32: two_pi_u24, the same value without FP64; the
             // hardware sine and cosine)
@@ -617,10 +682,14 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
             if constexpr (sizeof(T) == 4) ang = two_pi_u24(rs.next() >> 8);
             else ang = (T)(6.283185307179586 * (double)Rand<T>::u(rs));
             if constexpr (sizeof(T) == 4) __sincosf(ang, &vy, &vx);
-            else m_sincos(ang, &vy, &vx);
+            else {
+                m_sincos(ang, &vy, &vx);
+                rvx = 1.0 / vx;
+                rvy = 1.0 / vy;
+            }
         }
         // census: t = 0 and the state written back by finish()
-        if (dist == dist_cen) return 2;
+        if (at_cen) return 2;
         return 0;
     };
     auto finish = [&](int end) {

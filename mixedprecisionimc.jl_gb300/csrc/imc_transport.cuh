@@ -45,6 +45,15 @@ template <class T> __device__ __forceinline__ void nadd(T &s, T &c, T x) {
     else c += (x - t) + s;
     s = t;
 }
+// the same sums with the order chosen by the bits: four FP64 instructions
+// where the branches of the generic form issue up to eight
+template <> __device__ __forceinline__ void nadd<double>(double &s, double &c, double x) {
+    const bool ge = (long long)m64::bits(s) >= (long long)m64::bits(x);
+    const double big = ge ? s : x, small = ge ? x : s;
+    const double t = s + x;
+    c += (big - t) + small;
+    s = t;
+}
 
 // Limb adds into global memory (64-bit integer reductions in L2) or into the
 // block's private copy of the tally in shared memory.
@@ -217,22 +226,29 @@ constexpr int kSmtBlock64 = 512;
 constexpr int kGlbBlock32 = 1024;
 constexpr int kGlbBlock64 = 256;
 
-// 1D per-cell table: sigma_a f, effective scatter, width * distancescale,
-// width; the FP32 table adds the reciprocals its arithmetic multiplies by
+// 1D per-cell table: sigma_a f, effective scatter, width * distancescale;
+// the FP32 table adds the width and the reciprocals its arithmetic multiplies
+// by, the FP64 table 1/seff (its deposits are energies, not densities, so it
+// needs no width)
 template <class T> struct Tab1;
-template <> struct Tab1<double> { double saf, seff, dxs, dxT; };
+template <> struct Tab1<double> { double saf, seff, rseff, dxs; };
 template <> struct Tab1<float> { float saf, seff, dxs, dxT, rseff, rdxT, pad0, pad1; };
 static_assert(sizeof(Tab1<double>) == 32 && sizeof(Tab1<float>) == 32, "32-byte table rows");
 
+// The rows are written once per step by k_update (store_tab) and copied to
+// shared memory by every transport block (load_tab): built by each block,
+// they cost every SM the FP64 conversions and divisions of all cells.
 template <class T>
 __device__ __forceinline__ Tab1<T> make_tab1(double sa, double f, double ss, double dx, T ds) {
     Tab1<T> e;
     const T saT = (T)sa, fT = (T)f, ssT = (T)ss;
     e.saf = saT * fT;
     e.seff = saT * ((T)1 - fT) + ssT;
-    e.dxT = (T)dx;
-    e.dxs = e.dxT * ds;
-    if constexpr (sizeof(T) == 4) {
+    e.dxs = (T)dx * ds;
+    if constexpr (sizeof(T) == 8) {
+        e.rseff = 1.0 / e.seff;
+    } else {
+        e.dxT = (T)dx;
         e.rseff = 1.0f / e.seff;  // inf for a zero opacity: the flight is then inf, as seff/0 is
         e.rdxT = 1.0f / e.dxT;
         e.pad0 = e.pad1 = 0.0f;
@@ -240,25 +256,50 @@ __device__ __forceinline__ Tab1<T> make_tab1(double sa, double f, double ss, dou
     return e;
 }
 
-// Segment arithmetic of Transport.MC (src/imc_transport.jl:84-123).  FP64
-// evaluates the reference's expressions as written.  FP32 (and FP16 state)
-// evaluates the same quantities with fewer instructions: the collision
-// distance as -log(v) * (1/seff) with the hardware logarithm, the weight
-// after the segment as E + E expm1(-sigma_a f d) -- one transcendental for
-// both the attenuation and the deposit, so the two add up to E up to one
-// rounding -- and reciprocals instead of divisions.
+// Segment arithmetic of Transport.MC (src/imc_transport.jl:84-123).  FP32
+// (and FP16 state) evaluates the collision distance as -log(v) * (1/seff)
+// with the hardware logarithm, the weight after the segment as E + E
+// expm1(-sigma_a f d) -- one transcendental for both the attenuation and the
+// deposit, so the two add up to E up to one rounding -- and reciprocals
+// instead of divisions.  FP64 evaluates the same quantities from the functions
+// of imc_math64.cuh.  The FP64 pipe bounds it (16 cycles per warp instruction
+// and SM), so a segment holds as few FP64 instructions as its accuracy
+// allows: the deposits of a cell are summed as energies and divided by the
+// cell's volume once, when the tally is finalised, and comparisons run on the
+// bits.  Against CUDA's exp, expm1 and log, five divisions and FP64 compares:
+// 2000-cell slab at 2e6 histories 1.24 -> 0.65 ms per launch, 98 x 28 channel
+// 0.58 -> 0.21 ms.
 template <class T> struct SegMath;
 template <> struct SegMath<double> {
+    // inf for a zero opacity (rseff inf), as el / 0 is
+    static __device__ __forceinline__ double flight(Stream &rs, double seff, double rseff) {
+        const double el = Rand<double>::exp1(rs), q = el * rseff;
+        const double d = fma(fma(-q, seff, el), rseff, q);
+        return m64::hi32(rseff) < 0x7FE00000u ? d : el / seff;
+    }
     static __device__ __forceinline__ double flight(Stream &rs, const Tab1<double> &ce) {
-        return Rand<double>::exp1(rs) / ce.seff;
+        return flight(rs, ce.seff, ce.rseff);
     }
-    // new weight; *dep = the deposit per unit width
-    static __device__ __forceinline__ double attenuate(double E, const Tab1<double> &ce, double d, double *dep) {
-        *dep = -(E / ce.dxT) * expm1(-ce.saf * d);
-        return E * exp(-ce.saf * d);
+    // new weight; *dep = the energy deposited (d < 0, a history past its
+    // census time by a rounding, takes the general expm1)
+    static __device__ __forceinline__ double attenuate(double E, double saf, double d, bool odd, double *dep) {
+        const double em1 = odd ? expm1(-saf * d) : m64::expm1_neg(saf * d);
+        *dep = -(E * em1);
+        return fma(E, em1, E);
     }
-    static __device__ __forceinline__ double all_in(double E, const Tab1<double> &ce) { return E / ce.dxT; }
+    static __device__ __forceinline__ double all_in(double E, const Tab1<double> &) { return E; }
 };
+// The shortest of the distances of an FP64 segment, and which of them it is
+// (ties give every one): bit comparisons when all are in [+0, inf], else
+// (odd) the reference's NaN-propagating minimum.
+__device__ __forceinline__ bool plain64(double v) { return m64::hi32(v) <= 0x7FF00000u; }
+__device__ __forceinline__ double min64(double a, double b) {
+    const uint64_t x = m64::bits(a), y = m64::bits(b);
+    return m64::from_bits(x < y ? x : y);
+}
+// v > 0, a <= b and a >= b without the FP64 pipe (a and b not both negative)
+__device__ __forceinline__ bool pos64(double v) { return (long long)m64::bits(v) > 0; }
+__device__ __forceinline__ bool le64(double a, double b) { return (long long)m64::bits(a) <= (long long)m64::bits(b); }
 template <> struct SegMath<float> {
     static __device__ __forceinline__ float flight(Stream &rs, const Tab1<float> &ce) {
         const float v = (float)((rs.next() >> 8) | 1u) * 0x1p-24f;
@@ -278,6 +319,35 @@ template <> struct Tab2<double> { double saf, seff; };
 template <> struct Tab2<float> { float saf, seff, rseff, rarea; };
 static_assert(sizeof(Tab2<double>) == 16 && sizeof(Tab2<float>) == 16, "16-byte table rows");
 template <class T> struct Face { T ws, wT; };  // width * distancescale, width
+template <class T>
+__device__ __forceinline__ Tab2<T> make_tab2(double sa_, double f_, double ss_, double dx, double dy) {
+    const T sa = (T)sa_, f = (T)f_, ss = (T)ss_;
+    Tab2<T> e;
+    e.saf = sa * f;
+    e.seff = sa * ((T)1 - f) + ss;
+    if constexpr (sizeof(T) == 4) {
+        e.rseff = 1.0f / e.seff;
+        e.rarea = 1.0f / ((float)dx * (float)dy);
+    }
+    return e;
+}
+// row i of the table in global memory
+template <class T>
+__device__ __forceinline__ void store_tab(const CellArgs &ca, int i, double sa, double f, double ss) {
+    if (ca.geometry == 1) {
+        static_cast<Tab1<T> *>(ca.tab)[i] = make_tab1<T>(sa, f, ss, ca.dx[i], (T)ca.ds);
+    } else {
+        const Tab2<T> e = make_tab2<T>(sa, f, ss, ca.dx[i % ca.nx], ca.dy[i / ca.nx]);
+        static_cast<Tab2<T> *>(ca.tab)[i] = e;
+        if constexpr (sizeof(T) == 8) ca.tab_rs[i] = 1.0 / e.seff;
+    }
+}
+// `rows` table rows of R from global memory into shared memory
+template <class R> __device__ __forceinline__ void load_tab(R *dst, const void *src, int rows) {
+    const uint4 *s = static_cast<const uint4 *>(src);
+    uint4 *d = reinterpret_cast<uint4 *>(dst);
+    for (int v = threadIdx.x; v < rows * (int)(sizeof(R) / 16); v += blockDim.x) d[v] = s[v];
+}
 
 // end-of-kernel reduction of per-thread counters: one atomic per warp
 // (segments, histories removed from the list, error flags, and the census

@@ -212,11 +212,6 @@ __device__ __forceinline__ void load_queued(const SurrQueue &qq, long long e, un
     h.seg = 0;
 }
 
-template <class T>
-__device__ __forceinline__ void fill_table(const CellArgs &ca, Tab1<T> *tab, T ds) {
-    for (int i = threadIdx.x; i < ca.nx; i += blockDim.x) tab[i] = make_tab1<T>(ca.sa[i], ca.fleck[i], ca.ss[i], ca.dx[i], ds);
-}
-
 // ------------------------------------------------------------- query pass
 // One network query for every history of the ask queue of round `round`:
 // 32 histories per warp, two tensor-core passes of 16 rows, all lanes
@@ -245,7 +240,7 @@ __global__ void __launch_bounds__(kQueryBlock, 2) k_wave_query(CellArgs ca, Scal
         for (int v = threadIdx.x; v < kImageBytes / 16; v += blockDim.x) dst[v] = ca.surr_image[v];
         for (int v = threadIdx.x; v < kQueryWarps * kStageFloats; v += blockDim.x) stage_all[v] = 0.0f;
     }
-    fill_table<T>(ca, tab, ds);
+    load_tab(tab, ca.tab, N);
     __shared__ int s_sexp[16];
     load_scale_exps(ca, s_sexp);
     __syncthreads();
