@@ -59,6 +59,7 @@ struct ImcHandle {
     long long stats_cap = 0;
     int grid_transport = 0, block_transport = 256, grid_emit = 0;
     int grid_full = 0;  // resident transport blocks on the whole GPU
+    bool side_by_side = false;  // one of several handles running at once (imc_run_batch): smaller grids
     // learned surrogate: device image of the network (ca.surr_image points
     // into it while the surrogate is on) and its kernel's persistent grid
     void *d_surr_image = nullptr;
@@ -172,10 +173,13 @@ void drop_graphs(ImcHandle *h) {
 }
 
 // Transport blocks for this handle: the resident grid of the whole GPU, or
-// fewer for a small particle buffer (16 entries per thread at capacity), so
-// that the kernels of small decks run side by side in a batch.
+// fewer for a small particle buffer: one entry per thread at capacity for a
+// handle that has the GPU to itself (a step then waits for no more histories
+// per thread than it must), 16 in a batch of handles side by side, whose
+// kernels share the GPU and whose blocks each cost a table and a tally flush.
 int sized_grid(const ImcHandle *h, int full, int block) {
-    const long long want = (h->capacity + 16ll * block - 1) / (16ll * block);
+    const long long per = h->side_by_side ? 16 : 1;
+    const long long want = (h->capacity + per * block - 1) / (per * block);
     return (int)std::max<long long>(1, std::min<long long>(full, want));
 }
 
@@ -274,6 +278,14 @@ int grow(ImcHandle *h, long long need) {
     if (h->ca.surr_image && (rc = surr_queue_alloc(h))) return rc;
     drop_graphs(h);
     return IMC_OK;
+}
+
+// the handle's launch shapes for a run of its own or one among others
+void set_side_by_side(ImcHandle *h, bool on) {
+    if (h->side_by_side == on) return;
+    h->side_by_side = on;
+    h->grid_transport = sized_grid(h, h->grid_full, h->block_transport);
+    drop_graphs(h);
 }
 
 int read_scalars(ImcHandle *h, Scalars *sc) {
@@ -951,8 +963,7 @@ int imc_step(ImcHandle *h, ImcStepStats *stats, int *done) {
     return flags_status(h, ds.error_flags);
 }
 
-int imc_run(ImcHandle *h, int64_t max_steps, ImcStepStats *stats, int64_t *n_steps, double *device_ms) {
-    if (!h) return IMC_ERR_INVALID_ARG;
+static int run_steps(ImcHandle *h, int64_t max_steps, ImcStepStats *stats, int64_t *n_steps, double *device_ms) {
     if (n_steps) *n_steps = 0;
     if (device_ms) *device_ms = 0.0;
     // steps this run will take, from the host clock mirror
@@ -1017,6 +1028,12 @@ int imc_run(ImcHandle *h, int64_t max_steps, ImcStepStats *stats, int64_t *n_ste
     return flags_status(h, allflags);
 }
 
+int imc_run(ImcHandle *h, int64_t max_steps, ImcStepStats *stats, int64_t *n_steps, double *device_ms) {
+    if (!h) return IMC_ERR_INVALID_ARG;
+    set_side_by_side(h, false);
+    return run_steps(h, max_steps, stats, n_steps, device_ms);
+}
+
 int imc_run_batch(ImcHandle *const *hs, int32_t n, int64_t max_steps, int32_t n_threads, int64_t *steps,
                   double *wall_ms, int32_t *failed) {
     if (!hs || n < 0 || n_threads < 1) return IMC_ERR_INVALID_ARG;
@@ -1026,6 +1043,7 @@ int imc_run_batch(ImcHandle *const *hs, int32_t n, int64_t max_steps, int32_t n_
         for (int32_t j = 0; j < i; ++j)
             if (hs[i] == hs[j]) return IMC_ERR_INVALID_ARG;  // a handle is not thread-safe
     if (failed) *failed = -1;
+    const int nt = (int)std::min<int32_t>(n_threads, std::max<int32_t>(n, 1));
     std::atomic<int32_t> next(0);
     std::atomic<int> first_rc(IMC_OK);
     std::atomic<int32_t> first_bad(-1);
@@ -1035,7 +1053,8 @@ int imc_run_batch(ImcHandle *const *hs, int32_t n, int64_t max_steps, int32_t n_
             if (i >= n) return;
             ImcHandle *h = hs[i];
             int64_t st = 0;
-            int rc = cudaSetDevice(h->device) == cudaSuccess ? imc_run(h, max_steps, nullptr, &st, nullptr)
+            set_side_by_side(h, nt > 1);
+            int rc = cudaSetDevice(h->device) == cudaSuccess ? run_steps(h, max_steps, nullptr, &st, nullptr)
                                                              : fail(h, IMC_ERR_CUDA, "cudaSetDevice");
             if (steps) steps[i] = st;
             if (rc != IMC_OK) {
@@ -1045,7 +1064,6 @@ int imc_run_batch(ImcHandle *const *hs, int32_t n, int64_t max_steps, int32_t n_
         }
     };
     const auto t0 = std::chrono::steady_clock::now();
-    const int nt = (int)std::min<int32_t>(n_threads, std::max<int32_t>(n, 1));
     std::vector<std::thread> pool;
     for (int t = 1; t < nt; ++t) pool.emplace_back(worker);
     worker();

@@ -39,10 +39,11 @@ enum { kModePlain = 0, kModeList = 1, kModeResume = 2, kModeResumeLast = 3 };
 // (kTallyGlobal, kTallyShared, or kTallySharedDep: deposition tallies shared,
 // census tallies global; the plain pass only).  The block's shared tallies
 // and counters are flushed to the deck's before it returns; the caller puts a
-// barrier between two calls.
+// barrier between two calls.  chunk: list entries a warp takes at a time in the
+// short-history schedule (0: by the list's length, list_chunk).
 template <class St, int BLOCK, int TM, int MODE, class CA, class BP>
 __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, const BP &bufs, const SurrWave &w,
-                                                  int round, unsigned char *smem_raw) {
+                                                  int round, unsigned char *smem_raw, int chunk) {
     constexpr bool SMT = TM != kTallyGlobal;      // deposition flushes to shared memory
     constexpr bool RAD_SMT = TM == kTallyShared;  // census flushes to shared memory
     typedef typename St::T T;
@@ -51,6 +52,7 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
     constexpr bool kPause = MODE == kModeList || MODE == kModeResume;
     const long long n = kFromQueue ? (long long)sc->qcount[2 * round + 1] : sc->n_particles;
     if (kFromQueue && n == 0) return;
+    if (chunk == 0) chunk = list_chunk(n, kListChunk1D);
     PBuf<St> pb(bufs.b[sc->cur]);
     Tab1<T> *tab = reinterpret_cast<Tab1<T> *>(smem_raw);
     const int N = ca.nx;
@@ -341,15 +343,15 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
                 pa = e < n ? pb.alive[e] : (uint8_t)0;
                 if (pa) { pcs = pb.cs[e]; pt = pb.t[e]; px = pb.x[e]; pmu = pb.ux[e]; pE = pb.E[e]; pE0 = pb.E0[e]; }
             };
-            for (long long base = warp_counter_next(&sc->work_next) * kListChunk1D; base < n;
-                 base = warp_counter_next(&sc->work_next) * kListChunk1D) {
+            for (long long base = warp_counter_next(&sc->work_next) * chunk; base < n;
+                 base = warp_counter_next(&sc->work_next) * chunk) {
                 fetch(base + lane);
-                for (int r = 0; r < kListChunk1D; r += 32) {
+                for (int r = 0; r < chunk; r += 32) {
                     const long long e = base + r + lane;
                     const bool a = pa != 0;
                     const int ccs = pcs;
                     t = (T)pt; x = (T)px; mu = (T)pmu; E = (T)pE; E0 = (T)pE0;
-                    if (r + 32 < kListChunk1D) fetch(e + 32);
+                    if (r + 32 < chunk) fetch(e + 32);
                     if (a) {
                         i = e;
                         cs = ccs;
@@ -362,9 +364,9 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
             }
         } else {
             // the list (or a resume pass's queue) in chunks from the counter
-            for (long long base = warp_counter_next(&sc->work_next) * kListChunk1D; base < n;
-                 base = warp_counter_next(&sc->work_next) * kListChunk1D)
-                for (int r = 0; r < kListChunk1D; r += 32)
+            for (long long base = warp_counter_next(&sc->work_next) * chunk; base < n;
+                 base = warp_counter_next(&sc->work_next) * chunk)
+                for (int r = 0; r < chunk; r += 32)
                     if (base + r + lane < n) walk(base + r + lane);
         }
     } else {
@@ -443,7 +445,7 @@ template <class St, int BLOCK, int TM, int MODE>
 __global__ void __launch_bounds__(BLOCK) k_transport1d(CellArgs ca, Scalars *sc, PBufPair bufs, SurrWave w,
                                                        int round) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    transport1d_block<St, BLOCK, TM, MODE>(ca, sc, bufs, w, round, smem_raw);
+    transport1d_block<St, BLOCK, TM, MODE>(ca, sc, bufs, w, round, smem_raw, 0);
 }
 
 // One transport launch over the lists of many 1D decks (the fused batch,
@@ -475,7 +477,7 @@ __global__ void __launch_bounds__(BLOCK) k_transport1d_multi(int ndecks) {
         __syncthreads();
         if (s_go)
             transport1d_block<St, BLOCK, kTallyShared, kModePlain>(c_multi_ca[d], sc, c_multi_bufs[d], SurrWave{}, 0,
-                                                                    smem_raw);
+                                                                    smem_raw, kListChunk1D);
         __syncthreads();
     }
 }
@@ -738,10 +740,10 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
             finish(end);
         };
         // the list in chunks from the counter
-        const int lane = threadIdx.x & 31;
-        for (long long base = warp_counter_next(&sc->work_next) * kListChunk; base < n;
-             base = warp_counter_next(&sc->work_next) * kListChunk)
-            for (int r = 0; r < kListChunk; r += 32)
+        const int lane = threadIdx.x & 31, chunk = list_chunk(n, kListChunk);
+        for (long long base = warp_counter_next(&sc->work_next) * chunk; base < n;
+             base = warp_counter_next(&sc->work_next) * chunk)
+            for (int r = 0; r < chunk; r += 32)
                 if (base + r + lane < n) walk(base + r + lane);
     } else {
         // long histories: lanes refill from 32-entry chunks (see k_transport1d)
