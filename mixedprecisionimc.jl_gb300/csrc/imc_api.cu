@@ -770,6 +770,7 @@ int imc_create(const ImcDeck *d, ImcHandle **out) {
     ca.n_input = d->n_input; ca.n_max = d->n_max;
     ca.seg_cap = d->segment_cap > 0 ? d->segment_cap : 10000000;
     ca.seed = d->seed;
+    ca.rk.set(d->seed);
     double dxmin = *std::min_element(d->dx, d->dx + h->nx);
     double dymin = d->geometry == IMC_GEOM_2D ? *std::min_element(d->dy, d->dy + h->ny) : 1.0;
     ca.vol_min = h->prec == IMC_FP64 ? 1.0 : dxmin * dymin;  // least divisor of a deposit (FP64: energies)

@@ -19,6 +19,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 #include <cuda_fp16.h>
+#include "imc_device.cuh"
 
 namespace imc {
 
@@ -92,6 +93,7 @@ struct CellArgs {
     int linearized, marshak, sel_prec, timestepping;
     long long n_input, n_max, capacity, seg_cap;
     unsigned long long seed;
+    RoundKeys rk;                      // of seed
     double vol_min, scale_min;
     double t_end, dtmax, kfac;
     // the transport's per-cell table (imc_transport.cuh: Tab1 rows, or Tab2

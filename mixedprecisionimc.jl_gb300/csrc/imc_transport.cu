@@ -83,7 +83,9 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
     const int b_dep = sc->b_dep, b_rad = sc->b_rad, b_lost = sc->b_lost;
     const unsigned step = sc->step;
     const unsigned long long seed = ca.seed;
-    const long long cap = ca.seg_cap;
+    // segments are counted in 32 bits: a cap beyond them is out of any
+    // launch's reach
+    const unsigned cap = ca.seg_cap > 0xFFFFFFFEll ? 0xFFFFFFFEu : (unsigned)ca.seg_cap;
     const int nc = ca.nc;
     const bool reflect_r = ca.bc[1] == 1, reflect_l = ca.bc[0] == 1;
     unsigned long long *ask_count = &sc->qcount[kFromQueue ? 2 * round + 2 : 0];
@@ -101,12 +103,14 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
     int cs = 0, cell = 0, k = 0, acc_cell = 0, prv_cell = -1;
     T t = (T)0, x = (T)0, mu = (T)0, E = (T)0, E0 = (T)0, minenergy = (T)0, acc_s = (T)0, acc_c = (T)0, rmu = (T)0;
     T prv_s = (T)0, prv_c = (T)0;
-    long long seg = 0;
-    Stream rs;
+    unsigned seg = 0;
+    Stream rs;  // FP64
+    Words ws;   // FP32
     auto start = [&](int cs_now) {
         cell = cs_now & 0xFFFFFF;
         k = cs_now >> 24;
-        rs.init(seed, step, (uint32_t)i, stage);
+        if constexpr (sizeof(T) == 8) rs.init(seed, step, (uint32_t)i, stage);
+        else ws.init((uint32_t)i);
         minenergy = cutoff_energy(E0);  // (T)(0.01 * (double)E0), without FP64 in binary32
         acc_s = (T)0;
         acc_c = (T)0;
@@ -174,15 +178,18 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
             const Tab1<T> ce = tab[cell];
             T dist_b, dist_cen, dist;
             bool at_b, at_col, at_cen, odd = false;  // odd (FP64): a distance below +0 or not a number
-            const T dist_col = M::flight(rs, ce);
+            T dist_col;
             if constexpr (sizeof(T) == 4) {
+                if (ws.n < 2) ws.refill(round_keys(ca), step, stage);
+                dist_col = M::flight(ws.w0, ce);
                 dist_b = mu > (T)0 ? (ce.dxs - x) * rmu : m_abs(x * rmu);
                 dist_cen = c * (endsteptime - t) * ds;
-                dist = jmin(jmin(dist_b, dist_col), dist_cen);
+                dist = min3_nan(dist_b, dist_col, dist_cen);
                 at_b = dist == dist_b;
                 at_col = dist == dist_col;
                 at_cen = dist == dist_cen;
             } else {
+                dist_col = M::flight(rs, ce);
                 const bool fwd = pos64(mu);
                 dist_b = m64::div_r(fwd ? ce.dxs - x : x, mu, rmu);
                 if (!fwd) dist_b = m_abs(dist_b);
@@ -233,42 +240,42 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
                     }
                     E = newenergy;
                     if (at_b) {
-                        if (mu > (T)0) {
-                            if (cell == N - 1) {
-                                if (reflect_r) {
-                                    mu = -mu;
-                                    rmu = -rmu;
-                                } else {
-                                    end = 4;
-                                }
-                            }
-                            if (!end) {
-                                cell += 1;
-                                x = (T)0;
-                            }
-                        }
-                        if (!end && mu < (T)0) {
-                            if (cell == 0) {
-                                if (reflect_l) {
-                                    mu = -mu;
-                                    rmu = -rmu;
-                                } else {
-                                    end = 4;
-                                }
-                            } else {
-                                cell -= 1;
-                                x = tab[cell].dxs;
-                            }
+                        // through the right face (mu > 0) or the left one: the
+                        // next cell, or at the domain's end the escape or the
+                        // reflection, which leaves a right mover on its face
+                        // (the reference steps out and back in)
+                        const bool right = mu > (T)0;
+                        const int next = cell + (right ? 1 : -1);
+                        if ((unsigned)next < (unsigned)N) {
+                            cell = next;
+                            x = right ? (T)0 : tab[next].dxs;
+                        } else if (right ? reflect_r : reflect_l) {
+                            mu = -mu;
+                            rmu = -rmu;
+                            if (right) x = ce.dxs;
+                        } else {
+                            end = 4;
                         }
                     }
-                    if (!end && at_col) {
+                    const bool turn = !end && at_col;
+                    if (turn) {
                         // mu = 1 - 2*rand, redrawn while zero (src/imc_transport.jl:178-181);
                         // a zero needs rand == 0.5 exactly, so 64 redraws never run out
-                        mu = (T)0;
-                        for (int r = 0; r < 64 && mu == (T)0; ++r) mu = Rand<T>::cosine(rs);
+                        if constexpr (sizeof(T) == 4) {
+                            mu = Rand<T>::cosine(ws.w1);
+                            for (int r = 1; r < 64 && mu == (T)0; ++r) {
+                                ws.drop(false);
+                                if (ws.n < 2) ws.refill(round_keys(ca), step, stage);
+                                mu = Rand<T>::cosine(ws.w1);
+                            }
+                        } else {
+                            mu = (T)0;
+                            for (int r = 0; r < 64 && mu == (T)0; ++r) mu = Rand<T>::cosine(rs);
+                        }
                         if (mu == (T)0) mu = (T)1;
                         rmu = (T)1 / mu;
                     }
+                    if constexpr (sizeof(T) == 4) ws.drop(turn);
                     // census: t = 0 and the state written back by finish()
                     // (src/imc_transport.jl:185-193)
                     if (!end && at_cen) end = 2;

@@ -45,6 +45,12 @@ template <class T> __device__ __forceinline__ void nadd(T &s, T &c, T x) {
     else c += (x - t) + s;
     s = t;
 }
+// the same sums without a branch (two of them for lanes that part)
+template <> __device__ __forceinline__ void nadd<float>(float &s, float &c, float x) {
+    const float t = s + x;
+    c += (fmaxf(s, x) - t) + fminf(s, x);
+    s = t;
+}
 // the same sums with the order chosen by the bits: four FP64 instructions
 // where the branches of the generic form issue up to eight
 template <> __device__ __forceinline__ void nadd<double>(double &s, double &c, double x) {
@@ -297,6 +303,16 @@ template <> struct SegMath<double> {
     }
     static __device__ __forceinline__ double all_in(double E, const Tab1<double> &) { return E; }
 };
+// the least of three, NaN if one is NaN (jmin of jmin; one instruction)
+__device__ __forceinline__ float min3_nan(float a, float b, float c) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+// the round keys of a launch's seed
+__device__ __forceinline__ const RoundKeys &round_keys(const CellArgs &ca) { return ca.rk; }
+__device__ __forceinline__ SeedKeys round_keys(const Deck1DArgs &ca) { return SeedKeys(ca.seed); }
+
 // The shortest of the distances of an FP64 segment, and which of them it is
 // (ties give every one): bit comparisons when all are in [+0, inf], else
 // (odd) the reference's NaN-propagating minimum.
@@ -309,8 +325,8 @@ __device__ __forceinline__ double min64(double a, double b) {
 __device__ __forceinline__ bool pos64(double v) { return (long long)m64::bits(v) > 0; }
 __device__ __forceinline__ bool le64(double a, double b) { return (long long)m64::bits(a) <= (long long)m64::bits(b); }
 template <> struct SegMath<float> {
-    static __device__ __forceinline__ float flight(Stream &rs, const Tab1<float> &ce) {
-        const float v = (float)((rs.next() >> 8) | 1u) * 0x1p-24f;
+    static __device__ __forceinline__ float flight(uint32_t w, const Tab1<float> &ce) {
+        const float v = (float)((w >> 8) | 1u) * 0x1p-24f;
         return -__logf(v) * ce.rseff;
     }
     static __device__ __forceinline__ float attenuate(float E, const Tab1<float> &ce, float d, float *dep) {
