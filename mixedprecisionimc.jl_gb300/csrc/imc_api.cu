@@ -517,6 +517,7 @@ Deck1DArgs deck1d_args(const CellArgs &ca) {
     a.tab = ca.tab; a.scales = ca.scales;
     a.dep_acc = ca.dep_acc; a.rad_acc = ca.rad_acc; a.lost_acc = ca.lost_acc;
     a.c = ca.c; a.ds = ca.ds;
+    a.c_f = ca.c_f; a.ds_f = ca.ds_f; a.rdsc_f = ca.rdsc_f;
     a.seg_cap = ca.seg_cap;
     a.seed = ca.seed;
     return a;
@@ -763,6 +764,7 @@ int imc_create(const ImcDeck *d, ImcHandle **out) {
     if ((rc = upload<double>(h, &ca.part_tally, nullptr, (size_t)ca.nblk_cell * (K + 1) * 2))) return bail(rc);
     for (int b = 0; b < 4; ++b) ca.bc[b] = d->bc[b];
     ca.c = d->phys_c; ca.a = d->phys_a; ca.alpha = d->alpha; ca.ds = d->distancescale;
+    ca.c_f = (float)ca.c; ca.ds_f = (float)ca.ds; ca.rdsc_f = 1.0f / (ca.ds_f * ca.c_f);
     ca.temp_floor = d->temp_floor; ca.cellmin = d->cellmin;
     ca.linearized = d->linearized ? 1 : 0; ca.marshak = d->marshak_opacity ? 1 : 0;
     ca.sel_prec = d->scale_select_precision;

@@ -90,6 +90,10 @@ struct CellArgs {
     // physics / control
     int bc[4];
     double c, a, alpha, ds, temp_floor, cellmin;
+    // c, DISTANCESCALE and 1 / (DISTANCESCALE c) in binary32: converted in a
+    // kernel, they are converted again wherever registers are short, each time
+    // by the FP64 pipe
+    float c_f, ds_f, rdsc_f;
     int linearized, marshak, sel_prec, timestepping;
     long long n_input, n_max, capacity, seg_cap;
     unsigned long long seed;
@@ -205,6 +209,7 @@ struct Deck1DArgs {
     const double *scales;
     long long *dep_acc, *rad_acc, *lost_acc;
     double c, ds;
+    float c_f, ds_f, rdsc_f;
     long long seg_cap;
     unsigned long long seed;
 };

@@ -56,9 +56,9 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
     PBuf<St> pb(bufs.b[sc->cur]);
     Tab1<T> *tab = reinterpret_cast<Tab1<T> *>(smem_raw);
     const int N = ca.nx;
-    const T ds = (T)ca.ds, c = (T)ca.c;
+    const T ds = Consts<T>::ds(ca), c = Consts<T>::c(ca);
     const bool ds_one = ds == (T)1, c_one = c == (T)1;
-    const T rdsc = (T)1 / (ds * c);
+    const T rdsc = Consts<T>::rdsc(ca);
     const T rds = sizeof(T) == 8 ? (T)1 / ds : (T)0, rc = sizeof(T) == 8 ? (T)1 / c : (T)0;
     long long *dep_acc = ca.dep_acc, *rad_acc = ca.rad_acc;
     if (SMT) {
@@ -504,9 +504,9 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
     Tab2<T> *tab = reinterpret_cast<Tab2<T> *>(smem_raw);
     Face<T> *fx = reinterpret_cast<Face<T> *>(tab + nc);
     Face<T> *fy = fx + NX;
-    const T ds = (T)ca.ds, c = (T)ca.c;
+    const T ds = Consts<T>::ds(ca), c = Consts<T>::c(ca);
     const bool ds_one = ds == (T)1, c_one = c == (T)1;
-    const T rdsc = (T)1 / (ds * c);
+    const T rdsc = Consts<T>::rdsc(ca);
     const T rds = sizeof(T) == 8 ? (T)1 / ds : (T)0, rc = sizeof(T) == 8 ? (T)1 / c : (T)0;
     long long *dep_acc = ca.dep_acc, *rad_acc = ca.rad_acc;
     if (SMT) {

@@ -309,6 +309,18 @@ __device__ __forceinline__ float min3_nan(float a, float b, float c) {
     asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
     return r;
 }
+// c, DISTANCESCALE and 1 / (DISTANCESCALE c) in the arithmetic type
+template <class T> struct Consts;
+template <> struct Consts<float> {
+    template <class CA> static __device__ __forceinline__ float c(const CA &ca) { return ca.c_f; }
+    template <class CA> static __device__ __forceinline__ float ds(const CA &ca) { return ca.ds_f; }
+    template <class CA> static __device__ __forceinline__ float rdsc(const CA &ca) { return ca.rdsc_f; }
+};
+template <> struct Consts<double> {
+    template <class CA> static __device__ __forceinline__ double c(const CA &ca) { return ca.c; }
+    template <class CA> static __device__ __forceinline__ double ds(const CA &ca) { return ca.ds; }
+    template <class CA> static __device__ __forceinline__ double rdsc(const CA &) { return 0.0; }  // divides
+};
 // the round keys of a launch's seed
 __device__ __forceinline__ const RoundKeys &round_keys(const CellArgs &ca) { return ca.rk; }
 __device__ __forceinline__ SeedKeys round_keys(const Deck1DArgs &ca) { return SeedKeys(ca.seed); }

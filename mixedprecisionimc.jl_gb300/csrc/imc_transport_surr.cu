@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(kQueryBlock, 2) k_wave_query(CellArgs ca, Scal
     float *stage_all = reinterpret_cast<float *>(smem_raw + kImageBytes);
     Tab1<T> *tab = reinterpret_cast<Tab1<T> *>(smem_raw + kQueryHead);
     const int N = ca.nx, nc = ca.nc;
-    const T ds = (T)ca.ds, c = (T)ca.c;
+    const T ds = Consts<T>::ds(ca), c = Consts<T>::c(ca);
     const bool ds_one = ds == (T)1;
     {
         uint4 *dst = reinterpret_cast<uint4 *>(smem_raw);
