@@ -57,8 +57,8 @@ struct ImcHandle {
     long long *tile_cnt = nullptr, *tile_off = nullptr;
     DevStats *d_stats = nullptr;
     long long stats_cap = 0;
-    int grid_transport = 0, block_transport = 256, grid_emit = 0;
-    int grid_full = 0;  // resident transport blocks on the whole GPU
+    int block_transport = 256, block_transport_long = 256, grid_emit = 0;
+    TransportGrid grid_full{}, grid_transport{};  // resident blocks on the whole GPU; those of this handle's launches
     bool side_by_side = false;  // one of several handles running at once (imc_run_batch): smaller grids
     // learned surrogate: device image of the network (ca.surr_image points
     // into it while the surrogate is on) and its kernel's persistent grid
@@ -183,6 +183,11 @@ int sized_grid(const ImcHandle *h, int full, int block) {
     return (int)std::max<long long>(1, std::min<long long>(full, want));
 }
 
+void size_grids(ImcHandle *h) {
+    h->grid_transport.grid = sized_grid(h, h->grid_full.grid, h->block_transport);
+    h->grid_transport.grid_long = sized_grid(h, h->grid_full.grid_long, h->block_transport_long);
+}
+
 PBufPair pair(const ImcHandle *h) {
     PBufPair p;
     p.b[0] = h->buf[0];
@@ -273,7 +278,7 @@ int grow(ImcHandle *h, long long need) {
     sc.cur = 0;
     CK(h, hcopy(h, h->d_sc, &sc, sizeof(Scalars), cudaMemcpyHostToDevice));
     h->ca.capacity = ncap;
-    h->grid_transport = sized_grid(h, h->grid_full, h->block_transport);
+    size_grids(h);
     if ((rc = tile_alloc(h))) return rc;
     if (h->ca.surr_image && (rc = surr_queue_alloc(h))) return rc;
     drop_graphs(h);
@@ -284,7 +289,7 @@ int grow(ImcHandle *h, long long need) {
 void set_side_by_side(ImcHandle *h, bool on) {
     if (h->side_by_side == on) return;
     h->side_by_side = on;
-    h->grid_transport = sized_grid(h, h->grid_full, h->block_transport);
+    size_grids(h);
     drop_graphs(h);
 }
 
@@ -342,7 +347,8 @@ void host_timestep(const ImcDeck &d, double &t, double &dt, bool &finished) {
 void run_transport(ImcHandle *h, PBufPair bufs, cudaStream_t st) {
     if (h->ca.surr_image) {
         SurrShapes sh = h->sshape;
-        sh.analog_grid = sized_grid(h, sh.analog_grid, sh.analog_block);
+        sh.analog_grid.grid = sized_grid(h, sh.analog_grid.grid, sh.analog_block);
+        sh.analog_grid.grid_long = sized_grid(h, sh.analog_grid.grid_long, sh.analog_block_long);
         sh.query_grid = sized_grid(h, sh.query_grid, sh.query_block);
         launch_transport_surr(h->ca, h->d_sc, h->prec, bufs, h->wave, sh, st);
     }
@@ -555,18 +561,24 @@ int build_fused(FusedBatch &F, ImcHandle *const *hs, const std::vector<int> &mem
         smem = std::max(smem, transport_shape(h->ca, prec).smem);
     }
     CK(h0, set_transport_multi_decks(cas.data(), bufs.data(), scs.data(), n, F.st));
-    const void *kp = transport_multi_ptr(prec);
-    const int block = transport_multi_block(prec);
-    CK(h0, raise_smem_limit(kp, smem));
-    int per_sm = 0;
-    CK(h0, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kp, block, smem));
-    if (per_sm < 1) return fail(h0, IMC_ERR_CUDA, "fused transport: no block fits on an SM");
-    const int grid = per_sm * h0->sm_count;
+    // the short- and the long-history kernel, each over the decks it serves
+    // this step
+    const void *kp[2];
+    int block[2], grid[2];
+    for (int v = 0; v < 2; ++v) {
+        kp[v] = transport_multi_ptr(prec, v == 1);
+        block[v] = transport_multi_block(prec, v == 1);
+        CK(h0, raise_smem_limit(kp[v], smem));
+        int per_sm = 0;
+        CK(h0, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kp[v], block[v], smem));
+        if (per_sm < 1) return fail(h0, IMC_ERR_CUDA, "fused transport: no block fits on an SM");
+        grid[v] = per_sm * h0->sm_count;
+    }
     cudaGraph_t G = nullptr;
     CK(h0, cudaGraphCreate(&G, 0));
     int rc = IMC_OK;
     std::vector<cudaGraphNode_t> before((size_t)n);
-    cudaGraphNode_t tn = nullptr;
+    cudaGraphNode_t tn[2] = {nullptr, nullptr};
     auto add_half = [&](int j, bool first, const cudaGraphNode_t *deps, size_t ndeps, cudaGraphNode_t *node) {
         ImcHandle *h = hs[members[j]];
         cudaGraph_t g = nullptr;
@@ -579,22 +591,23 @@ int build_fused(FusedBatch &F, ImcHandle *const *hs, const std::vector<int> &mem
         }
     };
     for (int j = 0; j < n && !rc; ++j) add_half(j, true, nullptr, 0, &before[j]);
-    if (!rc) {
+    for (int v = 0; v < 2 && !rc; ++v) {
         int nd = n;
         void *args[] = {&nd};
         cudaKernelNodeParams p{};
-        p.func = const_cast<void *>(kp);
-        p.gridDim = dim3((unsigned)grid);
-        p.blockDim = dim3((unsigned)block);
+        p.func = const_cast<void *>(kp[v]);
+        p.gridDim = dim3((unsigned)grid[v]);
+        p.blockDim = dim3((unsigned)block[v]);
         p.sharedMemBytes = (unsigned)smem;
         p.kernelParams = args;
         p.extra = nullptr;
-        const cudaError_t e = cudaGraphAddKernelNode(&tn, G, before.data(), (size_t)n, &p);
+        const cudaError_t e = v == 0 ? cudaGraphAddKernelNode(&tn[0], G, before.data(), (size_t)n, &p)
+                                     : cudaGraphAddKernelNode(&tn[1], G, &tn[0], 1, &p);
         if (e != cudaSuccess) rc = fail(h0, IMC_ERR_CUDA, std::string("fused transport node: ") + cudaGetErrorString(e));
     }
     for (int j = 0; j < n && !rc; ++j) {
         cudaGraphNode_t after = nullptr;
-        add_half(j, false, &tn, 1, &after);
+        add_half(j, false, &tn[1], 1, &after);
     }
     if (!rc) {
         const cudaError_t e = cudaGraphInstantiate(&F.exec, G, 0);
@@ -803,17 +816,21 @@ int imc_create(const ImcDeck *d, ImcHandle **out) {
     TransportShape shape = transport_shape(ca, h->prec);
     const int smem = shape.smem;
     h->block_transport = shape.block;
-    const void *kp = transport_kernel_ptr(ca, h->prec);
+    h->block_transport_long = shape.block_long ? shape.block_long : shape.block;
     if (smem > 227 * 1024) return bail(fail(h, IMC_ERR_INVALID_ARG, "mesh too large for the shared-memory transport table"));
-    if (smem > 48 * 1024)
-        if (raise_smem_limit(kp, smem) != cudaSuccess)
-            return bail(fail(h, IMC_ERR_CUDA, "cudaFuncSetAttribute(smem)"));
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kp, h->block_transport, smem) != cudaSuccess || per_sm < 1)
-        return bail(fail(h, IMC_ERR_CUDA, "transport kernel cannot be resident"));
-    h->grid_full = h->sm_count * per_sm;
+    for (int v = 0; v < 2; ++v) {
+        const void *kp = transport_kernel_ptr(ca, h->prec, v == 1);
+        if (smem > 48 * 1024)
+            if (raise_smem_limit(kp, smem) != cudaSuccess)
+                return bail(fail(h, IMC_ERR_CUDA, "cudaFuncSetAttribute(smem)"));
+        int per_sm = 0;
+        const int block = v ? h->block_transport_long : h->block_transport;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kp, block, smem) != cudaSuccess || per_sm < 1)
+            return bail(fail(h, IMC_ERR_CUDA, "transport kernel cannot be resident"));
+        (v ? h->grid_full.grid_long : h->grid_full.grid) = h->sm_count * per_sm;
+    }
     ca.surr_min_calls = 2ll * h->sm_count * 1024;  // two queries per thread of the GPU
-    h->grid_transport = sized_grid(h, h->grid_full, h->block_transport);
+    size_grids(h);
     h->grid_emit = h->sm_count * 4;
     if (cudaEventCreate(&h->ev[0]) != cudaSuccess || cudaEventCreate(&h->ev[1]) != cudaSuccess)
         return bail(fail(h, IMC_ERR_CUDA, "cudaEventCreate"));
@@ -1569,18 +1586,21 @@ int imc_set_surrogate(ImcHandle *h, const float *params, int64_t n_params) {
     SurrShapes sh = surr_shapes(ca, h->prec);
     if (sh.analog_smem > 227 * 1024 || sh.query_smem > 227 * 1024)
         return fail(h, IMC_ERR_INVALID_ARG, "surrogate: mesh too large for shared memory");
-    int grids[4] = {0, 0, 0, 0};
-    for (int which = 0; which < 4; ++which) {
-        const void *kp = surr_kernel_ptr(ca, h->prec, which);
-        const int block = which == 3 ? sh.query_block : sh.analog_block;
+    int grids[7] = {0, 0, 0, 0, 0, 0, 0};  // short-history list, resume, last resume; query; long-history ones
+    for (int v = 0; v < 7; ++v) {
+        const int which = v < 4 ? v : v - 4;
+        const bool lng = v >= 4;
+        const void *kp = surr_kernel_ptr(ca, h->prec, which, lng);
+        const int block = which == 3 ? sh.query_block : lng ? sh.analog_block_long : sh.analog_block;
         const int smem = which == 3 ? sh.query_smem : sh.analog_smem;
         CK(h, raise_smem_limit(kp, smem));
         int per_sm = 0;
         CK(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kp, block, smem));
         if (per_sm < 1) return fail(h, IMC_ERR_CUDA, "surrogate transport kernel cannot be resident");
-        grids[which] = h->sm_count * per_sm;
+        grids[v] = h->sm_count * per_sm;
     }
-    sh.analog_grid = std::min(grids[0], std::min(grids[1], grids[2]));
+    sh.analog_grid.grid = std::min(grids[0], std::min(grids[1], grids[2]));
+    sh.analog_grid.grid_long = std::min(grids[4], std::min(grids[5], grids[6]));
     sh.query_grid = grids[3];
     int rc = surr_queue_alloc(h);
     if (rc) return rc;
@@ -1598,10 +1618,11 @@ int imc_get_surrogate_active(const ImcHandle *h, int *active) {
 
 int imc_kernels_per_step(const ImcHandle *h, int *count) {
     if (!h || !count) return IMC_ERR_INVALID_ARG;
-    // update, source x5, transport, compact x4, finalize + tally +
-    // energycheck + timestep; the surrogate transport is 1 + 2 kSurrRounds
-    // kernels
-    *count = 12 + (h->ca.surr_image ? 2 * kSurrRounds : 0);
+    // update, source x5, transport (in 1D the short- and the long-history
+    // kernel), compact x4, finalize + tally + energycheck + timestep; the
+    // surrogate transport is 1 + kSurrRounds analog passes, each both
+    // kernels, and kSurrRounds query passes
+    *count = h->geometry == IMC_GEOM_2D ? 12 : 13 + (h->ca.surr_image ? 3 * kSurrRounds : 0);
     return IMC_OK;
 }
 

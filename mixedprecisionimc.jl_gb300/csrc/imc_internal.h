@@ -142,9 +142,15 @@ struct TransportShape {
     bool dep_only;    // only the deposition tallies in shared memory
     int smem;         // dynamic shared memory bytes
     int block;        // threads per block
+    int block_long;   // of the long-history kernel (1D)
+};
+// blocks of a transport launch: of the only or the short-history kernel, and of
+// the 1D long-history kernel
+struct TransportGrid {
+    int grid, grid_long;
 };
 TransportShape transport_shape(const CellArgs &ca, int prec);
-void launch_transport(const CellArgs &ca, Scalars *sc, int prec, PBufPair bufs, int grid, cudaStream_t st);
+void launch_transport(const CellArgs &ca, Scalars *sc, int prec, PBufPair bufs, TransportGrid grid, cudaStream_t st);
 // 1D transport with the learned surrogate in thick cells (ca.surr_image set;
 // FP32 or FP16 state), as 1 + 2 kSurrRounds kernels per step: an analog pass
 // over the list that sets aside the histories that want a network query,
@@ -161,20 +167,21 @@ struct SurrWave {
     SurrQueue resume;   // continuing after a query
 };
 struct SurrShapes {
-    int analog_block, analog_smem, analog_grid;  // list pass
+    int analog_block, analog_block_long, analog_smem;  // list and resume passes
+    TransportGrid analog_grid;
     bool analog_smt;
     int query_block, query_smem, query_grid;     // query passes
 };
 SurrShapes surr_shapes(const CellArgs &ca, int prec);
 // the analog passes are the 1D transport kernel in its pass modes
 // (imc_transport.cu); which: 0 list pass, 1 resume pass, 2 last resume pass
-const void *surr_analog_ptr(const CellArgs &ca, int prec, int which);
+const void *surr_analog_ptr(const CellArgs &ca, int prec, int which, bool lng);
 int surr_analog_smem(const CellArgs &ca, int prec);
 void launch_surr_analog(const CellArgs &ca, Scalars *sc, int prec, PBufPair bufs, const SurrWave &w, int which,
-                        int round, int grid, int smem, cudaStream_t st);
+                        int round, TransportGrid grid, int smem, cudaStream_t st);
 // kernel pointers for attribute / occupancy set-up: which = 0 list pass,
 // 1 resume pass that sets aside, 2 last resume pass, 3 query pass
-const void *surr_kernel_ptr(const CellArgs &ca, int prec, int which);
+const void *surr_kernel_ptr(const CellArgs &ca, int prec, int which, bool lng);
 void launch_transport_surr(const CellArgs &ca, Scalars *sc, int prec, PBufPair bufs, const SurrWave &w,
                            const SurrShapes &sh, cudaStream_t st);
 // writes the tensor-core image of FP32 parameters into dst (device, kImageBytes)
@@ -198,7 +205,7 @@ void launch_finalize_tally(const CellArgs &ca, Scalars *sc, cudaStream_t st);
 void launch_tally_check_timestep(const CellArgs &ca, Scalars *sc, DevStats *stats, long long stats_cap,
                                  cudaStream_t st);
 void launch_prepare_transport(const CellArgs &ca, Scalars *sc, cudaStream_t st);
-const void *transport_kernel_ptr(const CellArgs &ca, int prec);
+const void *transport_kernel_ptr(const CellArgs &ca, int prec, bool lng);
 // One deck of the fused batch transport (1D): what the transport reads of
 // its CellArgs, and its two particle buffers' 1D arrays.  The fused kernel
 // reads them from constant memory (kFusedMaxDecks entries), so that, like a
@@ -226,8 +233,8 @@ constexpr int kFusedMaxDecks = 256;
 // of decks, launched (as a graph kernel node) with transport_multi_block
 // threads per block and the largest deck's dynamic shared memory over the
 // decks set by set_transport_multi_decks
-const void *transport_multi_ptr(int prec);
-int transport_multi_block(int prec);
+const void *transport_multi_ptr(int prec, bool lng);
+int transport_multi_block(int prec, bool lng);
 cudaError_t set_transport_multi_decks(const Deck1DArgs *ca, const PBufPair1D *bufs, Scalars *const *sc, int n,
                                       cudaStream_t st);
 

@@ -41,7 +41,7 @@ enum { kModePlain = 0, kModeList = 1, kModeResume = 2, kModeResumeLast = 3 };
 // and counters are flushed to the deck's before it returns; the caller puts a
 // barrier between two calls.  chunk: list entries a warp takes at a time in the
 // short-history schedule (0: by the list's length, list_chunk).
-template <class St, int BLOCK, int TM, int MODE, class CA, class BP>
+template <class St, int BLOCK, int TM, int MODE, bool LONG, class CA, class BP>
 __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, const BP &bufs, const SurrWave &w,
                                                   int round, unsigned char *smem_raw, int chunk) {
     constexpr bool SMT = TM != kTallyGlobal;      // deposition flushes to shared memory
@@ -322,7 +322,7 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
         segs += (unsigned long long)seg;
     };
     const int lane = threadIdx.x & 31;
-    if (sc->seg_per_hist < kRefillSegments) {
+    if constexpr (!LONG) {
         // Short histories (the last transport averaged fewer than
         // kRefillSegments segments each): each lane walks one history to its
         // end, and the warp moves on together to 32 consecutive entries, so
@@ -448,11 +448,17 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
     finish_counters(sc, segs, killed, flags, emax_e);
 }
 
-template <class St, int BLOCK, int TM, int MODE>
+// The two lane schedules are kernels of their own, so that neither holds the
+// other's registers and each has its own block size; a step launches both and
+// the one whose schedule the step does not take returns at once (~2 us).
+__device__ __forceinline__ bool long_histories(const Scalars *sc) { return sc->seg_per_hist >= kRefillSegments; }
+
+template <class St, int BLOCK, int TM, int MODE, bool LONG>
 __global__ void __launch_bounds__(BLOCK) k_transport1d(CellArgs ca, Scalars *sc, PBufPair bufs, SurrWave w,
                                                        int round) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    transport1d_block<St, BLOCK, TM, MODE>(ca, sc, bufs, w, round, smem_raw, 0);
+    if (long_histories(sc) != LONG) return;
+    transport1d_block<St, BLOCK, TM, MODE, LONG>(ca, sc, bufs, w, round, smem_raw, 0);
 }
 
 // One transport launch over the lists of many 1D decks (the fused batch,
@@ -467,7 +473,7 @@ __constant__ Deck1DArgs c_multi_ca[kFusedMaxDecks];
 __constant__ PBufPair1D c_multi_bufs[kFusedMaxDecks];
 __constant__ Scalars *c_multi_sc[kFusedMaxDecks];
 
-template <class St, int BLOCK>
+template <class St, int BLOCK, bool LONG>
 __global__ void __launch_bounds__(BLOCK) k_transport1d_multi(int ndecks) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int s_go;
@@ -478,12 +484,12 @@ __global__ void __launch_bounds__(BLOCK) k_transport1d_multi(int ndecks) {
             // the refill schedule (a stale, low counter only costs a setup)
             const long long n = *(volatile long long *)&sc->n_particles;
             const unsigned long long used = *(volatile unsigned long long *)&sc->work_next;
-            const long long per = *(volatile float *)&sc->seg_per_hist < kRefillSegments ? kListChunk1D : 32;
-            s_go = (long long)used * per < n;
+            const long long per = LONG ? 32 : kListChunk1D;
+            s_go = long_histories(sc) == LONG && (long long)used * per < n;
         }
         __syncthreads();
         if (s_go)
-            transport1d_block<St, BLOCK, kTallyShared, kModePlain>(c_multi_ca[d], sc, c_multi_bufs[d], SurrWave{}, 0,
+            transport1d_block<St, BLOCK, kTallyShared, kModePlain, LONG>(c_multi_ca[d], sc, c_multi_bufs[d], SurrWave{}, 0,
                                                                     smem_raw, kListChunk1D);
         __syncthreads();
     }
@@ -826,7 +832,7 @@ constexpr int kSmemBudget = 200 * 1024;
 constexpr int kSmemOptInMax = 227 * 1024;  // sm_100-family dynamic shared memory per block
 
 TransportShape transport_shape(const CellArgs &ca, int prec) {
-    TransportShape sh;
+    TransportShape sh{};
     const int tsz = prec == 0 ? 8 : 4;
     const int table = table_bytes(ca, tsz);
     const long long dep = 3ll * 8 * (long long)ca.K * ca.nc;
@@ -835,62 +841,78 @@ TransportShape transport_shape(const CellArgs &ca, int prec) {
     sh.smem = table + (int)(sh.smem_tally ? 2 * dep : sh.dep_only ? dep : 0);
     const bool shared = sh.smem_tally || sh.dep_only;
     sh.block = shared ? (prec == 0 ? kSmtBlock64 : kSmtBlock32) : (prec == 0 ? kGlbBlock64 : kGlbBlock32);
+    if (ca.geometry == 1) sh.block_long = prec == 0 ? sh.block : kLongBlock32;
     return sh;
 }
 
-// the plain 1D or 2D transport kernel of one state type, block size and
-// tally mode
-template <class St, int B, int TM> static const void *kptr(int geometry) {
-    if (geometry == 1) return (const void *)k_transport1d<St, B, TM, kModePlain>;
-    return (const void *)k_transport2d<St, B, TM>;
-}
-
-template <class St, int B, int TM>
-static void launch_one(const CellArgs &ca, Scalars *sc, PBufPair buf, int grid, int smem, cudaStream_t st) {
-    if (ca.geometry == 1) k_transport1d<St, B, TM, kModePlain><<<grid, B, smem, st>>>(ca, sc, buf, SurrWave{}, 0);
-    else k_transport2d<St, B, TM><<<grid, B, smem, st>>>(ca, sc, buf);
-}
-
 template <class St> struct StBlocks {
-    static constexpr int smt = sizeof(typename St::T) == 8 ? kSmtBlock64 : kSmtBlock32;
-    static constexpr int glb = sizeof(typename St::T) == 8 ? kGlbBlock64 : kGlbBlock32;
+    static constexpr bool fp64 = sizeof(typename St::T) == 8;
+    static constexpr int smt = fp64 ? kSmtBlock64 : kSmtBlock32;
+    static constexpr int glb = fp64 ? kGlbBlock64 : kGlbBlock32;
+    static constexpr int smt_long = fp64 ? kSmtBlock64 : kLongBlock32;
+    static constexpr int glb_long = fp64 ? kGlbBlock64 : kLongBlock32;
 };
 
-template <class St> static const void *kernel_of(const CellArgs &ca, const TransportShape &sh) {
-    if (sh.smem_tally) return kptr<St, StBlocks<St>::smt, kTallyShared>(ca.geometry);
-    if (sh.dep_only) return kptr<St, StBlocks<St>::smt, kTallySharedDep>(ca.geometry);
-    return kptr<St, StBlocks<St>::glb, kTallyGlobal>(ca.geometry);
+// the transport kernels of one state type and tally mode: 1D short histories,
+// 1D long histories, 2D
+template <class St, int TM> struct Kernels {
+    static constexpr int block = TM == kTallyGlobal ? StBlocks<St>::glb : StBlocks<St>::smt;
+    static constexpr int block_long = TM == kTallyGlobal ? StBlocks<St>::glb_long : StBlocks<St>::smt_long;
+    static const void *ptr(int geometry, bool lng) {
+        if (geometry == 2) return (const void *)k_transport2d<St, block, TM>;
+        if (lng) return (const void *)k_transport1d<St, block_long, TM, kModePlain, true>;
+        return (const void *)k_transport1d<St, block, TM, kModePlain, false>;
+    }
+    static void launch(const CellArgs &ca, Scalars *sc, PBufPair buf, TransportGrid g, int smem, cudaStream_t st) {
+        if (ca.geometry == 2) {
+            k_transport2d<St, block, TM><<<g.grid, block, smem, st>>>(ca, sc, buf);
+            return;
+        }
+        k_transport1d<St, block, TM, kModePlain, false><<<g.grid, block, smem, st>>>(ca, sc, buf, SurrWave{}, 0);
+        k_transport1d<St, block_long, TM, kModePlain, true><<<g.grid_long, block_long, smem, st>>>(ca, sc, buf,
+                                                                                                SurrWave{}, 0);
+    }
+};
+
+template <class St> static const void *kernel_of(const CellArgs &ca, const TransportShape &sh, bool lng) {
+    if (sh.smem_tally) return Kernels<St, kTallyShared>::ptr(ca.geometry, lng);
+    if (sh.dep_only) return Kernels<St, kTallySharedDep>::ptr(ca.geometry, lng);
+    return Kernels<St, kTallyGlobal>::ptr(ca.geometry, lng);
 }
 
 template <class St>
-static void launch_of(const CellArgs &ca, const TransportShape &sh, Scalars *sc, PBufPair buf, int grid,
+static void launch_of(const CellArgs &ca, const TransportShape &sh, Scalars *sc, PBufPair buf, TransportGrid g,
                       cudaStream_t st) {
-    if (sh.smem_tally) launch_one<St, StBlocks<St>::smt, kTallyShared>(ca, sc, buf, grid, sh.smem, st);
-    else if (sh.dep_only) launch_one<St, StBlocks<St>::smt, kTallySharedDep>(ca, sc, buf, grid, sh.smem, st);
-    else launch_one<St, StBlocks<St>::glb, kTallyGlobal>(ca, sc, buf, grid, sh.smem, st);
+    if (sh.smem_tally) Kernels<St, kTallyShared>::launch(ca, sc, buf, g, sh.smem, st);
+    else if (sh.dep_only) Kernels<St, kTallySharedDep>::launch(ca, sc, buf, g, sh.smem, st);
+    else Kernels<St, kTallyGlobal>::launch(ca, sc, buf, g, sh.smem, st);
 }
 
-const void *transport_kernel_ptr(const CellArgs &ca, int prec) {
+const void *transport_kernel_ptr(const CellArgs &ca, int prec, bool lng) {
     TransportShape sh = transport_shape(ca, prec);
-    if (prec == 0) return kernel_of<StF64>(ca, sh);
-    if (prec == 1) return kernel_of<StF32>(ca, sh);
-    return kernel_of<StF16>(ca, sh);
+    if (prec == 0) return kernel_of<StF64>(ca, sh, lng);
+    if (prec == 1) return kernel_of<StF32>(ca, sh, lng);
+    return kernel_of<StF16>(ca, sh, lng);
 }
 
-void launch_transport(const CellArgs &ca, Scalars *sc, int prec, PBufPair buf, int grid, cudaStream_t st) {
+void launch_transport(const CellArgs &ca, Scalars *sc, int prec, PBufPair buf, TransportGrid g, cudaStream_t st) {
     TransportShape sh = transport_shape(ca, prec);
-    if (prec == 0) launch_of<StF64>(ca, sh, sc, buf, grid, st);
-    else if (prec == 1) launch_of<StF32>(ca, sh, sc, buf, grid, st);
-    else launch_of<StF16>(ca, sh, sc, buf, grid, st);
+    if (prec == 0) launch_of<StF64>(ca, sh, sc, buf, g, st);
+    else if (prec == 1) launch_of<StF32>(ca, sh, sc, buf, g, st);
+    else launch_of<StF16>(ca, sh, sc, buf, g, st);
 }
 
-const void *transport_multi_ptr(int prec) {
-    if (prec == 0) return (const void *)k_transport1d_multi<StF64, kSmtBlock64>;
-    if (prec == 1) return (const void *)k_transport1d_multi<StF32, kSmtBlock32>;
-    return (const void *)k_transport1d_multi<StF16, kSmtBlock32>;
+template <class St> static const void *multi_ptr(bool lng) {
+    if (lng) return (const void *)k_transport1d_multi<St, StBlocks<St>::smt_long, true>;
+    return (const void *)k_transport1d_multi<St, StBlocks<St>::smt, false>;
+}
+const void *transport_multi_ptr(int prec, bool lng) {
+    return prec == 0 ? multi_ptr<StF64>(lng) : prec == 1 ? multi_ptr<StF32>(lng) : multi_ptr<StF16>(lng);
 }
 
-int transport_multi_block(int prec) { return prec == 0 ? kSmtBlock64 : kSmtBlock32; }
+int transport_multi_block(int prec, bool lng) {
+    return prec == 0 ? kSmtBlock64 : lng ? kLongBlock32 : kSmtBlock32;
+}
 
 cudaError_t set_transport_multi_decks(const Deck1DArgs *ca, const PBufPair1D *bufs, Scalars *const *sc, int n,
                                       cudaStream_t st) {
@@ -908,39 +930,53 @@ cudaError_t set_transport_multi_decks(const Deck1DArgs *ca, const PBufPair1D *bu
 
 // ------------------------------------------- analog passes of the surrogate transport
 // which: 0 the list pass, 1 a resume pass that sets aside, 2 the last resume pass
-template <class St, int B, bool SMT> static const void *wave_ptr(int which) {
-    if (which == 0) return (const void *)k_transport1d<St, B, SMT, kModeList>;
-    if (which == 1) return (const void *)k_transport1d<St, B, SMT, kModeResume>;
-    return (const void *)k_transport1d<St, B, SMT, kModeResumeLast>;
+template <class St, bool SMT, int MODE> struct WaveKernels {
+    static constexpr int tm = SMT ? kTallyShared : kTallyGlobal;
+    static constexpr int block = SMT ? kSmtBlock32 : kGlbBlock32;
+    static const void *ptr(bool lng) {
+        if (lng) return (const void *)k_transport1d<St, kLongBlock32, tm, MODE, true>;
+        return (const void *)k_transport1d<St, block, tm, MODE, false>;
+    }
+    static void launch(const CellArgs &ca, Scalars *sc, PBufPair bufs, const SurrWave &w, int round, TransportGrid g,
+                       int smem, cudaStream_t st) {
+        k_transport1d<St, block, tm, MODE, false><<<g.grid, block, smem, st>>>(ca, sc, bufs, w, round);
+        k_transport1d<St, kLongBlock32, tm, MODE, true><<<g.grid_long, kLongBlock32, smem, st>>>(ca, sc, bufs, w, round);
+    }
+};
+
+template <class St, bool SMT> static const void *wave_ptr(int which, bool lng) {
+    if (which == 0) return WaveKernels<St, SMT, kModeList>::ptr(lng);
+    if (which == 1) return WaveKernels<St, SMT, kModeResume>::ptr(lng);
+    return WaveKernels<St, SMT, kModeResumeLast>::ptr(lng);
 }
 
-const void *surr_analog_ptr(const CellArgs &ca, int prec, int which) {
+const void *surr_analog_ptr(const CellArgs &ca, int prec, int which, bool lng) {
     const bool smt = transport_shape(ca, prec).smem_tally;
-    if (prec == 2) return smt ? wave_ptr<StF16, kSmtBlock32, true>(which) : wave_ptr<StF16, kGlbBlock32, false>(which);
-    return smt ? wave_ptr<StF32, kSmtBlock32, true>(which) : wave_ptr<StF32, kGlbBlock32, false>(which);
+    if (prec == 2) return smt ? wave_ptr<StF16, true>(which, lng) : wave_ptr<StF16, false>(which, lng);
+    return smt ? wave_ptr<StF32, true>(which, lng) : wave_ptr<StF32, false>(which, lng);
 }
 
 int surr_analog_smem(const CellArgs &ca, int prec) {
     return analog1d_smem(ca, 4, transport_shape(ca, prec).smem_tally, true);
 }
 
-template <class St, int B, bool SMT>
+template <class St, bool SMT>
 static void wave_one(const CellArgs &ca, Scalars *sc, PBufPair bufs, const SurrWave &w, int which, int round,
-                     int grid, int smem, cudaStream_t st) {
-    if (which == 0) k_transport1d<St, B, SMT, kModeList><<<grid, B, smem, st>>>(ca, sc, bufs, w, round);
-    else if (which == 1) k_transport1d<St, B, SMT, kModeResume><<<grid, B, smem, st>>>(ca, sc, bufs, w, round);
-    else k_transport1d<St, B, SMT, kModeResumeLast><<<grid, B, smem, st>>>(ca, sc, bufs, w, round);
+                     TransportGrid g, int smem, cudaStream_t st) {
+    if (which == 0) WaveKernels<St, SMT, kModeList>::launch(ca, sc, bufs, w, round, g, smem, st);
+    else if (which == 1) WaveKernels<St, SMT, kModeResume>::launch(ca, sc, bufs, w, round, g, smem, st);
+    else WaveKernels<St, SMT, kModeResumeLast>::launch(ca, sc, bufs, w, round, g, smem, st);
 }
 
 void launch_surr_analog(const CellArgs &ca, Scalars *sc, int prec, PBufPair bufs, const SurrWave &w, int which,
-                        int round, int grid, int smem, cudaStream_t st) {
+                        int round, TransportGrid g, int smem, cudaStream_t st) {
     const bool smt = transport_shape(ca, prec).smem_tally;
     if (prec == 2) {
-        if (smt) wave_one<StF16, kSmtBlock32, true>(ca, sc, bufs, w, which, round, grid, smem, st);
-        else wave_one<StF16, kGlbBlock32, false>(ca, sc, bufs, w, which, round, grid, smem, st);
+        if (smt) wave_one<StF16, true>(ca, sc, bufs, w, which, round, g, smem, st);
+        else wave_one<StF16, false>(ca, sc, bufs, w, which, round, g, smem, st);
     } else {
-        if (smt) wave_one<StF32, kSmtBlock32, true>(ca, sc, bufs, w, which, round, grid, smem, st);
-        else wave_one<StF32, kGlbBlock32, false>(ca, sc, bufs, w, which, round, grid, smem, st);
+        if (smt) wave_one<StF32, true>(ca, sc, bufs, w, which, round, g, smem, st);
+        else wave_one<StF32, false>(ca, sc, bufs, w, which, round, g, smem, st);
     }
 }
 

@@ -238,6 +238,11 @@ constexpr int kSmtBlock64 = 512;
 // tallies do not fit): FP32 / FP16 state as one 1024-thread block per SM,
 // FP64 in 256-thread blocks
 constexpr int kGlbBlock32 = 1024;
+// the 1D long-history kernels of FP32 / FP16 state: 80 registers a thread keep
+// the history and its random words out of local memory, and the schedule loses
+// nothing by eight warps less (heat wave 163 -> 162 ms, thick slab 51.9 -> 50.3
+// ms at 768 against 1024 threads; the short-history kernel 402 -> 452 us)
+constexpr int kLongBlock32 = 768;
 constexpr int kGlbBlock64 = 256;
 
 // 1D per-cell table: sigma_a f, effective scatter, width * distancescale;

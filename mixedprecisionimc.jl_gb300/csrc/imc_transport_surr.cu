@@ -349,6 +349,7 @@ SurrShapes surr_shapes(const CellArgs &ca, int prec) {
     SurrShapes s{};
     const TransportShape ts = transport_shape(ca, prec);
     s.analog_block = ts.block;
+    s.analog_block_long = ts.block_long;
     s.analog_smem = surr_analog_smem(ca, prec);
     s.analog_smt = ts.smem_tally;
     s.query_block = kQueryBlock;
@@ -356,9 +357,9 @@ SurrShapes surr_shapes(const CellArgs &ca, int prec) {
     return s;
 }
 
-const void *surr_kernel_ptr(const CellArgs &ca, int prec, int which) {
+const void *surr_kernel_ptr(const CellArgs &ca, int prec, int which, bool lng) {
     if (which == 3) return prec == 2 ? (const void *)k_wave_query<StF16> : (const void *)k_wave_query<StF32>;
-    return surr_analog_ptr(ca, prec, which);
+    return surr_analog_ptr(ca, prec, which, lng);
 }
 
 void launch_transport_surr(const CellArgs &ca, Scalars *sc, int prec, PBufPair bufs, const SurrWave &w,
