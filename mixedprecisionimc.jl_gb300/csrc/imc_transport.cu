@@ -105,7 +105,8 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
     T prv_s = (T)0, prv_c = (T)0;
     unsigned seg = 0;
     Stream rs;  // FP64
-    Words ws;   // FP32
+    Words<LONG ? 7 : 5> ws;  // FP32
+    int need = 2;            // words a segment starts with: 2, or 2 and 4 in turn for the whole warp
     auto start = [&](int cs_now) {
         cell = cs_now & 0xFFFFFF;
         k = cs_now >> 24;
@@ -180,8 +181,8 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
             bool at_b, at_col, at_cen, odd = false;  // odd (FP64): a distance below +0 or not a number
             T dist_col;
             if constexpr (sizeof(T) == 4) {
-                if (ws.n < 2) ws.refill(round_keys(ca), step, stage);
-                dist_col = M::flight(ws.w0, ce);
+                if (ws.n < need) ws.refill(round_keys(ca), step, stage);
+                dist_col = M::flight(ws.w[0], ce);
                 dist_b = mu > (T)0 ? (ce.dxs - x) * rmu : m_abs(x * rmu);
                 dist_cen = c * (endsteptime - t) * ds;
                 dist = min3_nan(dist_b, dist_col, dist_cen);
@@ -262,11 +263,11 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
                         // mu = 1 - 2*rand, redrawn while zero (src/imc_transport.jl:178-181);
                         // a zero needs rand == 0.5 exactly, so 64 redraws never run out
                         if constexpr (sizeof(T) == 4) {
-                            mu = Rand<T>::cosine(ws.w1);
+                            mu = Rand<T>::cosine(ws.w[1]);
                             for (int r = 1; r < 64 && mu == (T)0; ++r) {
                                 ws.drop(false);
                                 if (ws.n < 2) ws.refill(round_keys(ca), step, stage);
-                                mu = Rand<T>::cosine(ws.w1);
+                                mu = Rand<T>::cosine(ws.w[1]);
                             }
                         } else {
                             mu = (T)0;
@@ -432,6 +433,7 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
                 idle = __ballot_sync(0xFFFFFFFFu, !has);
             }
             if (idle == 0xFFFFFFFFu) break;  // no history left for this warp
+            need ^= 6;
             if (!has) continue;
             const int end = segment();
             if (end) {
