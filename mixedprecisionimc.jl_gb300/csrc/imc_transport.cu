@@ -95,14 +95,10 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
     int emax_e = kNoExp;
     // Lane state of the history in flight (cs: as stored in the list; the
     // current cell and scale are cell, k).  Deposits go to the compensated
-    // pair (acc_s, acc_c) of the current cell acc_cell; the pair of the cell
-    // the history left last waits in (prv_s, prv_c, prv_cell) and is flushed
-    // only when a third cell is entered, so a history that visits at most
-    // two cells flushes both pairs at its end, with the warp converged.
+    // pair (acc_s, acc_c) of the current cell, flushed when it is left.
     long long i = 0;
-    int cs = 0, cell = 0, k = 0, acc_cell = 0, prv_cell = -1;
+    int cs = 0, cell = 0, k = 0;
     T t = (T)0, x = (T)0, mu = (T)0, E = (T)0, E0 = (T)0, minenergy = (T)0, acc_s = (T)0, acc_c = (T)0, rmu = (T)0;
-    T prv_s = (T)0, prv_c = (T)0;
     unsigned seg = 0;
     Stream rs;  // FP64
     Words<LONG ? 7 : 5> ws;  // FP32
@@ -115,8 +111,6 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
         minenergy = cutoff_energy(E0);  // (T)(0.01 * (double)E0), without FP64 in binary32
         acc_s = (T)0;
         acc_c = (T)0;
-        acc_cell = cell;
-        prv_cell = -1;
         seg = 0;
         rmu = (T)1 / mu;  // the face distance as a product (reset at each new direction)
     };
@@ -144,14 +138,9 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
         }
         return true;
     };
-    // the history is in `cell`: on a cell change the current pair moves to
-    // the waiting slot, whose earlier pair (a third cell) is flushed now
-    auto enter_cell = [&]() {
-        if (cell != acc_cell) {
-            if (prv_cell >= 0) flush_pair<T, SMT>(dep_acc, k * nc + prv_cell, prv_s, prv_c, b_dep + s_sexp[k], flags);
-            prv_cell = acc_cell; prv_s = acc_s; prv_c = acc_c;
-            acc_s = (T)0; acc_c = (T)0; acc_cell = cell;
-        }
+    // the deposits of the cell the history leaves, or ends in
+    auto flush_cell = [&]() {
+        flush_pair<T, SMT>(dep_acc, k * nc + cell, acc_s, acc_c, b_dep + s_sexp[k], flags);
     };
     // one pass of the reference's while loop; 0 = go on, 1 = killed, 2 =
     // census, 3 = set aside for a query (kPause), 4 = escaped through a
@@ -162,7 +151,6 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
             Query q;
             const int kind = surr_decide<T>(tab[cell], x, mu, t, E, minenergy, c, ds, endsteptime, q);
             if (kind == kCertainKill) {
-                enter_cell();
                 nadd(acc_s, acc_c, M::all_in(E, tab[cell]));
                 ++seg;
                 ++calls;
@@ -170,125 +158,140 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
             }
             if (kind == kAsk) return 3;
         }
-        int end = 0;
-        // one pass of the reference's while loop (src/imc_transport.jl:73-195)
         if (++seg > cap) {
             flags |= (1u << 2);
-            end = 1;
+            return 1;
+        }
+        const Tab1<T> ce = tab[cell];
+        int end = 0;
+        if constexpr (sizeof(T) == 4) {
+            // Written without branches but for the rare cases and the flush: a
+            // warp's lanes collide, cross and end in one and the same segment,
+            // and each branch would run for a few of them at a time.
+            if (ws.n < need) ws.refill(round_keys(ca), step, stage);
+            const bool right = mu > (T)0;
+            const T dist_col = M::flight(ws.w[0], ce);
+            const T dist_b = right ? (ce.dxs - x) * rmu : m_abs(x * rmu);
+            const T dist_cen = c * (endsteptime - t) * ds;
+            const T dist = min3_nan(dist_b, dist_col, dist_cen);
+            if (dist != dist) {
+                flags |= 1u;
+                return 1;
+            }
+            T dep;
+            const T newenergy = M::attenuate(E, ce, dist, &dep);
+            const bool dead = newenergy <= minenergy;
+            nadd(acc_s, acc_c, dead ? M::all_in(E, ce) : dep);
+            x += mu * dist;
+            t += dist * rdsc;
+            E = newenergy;
+            // the events in the reference's order: face, collision, census
+            const bool at_b = !dead && dist == dist_b;
+            const int next = cell + (right ? 1 : -1);
+            const bool inside = (unsigned)next < (unsigned)N;
+            if (at_b && inside) {
+                flush_cell();
+                acc_s = (T)0;
+                acc_c = (T)0;
+                cell = next;
+                x = right ? (T)0 : tab[next].dxs;
+            }
+            bool escaped = false;
+            if (at_b && !inside) {
+                // the escape, or the reflection, which leaves a right mover on
+                // its face (the reference steps out and back in)
+                escaped = !(right ? reflect_r : reflect_l);
+                mu = -mu;
+                rmu = -rmu;
+                if (right) x = ce.dxs;
+            }
+            const bool turn = dist == dist_col;
+            // mu = 1 - 2*rand, redrawn while zero (src/imc_transport.jl:178-181);
+            // a zero needs rand == 0.5 exactly, so 64 redraws never run out
+            T mu_new = Rand<T>::cosine(ws.w[1]);
+            if (turn && mu_new == (T)0) {
+                for (int r = 1; r < 64 && mu_new == (T)0; ++r) {
+                    ws.drop(false);
+                    if (ws.n < 2) ws.refill(round_keys(ca), step, stage);
+                    mu_new = Rand<T>::cosine(ws.w[1]);
+                }
+                if (mu_new == (T)0) mu_new = (T)1;
+            }
+            const T rmu_new = rcp_cosine(mu_new);
+            mu = turn ? mu_new : mu;
+            rmu = turn ? rmu_new : rmu;
+            ws.drop(turn);
+            // census: t = 0 and the state written back by finish()
+            // (src/imc_transport.jl:185-193)
+            end = dead ? 1 : escaped ? 4 : dist == dist_cen ? 2 : 0;
         } else {
-            const Tab1<T> ce = tab[cell];
-            T dist_b, dist_cen, dist;
-            bool at_b, at_col, at_cen, odd = false;  // odd (FP64): a distance below +0 or not a number
-            T dist_col;
-            if constexpr (sizeof(T) == 4) {
-                if (ws.n < need) ws.refill(round_keys(ca), step, stage);
-                dist_col = M::flight(ws.w[0], ce);
-                dist_b = mu > (T)0 ? (ce.dxs - x) * rmu : m_abs(x * rmu);
-                dist_cen = c * (endsteptime - t) * ds;
-                dist = min3_nan(dist_b, dist_col, dist_cen);
+            // FP64: every FP64 instruction costs more than a branch
+            T dist_b, dist_cen, dist, dep;
+            bool at_b, at_col, at_cen;
+            const T dist_col = M::flight(rs, ce);
+            const bool fwd = pos64(mu);
+            dist_b = m64::div_r(fwd ? ce.dxs - x : x, mu, rmu);
+            if (!fwd) dist_b = m_abs(dist_b);
+            dist_cen = endsteptime - t;
+            if (!c_one) dist_cen = c * dist_cen;
+            if (!ds_one) dist_cen = dist_cen * ds;
+            // odd: a distance below +0 or not a number
+            const bool odd = !(plain64(dist_b) && plain64(dist_col) && plain64(dist_cen));
+            if (!odd) {
+                dist = min64(min64(dist_b, dist_col), dist_cen);
+                at_b = m64::bits(dist) == m64::bits(dist_b);
+                at_col = m64::bits(dist) == m64::bits(dist_col);
+                at_cen = m64::bits(dist) == m64::bits(dist_cen);
+            } else {
+                dist_b = mu > (T)0 ? (ce.dxs - x) / mu : m_abs(x / mu);
+                dist = jmin(jmin(dist_b, dist_col), dist_cen);
                 at_b = dist == dist_b;
                 at_col = dist == dist_col;
                 at_cen = dist == dist_cen;
-            } else {
-                dist_col = M::flight(rs, ce);
-                const bool fwd = pos64(mu);
-                dist_b = m64::div_r(fwd ? ce.dxs - x : x, mu, rmu);
-                if (!fwd) dist_b = m_abs(dist_b);
-                dist_cen = endsteptime - t;
-                if (!c_one) dist_cen = c * dist_cen;
-                if (!ds_one) dist_cen = dist_cen * ds;
-                odd = !(plain64(dist_b) && plain64(dist_col) && plain64(dist_cen));
-                if (!odd) {
-                    dist = min64(min64(dist_b, dist_col), dist_cen);
-                    at_b = m64::bits(dist) == m64::bits(dist_b);
-                    at_col = m64::bits(dist) == m64::bits(dist_col);
-                    at_cen = m64::bits(dist) == m64::bits(dist_cen);
-                } else {
-                    dist_b = mu > (T)0 ? (ce.dxs - x) / mu : m_abs(x / mu);
-                    dist = jmin(jmin(dist_b, dist_col), dist_cen);
-                    at_b = dist == dist_b;
-                    at_col = dist == dist_col;
-                    at_cen = dist == dist_cen;
+                if (dist != dist) {
+                    flags |= 1u;
+                    return 1;
                 }
             }
-            if (odd ? dist != dist : sizeof(T) == 4 && dist != dist) {
-                flags |= 1u;
-                end = 1;
-            } else {
-                T dep, newenergy;
-                bool dead;
-                if constexpr (sizeof(T) == 4) {
-                    newenergy = M::attenuate(E, ce, dist, &dep);
-                    dead = newenergy <= minenergy;
+            const T newenergy = M::attenuate(E, ce.saf, dist, odd, &dep);
+            const bool dead = le64(newenergy, minenergy);
+            nadd(acc_s, acc_c, dead ? E : dep);
+            if (dead) return 1;
+            x = fma(mu, dist, x);
+            T dt_seg = ds_one ? dist : m64::div_r(dist, ds, rds);
+            if (!c_one) dt_seg = m64::div_r(dt_seg, c, rc);
+            t += dt_seg;
+            E = newenergy;
+            if (at_b) {
+                const bool right = mu > (T)0;
+                const int next = cell + (right ? 1 : -1);
+                if ((unsigned)next < (unsigned)N) {
+                    flush_cell();
+                    acc_s = (T)0;
+                    acc_c = (T)0;
+                    cell = next;
+                    x = right ? (T)0 : tab[next].dxs;
+                } else if (right ? reflect_r : reflect_l) {
+                    mu = -mu;
+                    rmu = -rmu;
+                    if (right) x = ce.dxs;
                 } else {
-                    newenergy = M::attenuate(E, ce.saf, dist, odd, &dep);
-                    dead = le64(newenergy, minenergy);
-                }
-                enter_cell();
-                if (dead) {
-                    nadd(acc_s, acc_c, M::all_in(E, ce));
-                    end = 1;
-                } else {
-                    nadd(acc_s, acc_c, dep);
-                    if constexpr (sizeof(T) == 4) {
-                        x += mu * dist;
-                        t += dist * rdsc;
-                    } else {
-                        x = fma(mu, dist, x);
-                        T dt_seg = ds_one ? dist : m64::div_r(dist, ds, rds);
-                        if (!c_one) dt_seg = m64::div_r(dt_seg, c, rc);
-                        t += dt_seg;
-                    }
-                    E = newenergy;
-                    if (at_b) {
-                        // through the right face (mu > 0) or the left one: the
-                        // next cell, or at the domain's end the escape or the
-                        // reflection, which leaves a right mover on its face
-                        // (the reference steps out and back in)
-                        const bool right = mu > (T)0;
-                        const int next = cell + (right ? 1 : -1);
-                        if ((unsigned)next < (unsigned)N) {
-                            cell = next;
-                            x = right ? (T)0 : tab[next].dxs;
-                        } else if (right ? reflect_r : reflect_l) {
-                            mu = -mu;
-                            rmu = -rmu;
-                            if (right) x = ce.dxs;
-                        } else {
-                            end = 4;
-                        }
-                    }
-                    const bool turn = !end && at_col;
-                    if (turn) {
-                        // mu = 1 - 2*rand, redrawn while zero (src/imc_transport.jl:178-181);
-                        // a zero needs rand == 0.5 exactly, so 64 redraws never run out
-                        if constexpr (sizeof(T) == 4) {
-                            mu = Rand<T>::cosine(ws.w[1]);
-                            for (int r = 1; r < 64 && mu == (T)0; ++r) {
-                                ws.drop(false);
-                                if (ws.n < 2) ws.refill(round_keys(ca), step, stage);
-                                mu = Rand<T>::cosine(ws.w[1]);
-                            }
-                        } else {
-                            mu = (T)0;
-                            for (int r = 0; r < 64 && mu == (T)0; ++r) mu = Rand<T>::cosine(rs);
-                        }
-                        if (mu == (T)0) mu = (T)1;
-                        rmu = (T)1 / mu;
-                    }
-                    if constexpr (sizeof(T) == 4) ws.drop(turn);
-                    // census: t = 0 and the state written back by finish()
-                    // (src/imc_transport.jl:185-193)
-                    if (!end && at_cen) end = 2;
+                    return 4;
                 }
             }
+            if (at_col) {
+                mu = (T)0;
+                for (int r = 0; r < 64 && mu == (T)0; ++r) mu = Rand<T>::cosine(rs);
+                if (mu == (T)0) mu = (T)1;
+                rmu = (T)1 / mu;
+            }
+            if (at_cen) end = 2;
         }
         return end;
     };
     auto finish = [&](int end) {
         const int se = s_sexp[k];
-        if (prv_cell >= 0) flush_pair<T, SMT>(dep_acc, k * nc + prv_cell, prv_s, prv_c, b_dep + se, flags);
-        flush_pair<T, SMT>(dep_acc, k * nc + acc_cell, acc_s, acc_c, b_dep + se, flags);
+        flush_cell();
         if (end == 2) {
             // census: t = 0, write the state back (src/imc_transport.jl:185-193)
             T Est = E;

@@ -27,15 +27,14 @@ __device__ __forceinline__ void m_sincos(double a, double *s, double *c) { sinco
 // of sigma_a f d below 1/16 -- every segment of the slab decks -- take the
 // series.  The oracle's FP32 path evaluates the same expression.
 __device__ __forceinline__ float expm1_seg(float x) {
-    if (fabsf(x) <= 0.0625f) {
-        float p = fmaf(x, 1.0f / 5040.0f, 1.0f / 720.0f);
-        p = fmaf(p, x, 1.0f / 120.0f);
-        p = fmaf(p, x, 1.0f / 24.0f);
-        p = fmaf(p, x, 1.0f / 6.0f);
-        p = fmaf(p, x, 0.5f);
-        return fmaf(p * x, x, x);
-    }
-    return expm1f(x);
+    float p = fmaf(x, 1.0f / 5040.0f, 1.0f / 720.0f);
+    p = fmaf(p, x, 1.0f / 120.0f);
+    p = fmaf(p, x, 1.0f / 24.0f);
+    p = fmaf(p, x, 1.0f / 6.0f);
+    p = fmaf(p, x, 0.5f);
+    p = fmaf(p * x, x, x);
+    if (fabsf(x) > 0.0625f) p = expm1f(x);
+    return p;
 }
 
 // Neumaier compensated add; all deposit terms are non-negative.
