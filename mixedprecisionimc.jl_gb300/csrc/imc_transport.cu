@@ -97,7 +97,10 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
     // current cell and scale are cell, k).  Deposits go to the compensated
     // pair (acc_s, acc_c) of the current cell, flushed when it is left.
     long long i = 0;
-    int cs = 0, cell = 0, k = 0;
+    int cs = 0, cell = 0, k = 0, se = 0;  // se: scale k's exponent
+    // shared tallies: scale k's deposition slots, and from there to its census slots
+    const unsigned dep_shared = SMT ? (unsigned)__cvta_generic_to_shared(dep_acc) : 0u;
+    unsigned slots_k = 0;
     T t = (T)0, x = (T)0, mu = (T)0, E = (T)0, E0 = (T)0, minenergy = (T)0, acc_s = (T)0, acc_c = (T)0, rmu = (T)0;
     unsigned seg = 0;
     Stream rs;  // FP64
@@ -106,13 +109,16 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
     auto start = [&](int cs_now) {
         cell = cs_now & 0xFFFFFF;
         k = cs_now >> 24;
+        se = s_sexp[k];
+        if constexpr (SMT) slots_k = dep_shared + 24u * (unsigned)(k * nc);
         if constexpr (sizeof(T) == 8) rs.init(seed, step, (uint32_t)i, stage);
-        else ws.init((uint32_t)i);
+        else if constexpr (LONG) ws.init((uint32_t)i);
+        else ws.init_full((uint32_t)i, round_keys(ca), step, stage);
         minenergy = cutoff_energy(E0);  // (T)(0.01 * (double)E0), without FP64 in binary32
         acc_s = (T)0;
         acc_c = (T)0;
         seg = 0;
-        rmu = (T)1 / mu;  // the face distance as a product (reset at each new direction)
+        rmu = rcp_any(mu);  // the face distance as a product (reset at each new direction)
     };
     // one entry of the list (or of the resume queue): false if it holds no history
     auto load = [&](long long e, int &cs_now, T &lt, T &lx, T &lmu, T &lE, T &lE0, long long &li, int &lcs) -> bool {
@@ -140,7 +146,10 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
     };
     // the deposits of the cell the history leaves, or ends in
     auto flush_cell = [&]() {
-        flush_pair<T, SMT>(dep_acc, k * nc + cell, acc_s, acc_c, b_dep + s_sexp[k], flags);
+        const T v = acc_s + acc_c;
+        if constexpr (SMT && sizeof(T) == 4)
+            if (add_f32_smem(slots_k + 24u * (unsigned)cell, v, b_dep + se)) return;
+        flush_rest<T, SMT>(dep_acc, k * nc + cell, v, b_dep + se, flags);
     };
     // one pass of the reference's while loop; 0 = go on, 1 = killed, 2 =
     // census, 3 = set aside for a query (kPause), 4 = escaped through a
@@ -208,19 +217,28 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
             const bool turn = dist == dist_col;
             // mu = 1 - 2*rand, redrawn while zero (src/imc_transport.jl:178-181);
             // a zero needs rand == 0.5 exactly, so 64 redraws never run out
-            T mu_new = Rand<T>::cosine(ws.w[1]);
-            if (turn && mu_new == (T)0) {
-                for (int r = 1; r < 64 && mu_new == (T)0; ++r) {
-                    ws.drop(false);
-                    if (ws.n < 2) ws.refill(round_keys(ca), step, stage);
-                    mu_new = Rand<T>::cosine(ws.w[1]);
+            auto new_direction = [&]() {
+                T m = Rand<T>::cosine(ws.w[1]);
+                if (turn && m == (T)0) {
+                    for (int r = 1; r < 64 && m == (T)0; ++r) {
+                        ws.drop(false);
+                        if (ws.n < 2) ws.refill(round_keys(ca), step, stage);
+                        m = Rand<T>::cosine(ws.w[1]);
+                    }
+                    if (m == (T)0) m = (T)1;
                 }
-                if (mu_new == (T)0) mu_new = (T)1;
+                const T rm = rcp_mid(m);
+                mu = turn ? m : mu;
+                rmu = turn ? rm : rmu;
+                ws.drop(turn);
+            };
+            if constexpr (LONG) {
+                new_direction();
+            } else {
+                // a short history seldom collides
+                if (turn) new_direction();
+                else ws.drop(false);
             }
-            const T rmu_new = rcp_cosine(mu_new);
-            mu = turn ? mu_new : mu;
-            rmu = turn ? rmu_new : rmu;
-            ws.drop(turn);
             // census: t = 0 and the state written back by finish()
             // (src/imc_transport.jl:185-193)
             end = dead ? 1 : escaped ? 4 : dist == dist_cen ? 2 : 0;
@@ -290,7 +308,6 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
         return end;
     };
     auto finish = [&](int end) {
-        const int se = s_sexp[k];
         flush_cell();
         if (end == 2) {
             // census: t = 0, write the state back (src/imc_transport.jl:185-193)
@@ -309,7 +326,10 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
                 pb.E[i] = (typename St::S)E;
             }
             if (cell != (cs & 0xFFFFFF)) pb.cs[i] = cell | (k << 24);
-            flush_one<T, RAD_SMT>(rad_acc, k * nc + cell, Est, b_rad + se, flags);
+            bool flushed = false;
+            if constexpr (RAD_SMT && sizeof(T) == 4)
+                flushed = add_f32_smem(slots_k + 24u * (unsigned)(ca.K * nc + cell), Est, b_rad + se);
+            if (!flushed) flush_rest<T, RAD_SMT>(rad_acc, k * nc + cell, Est, b_rad + se, flags);
             const int ee = exp_bound(Est) - se;
             emax_e = ee > emax_e ? ee : emax_e;
         } else if (end == 3) {

@@ -104,13 +104,16 @@ __device__ __forceinline__ void add_words_u(unsigned addr, unsigned lo, unsigned
                  "@r red.shared.add.u32 [%0 + 8], 1;\n\t}"
                  :: "r"(addr), "r"(lo), "r"(hi) : "memory");
 }
-__device__ __forceinline__ bool add_f32_smem(long long *slot, float v, int b) {
+// slot: its address in the shared window
+__device__ __forceinline__ bool add_f32_smem(unsigned slot, float v, int b) {
     int j;
     uint32_t lo, hi;
     if (!f32_words(v, b, j, lo, hi)) return false;
-    const unsigned a = (unsigned)__cvta_generic_to_shared(slot) + 8u - 4u * (unsigned)j;
-    add_words_u(a, lo, hi);
+    add_words_u(slot + 8u - 4u * (unsigned)j, lo, hi);
     return true;
+}
+__device__ __forceinline__ bool add_f32_smem(long long *slot, float v, int b) {
+    return add_f32_smem((unsigned)__cvta_generic_to_shared(slot), v, b);
 }
 
 template <bool SMT> __device__ __forceinline__ void add_limbs(long long *a, const Limbs &L) {
@@ -182,13 +185,11 @@ __device__ __forceinline__ void flush_block_tallies(const CA &ca, const long lon
     }
 }
 
-// flush a compensated pair: the Neumaier result s + c, converted once
+// a value that add_f32_smem did not take: its exact conversion and adds in the
+// general form
 template <class T, bool SMT>
-__device__ __forceinline__ void flush_pair(long long *acc, int slot, T s, T c, int b, unsigned &flags) {
-    const T v = s + c;
+__device__ __forceinline__ void flush_rest(long long *acc, int slot, T v, int b, unsigned &flags) {
     if (v == (T)0) return;
-    if constexpr (SMT && sizeof(T) == 4)
-        if (add_f32_smem(acc + 3 * (size_t)slot, v, b)) return;
     Limbs A;
     if (!fix_split(v, b, A)) {
         flags |= (v != v) ? 1u /*NAN*/ : (1u << 5) /*FIXPOINT_RANGE*/;
@@ -199,15 +200,15 @@ __device__ __forceinline__ void flush_pair(long long *acc, int slot, T s, T c, i
 
 template <class T, bool SMT>
 __device__ __forceinline__ void flush_one(long long *acc, int slot, T v, int b, unsigned &flags) {
-    if (v == (T)0) return;
     if constexpr (SMT && sizeof(T) == 4)
         if (add_f32_smem(acc + 3 * (size_t)slot, v, b)) return;
-    Limbs A;
-    if (!fix_split(v, b, A)) {
-        flags |= (v != v) ? 1u : (1u << 5);
-        return;
-    }
-    add_limbs<SMT>(acc + 3 * (size_t)slot, A);
+    flush_rest<T, SMT>(acc, slot, v, b, flags);
+}
+
+// flush a compensated pair: the Neumaier result s + c, converted once
+template <class T, bool SMT>
+__device__ __forceinline__ void flush_pair(long long *acc, int slot, T s, T c, int b, unsigned &flags) {
+    flush_one<T, SMT>(acc, slot, s + c, b, flags);
 }
 
 // Work split of the transport over the particle list (or a resume pass's
@@ -355,7 +356,7 @@ __device__ __forceinline__ bool le64(double a, double b) { return (long long)m64
 template <> struct SegMath<float> {
     static __device__ __forceinline__ float flight(uint32_t w, const Tab1<float> &ce) {
         const float v = (float)((w >> 8) | 1u) * 0x1p-24f;
-        return -__logf(v) * ce.rseff;
+        return -log_fast(v) * ce.rseff;
     }
     static __device__ __forceinline__ float attenuate(float E, const Tab1<float> &ce, float d, float *dep) {
         const float em1 = expm1_seg(-ce.saf * d);
