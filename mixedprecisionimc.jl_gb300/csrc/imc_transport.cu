@@ -351,24 +351,15 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
         // kRefillSegments segments each): each lane walks one history to its
         // end, and the warp moves on together to 32 consecutive entries, so
         // every load and store of the list is coalesced.
-        auto walk = [&](long long e) {
-            int cs_now;
-            if (!load(e, cs_now, t, x, mu, E, E0, i, cs)) return;
-            start(cs_now);
-            int end;
-            do end = segment(); while (!end);
-            finish(end);
-        };
-        if constexpr (!kFromQueue && !St::half) {
+        if constexpr (!kFromQueue) {
             // the list in chunks from the counter; the next entry's fields
-            // are loaded while the current history walks (FP32 / FP64 state:
-            // their stored fields are the arithmetic values; measured on the
+            // are loaded while the current history walks (measured on the
             // 2000-cell slab, 0.496 -> 0.474 ms per launch)
             typedef typename St::S S;
             typedef typename St::E0S E0S;
             uint8_t pa = 0;
             int pcs = 0;
-            S pt = (S)0, px = (S)0, pmu = (S)0, pE = (S)0;
+            S pt = (S)0.0f, px = (S)0.0f, pmu = (S)0.0f, pE = (S)0.0f;
             E0S pE0 = (E0S)0;
             auto fetch = [&](long long e) {
                 pa = e < n ? pb.alive[e] : (uint8_t)0;
@@ -381,7 +372,15 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
                     const long long e = base + r + lane;
                     const bool a = pa != 0;
                     const int ccs = pcs;
-                    t = (T)pt; x = (T)px; mu = (T)pmu; E = (T)pE; E0 = (T)pE0;
+                    E0 = (T)pE0;
+                    if constexpr (St::half) {
+                        t = __half2float(pt) * endsteptime;
+                        x = a ? __half2float(px) * tab[ccs & 0xFFFFFF].dxs : 0.0f;
+                        mu = __half2float(pmu);
+                        E = __half2float(pE) * E0;
+                    } else {
+                        t = (T)pt; x = (T)px; mu = (T)pmu; E = (T)pE;
+                    }
                     if (r + 32 < chunk) fetch(e + 32);
                     if (a) {
                         i = e;
@@ -394,11 +393,18 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
                 }
             }
         } else {
-            // the list (or a resume pass's queue) in chunks from the counter
+            // a resume pass's queue in chunks from the counter
             for (long long base = warp_counter_next(&sc->work_next) * chunk; base < n;
                  base = warp_counter_next(&sc->work_next) * chunk)
-                for (int r = 0; r < chunk; r += 32)
-                    if (base + r + lane < n) walk(base + r + lane);
+                for (int r = 0; r < chunk; r += 32) {
+                    const long long e = base + r + lane;
+                    int cs_now;
+                    if (e >= n || !load(e, cs_now, t, x, mu, E, E0, i, cs)) continue;
+                    start(cs_now);
+                    int end;
+                    do end = segment(); while (!end);
+                    finish(end);
+                }
         }
     } else {
         // Long histories of unequal length: each lane starts the next history
