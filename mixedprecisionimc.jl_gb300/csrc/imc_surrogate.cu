@@ -8,8 +8,9 @@
 //   k_surr_grad     forward + backward of a 64-sample slice in FP32: the loss
 //                   (cross entropy of the outcome + pinball losses of the
 //                   outcome's quantile heads) and per-block weight gradients
-//   k_surr_reduce   sums the per-block gradients in block order (deterministic)
-//   k_surr_adam     Adam step on FP32 master weights
+//   k_surr_adam     sums the per-block gradients in block order (deterministic)
+//                   and takes the Adam step on FP32 master weights
+//   k_surr_reduce   the sums alone
 //   k_surr_forward  the transport kernel's tensor-core forward pass on given
 //                   inputs (for the tests)
 //   k_surr_sample   inverse-transform sampling of the network's outputs, as
@@ -123,173 +124,283 @@ __global__ void k_surr_datagen(unsigned long long seed, long long n, const float
 // ------------------------------------------------------------- training
 constexpr int kSlice = 64;        // samples per block
 constexpr int kTrainThreads = 256;
+constexpr int kQMax = kQL + kQM;  // knots of an outcome's two heads, at most
 
-// gradient of the loss w.r.t. the 64 raw outputs of one sample; returns the loss
-__device__ float output_grad(const float *out, int c, float y0, float y1, float *dout) {
-    for (int j = 0; j < kOut; ++j) dout[j] = 0.0f;
-    // cross entropy of the outcome
-    const float m = fmaxf(out[0], fmaxf(out[1], out[2]));
-    const float e0 = expf(out[0] - m), e1 = expf(out[1] - m), e2 = expf(out[2] - m);
-    const float z = e0 + e1 + e2;
-    float loss = -(out[c] - m - logf(z));
-    dout[0] = e0 / z - (c == 0 ? 1.0f : 0.0f);
-    dout[1] = e1 / z - (c == 1 ? 1.0f : 0.0f);
-    dout[2] = e2 / z - (c == 2 ? 1.0f : 0.0f);
-    // pinball losses of the outcome's two quantile heads
-    int h0, k0, h1, k1;
+// shared-memory layout of k_surr_grad (floats).  Weights W2..W4 as they are in
+// the parameters and activations by sample, both with rows of 68 floats: 16
+// threads reading one float4 each from 16 consecutive rows (weights) or from
+// one row meet no bank twice, and two rows four apart lie 16 banks apart.
+constexpr int kLd = 68;
+constexpr int kSmW1 = 0;                           // [64][4]
+constexpr int kSmW2 = kSmW1 + kHid * kIn;          // [64][68] each
+constexpr int kSmW3 = kSmW2 + kHid * kLd;
+constexpr int kSmW4 = kSmW3 + kHid * kLd;
+constexpr int kSmB = kSmW4 + kHid * kLd;           // biases b1..b4 (256)
+constexpr int kSmX = kSmB + 4 * kHid;              // inputs [64][4]
+constexpr int kSmA1 = kSmX + kSlice * kIn;         // activations [64][68] x 3
+constexpr int kSmA2 = kSmA1 + kSlice * kLd;
+constexpr int kSmA3 = kSmA2 + kSlice * kLd;
+constexpr int kSmO = kSmA3 + kSlice * kLd;         // outputs, then their gradients
+constexpr int kSmD = kSmO + kSlice * kLd;          // back-propagated deltas
+constexpr int kSmQ = kSmD + kSlice * kLd;          // per sample and knot: softplus, sigmoid, loss term
+constexpr int kSmTotal = kSmQ + 3 * kSlice * kQMax;
+constexpr int kGradSmemBytes = kSmTotal * 4;
+static_assert(kSmW2 % 4 == 0 && kSmB % 4 == 0 && kSmX % 4 == 0 && kSmA1 % 4 == 0, "float4 rows");
+
+// Gradient of the loss with respect to the 64 raw outputs of one sample, in
+// place (O: its row), by four neighbouring threads (q = 0..3); thread 0
+// returns the loss.  The transcendentals of the knots are spread over the four
+// threads; the two heads' sums run in the order of a single thread, one thread
+// each.  sp, sg, tm: the sample's kQMax entries of each.  valid: the sample
+// exists (a padding row's gradient is zero).
+__device__ float output_grad(float *O, int q, bool valid, int c, float y0, float y1, float *sp, float *sg, float *tm) {
+    int h0 = 0, k0 = 0, h1 = 0, k1 = 0;
     heads_of(c, &h0, &k0, &h1, &k1);
-    const int heads[2] = {h0, h1}, ks[2] = {k0, k1};
-    const float ys[2] = {y0, y1};
-    for (int hh = 0; hh < 2; ++hh) {
-        const float *h = out + heads[hh];
-        const int K = ks[hh];
-        float q[kQL], dq[kQL];
-        knots(h, K, q);
+    float d0 = 0.0f, d1 = 0.0f, d2 = 0.0f, loss = 0.0f;
+    if (valid) {
+        for (int e = q; e < k0 + k1; e += 4) {
+            const float h = O[e < k0 ? h0 + e : h1 + e - k0];
+            if (e != 0 && e != k0) {
+                sp[e] = softplusf(h);
+                sg[e] = 1.0f / (1.0f + expf(-h));
+            } else {
+                sp[e] = h;  // the head's first knot
+            }
+        }
+        if (q == 0) {
+            // cross entropy of the outcome
+            const float m = fmaxf(O[0], fmaxf(O[1], O[2]));
+            const float e0 = expf(O[0] - m), e1 = expf(O[1] - m), e2 = expf(O[2] - m);
+            const float z = e0 + e1 + e2;
+            loss = -(O[c] - m - logf(z));
+            d0 = e0 / z - (c == 0 ? 1.0f : 0.0f);
+            d1 = e1 / z - (c == 1 ? 1.0f : 0.0f);
+            d2 = e2 / z - (c == 2 ? 1.0f : 0.0f);
+        }
+    }
+    __syncwarp();
+    for (int j = 4 * q; j < kOut; j += 16) *reinterpret_cast<float4 *>(O + j) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    __syncwarp();
+    if (valid && q < 2) {
+        // pinball losses of one of the outcome's two quantile heads; tm holds
+        // the loss terms, sp is overwritten by d loss / d q_k
+        const int off = q == 0 ? 0 : k0, K = q == 0 ? k0 : k1, head = q == 0 ? h0 : h1;
+        const float y = q == 0 ? y0 : y1;
+        float acc = 0.0f;
         for (int k = 0; k < K; ++k) {
-            const float tau = level(k, K), u = ys[hh] - q[k];
-            loss += u >= 0.0f ? tau * u : (tau - 1.0f) * u;
-            dq[k] = (u < 0.0f ? 1.0f : 0.0f) - tau;  // d loss / d q_k
+            acc = k == 0 ? sp[off] : acc + sp[off + k];
+            const float tau = level(k, K), u = y - acc;
+            tm[off + k] = u >= 0.0f ? tau * u : (tau - 1.0f) * u;
+            sp[off + k] = (u < 0.0f ? 1.0f : 0.0f) - tau;
         }
         // back through q_k = h_0 + sum_{j<=k, j>=1} softplus(h_j)
         float tail = 0.0f;
         for (int k = K - 1; k >= 1; --k) {
-            tail += dq[k];
-            const float sg = 1.0f / (1.0f + expf(-h[k]));
-            dout[heads[hh] + k] = tail * sg;
+            tail += sp[off + k];
+            O[head + k] = tail * sg[off + k];
         }
-        dout[heads[hh]] = tail + dq[0];
+        O[head] = tail + sp[off];
+    }
+    __syncwarp();
+    if (valid && q == 0) {
+        O[0] = d0; O[1] = d1; O[2] = d2;
+        for (int k = 0; k < k0 + k1; ++k) loss += tm[k];
     }
     return loss;
 }
 
-// shared-memory layout of k_surr_grad (floats)
-constexpr int kSmWT = 0;                          // W1..W4 transposed: WT[k][j]
-constexpr int kSmB = kSmWT + kParams - 4 * kHid;  // biases b1..b4 (256)
-constexpr int kSmX = kSmB + 4 * kHid;             // inputs [64][4]
-constexpr int kSmA1 = kSmX + kSlice * kIn;        // activations [64][64] x 3
-constexpr int kSmA2 = kSmA1 + kSlice * kHid;
-constexpr int kSmA3 = kSmA2 + kSlice * kHid;
-constexpr int kSmO = kSmA3 + kSlice * kHid;       // outputs, then their gradients
-constexpr int kSmD = kSmO + kSlice * kOut;        // back-propagated deltas
-constexpr int kSmTotal = kSmD + kSlice * kHid;
-constexpr int kGradSmemBytes = kSmTotal * 4;
+// The three products of a layer, each thread a 4 x 4 tile of the result in
+// registers: two shared float4 loads feed 32 multiplies and adds, where one
+// result per thread and step loaded two floats for one of each.  Every sum runs
+// over its index in order, one product at a time.  (FP32 issue bounds them:
+// 256 threads x 16 sums x 64 products x 2 instructions are 4.1 us a product on
+// an SM.)
+__device__ __forceinline__ float lane4(const float4 &v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
 
-// z[s][j] = b[j] + sum_k WT[k][j] a[s][k] for the 64 x 64 outputs of a layer
-__device__ __forceinline__ void dense_fwd(const float *WT, const float *b, const float *a, int K, float *z, bool relu) {
-    const int j = threadIdx.x & 63;
-    for (int s = threadIdx.x >> 6; s < kSlice; s += kTrainThreads / 64) {
-        float acc = b[j];
-        for (int k = 0; k < K; ++k) acc += WT[k * kHid + j] * a[s * K + k];
-        z[s * kHid + j] = relu ? fmaxf(acc, 0.0f) : acc;
+// z[s][j] = b[j] + sum_k W[j][k] a[s][k], the 64 x 64 outputs of a layer:
+// outputs tj + 16 jj, samples 4 ts + i
+template <int K>
+__device__ __forceinline__ void dense_fwd(const float *W, int ldw, const float *b, const float *a, int lda, float *z,
+                                          bool relu) {
+    const int tj = threadIdx.x & 15, ts = threadIdx.x >> 4;
+    float acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) acc[i][jj] = b[tj + 16 * jj];
+#pragma unroll 4
+    for (int k = 0; k < K; k += 4) {
+        float4 w[4], v[4];
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) w[jj] = *reinterpret_cast<const float4 *>(W + (tj + 16 * jj) * ldw + k);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const float4 *>(a + (4 * ts + i) * lda + k);
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int jj = 0; jj < 4; ++jj) acc[i][jj] += lane4(w[jj], kk) * lane4(v[i], kk);
     }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) z[(4 * ts + i) * kLd + tj + 16 * jj] = relu ? fmaxf(acc[i][jj], 0.0f) : acc[i][jj];
     __syncthreads();
 }
 
 // weight / bias gradients of one layer: gW[j][k] = sum_s dz[s][j] a[s][k]
-__device__ __forceinline__ void dense_wgrad(const float *dz, const float *a, int K, float *gW, float *gb) {
-    for (int e = threadIdx.x; e < kHid * K; e += kTrainThreads) {
-        const int j = e / K, k = e % K;
-        float acc = 0.0f;
-        for (int s = 0; s < kSlice; ++s) acc += dz[s * kHid + j] * a[s * K + k];
-        gW[e] = acc;
+template <int K>
+__device__ __forceinline__ void dense_wgrad(const float *dz, const float *a, int lda, float *gW, float *gb) {
+    constexpr int nk = K / 4;  // column tiles
+    if ((int)threadIdx.x < 16 * nk) {
+        const int tk = threadIdx.x % nk, tj = threadIdx.x / nk;
+        float acc[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) acc[i][kk] = 0.0f;
+#pragma unroll 8
+        for (int s = 0; s < kSlice; ++s) {
+            const float4 d = *reinterpret_cast<const float4 *>(dz + s * kLd + 4 * tj);
+            const float4 v = *reinterpret_cast<const float4 *>(a + s * lda + 4 * tk);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) acc[i][kk] += lane4(d, i) * lane4(v, kk);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            *reinterpret_cast<float4 *>(gW + (4 * tj + i) * K + 4 * tk) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
     }
-    for (int j = threadIdx.x; j < kHid; j += kTrainThreads) {
+    if (threadIdx.x < kHid) {
         float acc = 0.0f;
-        for (int s = 0; s < kSlice; ++s) acc += dz[s * kHid + j];
-        gb[j] = acc;
+#pragma unroll 16
+        for (int s = 0; s < kSlice; ++s) acc += dz[s * kLd + threadIdx.x];
+        gb[threadIdx.x] = acc;
     }
 }
 
 // delta of the layer below: da[s][k] = sum_j W[j][k] dz[s][j], masked by ReLU
 __device__ __forceinline__ void dense_bwd(const float *W, const float *dz, const float *a_below, float *da) {
-    const int k = threadIdx.x & 63;
-    for (int s = threadIdx.x >> 6; s < kSlice; s += kTrainThreads / 64) {
-        float acc = 0.0f;
-        for (int j = 0; j < kHid; ++j) acc += W[j * kHid + k] * dz[s * kHid + j];
-        da[s * kHid + k] = a_below[s * kHid + k] > 0.0f ? acc : 0.0f;
+    const int tk = threadIdx.x & 15, ts = threadIdx.x >> 4;
+    float acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) acc[i][kk] = 0.0f;
+#pragma unroll 4
+    for (int j = 0; j < kHid; j += 4) {
+        float4 w[4], d[4];
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) w[jj] = *reinterpret_cast<const float4 *>(W + (j + jj) * kLd + 4 * tk);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) d[i] = *reinterpret_cast<const float4 *>(dz + (4 * ts + i) * kLd + j);
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) acc[i][kk] += lane4(w[jj], kk) * lane4(d[i], jj);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float4 m = *reinterpret_cast<const float4 *>(a_below + (4 * ts + i) * kLd + 4 * tk);
+        *reinterpret_cast<float4 *>(da + (4 * ts + i) * kLd + 4 * tk) =
+            make_float4(m.x > 0.0f ? acc[i][0] : 0.0f, m.y > 0.0f ? acc[i][1] : 0.0f, m.z > 0.0f ? acc[i][2] : 0.0f,
+                        m.w > 0.0f ? acc[i][3] : 0.0f);
     }
     __syncthreads();
 }
 
 // Forward + backward of samples [off + 64 b, off + 64 b + 64) clipped to n;
-// writes this block's gradient sums (kParams floats) and loss sum.
+// writes this block's gradient sums (kParams floats) and loss sum.  One block
+// an SM; a batch of 8192 walks is 128 of them.
 __global__ void __launch_bounds__(kTrainThreads) k_surr_grad(const float *P, const float *x, const int *cls,
                                                              const float *tgt, long long n, long long off,
                                                              float *gpart, float *lpart) {
-    extern __shared__ float sm[];
-    float *WT = sm + kSmWT, *B = sm + kSmB, *X = sm + kSmX;
+    extern __shared__ __align__(16) float sm[];
+    float *W1 = sm + kSmW1, *W2 = sm + kSmW2, *W3 = sm + kSmW3, *W4 = sm + kSmW4, *B = sm + kSmB, *X = sm + kSmX;
     float *A1 = sm + kSmA1, *A2 = sm + kSmA2, *A3 = sm + kSmA3, *O = sm + kSmO, *D = sm + kSmD;
-    // transposed weights: WT1 [4][64], WT2..WT4 [64][64]
-    float *WT1 = WT, *WT2 = WT + kIn * kHid, *WT3 = WT2 + kHid * kHid, *WT4 = WT3 + kHid * kHid;
-    for (int e = threadIdx.x; e < kHid * kIn; e += kTrainThreads) {
-        const int j = e / kIn, k = e % kIn;
-        WT1[k * kHid + j] = P[kW1 + e];
+    for (int e = 4 * threadIdx.x; e < kHid * kHid; e += 4 * kTrainThreads) {
+        const int at = (e / kHid) * kLd + e % kHid;
+        *reinterpret_cast<float4 *>(W2 + at) = *reinterpret_cast<const float4 *>(P + kW2 + e);
+        *reinterpret_cast<float4 *>(W3 + at) = *reinterpret_cast<const float4 *>(P + kW3 + e);
+        *reinterpret_cast<float4 *>(W4 + at) = *reinterpret_cast<const float4 *>(P + kW4 + e);
     }
-    for (int e = threadIdx.x; e < kHid * kHid; e += kTrainThreads) {
-        const int j = e / kHid, k = e % kHid;
-        WT2[k * kHid + j] = P[kW2 + e];
-        WT3[k * kHid + j] = P[kW3 + e];
-        WT4[k * kHid + j] = P[kW4 + e];
-    }
-    for (int j = threadIdx.x; j < kHid; j += kTrainThreads) {
+    static_assert(kHid * kIn == kTrainThreads && kSlice * kIn == kTrainThreads, "one element a thread");
+    W1[threadIdx.x] = P[kW1 + threadIdx.x];
+    if (threadIdx.x < kHid) {
+        const int j = threadIdx.x;
         B[j] = P[kB1 + j]; B[kHid + j] = P[kB2 + j]; B[2 * kHid + j] = P[kB3 + j]; B[3 * kHid + j] = P[kB4 + j];
     }
     const long long s0 = off + (long long)blockIdx.x * kSlice;
-    for (int e = threadIdx.x; e < kSlice * kIn; e += kTrainThreads) {
-        const long long i = s0 + e / kIn;
-        X[e] = i < n ? x[i * kIn + e % kIn] : 0.0f;
+    {
+        const long long i = s0 + threadIdx.x / kIn;
+        X[threadIdx.x] = i < n ? x[i * kIn + threadIdx.x % kIn] : 0.0f;
     }
+    // this thread's sample of the output gradient
+    const int smp = threadIdx.x >> 2;
+    const bool valid = s0 + smp < n;
+    const int c = valid ? cls[s0 + smp] : 0;
+    const float y0 = valid ? tgt[2 * (s0 + smp)] : 0.0f, y1 = valid ? tgt[2 * (s0 + smp) + 1] : 0.0f;
     __syncthreads();
-    dense_fwd(WT1, B, X, kIn, A1, true);
-    dense_fwd(WT2, B + kHid, A1, kHid, A2, true);
-    dense_fwd(WT3, B + 2 * kHid, A2, kHid, A3, true);
-    dense_fwd(WT4, B + 3 * kHid, A3, kHid, O, false);
-    // output gradients, one thread per sample (zero for padding rows)
+    dense_fwd<kIn>(W1, kIn, B, X, kIn, A1, true);
+    dense_fwd<kHid>(W2, kLd, B + kHid, A1, kLd, A2, true);
+    dense_fwd<kHid>(W3, kLd, B + 2 * kHid, A2, kLd, A3, true);
+    dense_fwd<kHid>(W4, kLd, B + 3 * kHid, A3, kLd, O, false);
     __shared__ float sloss[kSlice];
-    if (threadIdx.x < kSlice) {
-        const long long i = s0 + threadIdx.x;
-        float dout[kOut];
-        float l = 0.0f;
-        if (i < n) {
-            l = output_grad(O + threadIdx.x * kOut, cls[i], tgt[2 * i], tgt[2 * i + 1], dout);
-        } else {
-            for (int j = 0; j < kOut; ++j) dout[j] = 0.0f;
-        }
-        for (int j = 0; j < kOut; ++j) O[threadIdx.x * kOut + j] = dout[j];
-        sloss[threadIdx.x] = l;
+    {
+        float *Q = sm + kSmQ + smp * kQMax;
+        const float l = output_grad(O + smp * kLd, threadIdx.x & 3, valid, c, y0, y1, Q, Q + kSlice * kQMax,
+                                    Q + 2 * kSlice * kQMax);
+        if ((threadIdx.x & 3) == 0) sloss[smp] = l;
     }
     __syncthreads();
     float *g = gpart + (size_t)blockIdx.x * kParams;
-    dense_wgrad(O, A3, kHid, g + kW4, g + kB4);
-    dense_bwd(P + kW4, O, A3, D);                 // delta at layer 3 output
-    dense_wgrad(D, A2, kHid, g + kW3, g + kB3);
-    __syncthreads();
-    dense_bwd(P + kW3, D, A2, O);                 // delta at layer 2 output (reuses O)
-    dense_wgrad(O, A1, kHid, g + kW2, g + kB2);
-    __syncthreads();
-    dense_bwd(P + kW2, O, A1, D);                 // delta at layer 1 output
-    dense_wgrad(D, X, kIn, g + kW1, g + kB1);
+    dense_wgrad<kHid>(O, A3, kLd, g + kW4, g + kB4);
+    dense_bwd(W4, O, A3, D);                      // delta at layer 3 output
+    dense_wgrad<kHid>(D, A2, kLd, g + kW3, g + kB3);
+    dense_bwd(W3, D, A2, O);                      // delta at layer 2 output (reuses O)
+    dense_wgrad<kHid>(O, A1, kLd, g + kW2, g + kB2);
+    dense_bwd(W2, O, A1, D);                      // delta at layer 1 output
+    dense_wgrad<kIn>(D, X, kIn, g + kW1, g + kB1);
     if (threadIdx.x == 0) {
         float l = 0.0f;
+#pragma unroll 16
         for (int s = 0; s < kSlice; ++s) l += sloss[s];
         lpart[blockIdx.x] = l;
     }
 }
 
-// grad[p] = scale * sum_b gpart[b][p], in block order
-__global__ void k_surr_reduce(const float *gpart, int nblk, float scale, float *grad) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= kParams) return;
+// scale * sum_b gpart[b][p], in block order (the loads of 16 blocks in flight)
+constexpr int kReduceThreads = 64;
+__device__ __forceinline__ float reduce_param(const float *gpart, int nblk, float scale, int p) {
     float acc = 0.0f;
-    for (int b = 0; b < nblk; ++b) acc += gpart[(size_t)b * kParams + p];
-    grad[p] = acc * scale;
+    int b = 0;
+    for (; b + 16 <= nblk; b += 16) {
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = gpart[(size_t)(b + i) * kParams + p];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc += v[i];
+    }
+    for (; b < nblk; ++b) acc += gpart[(size_t)b * kParams + p];
+    return acc * scale;
 }
 
-__global__ void k_surr_adam(float *P, float *m, float *v, const float *grad, float lr, float b1t, float b2t) {
+__global__ void __launch_bounds__(kReduceThreads) k_surr_reduce(const float *gpart, int nblk, float scale, float *grad) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < kParams) grad[p] = reduce_param(gpart, nblk, scale, p);
+}
+
+// the reduction and the Adam step of each parameter
+__global__ void __launch_bounds__(kReduceThreads) k_surr_adam(float *P, float *m, float *v, const float *gpart, int nblk,
+                                                              float scale, float lr, float b1t, float b2t) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= kParams) return;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    const float gr = grad[p];
+    const float gr = reduce_param(gpart, nblk, scale, p);
     const float mm = b1 * m[p] + (1.0f - b1) * gr;
     const float vv = b2 * v[p] + (1.0f - b2) * gr * gr;
     m[p] = mm;
@@ -440,7 +551,8 @@ int launch_grad(const float *P, const float *x, const int *cls, const float *tgt
                 float *gpart, float *lpart, float *grad, cudaStream_t s) {
     const int nblk = (int)((n + kSlice - 1) / kSlice);
     k_surr_grad<<<nblk, kTrainThreads, kGradSmemBytes, s>>>(P, x, cls, tgt, off + n, off, gpart, lpart);
-    k_surr_reduce<<<(kParams + 255) / 256, 256, 0, s>>>(gpart, nblk, 1.0f / (float)n, grad);
+    k_surr_reduce<<<(kParams + kReduceThreads - 1) / kReduceThreads, kReduceThreads, 0, s>>>(gpart, nblk,
+                                                                                             1.0f / (float)n, grad);
     return cudaGetLastError() == cudaSuccess ? IMC_OK : IMC_ERR_CUDA;
 }
 
@@ -530,9 +642,9 @@ int imc_surrogate_train(const ImcSurrogateTrainConfig *cfg, float *params, float
     float *dx = ds.alloc<float>(kIn * n), *dt = ds.alloc<float>(2 * n);
     int *dc = ds.alloc<int>(n);
     float *dP = ds.alloc<float>(kParams), *dm = ds.alloc<float>(kParams), *dv = ds.alloc<float>(kParams);
-    float *gpart = ds.alloc<float>((size_t)nblk * kParams), *dg = ds.alloc<float>(kParams);
+    float *gpart = ds.alloc<float>((size_t)nblk * kParams);
     float *lpart = ds.alloc<float>((size_t)nblk * cfg->iterations);
-    if (!dx || !dt || !dc || !dP || !dm || !dv || !gpart || !dg || !lpart) return IMC_ERR_OOM;
+    if (!dx || !dt || !dc || !dP || !dm || !dv || !gpart || !lpart) return IMC_ERR_OOM;
     k_surr_datagen<<<grid_of(n, 256, 8192), 256, 0, ds.stream>>>(cfg->seed, n, nullptr, dx, dc, dt);
     k_surr_init<<<(kParams + 255) / 256, 256, 0, ds.stream>>>(dP, cfg->seed);
     if (cudaMemsetAsync(dm, 0, 4 * (size_t)kParams, ds.stream) != cudaSuccess ||
@@ -544,11 +656,11 @@ int imc_surrogate_train(const ImcSurrogateTrainConfig *cfg, float *params, float
         const long long off = ((long long)it * B) % n;
         k_surr_grad<<<nblk, kTrainThreads, kGradSmemBytes, ds.stream>>>(dP, dx, dc, dt, off + B, off, gpart,
                                                                         lpart + (size_t)it * nblk);
-        k_surr_reduce<<<(kParams + 255) / 256, 256, 0, ds.stream>>>(gpart, nblk, 1.0f / (float)B, dg);
         b1t *= 0.9;
         b2t *= 0.999;
         const double lr = cfg->lr_min + 0.5 * (cfg->lr - cfg->lr_min) * (1.0 + cos(pi * it / cfg->iterations));
-        k_surr_adam<<<(kParams + 255) / 256, 256, 0, ds.stream>>>(dP, dm, dv, dg, (float)lr, (float)b1t, (float)b2t);
+        k_surr_adam<<<(kParams + kReduceThreads - 1) / kReduceThreads, kReduceThreads, 0, ds.stream>>>(
+            dP, dm, dv, gpart, nblk, 1.0f / (float)B, (float)lr, (float)b1t, (float)b2t);
         if (cudaGetLastError() != cudaSuccess) return IMC_ERR_CUDA;
     }
     if ((rc = d2h(params, dP, 4 * (size_t)kParams, ds.stream))) return rc;
