@@ -38,22 +38,51 @@ constexpr int kWalkCapFactor = 8;        // flight cap: 8 * lmax + 64
 
 // ----------------------------------------------------------- in-cell walk
 // Analog walk from (d_n, d_f, mu', lmax), all in mean free paths, near face at
-// 0, far face at d_n + d_f.  Returns the outcome and the two targets: for an
-// exit ln(path / lmax) and |mu|, for truncation the displacement toward the
-// far face / sqrt(lmax) and the final mu'.
-__device__ int walk(Stream &rs, float d_n, float d_f, float mu, float lmax, float *y0, float *y1) {
-    const float W = d_n + d_f;
-    float pos = d_n, path = 0.0f;
-    const int cap = kWalkCapFactor * (int)lmax + 64;
-    for (int it = 0; it < cap; ++it) {
-        const float s = Rand<float>::exp1(rs);
-        const float dface = mu > 0.0f ? (W - pos) / mu : pos / (-mu);
+// 0, far face at d_n + d_f, one flight at a time.  Ends with the outcome and
+// its two targets: for an exit ln(path / lmax) and |mu|, for truncation the
+// displacement toward the far face / sqrt(lmax) and the final mu'.
+struct Walk {
+    float d_n, W, mu, lmax, pos, path;
+    float den, rden;  // |mu| as the divisor of the face distance, and 1 / den where that serves (inf otherwise)
+    int left;         // flights left before the cap
+    Words<5> ws;
+    __device__ __forceinline__ void aim(float m) {
+        mu = m;
+        den = m > 0.0f ? m : -m;
+        rden = den >= 0x1p-40f && den <= 1.0f ? rcp_mid(den) : INFINITY;
+    }
+    __device__ __forceinline__ void start(float dn, float df, float m, float L, const Stream &rs) {
+        d_n = dn; W = dn + df; lmax = L; pos = dn; path = 0.0f;
+        left = kWalkCapFactor * (int)L + 64;
+        aim(m);
+        // the rest of the stream's block, then its next ones
+        ws.pid = rs.pid; ws.block = rs.block; ws.n = 4 - rs.idx;
+        ws.w[0] = rs.idx == 0 ? rs.buf[0] : rs.idx == 1 ? rs.buf[1] : rs.idx == 2 ? rs.buf[2] : rs.buf[3];
+        ws.w[1] = rs.idx == 0 ? rs.buf[1] : rs.idx == 1 ? rs.buf[2] : rs.buf[3];
+        ws.w[2] = rs.idx == 0 ? rs.buf[2] : rs.buf[3];
+        ws.w[3] = rs.buf[3];
+    }
+    __device__ __forceinline__ int truncated(float *y0, float *y1) const {
+        *y0 = (pos - d_n) / sqrtf(lmax);
+        *y1 = mu;
+        return kTrunc;
+    }
+    // one flight; the outcome, or -1 while the walk goes on
+    __device__ __forceinline__ int flight(const SeedKeys &key, float *y0, float *y1) {
+        if (left <= 0) return truncated(y0, y1);
+        if (ws.n < 2) ws.refill(key, 0u, kStageSurrData);
+        const float s = -logf((float)((ws.w[0] >> 8) | 1u) * 0x1p-24f);
+        // the distance to the face ahead, num / den: the quotient's residual
+        // corrects num * rden to the IEEE quotient (Markstein, IBM J. Res.
+        // Dev. 34, 1990) while nothing leaves binary32's middle range
+        const float num = mu > 0.0f ? W - pos : pos;
+        const float q = num * rden;
+        float dface = fmaf(fmaf(-q, den, num), rden, q);
+        if (!(fabsf(q) >= 0x1p-60f && fabsf(q) <= 0x1p60f)) dface = num / den;
         const float rem = lmax - path;
         if (rem <= s && rem <= dface) {
             pos += mu * rem;
-            *y0 = (pos - d_n) / sqrtf(lmax);
-            *y1 = mu;
-            return kTrunc;
+            return truncated(y0, y1);
         }
         if (dface <= s) {
             path += dface;
@@ -63,14 +92,18 @@ __device__ int walk(Stream &rs, float d_n, float d_f, float mu, float lmax, floa
         }
         pos += mu * s;
         path += s;
-        mu = 0.0f;
-        for (int r = 0; r < 64 && mu == 0.0f; ++r) mu = 1.0f - 2.0f * Rand<float>::u(rs);
-        if (mu == 0.0f) mu = 1.0f;
+        float m = Rand<float>::cosine(ws.w[1]);
+        for (int r = 1; r < 64 && m == 0.0f; ++r) {
+            ws.drop(false);
+            if (ws.n < 2) ws.refill(key, 0u, kStageSurrData);
+            m = Rand<float>::cosine(ws.w[1]);
+        }
+        aim(m == 0.0f ? 1.0f : m);
+        ws.drop(true);
+        --left;
+        return -1;
     }
-    *y0 = (pos - d_n) / sqrtf(lmax);
-    *y1 = mu;
-    return kTrunc;
-}
+};
 
 // Random walk states covering the states the transport kernel asks about
 // (lmax >= 32, cells >= 8 mean free paths, expected collisions
@@ -98,26 +131,60 @@ __device__ void draw_state(Stream &rs, float *d_n, float *d_f, float *mu, float 
     *d_n = dn; *d_f = W - dn; *mu = m; *lmax = L;
 }
 
-__global__ void k_surr_datagen(unsigned long long seed, long long n, const float *state_in, float *x, int *cls,
-                               float *tgt) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
-        Stream rs;
-        rs.init(seed, 0u, (uint32_t)i, kStageSurrData);
-        float dn, df, mu, L;
-        if (state_in) {
-            dn = state_in[4 * i]; df = state_in[4 * i + 1]; mu = state_in[4 * i + 2]; L = state_in[4 * i + 3];
-        } else {
-            draw_state(rs, &dn, &df, &mu, &L);
+// The walks, a lane each: a lane whose walk has ended takes the next sample from
+// the counter, once four of a warp's lanes wait (walks are 1 to 1e4 flights
+// long; a thread per sample left most lanes waiting for the longest walk of
+// their warp: 2^18 walks 12.3 ms).  Every sample has its own stream, so who walks it
+// changes nothing.
+constexpr int kDatagenThreads = 256;
+// samples a lane walks before the grid grows past one block an SM: fewer leave
+// the lanes idle behind the longest walks (3: 9.2 ms for 2^18 walks), more leave
+// SMs short of warps (12: 11.2 ms); 8.4 ms
+constexpr int kDatagenPerLane = 6;
+__global__ void __launch_bounds__(kDatagenThreads, 4) k_surr_datagen(unsigned long long seed, long long n,
+                                                                     const float *state_in, float *x, int *cls,
+                                                                     float *tgt, unsigned long long *counter) {
+    const int lane = threadIdx.x & 31;
+    const SeedKeys key(seed);
+    Walk w{};
+    long long i = -1;   // the sample under way (-1: none)
+    bool more = true;   // warp-uniform: the counter has samples left
+    while (true) {
+        const unsigned idle = __ballot_sync(0xFFFFFFFFu, i < 0);
+        if (more && (__popc(idle) >= 4)) {
+            unsigned long long base = 0;
+            if (lane == 0) base = atomicAdd(counter, (unsigned long long)__popc(idle));
+            base = __shfl_sync(0xFFFFFFFFu, base, 0);
+            more = (long long)base + __popc(idle) < n;
+            const long long mine = (long long)base + __popc(idle & ((1u << lane) - 1u));
+            if (i < 0 && mine < n) {
+                i = mine;
+                Stream rs;
+                rs.init(seed, 0u, (uint32_t)i, kStageSurrData);
+                float dn, df, mu, L;
+                if (state_in) {
+                    dn = state_in[4 * i]; df = state_in[4 * i + 1]; mu = state_in[4 * i + 2]; L = state_in[4 * i + 3];
+                } else {
+                    draw_state(rs, &dn, &df, &mu, &L);
+                }
+                float f[kIn];
+                features(dn, df, mu, L, f);
+                for (int k = 0; k < kIn; ++k) x[kIn * i + k] = f[k];
+                w.start(dn, df, mu, L, rs);
+            }
+        } else if (idle == 0xFFFFFFFFu) {
+            return;
         }
-        float y0, y1;
-        const int c = walk(rs, dn, df, mu, L, &y0, &y1);
-        float f[kIn];
-        features(dn, df, mu, L, f);
-        for (int k = 0; k < kIn; ++k) x[kIn * i + k] = f[k];
-        cls[i] = c;
-        tgt[2 * i] = y0;
-        tgt[2 * i + 1] = y1;
+        if (i >= 0) {
+            float y0, y1;
+            const int c = w.flight(key, &y0, &y1);
+            if (c >= 0) {
+                cls[i] = c;
+                tgt[2 * i] = y0;
+                tgt[2 * i + 1] = y1;
+                i = -1;
+            }
+        }
     }
 }
 
@@ -546,6 +613,21 @@ int grid_of(long long n, int per_block, int cap) {
     return (int)(b < 1 ? 1 : (b > cap ? cap : b));
 }
 
+// n walks on a grid of at most four blocks an SM
+int launch_datagen(DevScope &ds, unsigned long long seed, long long n, const float *state, float *x, int *cls,
+                   float *tgt) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return IMC_ERR_CUDA;
+    unsigned long long *counter = ds.alloc<unsigned long long>(1);
+    if (!counter) return IMC_ERR_OOM;
+    if (cudaMemsetAsync(counter, 0, sizeof(*counter), ds.stream) != cudaSuccess) return IMC_ERR_CUDA;
+    k_surr_datagen<<<grid_of(n, kDatagenPerLane * kDatagenThreads, 4 * sms), kDatagenThreads, 0, ds.stream>>>(seed, n, state, x, cls, tgt,
+                                                                                          counter);
+    return IMC_OK;
+}
+
 // per-slice gradients and the block-order reduction: grad = mean over n
 int launch_grad(const float *P, const float *x, const int *cls, const float *tgt, long long n, long long off,
                 float *gpart, float *lpart, float *grad, cudaStream_t s) {
@@ -589,7 +671,7 @@ int imc_surrogate_walk(uint64_t seed, const float *state, int64_t n, float *x, i
     float *dx = ds.alloc<float>(kIn * n), *dt = ds.alloc<float>(2 * n);
     int *dc = ds.alloc<int>(n);
     if (!dx || !dt || !dc) return IMC_ERR_OOM;
-    k_surr_datagen<<<grid_of(n, 256, 4096), 256, 0, ds.stream>>>(seed, n, dstate, dx, dc, dt);
+    if ((rc = launch_datagen(ds, seed, n, dstate, dx, dc, dt))) return rc;
     if ((rc = d2h(x, dx, 4 * kIn * (size_t)n, ds.stream)) || (rc = d2h(cls, dc, 4 * (size_t)n, ds.stream)) ||
         (rc = d2h(tgt, dt, 8 * (size_t)n, ds.stream)))
         return rc;
@@ -645,7 +727,7 @@ int imc_surrogate_train(const ImcSurrogateTrainConfig *cfg, float *params, float
     float *gpart = ds.alloc<float>((size_t)nblk * kParams);
     float *lpart = ds.alloc<float>((size_t)nblk * cfg->iterations);
     if (!dx || !dt || !dc || !dP || !dm || !dv || !gpart || !lpart) return IMC_ERR_OOM;
-    k_surr_datagen<<<grid_of(n, 256, 8192), 256, 0, ds.stream>>>(cfg->seed, n, nullptr, dx, dc, dt);
+    if ((rc = launch_datagen(ds, cfg->seed, n, nullptr, dx, dc, dt))) return rc;
     k_surr_init<<<(kParams + 255) / 256, 256, 0, ds.stream>>>(dP, cfg->seed);
     if (cudaMemsetAsync(dm, 0, 4 * (size_t)kParams, ds.stream) != cudaSuccess ||
         cudaMemsetAsync(dv, 0, 4 * (size_t)kParams, ds.stream) != cudaSuccess)
