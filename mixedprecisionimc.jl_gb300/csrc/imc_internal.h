@@ -199,8 +199,6 @@ void launch_finalize(const CellArgs &ca, Scalars *sc, cudaStream_t st);
 void launch_tally(const CellArgs &ca, Scalars *sc, cudaStream_t st);
 void launch_energycheck(const CellArgs &ca, Scalars *sc, DevStats *stats, long long stats_cap, cudaStream_t st);
 void launch_timestep(const CellArgs &ca, Scalars *sc, cudaStream_t st);
-// the step sequence's fused launches: finalize + tally, energycheck + timestep
-void launch_finalize_tally(const CellArgs &ca, Scalars *sc, cudaStream_t st);
 // finalize + tally + energycheck + timestep in one launch (the step sequence)
 void launch_tally_check_timestep(const CellArgs &ca, Scalars *sc, DevStats *stats, long long stats_cap,
                                  cudaStream_t st);

@@ -30,27 +30,91 @@ constexpr int kPlanThreads = 1024;
 // double-double per block over a fixed partition of the cells, combined in
 // block order.
 
-__device__ __forceinline__ DD block_reduce_dd(DD v, DD *sh) {
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for (int w = kCellThreads / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) {
-            DD x = sh[threadIdx.x];
-            x.add(sh[threadIdx.x + w]);
-            sh[threadIdx.x] = x;
+// ---- sums over the lanes of a warp
+// A double as up to 93 bits of a fixed-point number whose top bit is that of
+// the largest exponent present: four signed 24-bit digits.  32 or more such
+// digits add up in 32 bits with the warp's integer reduction, so a sum costs a
+// handful of FP64 instructions (the digits back to two doubles) where a tree
+// of double-double adds took 40 (64 cycles each for a warp: half of the step's
+// tail).  What lies 93 bits below the largest term is rounded away, as a
+// double-double sum's is.
+struct Digits {
+    int d[4];
+    __device__ __forceinline__ void clear() { d[0] = d[1] = d[2] = d[3] = 0; }
+    // emax: the largest biased exponent (1..2046)
+    __device__ __forceinline__ void add(double x, int emax) {
+        const uint64_t b = d2u(x);
+        const int ex = (int)((b >> 52) & 0x7FFu);
+        uint64_t man = b & 0xFFFFFFFFFFFFFull;
+        if (ex) man |= 0x10000000000000ull;
+        const int sh = emax - (ex ? ex : 1);
+        uint64_t hi = man >> 24, lo = man << 40;  // man 2^40 in 128 bits
+        if (sh >= 64) {
+            lo = sh < 128 ? hi >> (sh - 64) : 0ull;
+            hi = 0ull;
+        } else if (sh > 0) {
+            lo = (lo >> sh) | (hi << (64 - sh));
+            hi >>= sh;
         }
-        __syncthreads();
+        const int sg = (long long)b < 0 ? -1 : 1;
+        d[0] += sg * (int)(lo & 0xFFFFFFull);
+        d[1] += sg * (int)((lo >> 24) & 0xFFFFFFull);
+        d[2] += sg * (int)((lo >> 48) | ((hi & 0xFFull) << 16));
+        d[3] += sg * (int)(hi >> 8);
     }
-    DD r = sh[0];
-    __syncthreads();
-    return r;
+    __device__ __forceinline__ void warp_sum() {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) d[i] = __reduce_add_sync(0xFFFFFFFFu, d[i]);
+    }
+    // emax as in add, at least kDigitsExpMin: the scales are normal numbers
+    __device__ __forceinline__ DD value(int emax) const {
+        const long long top = ((long long)d[3] << 24) + d[2], low = ((long long)d[1] << 24) + d[0];
+        // units 2^(emax - 1075 - 40) and, of top, 2^48 of them
+        const double u = m64::from_bits((uint64_t)(emax - 1075 - 40 + 1023) << 52);
+        const double a = (double)top * (u * 0x1p48), c = (double)low * u;
+        DD r;
+        r.hi = a + c;
+        r.lo = c - (r.hi - a);
+        return r;
+    }
+};
+constexpr int kDigitsExpMin = 128;
+__device__ __forceinline__ int biased_exp(double x) { return (int)((d2u(x) >> 52) & 0x7FFu); }
+// digits serve for finite terms that are not all tiny
+__device__ __forceinline__ bool digits_serve(int emax) { return emax >= kDigitsExpMin && emax < 0x7FF; }
+
+// sum of one double-double a lane over the warp, by shuffles (any values)
+__device__ __forceinline__ DD warp_sum_tree(DD d) {
+    for (int off = 16; off > 0; off >>= 1) {
+        DD o;
+        o.hi = __shfl_down_sync(0xFFFFFFFFu, d.hi, off);
+        o.lo = __shfl_down_sync(0xFFFFFFFFu, d.lo, off);
+        if ((int)(threadIdx.x & 31) < off) d.add(o);
+    }
+    d.hi = __shfl_sync(0xFFFFFFFFu, d.hi, 0);
+    d.lo = __shfl_sync(0xFFFFFFFFu, d.lo, 0);
+    return d;
 }
 
-__device__ __forceinline__ DD dd_of(double x) {
-    DD d;
-    d.hi = x;
-    d.lo = 0.0;
-    return d;
+// sum of one double a lane over the warp, on every lane
+__device__ __forceinline__ DD warp_sum(double x) {
+    const int emax = __reduce_max_sync(0xFFFFFFFFu, biased_exp(x));
+    if (!__any_sync(0xFFFFFFFFu, x != 0.0)) {
+        DD z;
+        z.clear();
+        return z;
+    }
+    if (!digits_serve(emax)) {
+        DD d;
+        d.hi = x;
+        d.lo = 0.0;
+        return warp_sum_tree(d);
+    }
+    Digits g;
+    g.clear();
+    g.add(x, emax);
+    g.warp_sum();
+    return g.value(emax);
 }
 
 // ------------------------------------------------------------------ update
@@ -127,7 +191,6 @@ __device__ __forceinline__ int slot_group(const CellArgs &ca, int s) {
 // also leaves double-double partial sums of e/escale per slot group.
 template <int G, int SEL>
 __global__ void __launch_bounds__(kCellThreads) k_source_slots(CellArgs ca, Scalars *sc) {
-    __shared__ DD sh[kCellThreads];
     const double a = ca.a, c = ca.c, ds = ca.ds, dt = sc->dt;
     const int ns = nsurf_slots(ca), nc = ca.nc, K = ca.K;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -189,14 +252,9 @@ __global__ void __launch_bounds__(kCellThreads) k_source_slots(CellArgs ca, Scal
     }
     for (int g = 0; g < 6; ++g) {
         // most blocks hold one group: reduce only the groups present
-        if (!__syncthreads_or(grp == g)) {
-            if (threadIdx.x == 0) {
-                ca.part_src[(blockIdx.x * 6 + g) * 2] = 0.0;
-                ca.part_src[(blockIdx.x * 6 + g) * 2 + 1] = 0.0;
-            }
-            continue;
-        }
-        DD r = block_reduce_dd(dd_of(grp == g ? q : 0.0), sh);
+        DD r;
+        r.clear();
+        if (__any_sync(0xFFFFFFFFu, grp == g)) r = warp_sum(grp == g ? q : 0.0);
         if (threadIdx.x == 0) {
             ca.part_src[(blockIdx.x * 6 + g) * 2] = r.hi;
             ca.part_src[(blockIdx.x * 6 + g) * 2 + 1] = r.lo;
@@ -211,10 +269,25 @@ __device__ __forceinline__ long long round_count(double q, double n_source, doub
     return (long long)r;
 }
 
-// Sum of the double-double block partials of one group by one warp: lane l
-// takes blocks l, l+32, ..., then a fixed shuffle tree.  Deterministic.
+// Sum of the double-double partials of one group by one warp (lane l takes
+// partials l, l + 32, ...), on every lane.  Deterministic.
 __device__ __forceinline__ double warp_sum_partials(const double *part, int nb, int stride, int g) {
     const int lane = threadIdx.x & 31;
+    int emax = 0;
+    for (int bb = lane; bb < nb; bb += 32) emax = max(emax, biased_exp(part[(bb * stride + g) * 2]));
+    emax = __reduce_max_sync(0xFFFFFFFFu, emax);
+    // a lane's digits hold 4 terms: 64 partials (hi and lo), 2^24 4 32 = 2^31
+    if (nb <= 64 && digits_serve(emax)) {
+        Digits d;
+        d.clear();
+        for (int bb = lane; bb < nb; bb += 32) {
+            d.add(part[(bb * stride + g) * 2], emax);
+            d.add(part[(bb * stride + g) * 2 + 1], emax);
+        }
+        // (|lo| < |hi| / 2^52: the sums stay below 2^31)
+        d.warp_sum();
+        return d.value(emax).val();
+    }
     DD d;
     d.clear();
     for (int bb = lane; bb < nb; bb += 32) {
@@ -223,13 +296,7 @@ __device__ __forceinline__ double warp_sum_partials(const double *part, int nb, 
         p.lo = part[(bb * stride + g) * 2 + 1];
         d.add(p);
     }
-    for (int off = 16; off > 0; off >>= 1) {
-        DD o;
-        o.hi = __shfl_down_sync(0xFFFFFFFFu, d.hi, off);
-        o.lo = __shfl_down_sync(0xFFFFFFFFu, d.lo, off);
-        if (lane < off) d.add(o);
-    }
-    return __shfl_sync(0xFFFFFFFFu, d.val(), 0);
+    return warp_sum_tree(d).val();
 }
 
 // Sums of the slot groups (src/imc_sourcing.jl:121): one one-warp block per
@@ -786,50 +853,74 @@ __device__ __forceinline__ double cell_vol(const CellArgs &ca, int i) {
     return ca.geometry == 1 ? ca.dx[i] : ca.dx[i % ca.nx] * ca.dy[i / ca.nx];
 }
 
+// x / s for an energy scale s: the scales in use are 1 and powers of two, whose
+// quotients need no division
+__device__ __forceinline__ double div_scale(double x, double s) {
+    const uint64_t b = d2u(s);
+    if (b == 0x3FF0000000000000ull) return x;
+    const int ex = (int)(b >> 52);  // s > 0
+    if ((b & 0xFFFFFFFFFFFFFull) == 0 && ex >= 1 && ex <= 2045) return x * m64::from_bits((uint64_t)(2046 - ex) << 52);
+    return x / s;
+}
+// fix_value with the power of two applied to its two halves
+__device__ __forceinline__ double fix_value_fast(const long long *a, int b) {
+    if (b < -960 || b > 800) return fix_value(a, b);
+    uint64_t hi = (uint64_t)a[0], lo = 0;
+    const uint64_t lo1 = (uint64_t)a[1] << 32, lo2 = (uint64_t)a[2];
+    lo = lo1 + lo2;
+    hi += (uint64_t)(a[1] >> 32) + (a[2] < 0 ? ~0ull : 0ull) + (lo < lo1 ? 1ull : 0ull);
+    const double u = m64::from_bits((uint64_t)(1023 + b) << 52);
+    return (double)(long long)hi * (u * 0x1p64) + (double)lo * u;
+}
+
 // Converts this transport's fixed-point tallies to FP64 mesh fields and
-// clears the accumulators: energydep and the escaped energy as
-// Transport.MC leaves them (src/imc_transport.jl:198-205), and the census
-// radiation energy density of src/imc_tally.jl:81-113.  Cell i, and the
-// escaped energy and segment statistics in block 0, thread 0.
+// clears the accumulators: energydep as Transport.MC leaves it
+// (src/imc_transport.jl:198-205), and the census radiation energy density of
+// src/imc_tally.jl:81-113, for cell i.
 __device__ __forceinline__ void finalize_cell(const CellArgs &ca, Scalars *sc, int i) {
     const int nc = ca.nc, K = ca.K;
-    const int b_dep = sc->b_dep, b_rad = sc->b_rad, b_lost = sc->b_lost;
+    const int b_dep = sc->b_dep, b_rad = sc->b_rad;
     if (i < nc) {
         const double vol = cell_vol(ca, i);
         double r = 0.0;
         for (int k = 0; k < K; ++k) {
             const size_t idx = (size_t)k * nc + i;
-            const int se = scale_exp(ca.scales[k]);
+            const double s = ca.scales[k];
+            const int se = scale_exp(s);
             long long *d = ca.dep_acc + 3 * idx;
             // FP64 histories deposit energies, FP32 ones densities
-            const double dep = fix_value(d, b_dep + se);
+            const double dep = fix_value_fast(d, b_dep + se);
             ca.energydep[idx] = ca.prec == 0 ? dep / vol : dep;
             d[0] = d[1] = d[2] = 0;
             long long *g = ca.rad_acc + 3 * idx;
-            r += fix_value(g, b_rad + se) / (vol * ca.scales[k]);
+            r += fix_value_fast(g, b_rad + se) / (d2u(s) == 0x3FF0000000000000ull ? vol : vol * s);
             g[0] = g[1] = g[2] = 0;
         }
         ca.radenergydens[i] = r;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        double lost = 0.0;
-        for (int k = 0; k < K; ++k) {
-            long long *d = ca.lost_acc + 3 * k;
-            lost += fix_value(d, b_lost + scale_exp(ca.scales[k])) / ca.scales[k];
-            d[0] = d[1] = d[2] = 0;
-        }
-        sc->lost_step = lost;
-        // mean transport segments per history of this step: the next
-        // transport picks its lane schedule from it
-        const double hist = (double)(sc->n_census_in + sc->n_sourced);
-        sc->seg_per_hist = hist > 0.0 ? (float)((double)sc->segments / hist) : 0.0f;
-        sc->lostenergy += lost;
-    }
 }
 
-// Tally.tally per cell (src/imc_tally.jl:29-75); each block leaves partial
-// sums of the deposited energy per scale and of the radiation energy.
-__device__ __forceinline__ void tally_cell(const CellArgs &ca, Scalars *sc, int i, DD *sh) {
+// the escaped energy and the segment statistics, by one thread
+__device__ __forceinline__ void finalize_scalars(const CellArgs &ca, Scalars *sc) {
+    const int b_lost = sc->b_lost;
+    double lost = 0.0;
+    for (int k = 0; k < ca.K; ++k) {
+        long long *d = ca.lost_acc + 3 * k;
+        const double s = ca.scales[k];
+        if (d[0] | d[1] | d[2]) lost += div_scale(fix_value_fast(d, b_lost + scale_exp(s)), s);
+        d[0] = d[1] = d[2] = 0;
+    }
+    sc->lost_step = lost;
+    // mean transport segments per history of this step: the next
+    // transport picks its lane schedule from it
+    const double hist = (double)(sc->n_census_in + sc->n_sourced);
+    sc->seg_per_hist = hist > 0.0 ? (float)((double)sc->segments / hist) : 0.0f;
+    sc->lostenergy += lost;
+}
+
+// Tally.tally per cell (src/imc_tally.jl:29-75); each unit of 32 cells leaves
+// partial sums of the deposited energy per scale and of the radiation energy.
+__device__ __forceinline__ void tally_cell(const CellArgs &ca, Scalars *sc, int i, int unit) {
     const int nc = ca.nc, K = ca.K;
     const double a = ca.a, c = ca.c, dt = sc->dt;
     const bool first = sc->t == 0.0;
@@ -845,45 +936,34 @@ __device__ __forceinline__ void tally_cell(const CellArgs &ca, Scalars *sc, int 
         }
         double inc = 0.0;
         for (int k = 0; k < K; ++k)
-            inc += (ca.energydep[(size_t)k * nc + i] - ca.emitted[(size_t)k * nc + i]) / ca.scales[k];
+            inc += div_scale(ca.energydep[(size_t)k * nc + i] - ca.emitted[(size_t)k * nc + i], ca.scales[k]);
         double m = ca.matenergydens[i] + inc;
         ca.matenergydens[i] = m;
-        if (ca.linearized) ca.temp[i] = pow(m, 0.25);
+        // the fourth root as two square roots: 3/4 of a unit in the last place
+        // at most, in a third of pow's instructions
+        if (ca.linearized) ca.temp[i] = sqrt(sqrt(m));
         else ca.temp[i] = ca.temp[i] + inc / ca.bee[i];
     }
     const int np = K + 1;
-    for (int k = 0; k < K; ++k) {
-        double x = i < nc ? (ca.energydep[(size_t)k * nc + i] * vol) / ca.scales[k] : 0.0;
-        DD r = block_reduce_dd(dd_of(x), sh);
-        if (threadIdx.x == 0) {
-            ca.part_tally[(blockIdx.x * np + k) * 2] = r.hi;
-            ca.part_tally[(blockIdx.x * np + k) * 2 + 1] = r.lo;
+    for (int k = 0; k <= K; ++k) {
+        double x = 0.0;
+        if (i < nc)
+            x = k < K ? div_scale(ca.energydep[(size_t)k * nc + i] * vol, ca.scales[k]) : ca.radenergydens[i] * vol;
+        const DD r = warp_sum(x);
+        if ((threadIdx.x & 31) == 0) {
+            ca.part_tally[(unit * np + k) * 2] = r.hi;
+            ca.part_tally[(unit * np + k) * 2 + 1] = r.lo;
         }
-    }
-    DD r = block_reduce_dd(dd_of(i < nc ? ca.radenergydens[i] * vol : 0.0), sh);
-    if (threadIdx.x == 0) {
-        ca.part_tally[(blockIdx.x * np + K) * 2] = r.hi;
-        ca.part_tally[(blockIdx.x * np + K) * 2 + 1] = r.lo;
     }
 }
 
 __global__ void __launch_bounds__(kCellThreads) k_finalize(CellArgs ca, Scalars *sc) {
     finalize_cell(ca, sc, blockIdx.x * blockDim.x + threadIdx.x);
+    if (blockIdx.x == 0 && threadIdx.x == 0) finalize_scalars(ca, sc);
 }
 
 __global__ void __launch_bounds__(kCellThreads) k_tally(CellArgs ca, Scalars *sc) {
-    __shared__ DD sh[kCellThreads];
-    tally_cell(ca, sc, blockIdx.x * blockDim.x + threadIdx.x, sh);
-}
-
-// Both in one launch (the step sequence): the tally of cell i reads only
-// what the finalize of cell i wrote, in the same thread, and nothing that
-// the compaction between them in the reference's order changes.
-__global__ void __launch_bounds__(kCellThreads) k_finalize_tally(CellArgs ca, Scalars *sc) {
-    __shared__ DD sh[kCellThreads];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    finalize_cell(ca, sc, i);
-    tally_cell(ca, sc, i, sh);
+    tally_cell(ca, sc, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.x);
 }
 
 void launch_finalize(const CellArgs &ca, Scalars *sc, cudaStream_t st) {
@@ -892,10 +972,6 @@ void launch_finalize(const CellArgs &ca, Scalars *sc, cudaStream_t st) {
 
 void launch_tally(const CellArgs &ca, Scalars *sc, cudaStream_t st) {
     k_tally<<<ca.nblk_cell, kCellThreads, 0, st>>>(ca, sc);
-}
-
-void launch_finalize_tally(const CellArgs &ca, Scalars *sc, cudaStream_t st) {
-    k_finalize_tally<<<ca.nblk_cell, kCellThreads, 0, st>>>(ca, sc);
 }
 
 // timestep (src/MixedPrecisionIMC.jl:181-222), FP64 on the device so a run
@@ -992,29 +1068,38 @@ __global__ void __launch_bounds__(544) k_energycheck(CellArgs ca, Scalars *sc, D
 }
 
 // Finalize + tally per cell, then, in the block that finishes last, the
-// energy check and the timestep: one launch for the step's tail.  Each
-// block publishes its partial sums before taking a ticket; the last block
-// sums every block's partials in block order (the same fixed order as
-// k_energycheck, so the same values).
-__global__ void __launch_bounds__(kCellThreads) k_tally_check(CellArgs ca, Scalars *sc, DevStats *stats,
+// energy check and the timestep: one launch for the step's tail.  The tally of
+// cell i reads only what the finalize of cell i wrote, in the same thread, and
+// nothing that the compaction between them in the reference's order changes.
+// Blocks of four warps, one for each of an SM's FP64 units; each publishes its
+// partial sums before taking a ticket, and the last block's warps sum a group
+// each over every unit of cells.  (FP64 latency bounds it, a warp's FP64
+// instruction taking 64 cycles: 2000 cells 24 us with double-double trees,
+// pow and divisions by the scales, one warp a block.)
+constexpr int kTailThreads = 128;
+__global__ void __launch_bounds__(kTailThreads) k_tally_check(CellArgs ca, Scalars *sc, DevStats *stats,
                                                              long long stats_cap) {
-    static_assert(kCellThreads == 32, "one-warp blocks");
-    __shared__ DD sh[kCellThreads];
     __shared__ double g[17];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    finalize_cell(ca, sc, i);
-    tally_cell(ca, sc, i, sh);
+    __shared__ int s_last;
+    const int warp = threadIdx.x >> 5, unit = blockIdx.x * (kTailThreads / 32) + warp;
+    if (unit < ca.nblk_cell) {
+        const int i = unit * 32 + (threadIdx.x & 31);
+        finalize_cell(ca, sc, i);
+        tally_cell(ca, sc, i, unit);
+    }
     __threadfence();
-    unsigned ticket = 0;
-    if (threadIdx.x == 0) ticket = atomicAdd(&sc->tally_blocks_done, 1u);
-    ticket = __shfl_sync(0xFFFFFFFFu, ticket, 0);
-    if (ticket != gridDim.x - 1u) return;
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&sc->tally_blocks_done, 1u) == gridDim.x - 1u;
+    __syncthreads();
+    if (!s_last) return;
     __threadfence();
     const int np = ca.K + 1;
-    for (int q = 0; q < np; ++q) {
+    if (warp == 3 && (threadIdx.x & 31) == 0) finalize_scalars(ca, sc);
+    for (int q = warp; q < np; q += kTailThreads / 32) {
         const double v = warp_sum_partials(ca.part_tally, ca.nblk_cell, np, q);
-        if (threadIdx.x == 0) g[q] = v;
+        if ((threadIdx.x & 31) == 0) g[q] = v;
     }
+    __syncthreads();
     if (threadIdx.x == 0) {
         sc->tally_blocks_done = 0u;
         energycheck_done(ca, sc, stats, stats_cap, g, true);
@@ -1031,7 +1116,8 @@ void launch_energycheck(const CellArgs &ca, Scalars *sc, DevStats *stats, long l
 
 void launch_tally_check_timestep(const CellArgs &ca, Scalars *sc, DevStats *stats, long long stats_cap,
                                  cudaStream_t st) {
-    k_tally_check<<<ca.nblk_cell, kCellThreads, 0, st>>>(ca, sc, stats, stats_cap);
+    const int warps = kTailThreads / 32;
+    k_tally_check<<<(ca.nblk_cell + warps - 1) / warps, kTailThreads, 0, st>>>(ca, sc, stats, stats_cap);
 }
 
 // Transport of a list that was set directly (no sourcing this step): take the
