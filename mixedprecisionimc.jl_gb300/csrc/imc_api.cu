@@ -361,8 +361,7 @@ void run_transport(ImcHandle *h, PBufPair bufs, cudaStream_t st) {
 // cell field and the tally no particle) and finalize + tally + energycheck +
 // timestep in one launch.
 void enqueue_before_transport(ImcHandle *h, cudaStream_t st) {
-    launch_update(h->ca, h->d_sc, st);
-    launch_source(h->ca, h->d_sc, h->prec, pair(h), h->grid_emit, st);
+    launch_source(h->ca, h->d_sc, h->prec, pair(h), h->grid_emit, true, st);
 }
 void enqueue_after_transport(ImcHandle *h, cudaStream_t st) {
     launch_compact(h->ca, h->d_sc, h->prec, pair(h), h->tile_cnt, h->tile_off, h->ntiles_cap, false, st);
@@ -754,11 +753,12 @@ int imc_create(const ImcDeck *d, ImcHandle **out) {
     if ((rc = upload<long long>(h, &ca.lost_acc, nullptr, 3 * (size_t)K))) return bail(rc);
     ca.nslots = h->nslots;
     if ((rc = upload<double>(h, &ca.slot_e, nullptr, h->nslots))) return bail(rc);
-    if ((rc = upload<double>(h, &ca.slot_s, nullptr, h->nslots))) return bail(rc);
     if ((rc = upload<double>(h, &ca.slot_nrg, nullptr, h->nslots))) return bail(rc);
     if ((rc = upload<float>(h, &ca.slot_nrg_f, nullptr, h->nslots))) return bail(rc);
     if ((rc = upload<int>(h, &ca.slot_j, nullptr, h->nslots))) return bail(rc);
-    if ((rc = upload<long long>(h, &ca.slot_n, nullptr, h->nslots))) return bail(rc);
+    ca.nblk_count = (h->nslots + kCountThreads - 1) / kCountThreads;
+    if ((rc = upload<long long>(h, &ca.blk_off, nullptr, ca.nblk_count))) return bail(rc);
+    if ((rc = upload<unsigned>(h, &ca.src_flags, nullptr, 1))) return bail(rc);
     if ((rc = upload<long long>(h, &ca.slot_off, nullptr, h->nslots))) return bail(rc);
     if ((rc = upload<double>(h, &ca.slot_q, nullptr, h->nslots))) return bail(rc);
     ca.prec = h->prec;
@@ -773,7 +773,7 @@ int imc_create(const ImcDeck *d, ImcHandle **out) {
     ca.nblk_slot = (h->nslots + kCellThreads - 1) / kCellThreads;
     ca.nblk_cell = (nc + kCellThreads - 1) / kCellThreads;
     if ((rc = upload<double>(h, &ca.part_src, nullptr, (size_t)ca.nblk_slot * 12))) return bail(rc);
-    if ((rc = upload<double>(h, &ca.part_emax, nullptr, (size_t)ca.nblk_slot))) return bail(rc);
+    if ((rc = upload<double>(h, &ca.part_emax, nullptr, (size_t)ca.nblk_count))) return bail(rc);
     if ((rc = upload<double>(h, &ca.part_tally, nullptr, (size_t)ca.nblk_cell * (K + 1) * 2))) return bail(rc);
     for (int b = 0; b < 4; ++b) ca.bc[b] = d->bc[b];
     ca.c = d->phys_c; ca.a = d->phys_a; ca.alpha = d->alpha; ca.ds = d->distancescale;
@@ -869,7 +869,7 @@ int imc_sourcing(ImcHandle *h) {
     int rc = read_scalars(h, &sc);
     if (rc) return rc;
     if ((rc = grow(h, sc.n_particles + births_bound(h, sc.n_particles)))) return rc;
-    launch_source(h->ca, h->d_sc, h->prec, pair(h), h->grid_emit, h->stream);
+    launch_source(h->ca, h->d_sc, h->prec, pair(h), h->grid_emit, false, h->stream);
     CKL(h);
     if ((rc = read_scalars(h, &sc))) return rc;
     h->stage = Stage::Sourced;
@@ -1618,11 +1618,11 @@ int imc_get_surrogate_active(const ImcHandle *h, int *active) {
 
 int imc_kernels_per_step(const ImcHandle *h, int *count) {
     if (!h || !count) return IMC_ERR_INVALID_ARG;
-    // update, source x5, transport (in 1D the short- and the long-history
+    // update + source x3, transport (in 1D the short- and the long-history
     // kernel), compact x4, finalize + tally + energycheck + timestep; the
     // surrogate transport is 1 + kSurrRounds analog passes, each both
     // kernels, and kSurrRounds query passes
-    *count = h->geometry == IMC_GEOM_2D ? 12 : 13 + (h->ca.surr_image ? 3 * kSurrRounds : 0);
+    *count = h->geometry == IMC_GEOM_2D ? 9 : 10 + (h->ca.surr_image ? 3 * kSurrRounds : 0);
     return IMC_OK;
 }
 

@@ -69,7 +69,7 @@ struct CellArgs {
     long long *dep_acc, *rad_acc, *lost_acc;   // 3 limbs per slot
     // sourcing scratch (per source slot)
     int nslots;
-    double *slot_e, *slot_s, *slot_nrg, *slot_q;
+    double *slot_e, *slot_nrg, *slot_q;
     float *slot_nrg_f;                 // slot_nrg rounded to binary32 (FP32 / FP16 births)
     const float *dxf, *dyf;            // cell widths rounded to binary32 (FP32 / FP16 births)
     // fixed positions of the surface births, in binary32 (FP32 / FP16 state)
@@ -81,11 +81,13 @@ struct CellArgs {
     float surf_f[6];
     double surf_d[6];
     int *slot_j;
-    long long *slot_n, *slot_off;
+    long long *slot_off, *blk_off;     // first birth of a slot in its block of kCountThreads slots; of a block
+    int nblk_count;                    // blocks of kCountThreads slots
+    unsigned *src_flags;               // error flags of the step's first kernel
     // per-block partial sums (double-double pairs) and maxima
-    int nblk_slot, nblk_cell;          // kCellThreads-thread blocks over slots / cells
+    int nblk_slot, nblk_cell;          // units of kCellThreads slots / cells
     double *part_src;                  // [nblk_slot][6 groups][hi, lo]
-    double *part_emax;                 // [nblk_slot]
+    double *part_emax;                 // [nblk_count]
     double *part_tally;                // [nblk_cell][K + 1][hi, lo]
     // physics / control
     int bc[4];
@@ -136,7 +138,8 @@ void launch_update(const CellArgs &ca, Scalars *sc, cudaStream_t st);
 // the transport's per-cell table from the cell fields as they are now (the
 // stage-by-stage entry point: they may have been set since the update)
 void launch_table(const CellArgs &ca, cudaStream_t st);
-void launch_source(const CellArgs &ca, Scalars *sc, int prec, PBufPair bufs, int grid, cudaStream_t st);
+// update: with Update.update in the first launch
+void launch_source(const CellArgs &ca, Scalars *sc, int prec, PBufPair bufs, int grid, bool update, cudaStream_t st);
 struct TransportShape {
     bool smem_tally;  // block-private tallies in shared memory
     bool dep_only;    // only the deposition tallies in shared memory
@@ -240,6 +243,7 @@ cudaError_t set_transport_multi_decks(const Deck1DArgs *ca, const PBufPair1D *bu
 // a 2000-cell mesh spreads over 63 SMs (FP64 runs at 1/64 of the FP32 rate,
 // and these kernels are latency bound)
 constexpr int kCellThreads = 32;
+constexpr int kCountThreads = 128;     // threads per block of the birth counts
 constexpr int kCompactTile = 4096;     // particles per compaction tile
 constexpr int kCompactThreads = 256;
 
