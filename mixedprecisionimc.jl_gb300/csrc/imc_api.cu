@@ -1619,10 +1619,10 @@ int imc_get_surrogate_active(const ImcHandle *h, int *active) {
 int imc_kernels_per_step(const ImcHandle *h, int *count) {
     if (!h || !count) return IMC_ERR_INVALID_ARG;
     // update + source x3, transport (in 1D the short- and the long-history
-    // kernel), compact x4, finalize + tally + energycheck + timestep; the
+    // kernel), compact x2, finalize + tally + energycheck + timestep; the
     // surrogate transport is 1 + kSurrRounds analog passes, each both
     // kernels, and kSurrRounds query passes
-    *count = h->geometry == IMC_GEOM_2D ? 9 : 10 + (h->ca.surr_image ? 3 * kSurrRounds : 0);
+    *count = h->geometry == IMC_GEOM_2D ? 7 : 8 + (h->ca.surr_image ? 3 * kSurrRounds : 0);
     return IMC_OK;
 }
 

@@ -38,6 +38,14 @@ __device__ __forceinline__ double div_scale(double x, double s) {
     return x / s;
 }
 
+// v 2^e: by the exponent bits where both are normal numbers
+__device__ __forceinline__ double times_pow2(double v, int e) {
+    const uint64_t b = d2u(v);
+    const int ex = (int)((b >> 52) & 0x7FFu), to = ex + e;
+    if (ex == 0 || ex == 0x7FF || to <= 0 || to >= 0x7FF) return ldexp(v, e);
+    return m64::from_bits(b + ((uint64_t)(int64_t)e << 52));
+}
+
 // ---- sums over the lanes of a warp
 // A double as up to 93 bits of a fixed-point number whose top bit is that of
 // the largest exponent present: four signed 24-bit digits.  32 or more such
@@ -428,40 +436,45 @@ __global__ void __launch_bounds__(kCountThreads) k_source_counts(CellArgs ca, Sc
     __shared__ int s_last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ns = nsurf_slots(ca), nc = ca.nc;
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    // everything the slot needs, asked for before the first use
+    const bool slot = q < ca.nslots;
+    const double eq = slot ? ca.slot_e[q] : 0.0, qq = slot ? ca.slot_q[q] : 0.0;
+    const double qb = slot && ca.geometry == 2 && q >= ns + nc ? ca.slot_q[q - nc] : 0.0;
+    const int jq = slot ? ca.slot_j[q] : -1;
     double E, n_source;
     source_total(ca, sc, E, n_source);
+    const double scale = jq >= 0 ? ca.scales[jq] : 1.0;
     const bool ok = (E > 0.0) && isfinite(E);
+    double my = 0.0;
+    long long n = 0;
+    if (slot) {
+        long long nd = 0;
+        if (ok) {
+            if (q < ns) {
+                if (eq > 0) n = round_count(qq, n_source, E, ca.geometry == 2, ca.cellmin);
+                nd = n;
+            } else if (q < ns + nc) {
+                n = round_count(qq, n_source, E, true, ca.cellmin);
+                nd = n;
+            } else if (eq > 0) {
+                n = round_count(qq, n_source, E, true, ca.cellmin);
+                nd = n;
+                // 2D births n_body particles per source cell (src/imc_sourcing.jl:357)
+                if (ca.geometry == 2 && n > 0) n = round_count(qb, n_source, E, true, ca.cellmin);
+            }
+            if (n < 0) n = 0;
+        }
+        const double nrg = n > 0 ? eq / (double)nd : 0.0;
+        ca.slot_nrg[q] = nrg;
+        ca.slot_nrg_f[q] = (float)nrg;
+        // the largest birth energy in true units (see scale_exp)
+        if (n > 0) my = times_pow2(nrg, -scale_exp(scale));
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         sc->totalenergy = E;
         sc->n_source = n_source;
         if (!ok) atomicOr(&sc->flags, 1u << 4);
-    }
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    double my = 0.0;
-    long long n = 0;
-    if (q < ca.nslots) {
-        const double *e = ca.slot_e, *qv = ca.slot_q;
-        long long nd = 0;
-        if (ok) {
-            if (q < ns) {
-                if (e[q] > 0) n = round_count(qv[q], n_source, E, ca.geometry == 2, ca.cellmin);
-                nd = n;
-            } else if (q < ns + nc) {
-                n = round_count(qv[q], n_source, E, true, ca.cellmin);
-                nd = n;
-            } else if (e[q] > 0) {
-                n = round_count(qv[q], n_source, E, true, ca.cellmin);
-                nd = n;
-                // 2D births n_body particles per source cell (src/imc_sourcing.jl:357)
-                if (ca.geometry == 2 && n > 0) n = round_count(qv[q - nc], n_source, E, true, ca.cellmin);
-            }
-            if (n < 0) n = 0;
-        }
-        const double nrg = n > 0 ? e[q] / (double)nd : 0.0;
-        ca.slot_nrg[q] = nrg;
-        ca.slot_nrg_f[q] = (float)nrg;
-        // the largest birth energy in true units (see scale_exp)
-        if (n > 0) my = ldexp(nrg, -scale_exp(ca.scales[ca.slot_j[q]]));
     }
     // the block's scan and maximum
     long long x = n;
@@ -543,9 +556,10 @@ __global__ void __launch_bounds__(kCountThreads) k_source_counts(CellArgs ca, Sc
         sc->killed = 0ull;
         sc->work_next = 0ull;
         for (int r = 0; r <= 2 * kSurrRounds; ++r) sc->qcount[r] = 0ull;
-        sc->b_dep = fix_exponent(emax / ca.vol_min);
-        sc->b_lost = fix_exponent(emax);
-        sc->b_rad = fix_exponent(emax);
+        const int b = fix_exponent(emax);
+        sc->b_dep = ca.vol_min == 1.0 ? b : fix_exponent(emax / ca.vol_min);
+        sc->b_lost = b;
+        sc->b_rad = b;
         if (fl) atomicOr(&sc->flags, fl);
     }
 }
@@ -765,85 +779,93 @@ void launch_source(const CellArgs &ca, Scalars *sc, int prec, PBufPair buf, int 
 }
 
 // ------------------------------------------------------------- compaction
-// Stable three-pass compaction: per-tile alive counts, one-block exclusive
-// scan of the tile counts, then a per-tile block scan that scatters the
-// survivors in order into the other buffer.
-__global__ void __launch_bounds__(kCompactThreads) k_compact_count(const Scalars *sc, PBufPair bufs,
-                                                                   long long *tile_cnt) {
-    if (!sc->compact_now) return;
-    const uint8_t *alive = bufs.b[sc->cur].alive;
+// Stable compaction in two launches: per-tile alive counts and, in the block
+// that finishes last, their exclusive scan; then a per-tile block scan that
+// scatters the survivors in order into the other buffer.  Whether this step
+// compacts follows from the transport's kills (census carried in + births -
+// removed), so the holes are known without reading the alive bytes and every
+// block decides alike; a step that does not compact leaves at once.  The blocks
+// stride over the tiles: one per tile of the buffer's capacity, the launches
+// cost 5 us each on the 2000-cell slab's 5900 tiles with nothing to do.
+constexpr int kCompactGrid = 152 * 8;
+__global__ void __launch_bounds__(kCompactThreads) k_compact_count(Scalars *sc, PBufPair bufs, long long *tile_cnt,
+                                                                   long long *tile_off, long long *n_before, int force) {
+    constexpr int W = kCompactThreads / 32;
+    __shared__ int wt[W];
+    __shared__ long long s_tot[W], s_run;
+    __shared__ int s_last;
     const long long n = sc->n_particles;
-    const long long base = (long long)blockIdx.x * kCompactTile;
-    if (base >= n) return;
-    int cnt = 0;
-    if (base + kCompactTile <= n) {
-        // a full tile: 16 alive bytes per thread in one 16-byte load (tiles
-        // start at multiples of 4096 bytes, so every load is aligned)
-        static_assert(kCompactTile == 16 * kCompactThreads, "one uint4 per thread");
-        const uint4 v = reinterpret_cast<const uint4 *>(alive + base)[threadIdx.x];
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-        for (int q = 0; q < 4; ++q)
-            for (int b = 0; b < 4; ++b) cnt += ((w[q] >> (8 * b)) & 0xFFu) != 0u;
-    } else {
-        for (int r = threadIdx.x; r < kCompactTile; r += blockDim.x) {
-            long long i = base + r;
-            if (i < n && alive[i]) ++cnt;
+    const long long live = sc->n_census_in + sc->n_sourced - (long long)sc->killed;
+    if (!force && (n - live) * kDeferHoles <= n) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            sc->compact_now = 0;
+            sc->n_census = live;
         }
+        return;
     }
-    cnt = __reduce_add_sync(0xFFFFFFFFu, (unsigned)cnt);
-    __shared__ int wt[kCompactThreads / 32];
-    if ((threadIdx.x & 31) == 0) wt[threadIdx.x >> 5] = cnt;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        long long s = 0;
-        for (int w = 0; w < kCompactThreads / 32; ++w) s += wt[w];
-        tile_cnt[blockIdx.x] = s;
-    }
-}
-
-__global__ void __launch_bounds__(1024) k_compact_scan(Scalars *sc, const long long *tile_cnt, long long *tile_off,
-                                                      int force) {
-    __shared__ long long warp_tot[32];
-    __shared__ long long s_run;
-    if (!sc->compact_now) return;  // k_compact_decide set the live count
-    const long long n = sc->n_particles;
-    const long long ntiles = (n + kCompactTile - 1) / kCompactTile;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) s_run = 0;
+    const uint8_t *alive = bufs.b[sc->cur].alive;
+    const long long ntiles = (n + kCompactTile - 1) / kCompactTile;
+    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const long long base = tile * kCompactTile;
+        int cnt = 0;
+        if (base + kCompactTile <= n) {
+            // a full tile: 16 alive bytes per thread in one 16-byte load (tiles
+            // start at multiples of 4096 bytes, so every load is aligned)
+            static_assert(kCompactTile == 16 * kCompactThreads, "one uint4 per thread");
+            const uint4 v = reinterpret_cast<const uint4 *>(alive + base)[threadIdx.x];
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+            for (int q = 0; q < 4; ++q)
+                for (int b = 0; b < 4; ++b) cnt += ((w[q] >> (8 * b)) & 0xFFu) != 0u;
+        } else {
+            for (int r = threadIdx.x; r < kCompactTile; r += blockDim.x) {
+                long long i = base + r;
+                if (i < n && alive[i]) ++cnt;
+            }
+        }
+        cnt = __reduce_add_sync(0xFFFFFFFFu, (unsigned)cnt);
+        if (lane == 0) wt[warp] = cnt;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            long long t = 0;
+            for (int w = 0; w < W; ++w) t += wt[w];
+            tile_cnt[tile] = t;
+        }
+        __syncthreads();
+    }
+    __threadfence();
     __syncthreads();
-    for (long long base = 0; base < ntiles; base += blockDim.x) {
-        long long q = base + threadIdx.x;
-        long long v = q < ntiles ? tile_cnt[q] : 0;
+    if (threadIdx.x == 0) s_last = atomicAdd(&sc->tally_blocks_done, 1u) == gridDim.x - 1u;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    if (threadIdx.x == 0) s_run = 0;
+    for (long long base = 0; base < ntiles; base += kCompactThreads) {
+        const long long q = base + threadIdx.x;
+        const long long v = q < ntiles ? tile_cnt[q] : 0;
         long long x = v;
         for (int off = 1; off < 32; off <<= 1) {
-            long long y = __shfl_up_sync(0xFFFFFFFFu, x, off);
+            const long long y = __shfl_up_sync(0xFFFFFFFFu, x, off);
             if (lane >= off) x += y;
         }
-        if (lane == 31) warp_tot[warp] = x;
+        __syncthreads();  // s_tot and s_run as the round before left them
+        if (lane == 31) s_tot[warp] = x;
         __syncthreads();
-        if (warp == 0) {
-            long long w = warp_tot[lane];
-            for (int off = 1; off < 32; off <<= 1) {
-                long long y = __shfl_up_sync(0xFFFFFFFFu, w, off);
-                if (lane >= off) w += y;
-            }
-            warp_tot[lane] = w;
-        }
+        long long start = s_run;
+        for (int w = 0; w < warp; ++w) start += s_tot[w];
+        if (q < ntiles) tile_off[q] = start + x - v;
         __syncthreads();
-        long long excl = s_run + (warp > 0 ? warp_tot[warp - 1] : 0) + x - v;
-        if (q < ntiles) tile_off[q] = excl;
-        __syncthreads();
-        if (threadIdx.x == blockDim.x - 1) s_run = excl + v;
-        __syncthreads();
+        if (threadIdx.x == kCompactThreads - 1) s_run = start + x;
     }
+    __syncthreads();
     if (threadIdx.x == 0) {
-        // compact when forced (Clean.clean) or when the holes exceed 1/16 of the list
-        const long long alive = s_run;
-        (void)force;
-        sc->n_census = alive;
+        sc->tally_blocks_done = 0u;
+        sc->compact_now = 1;
+        *n_before = n;
+        sc->n_census = s_run;
         sc->compact_src = sc->cur;
         sc->cur ^= 1;
-        sc->n_particles = alive;
+        sc->n_particles = s_run;
     }
 }
 
@@ -857,8 +879,8 @@ __global__ void __launch_bounds__(kCompactThreads) k_compact_scatter(int geometr
     __shared__ int wt[kCompactThreads / 32];
     __shared__ int s_tot;
     const long long n = *n_before;
-    const long long base = (long long)blockIdx.x * kCompactTile;
-    if (base >= n) return;
+    for (long long tile = blockIdx.x; tile * kCompactTile < n; tile += gridDim.x) {
+    const long long base = tile * kCompactTile;
     const int tile_n = (int)((n - base) < kCompactTile ? (n - base) : kCompactTile);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // survivor list of the tile, in order: thread t owns tile positions
@@ -896,7 +918,7 @@ __global__ void __launch_bounds__(kCompactThreads) k_compact_scatter(int geometr
     const int run = s_tot;
     __syncthreads();
     const int cnt = run;
-    const long long out = tile_off[blockIdx.x];
+    const long long out = tile_off[tile];
     // Every field of a survivor in one pass: stores coalesced, loads gathered
     // from the tile (whole sectors when most entries survive; when most are
     // holes, only the sectors that hold a survivor), all fields' loads of a
@@ -918,34 +940,22 @@ __global__ void __launch_bounds__(kCompactThreads) k_compact_scatter(int geometr
         dst.cs[d] = cs;
         dst.alive[d] = 1;
     }
-}
-
-// Before compaction: the list length (for the scatter) and whether this step
-// compacts.  The live count follows from the transport's kills (census
-// carried in + births - removed), so the holes are known without reading the
-// alive bytes; they are counted per tile only when the list is compacted.
-__global__ void k_compact_decide(Scalars *sc, long long *n_before, int force) {
-    const long long n = sc->n_particles;
-    *n_before = n;
-    const long long live = sc->n_census_in + sc->n_sourced - (long long)sc->killed;
-    const bool compact = force || (n - live) * kDeferHoles > n;
-    sc->compact_now = compact ? 1 : 0;
-    if (!compact) sc->n_census = live;
+    __syncthreads();  // the tile's shared arrays are read
+    }
 }
 
 void launch_compact(const CellArgs &ca, Scalars *sc, int prec, PBufPair bufs, long long *tile_cnt,
                     long long *tile_off, long long ntiles_cap, bool force, cudaStream_t st) {
     // tile_off has ntiles_cap + 1 entries; the last holds the pre-compaction length
     long long *n_before = tile_off + ntiles_cap;
-    k_compact_decide<<<1, 1, 0, st>>>(sc, n_before, force ? 1 : 0);
-    k_compact_count<<<(unsigned)ntiles_cap, kCompactThreads, 0, st>>>(sc, bufs, tile_cnt);
-    k_compact_scan<<<1, 1024, 0, st>>>(sc, tile_cnt, tile_off, force ? 1 : 0);
+    const unsigned grid = (unsigned)(ntiles_cap < kCompactGrid ? ntiles_cap : kCompactGrid);
+    k_compact_count<<<grid, kCompactThreads, 0, st>>>(sc, bufs, tile_cnt, tile_off, n_before, force ? 1 : 0);
     if (prec == 0)
-        k_compact_scatter<StF64><<<(unsigned)ntiles_cap, kCompactThreads, 0, st>>>(ca.geometry, sc, tile_off, bufs, n_before);
+        k_compact_scatter<StF64><<<grid, kCompactThreads, 0, st>>>(ca.geometry, sc, tile_off, bufs, n_before);
     else if (prec == 1)
-        k_compact_scatter<StF32><<<(unsigned)ntiles_cap, kCompactThreads, 0, st>>>(ca.geometry, sc, tile_off, bufs, n_before);
+        k_compact_scatter<StF32><<<grid, kCompactThreads, 0, st>>>(ca.geometry, sc, tile_off, bufs, n_before);
     else
-        k_compact_scatter<StF16><<<(unsigned)ntiles_cap, kCompactThreads, 0, st>>>(ca.geometry, sc, tile_off, bufs, n_before);
+        k_compact_scatter<StF16><<<grid, kCompactThreads, 0, st>>>(ca.geometry, sc, tile_off, bufs, n_before);
 }
 
 void launch_compact(const CellArgs &ca, Scalars *sc, int prec, PBufRaw src, PBufRaw dst, long long *tile_cnt,
