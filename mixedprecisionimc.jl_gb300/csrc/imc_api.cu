@@ -816,7 +816,7 @@ int imc_create(const ImcDeck *d, ImcHandle **out) {
     TransportShape shape = transport_shape(ca, h->prec);
     const int smem = shape.smem;
     h->block_transport = shape.block;
-    h->block_transport_long = shape.block_long ? shape.block_long : shape.block;
+    h->block_transport_long = shape.block_long;
     if (smem > 227 * 1024) return bail(fail(h, IMC_ERR_INVALID_ARG, "mesh too large for the shared-memory transport table"));
     for (int v = 0; v < 2; ++v) {
         const void *kp = transport_kernel_ptr(ca, h->prec, v == 1);
@@ -1618,11 +1618,11 @@ int imc_get_surrogate_active(const ImcHandle *h, int *active) {
 
 int imc_kernels_per_step(const ImcHandle *h, int *count) {
     if (!h || !count) return IMC_ERR_INVALID_ARG;
-    // update + source x3, transport (in 1D the short- and the long-history
-    // kernel), compact x2, finalize + tally + energycheck + timestep; the
+    // update + source x3, transport (the short- and the long-history
+    // kernel, but in FP64 2D), compact x2, finalize + tally + energycheck + timestep; the
     // surrogate transport is 1 + kSurrRounds analog passes, each both
     // kernels, and kSurrRounds query passes
-    *count = h->geometry == IMC_GEOM_2D ? 7 : 8 + (h->ca.surr_image ? 3 * kSurrRounds : 0);
+    *count = (h->geometry == IMC_GEOM_2D && h->prec == IMC_FP64 ? 7 : 8) + (h->ca.surr_image ? 3 * kSurrRounds : 0);
     return IMC_OK;
 }
 

@@ -145,10 +145,9 @@ struct TransportShape {
     bool dep_only;    // only the deposition tallies in shared memory
     int smem;         // dynamic shared memory bytes
     int block;        // threads per block
-    int block_long;   // of the long-history kernel (1D)
+    int block_long;   // of the long-history kernel
 };
-// blocks of a transport launch: of the only or the short-history kernel, and of
-// the 1D long-history kernel
+// blocks of a transport launch: of the short- and of the long-history kernel
 struct TransportGrid {
     int grid, grid_long;
 };

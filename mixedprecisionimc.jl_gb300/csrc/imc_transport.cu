@@ -479,6 +479,7 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
     finish_counters(sc, segs, killed, flags, emax_e);
 }
 
+enum { kShortSchedule = 0, kLongSchedule = 1, kBothSchedules = 2 };
 // The two lane schedules are kernels of their own, so that neither holds the
 // other's registers and each has its own block size; a step launches both and
 // the one whose schedule the step does not take returns at once (~2 us).
@@ -530,8 +531,12 @@ __global__ void __launch_bounds__(BLOCK) k_transport1d_multi(int ndecks) {
 // census tallies block-private in shared memory) or kTallySharedDep (the
 // deposition tallies only; census energy, one flush per census particle, to
 // global memory)
-template <class St, int BLOCK, int TM>
+// SCHED: the short- or the long-history schedule, or both in one kernel (FP64,
+// whose registers hold both; the launch that does nothing costs it 3 %).
+template <class St, int BLOCK, int TM, int SCHED>
 __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc, PBufPair bufs) {
+    const bool long_step = long_histories(sc);
+    if (SCHED != kBothSchedules && long_step != (SCHED == kLongSchedule)) return;
     constexpr bool SMT = TM != kTallyGlobal;        // deposition flushes to shared memory
     constexpr bool RAD_SMT = TM == kTallyShared;    // census flushes to shared memory
     typedef typename St::T T;
@@ -562,34 +567,42 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
     const int b_dep = sc->b_dep, b_rad = sc->b_rad, b_lost = sc->b_lost;
     const unsigned step = sc->step;
     const unsigned long long seed = ca.seed;
-    const long long cap = ca.seg_cap;
+    const unsigned cap = ca.seg_cap > 0xFFFFFFFEll ? 0xFFFFFFFEu : (unsigned)ca.seg_cap;
     const bool refl_l = ca.bc[0] == 1, refl_r = ca.bc[1] == 1, refl_t = ca.bc[2] == 1, refl_b = ca.bc[3] == 1;
     unsigned long long segs = 0, killed = 0;
     unsigned flags = 0;
     int emax_e = kNoExp;
     // Lane state of the history in flight.
     long long i = 0;
-    int cs = 0, xi = 0, yi = 0, k = 0, acc_cell = 0;
+    int cs = 0, xi = 0, yi = 0, k = 0, se = 0;  // se: scale k's exponent
+    const unsigned dep_shared = SMT ? (unsigned)__cvta_generic_to_shared(dep_acc) : 0u;
+    unsigned slots_k = 0;  // shared tallies: scale k's deposition slots
+    // c / NX as the high word of c times this (exact: c NX < 2^32, as the
+    // table of all cells fits in shared memory)
+    const unsigned rNX = NX > 1 ? 0xFFFFFFFFu / (unsigned)NX + 1u : 0u;
+    auto row_of = [&](int c) { return NX > 1 ? (int)__umulhi((unsigned)c, rNX) : c; };
     T t = (T)0, xp = (T)0, yp = (T)0, vx = (T)0, vy = (T)0, E = (T)0, E0 = (T)0, minenergy = (T)0;
     T acc_s = (T)0, acc_c = (T)0;
-    T rvx = (T)0, rvy = (T)0;  // FP64: 1/vx, 1/vy
-    long long seg = 0;
-    Stream rs;
+    T rvx = (T)0, rvy = (T)0;  // 1/vx, 1/vy (FP32: inf where div_mid is to divide)
+    unsigned seg = 0;
+    Stream rs;     // FP64
+    Words<5> ws;   // FP32
     auto start = [&]() {
         const int cell0 = cs & 0xFFFFFF;
         k = cs >> 24;
-        xi = cell0 % NX;
-        yi = cell0 / NX;
-        rs.init(seed, step, (uint32_t)i, kStageTransport);
+        yi = row_of(cell0);
+        xi = cell0 - yi * NX;
+        se = s_sexp[k];
+        if constexpr (SMT) slots_k = dep_shared + 24u * (unsigned)(k * nc);
+        if constexpr (sizeof(T) == 8) rs.init(seed, step, (uint32_t)i, kStageTransport);
+        else if constexpr (SCHED == kLongSchedule) ws.init((uint32_t)i);
+        else ws.init_full((uint32_t)i, round_keys(ca), step, kStageTransport);
         minenergy = cutoff_energy(E0);  // (T)(0.01 * (double)E0), without FP64 in binary32
         acc_s = (T)0;
         acc_c = (T)0;
-        acc_cell = cell0;
         seg = 0;
-        if constexpr (sizeof(T) == 8) {
-            rvx = 1.0 / vx;
-            rvy = 1.0 / vy;
-        }
+        rvx = face_rcp(vx);
+        rvy = face_rcp(vy);
     };
     auto load = [&](long long e, int &lcs, T &lt, T &lx, T &ly, T &lvx, T &lvy, T &lE, T &lE0) -> bool {
         if (!pb.alive[e]) return false;
@@ -598,8 +611,9 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
         lE0 = (T)pb.E0[e];
         if (St::half) {
             lt = ld_f(pb.t + e) * (float)dtT;
-            lx = ld_f(pb.x + e) * (float)fx[c0 % NX].ws;
-            ly = ld_f(pb.y + e) * (float)fy[c0 / NX].ws;
+            const int r0 = row_of(c0);
+            lx = ld_f(pb.x + e) * (float)fx[c0 - r0 * NX].ws;
+            ly = ld_f(pb.y + e) * (float)fy[r0].ws;
             lvx = ld_f(pb.ux + e);
             lvy = ld_f(pb.uy + e);
             lE = ld_f(pb.E + e) * (float)lE0;
@@ -609,36 +623,38 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
         }
         return true;
     };
+    // the deposits of the cell the history leaves, or ends in
+    auto flush_cell = [&]() {
+        const int cell = xi + yi * NX;
+        const T v = acc_s + acc_c;
+        if constexpr (SMT && sizeof(T) == 4)
+            if (add_f32_smem(slots_k + 24u * (unsigned)cell, v, b_dep + se)) return;
+        flush_rest<T, SMT>(dep_acc, k * nc + cell, v, b_dep + se, flags);
+    };
     // one pass of the reference's while loop (src/imc_transport.jl:533-717);
     // 0 = go on, 1 = killed, 2 = census, 4 = escaped through a vacuum face.
     // The census write and the escape tally are left to finish(), which
-    // the warp runs converged once per history.
+    // the warp runs converged once per history.  Both axes and both directions
+    // share one path through the face: a warp's lanes cross all four.
     auto segment = [&]() -> int {
         if (++seg > cap) { flags |= (1u << 2); return 1; }
         const int cell = xi + yi * NX;
         const Tab2<T> ce = tab[cell];
         T dist_bx, dist_by, dist_col, dist_cen, dist, Edens, newenergy, dep;
         bool at_b, at_col, at_cen, dead;
-        // the distances by the reference's expressions and order
-        auto general = [&]() {
-            dist_bx = vx > (T)0 ? m_abs((fx[xi].ws - xp) / vx) : m_abs(xp / vx);
-            dist_by = vy > (T)0 ? m_abs((fy[yi].ws - yp) / vy) : m_abs(yp / vy);
-            T dist_b;
-            if (dist_bx != dist_bx) dist_b = dist_by;
-            else if (dist_by != dist_by) dist_b = dist_bx;
-            else dist_b = jmin(dist_bx, dist_by);
-            dist = jmin(jmin(dist_b, dist_col), dist_cen);
+        const bool right = vx > (T)0, up = vy > (T)0;
+        if constexpr (sizeof(T) == 4) {
+            if (ws.n < 2) ws.refill(round_keys(ca), step, kStageTransport);
+            dist_col = SegMath<T>::flight(ws.w[0], ce.rseff);
+            dist_cen = c * (dtT - t) * ds;
+            // the reference's quotients |num / v|
+            dist_bx = m_abs(div_mid(right ? fx[xi].ws - xp : xp, vx, rvx));
+            dist_by = m_abs(div_mid(up ? fy[yi].ws - yp : yp, vy, rvy));
+            dist = min3_nan(fminf(dist_bx, dist_by), dist_col, dist_cen);
+            if (dist != dist) { flags |= 1u; return 1; }
             at_b = dist == dist_bx || dist == dist_by;
             at_col = dist == dist_col;
             at_cen = dist == dist_cen;
-        };
-        if constexpr (sizeof(T) == 4) {
-            // FP32: the 1D kernels' formulation (SegMath<float>)
-            const float v = (float)((rs.next() >> 8) | 1u) * 0x1p-24f;
-            dist_col = -__logf(v) * ce.rseff;
-            dist_cen = c * (dtT - t) * ds;
-            general();
-            if (dist != dist) { flags |= 1u; return 1; }
             const float em1 = expm1_seg(-ce.saf * dist);
             newenergy = E + E * em1;
             Edens = E * ce.rarea;
@@ -650,8 +666,8 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
             dist_cen = dtT - t;
             if (!c_one) dist_cen = c * dist_cen;
             if (!ds_one) dist_cen = dist_cen * ds;
-            dist_bx = m_abs(m64::div_r(pos64(vx) ? fx[xi].ws - xp : xp, vx, rvx));
-            dist_by = m_abs(m64::div_r(pos64(vy) ? fy[yi].ws - yp : yp, vy, rvy));
+            dist_bx = m_abs(m64::div_r(right ? fx[xi].ws - xp : xp, vx, rvx));
+            dist_by = m_abs(m64::div_r(up ? fy[yi].ws - yp : yp, vy, rvy));
             const bool odd = !(plain64(dist_bx) && plain64(dist_by) && plain64(dist_col) && plain64(dist_cen));
             if (!odd) {
                 dist = min64(min64(dist_bx, dist_by), min64(dist_col, dist_cen));
@@ -660,22 +676,25 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
                 at_col = b == m64::bits(dist_col);
                 at_cen = b == m64::bits(dist_cen);
             } else {
-                general();
+                // by the reference's expressions and order
+                dist_bx = vx > (T)0 ? m_abs((fx[xi].ws - xp) / vx) : m_abs(xp / vx);
+                dist_by = vy > (T)0 ? m_abs((fy[yi].ws - yp) / vy) : m_abs(yp / vy);
+                T dist_b;
+                if (dist_bx != dist_bx) dist_b = dist_by;
+                else if (dist_by != dist_by) dist_b = dist_bx;
+                else dist_b = jmin(dist_bx, dist_by);
+                dist = jmin(jmin(dist_b, dist_col), dist_cen);
+                at_b = dist == dist_bx || dist == dist_by;
+                at_col = dist == dist_col;
+                at_cen = dist == dist_cen;
                 if (dist != dist) { flags |= 1u; return 1; }
             }
             Edens = E;
             newenergy = SegMath<double>::attenuate(E, ce.saf, dist, odd, &dep);
             dead = le64(newenergy, minenergy);
         }
-        if (cell != acc_cell) {
-            flush_pair<T, SMT>(dep_acc, k * nc + acc_cell, acc_s, acc_c, b_dep + s_sexp[k], flags);
-            acc_s = (T)0; acc_c = (T)0; acc_cell = cell;
-        }
-        if (dead) {
-            nadd(acc_s, acc_c, Edens);
-            return 1;
-        }
-        nadd(acc_s, acc_c, dep);
+        nadd(acc_s, acc_c, dead ? Edens : dep);
+        if (dead) return 1;
         if constexpr (sizeof(T) == 4) {
             xp += dist * vx;
             yp += dist * vy;
@@ -689,57 +708,42 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
         }
         E = newenergy;
         if (at_b) {
-            if (dist_bx < dist_by) {
-                if (vx > (T)0) {
-                    if (xi == NX - 1) {
-                        if (refl_r) { vx = -vx; rvx = -rvx; return 0; }
-                        return 4;
-                    }
-                    xi += 1; xp = (T)0;
-                } else {
-                    if (xi == 0) {
-                        if (refl_l) { vx = -vx; rvx = -rvx; return 0; }
-                        return 4;
-                    }
-                    xi -= 1; xp = fx[xi].ws;
-                }
-            } else {
-                if (vy > (T)0) {
-                    if (yi == NY - 1) {
-                        if (refl_t) { vy = -vy; rvy = -rvy; return 0; }
-                        return 4;
-                    }
-                    yi += 1; yp = (T)0;
-                } else {
-                    if (yi == 0) {
-                        if (refl_b) { vy = -vy; rvy = -rvy; return 0; }
-                        return 4;
-                    }
-                    yi -= 1; yp = fy[yi].ws;
-                }
+            if constexpr (sizeof(T) == 4) ws.drop(false);
+            const bool ax = dist_bx < dist_by, fwd = ax ? right : up;
+            const int next = (ax ? xi : yi) + (fwd ? 1 : -1);
+            if ((unsigned)next < (unsigned)(ax ? NX : NY)) {
+                flush_cell();
+                acc_s = (T)0;
+                acc_c = (T)0;
+                const T at = fwd ? (T)0 : (ax ? fx : fy)[next].ws;
+                if (ax) { xi = next; xp = at; }
+                else { yi = next; yp = at; }
+                return 0;
             }
+            if (!(ax ? (fwd ? refl_r : refl_l) : (fwd ? refl_t : refl_b))) return 4;
+            if (ax) { vx = -vx; rvx = -rvx; }
+            else { vy = -vy; rvy = -rvy; }
             return 0;
         }
         if (at_col) {
             // isotropic re-emission: angle 2*pi*rand in Float64, rounded to T
             // (binary32: two_pi_u24, the same value without FP64; the
             // hardware sine and cosine)
-            T ang;
-            if constexpr (sizeof(T) == 4) ang = two_pi_u24(rs.next() >> 8);
-            else ang = (T)(6.283185307179586 * (double)Rand<T>::u(rs));
-            if constexpr (sizeof(T) == 4) __sincosf(ang, &vy, &vx);
-            else {
-                m_sincos(ang, &vy, &vx);
-                rvx = 1.0 / vx;
-                rvy = 1.0 / vy;
+            if constexpr (sizeof(T) == 4) {
+                __sincosf(two_pi_u24(ws.w[1] >> 8), &vy, &vx);
+                ws.drop(true);
+            } else {
+                m_sincos((T)(6.283185307179586 * (double)Rand<T>::u(rs)), &vy, &vx);
             }
+            rvx = face_rcp(vx);
+            rvy = face_rcp(vy);
         }
         // census: t = 0 and the state written back by finish()
         if (at_cen) return 2;
         return 0;
     };
     auto finish = [&](int end) {
-        flush_pair<T, SMT>(dep_acc, k * nc + acc_cell, acc_s, acc_c, b_dep + s_sexp[k], flags);
+        flush_cell();
         if (end == 2) {
             // census: t = 0, write the state back (src/imc_transport.jl:700-717)
             const int cellf = xi + yi * NX;
@@ -762,18 +766,23 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
                 pb.E[i] = (typename St::S)E;
             }
             if (cellf != (cs & 0xFFFFFF)) pb.cs[i] = cellf | (k << 24);
-            flush_one<T, RAD_SMT>(rad_acc, k * nc + cellf, Est, b_rad + s_sexp[k], flags);
-            const int ee = exp_bound(Est) - s_sexp[k];
+            bool flushed = false;
+            if constexpr (sizeof(T) == 4) {
+                if constexpr (RAD_SMT) flushed = add_f32_smem(slots_k + 24u * (unsigned)(ca.K * nc + cellf), Est, b_rad + se);
+                else flushed = add_f32_global(rad_acc + 3 * (size_t)(k * nc + cellf), Est, b_rad + se);
+            }
+            if (!flushed) flush_rest<T, RAD_SMT>(rad_acc, k * nc + cellf, Est, b_rad + se, flags);
+            const int ee = exp_bound(Est) - se;
             emax_e = ee > emax_e ? ee : emax_e;
         } else {
             // killed, or escaped with E through a vacuum face
-            if (end == 4) flush_one<T, false>(ca.lost_acc, k, E, b_lost + s_sexp[k], flags);
+            if (end == 4) flush_one<T, false>(ca.lost_acc, k, E, b_lost + se, flags);
             pb.alive[i] = 0;
             ++killed;
         }
         segs += (unsigned long long)seg;
     };
-    if (sc->seg_per_hist < kRefillSegments) {
+    if (SCHED == kShortSchedule || (SCHED == kBothSchedules && !long_step)) {
         // short histories: one history per lane to its end (see k_transport1d)
         auto walk = [&](long long e) {
             if (!load(e, cs, t, xp, yp, vx, vy, E, E0)) return;
@@ -872,7 +881,7 @@ TransportShape transport_shape(const CellArgs &ca, int prec) {
     sh.smem = table + (int)(sh.smem_tally ? 2 * dep : sh.dep_only ? dep : 0);
     const bool shared = sh.smem_tally || sh.dep_only;
     sh.block = shared ? (prec == 0 ? kSmtBlock64 : kSmtBlock32) : (prec == 0 ? kGlbBlock64 : kGlbBlock32);
-    if (ca.geometry == 1) sh.block_long = prec == 0 ? sh.block : kLongBlock32;
+    sh.block_long = prec == 0 ? sh.block : kLongBlock32;
     return sh;
 }
 
@@ -884,19 +893,23 @@ template <class St> struct StBlocks {
     static constexpr int glb_long = fp64 ? kGlbBlock64 : kLongBlock32;
 };
 
-// the transport kernels of one state type and tally mode: 1D short histories,
-// 1D long histories, 2D
+// the transport kernels of one state type and tally mode: short histories, long
+// histories
 template <class St, int TM> struct Kernels {
     static constexpr int block = TM == kTallyGlobal ? StBlocks<St>::glb : StBlocks<St>::smt;
     static constexpr int block_long = TM == kTallyGlobal ? StBlocks<St>::glb_long : StBlocks<St>::smt_long;
+    static constexpr bool two = !StBlocks<St>::fp64;  // 2D: a kernel for each schedule
     static const void *ptr(int geometry, bool lng) {
-        if (geometry == 2) return (const void *)k_transport2d<St, block, TM>;
+        if (geometry == 2)
+            return lng ? (const void *)k_transport2d<St, block_long, TM, two ? kLongSchedule : kBothSchedules>
+                       : (const void *)k_transport2d<St, block, TM, two ? kShortSchedule : kBothSchedules>;
         if (lng) return (const void *)k_transport1d<St, block_long, TM, kModePlain, true>;
         return (const void *)k_transport1d<St, block, TM, kModePlain, false>;
     }
     static void launch(const CellArgs &ca, Scalars *sc, PBufPair buf, TransportGrid g, int smem, cudaStream_t st) {
         if (ca.geometry == 2) {
-            k_transport2d<St, block, TM><<<g.grid, block, smem, st>>>(ca, sc, buf);
+            k_transport2d<St, block, TM, two ? kShortSchedule : kBothSchedules><<<g.grid, block, smem, st>>>(ca, sc, buf);
+            if constexpr (two) k_transport2d<St, block_long, TM, kLongSchedule><<<g.grid_long, block_long, smem, st>>>(ca, sc, buf);
             return;
         }
         k_transport1d<St, block, TM, kModePlain, false><<<g.grid, block, smem, st>>>(ca, sc, buf, SurrWave{}, 0);

@@ -116,6 +116,18 @@ __device__ __forceinline__ bool add_f32_smem(long long *slot, float v, int b) {
     return add_f32_smem((unsigned)__cvta_generic_to_shared(slot), v, b);
 }
 
+// the same two words into a global slot's 64-bit accumulators (one flush per
+// census particle, seldom two of a warp's to one slot at once)
+__device__ __forceinline__ bool add_f32_global(long long *slot, float v, int b) {
+    int j;
+    uint32_t lo, hi;
+    if (!f32_words(v, b, j, lo, hi)) return false;
+    unsigned long long *a = reinterpret_cast<unsigned long long *>(slot) + 2 - j;
+    atomicAdd(a, (unsigned long long)lo);
+    if (hi) atomicAdd(a - 1, (unsigned long long)hi);
+    return true;
+}
+
 template <bool SMT> __device__ __forceinline__ void add_limbs(long long *a, const Limbs &L) {
     if (SMT) {
         // the pointer is known to address shared memory
@@ -354,9 +366,12 @@ __device__ __forceinline__ double min64(double a, double b) {
 __device__ __forceinline__ bool pos64(double v) { return (long long)m64::bits(v) > 0; }
 __device__ __forceinline__ bool le64(double a, double b) { return (long long)m64::bits(a) <= (long long)m64::bits(b); }
 template <> struct SegMath<float> {
-    static __device__ __forceinline__ float flight(uint32_t w, const Tab1<float> &ce) {
+    static __device__ __forceinline__ float flight(uint32_t w, float rseff) {
         const float v = (float)((w >> 8) | 1u) * 0x1p-24f;
-        return -log_fast(v) * ce.rseff;
+        return -log_fast(v) * rseff;
+    }
+    static __device__ __forceinline__ float flight(uint32_t w, const Tab1<float> &ce) {
+        return flight(w, ce.rseff);
     }
     static __device__ __forceinline__ float attenuate(float E, const Tab1<float> &ce, float d, float *dep) {
         const float em1 = expm1_seg(-ce.saf * d);
