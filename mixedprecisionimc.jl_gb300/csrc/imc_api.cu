@@ -831,7 +831,7 @@ int imc_create(const ImcDeck *d, ImcHandle **out) {
     }
     ca.surr_min_calls = 2ll * h->sm_count * 1024;  // two queries per thread of the GPU
     size_grids(h);
-    h->grid_emit = h->sm_count * 4;
+    h->grid_emit = h->sm_count * 8;
     if (cudaEventCreate(&h->ev[0]) != cudaSuccess || cudaEventCreate(&h->ev[1]) != cudaSuccess)
         return bail(fail(h, IMC_ERR_CUDA, "cudaEventCreate"));
     *out = h;

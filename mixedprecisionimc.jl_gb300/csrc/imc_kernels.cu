@@ -568,193 +568,261 @@ template <class T> struct RT;
 template <> struct RT<float> { static __device__ float sqrt_(float x) { return sqrtf(x); } };
 template <> struct RT<double> { static __device__ double sqrt_(double x) { return sqrt(x); } };
 
+// What every birth of a slot has in common, found once per slot.
+enum { kLeft1D, kRight1D, kBody1D, kBottom2D, kTop2D, kLeft2D, kRight2D, kBody2D };
+template <class T> struct BirthSlot {
+    int kind, cell, k;
+    T E0;
+    T wx, wy;      // widths that the drawn coordinates are multiplied by
+    T x0, y0;      // fixed coordinates of the surface births
+    T cx, cy;      // the cell's widths * DISTANCESCALE (FP16 state: the stored unit)
+};
+// binary32 copies of the widths for FP32 / FP16 births
+template <class T> __device__ __forceinline__ T width_x(const CellArgs &ca, int i) { return sizeof(T) == 4 ? (T)ca.dxf[i] : (T)ca.dx[i]; }
+template <class T> __device__ __forceinline__ T width_y(const CellArgs &ca, int i) { return sizeof(T) == 4 ? (T)ca.dyf[i] : (T)ca.dy[i]; }
+
 template <class St>
-__device__ __forceinline__ void store_birth(const CellArgs &ca, PBuf<St> &pb, long long pid, typename St::T t,
+__device__ __forceinline__ BirthSlot<typename St::T> birth_slot(const CellArgs &ca, int q) {
+    typedef typename St::T T;
+    const int ns = nsurf_slots(ca), nc = ca.nc, nx = ca.nx, ny = ca.ny;
+    // the surface births' fixed positions, the same for every birth of a
+    // face (computed on the host, CellArgs::surf_f / surf_d)
+    auto surf = [&](int w) -> T { return sizeof(T) == 4 ? (T)ca.surf_f[w] : (T)ca.surf_d[w]; };
+    BirthSlot<T> b;
+    b.E0 = sizeof(T) == 4 ? (T)ca.slot_nrg_f[q] : (T)ca.slot_nrg[q];
+    const int j = ca.slot_j[q];
+    b.k = j < 0 ? 0 : j;
+    b.wx = b.wy = b.x0 = b.y0 = b.cx = b.cy = (T)0;
+    int ix, iy = 0;
+    if (ca.geometry == 1) {
+        if (q < 2) {
+            b.kind = q == 0 ? kLeft1D : kRight1D;
+            ix = q == 0 ? 0 : nx - 1;
+            b.x0 = surf(q);
+        } else {
+            b.kind = kBody1D;
+            ix = q < ns + nc ? q - ns : q - ns - nc;
+            b.wx = width_x<T>(ca, ix);
+        }
+    } else if (q < ns) {
+        if (q < 2 * nx) {
+            const bool top = q >= nx;
+            b.kind = top ? kTop2D : kBottom2D;
+            ix = top ? q - nx : q;
+            iy = top ? ny - 1 : 0;
+            b.wx = width_x<T>(ca, ix);
+            b.y0 = surf(top ? 5 : 4);
+        } else {
+            const bool right = q >= 2 * nx + ny;
+            b.kind = right ? kRight2D : kLeft2D;
+            iy = right ? q - 2 * nx - ny : q - 2 * nx;
+            ix = right ? nx - 1 : 0;
+            b.x0 = surf(right ? 3 : 2);
+            // the reference scales y by mesh.dx[j] (src/imc_sourcing.jl:301,316)
+            b.wy = iy < nx ? width_x<T>(ca, iy) : width_y<T>(ca, iy);
+        }
+    } else {
+        const int cell = q < ns + nc ? q - ns : q - ns - nc;
+        b.kind = kBody2D;
+        iy = cell / nx;
+        ix = cell - iy * nx;
+        b.wx = width_x<T>(ca, ix);
+        b.wy = width_y<T>(ca, iy);
+    }
+    b.cell = ix + iy * nx;
+    if (St::half) {
+        b.cx = width_x<T>(ca, ix) * (T)ca.ds_f;
+        if (ca.geometry == 2) b.cy = width_y<T>(ca, iy) * (T)ca.ds_f;
+    }
+    return b;
+}
+
+template <class St>
+__device__ __forceinline__ void store_birth(int geometry, PBuf<St> &pb, long long pid, typename St::T t,
                                             typename St::T x, typename St::T y, typename St::T ux,
-                                            typename St::T uy, typename St::T E0, int cell, int k, float dtf) {
+                                            typename St::T uy, const BirthSlot<typename St::T> &b, float dtf) {
     typedef typename St::S S;
     if (St::half) {
-        const int ix = ca.geometry == 1 ? cell : cell % ca.nx;
-        float dxs = (float)ca.dx[ix] * (float)ca.ds;
-        st_v(pb.x + pid, (float)x / dxs);
-        if (ca.geometry == 2) {
-            const int iy = cell / ca.nx;
-            float dys = (float)ca.dy[iy] * (float)ca.ds;
-            st_v(pb.y + pid, (float)y / dys);
+        st_v(pb.x + pid, (float)x / (float)b.cx);
+        if (geometry == 2) {
+            st_v(pb.y + pid, (float)y / (float)b.cy);
             st_v(pb.uy + pid, (float)uy);
         }
         st_v(pb.t + pid, (float)t / dtf);
         st_v(pb.ux + pid, (float)ux);
         st_v(pb.E + pid, 1.0f);
-        pb.E0[pid] = (float)E0;
+        pb.E0[pid] = (float)b.E0;
     } else {
         pb.t[pid] = (S)t;
         pb.x[pid] = (S)x;
         pb.ux[pid] = (S)ux;
-        if (ca.geometry == 2) { pb.y[pid] = (S)y; pb.uy[pid] = (S)uy; }
-        pb.E[pid] = (S)E0;
-        pb.E0[pid] = (typename St::E0S)E0;
+        if (geometry == 2) { pb.y[pid] = (S)y; pb.uy[pid] = (S)uy; }
+        pb.E[pid] = (S)b.E0;
+        pb.E0[pid] = (typename St::E0S)b.E0;
     }
-    pb.cs[pid] = cell | (k << 24);
+    pb.cs[pid] = b.cell | (b.k << 24);
     pb.alive[pid] = 1;
 }
 
+// the uniforms of one birth, in the stream's order: for binary32 the words of a
+// block made at once (four serve a birth but for a redraw)
+template <class T> struct BirthDraws;
+template <> struct BirthDraws<float> {
+    Words<5> ws;
+    const CellArgs &ca;
+    unsigned step;
+    __device__ __forceinline__ BirthDraws(const CellArgs &c, unsigned st, uint32_t pid) : ca(c), step(st) {
+        ws.init_full(pid, ca.rk, step, kStageSource);
+    }
+    __device__ __forceinline__ uint32_t word() {
+        if (ws.n == 0) ws.refill(ca.rk, step, kStageSource);
+        const uint32_t w = ws.w[0];
+        ws.drop(false);
+        return w;
+    }
+    __device__ __forceinline__ float u() { return Rand<float>::u(word()); }
+    __device__ __forceinline__ float cosine() { return Rand<float>::cosine(word()); }
+};
+template <> struct BirthDraws<double> {
+    Stream rs;
+    __device__ __forceinline__ BirthDraws(const CellArgs &ca, unsigned step, uint32_t pid) {
+        rs.init(ca.seed, step, pid, kStageSource);
+    }
+    __device__ __forceinline__ double u() { return Rand<double>::u(rs); }
+    __device__ __forceinline__ double cosine() { return Rand<double>::cosine(rs); }
+};
+
 // One thread per newborn particle; its stream is keyed by its list index.
-template <class St>
+// (Instruction issue bounds it: 33 B are stored for 250 instructions a warp's
+// birth with the slot looked up and decoded for each, 49 us for the channel's
+// 4e6 births.)
+template <class St, int G>
 __global__ void __launch_bounds__(256) k_source_emit(CellArgs ca, Scalars *sc, PBufPair bufs) {
     typedef typename St::T T;
     PBuf<St> pb(bufs.b[sc->cur]);
     const long long n_new = sc->n_sourced, n_census = sc->birth_base;
     const unsigned step = sc->step;
-    const double dtd = sc->dt;
-    const T dtT = (T)dtd, dsT = (T)ca.ds;
-    const int ns = nsurf_slots(ca), nc = ca.nc, nslots = ca.nslots;
+    const T dtT = (T)sc->dt, dsT = Consts<T>::ds(ca);
+    const int nslots = ca.nslots;
     const double pd = 3.141592653589793;
-    // the surface births' fixed positions, the same for every birth of a
-    // face (computed on the host, CellArgs::surf_f / surf_d)
-    auto surf = [&](int w) -> T { return sizeof(T) == 4 ? (T)ca.surf_f[w] : (T)ca.surf_d[w]; };
-    const T x1_l = surf(0), x1_r = surf(1), x2_l = surf(2), x2_r = surf(3), y2_b = surf(4), y2_t = surf(5);
     // Each warp takes `run` consecutive births at a time, lane l the births
     // base + l + 32 i (every store coalesced).  A lane finds the slot of its
-    // first birth by binary search over the slot offsets (slot = last q with
-    // slot_off[q] <= j) and the later ones by galloping forward from there
-    // (q + 1, q + 2, q + 4, ... then bisection): one or two loads where the
-    // slot holds many births (the channel's surface segment), a few where
-    // it holds a handful (the CELLMIN births of every body cell).  The run
-    // is the births per warp of the grid, rounded up to a multiple of 32 in
-    // [32, 256], so a small step's births still spread over every warp.
+    // first birth by binary search over the slot offsets (slot = last q whose
+    // first birth is at or below j) and the later ones by galloping forward
+    // from there (q + 1, q + 2, q + 4, ... then bisection) once the slot's
+    // last birth is behind it.  The run is the births per warp of the grid,
+    // rounded up to a multiple of 32 in [32, 1024], so a small step's births
+    // still spread over every warp.
     auto off = [&](int s) { return ca.slot_off[s] + ca.blk_off[s / kCountThreads]; };
     const int lane = threadIdx.x & 31;
     const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
     const long long per_warp = (n_new + nw - 1) / nw;
-    const int run = per_warp >= 256 ? 256 : per_warp <= 32 ? 32 : (int)((per_warp + 31) & ~31ll);
-    for (long long base = wid * run; base < n_new; base += nw * run)
-    for (int q = -1, r = 0; r < run; r += 32) {
-        const long long j = base + r + lane;
-        if (j >= n_new) break;
-        if (q < 0) {
-            // the last block that starts at or below j, then its last such slot
-            int lo = 0, hi = ca.nblk_count;
-            while (hi - lo > 1) {
-                int mid = (lo + hi) >> 1;
-                if (ca.blk_off[mid] <= j) lo = mid;
-                else hi = mid;
-            }
-            const long long rest = j - ca.blk_off[lo];
-            lo *= kCountThreads;
-            hi = min(lo + kCountThreads, nslots);
-            while (hi - lo > 1) {
-                int mid = (lo + hi) >> 1;
-                if (ca.slot_off[mid] <= rest) lo = mid;
-                else hi = mid;
-            }
-            q = lo;
-        } else if (q + 1 < nslots && off(q + 1) <= j) {
-            int lo = q + 1, step = 2, hi = q + 2;  // slot_off[lo] <= j
-            while (hi < nslots && off(hi) <= j) {
-                lo = hi;
-                step <<= 1;
-                hi = q + step;
-            }
-            if (hi > nslots) hi = nslots;  // slot_off[hi] > j, or hi == nslots
-            while (hi - lo > 1) {
-                const int mid = (lo + hi) >> 1;
-                if (off(mid) <= j) lo = mid;
-                else hi = mid;
-            }
-            q = lo;
-        }
-        const long long pid = n_census + j;
-        Stream rs;
-        rs.init(ca.seed, step, (uint32_t)pid, kStageSource);
-        const T E0 = sizeof(T) == 4 ? (T)ca.slot_nrg_f[q] : (T)ca.slot_nrg[q];
-        const int k = ca.slot_j[q] < 0 ? 0 : ca.slot_j[q];
-        if (ca.geometry == 1) {
-            if (q < 2) {
-                // surface births (src/imc_sourcing.jl:161-189)
-                const int cell = q == 0 ? 0 : ca.nx - 1;
-                T xpos = q == 0 ? x1_l : x1_r;
-                T mu = (T)0;
-                for (int r = 0; r < 64 && mu == (T)0; ++r) {
-                    T rr = RT<T>::sqrt_(Rand<T>::u(rs));
-                    mu = q == 0 ? rr : -rr;
-                }
-                if (mu == (T)0) mu = q == 0 ? (T)1 : (T)-1;
-                T st = dtT * Rand<T>::u(rs);
-                store_birth<St>(ca, pb, pid, st, xpos, (T)0, mu, (T)0, E0, cell, k, (float)dtT);
-            } else {
-                // body / source births (src/imc_sourcing.jl:193-236)
-                const int cell = q < ns + nc ? q - ns : q - ns - nc;
-                T xpos = (sizeof(T) == 4 ? (T)ca.dxf[cell] : (T)ca.dx[cell]) * Rand<T>::u(rs) * dsT;
-                T mu = (T)0;
-                for (int r = 0; r < 64 && mu == (T)0; ++r) mu = (T)1 - (T)2 * Rand<T>::u(rs);
-                if (mu == (T)0) mu = (T)1;
-                T st = dtT * Rand<T>::u(rs);
-                store_birth<St>(ca, pb, pid, st, xpos, (T)0, mu, (T)0, E0, cell, k, (float)dtT);
-            }
-        } else {
-            T st, xpos, ypos, ang;
-            int ix, iy;
-            if (q < ns) {
-                // surface births (src/imc_sourcing.jl:265-323)
-                const int nx = ca.nx, ny = ca.ny;
-                int face, idx;
-                if (q < nx) { face = 0; idx = q; }
-                else if (q < 2 * nx) { face = 1; idx = q - nx; }
-                else if (q < 2 * nx + ny) { face = 2; idx = q - 2 * nx; }
-                else { face = 3; idx = q - 2 * nx - ny; }
-                st = dtT * Rand<T>::u(rs);
-                // the angles are the reference's Float64 products rounded to T
-                // (binary32: pi_n24 of the uniform's integer m, the same value
-                // without FP64; the widths binary32 copies)
-                if (face < 2) {
-                    ix = idx;
-                    iy = face == 0 ? 0 : ny - 1;
-                    xpos = (sizeof(T) == 4 ? (T)ca.dxf[ix] : (T)ca.dx[ix]) * Rand<T>::u(rs) * dsT;
-                    ypos = face == 0 ? y2_b : y2_t;
-                    if constexpr (sizeof(T) == 4) {
-                        const uint32_t m = rs.next() >> 8;
-                        ang = face == 0 ? (T)pd * ((T)m * 0x1p-24f) : -pi_n24((int)m);
-                    } else {
-                        T u = Rand<T>::u(rs);
-                        ang = face == 0 ? (T)((T)pd * u) : (T)(-pd * (double)u);
+    const int run = per_warp >= 1024 ? 1024 : per_warp <= 32 ? 32 : (int)((per_warp + 31) & ~31ll);
+    for (long long base = wid * run; base < n_new; base += nw * run) {
+        int q = -1;
+        long long next = -1;  // the first birth beyond slot q
+        BirthSlot<T> b{};
+        for (int r = 0; r < run; r += 32) {
+            const long long j = base + r + lane;
+            if (j >= n_new) break;
+            if (next <= j) {
+                int lo, hi;
+                if (q < 0) {
+                    // the last block that starts at or below j, then its last such slot
+                    lo = 0;
+                    hi = ca.nblk_count;
+                    while (hi - lo > 1) {
+                        const int mid = (lo + hi) >> 1;
+                        if (ca.blk_off[mid] <= j) lo = mid;
+                        else hi = mid;
+                    }
+                    const long long rest = j - ca.blk_off[lo];
+                    lo *= kCountThreads;
+                    hi = min(lo + kCountThreads, nslots);
+                    while (hi - lo > 1) {
+                        const int mid = (lo + hi) >> 1;
+                        if (ca.slot_off[mid] <= rest) lo = mid;
+                        else hi = mid;
                     }
                 } else {
-                    iy = idx;
-                    ix = face == 2 ? 0 : nx - 1;
-                    xpos = face == 2 ? x2_l : x2_r;
-                    // the reference scales y by mesh.dx[j] (src/imc_sourcing.jl:301,316)
-                    if constexpr (sizeof(T) == 4) {
-                        ypos = (iy < nx ? ca.dxf[iy] : ca.dyf[iy]) * Rand<T>::u(rs) * dsT;
-                        const uint32_t m = rs.next() >> 8;
-                        ang = face == 2 ? pi_n24((1 << 23) - (int)m)
-                                        : (T)(pd * (0.5 + (double)((T)m * 0x1p-24f)));
-                    } else {
-                        const double wq = iy < nx ? ca.dx[iy] : ca.dy[iy];
-                        ypos = (T)wq * Rand<T>::u(rs) * dsT;
-                        T u = Rand<T>::u(rs);
-                        ang = face == 2 ? (T)(pd * (0.5 - (double)u)) : (T)(pd * (0.5 + (double)u));
+                    int stride = 2;
+                    lo = q + 1;  // off(lo) <= j
+                    hi = q + 2;
+                    while (hi < nslots && off(hi) <= j) {
+                        lo = hi;
+                        stride <<= 1;
+                        hi = q + stride;
+                    }
+                    if (hi > nslots) hi = nslots;  // off(hi) > j, or hi == nslots
+                    while (hi - lo > 1) {
+                        const int mid = (lo + hi) >> 1;
+                        if (off(mid) <= j) lo = mid;
+                        else hi = mid;
                     }
                 }
-            } else {
-                // body / source births (src/imc_sourcing.jl:326-366)
-                const int cell = q < ns + nc ? q - ns : q - ns - nc;
-                ix = cell % ca.nx;
-                iy = cell / ca.nx;
-                // binary32 widths precomputed (no per-birth conversion); the
-                // angle is the reference's Float64 2 pi rand rounded to T
-                // (binary32: two_pi_u24, the same value without FP64)
-                xpos = (sizeof(T) == 4 ? (T)ca.dxf[ix] : (T)ca.dx[ix]) * Rand<T>::u(rs) * dsT;
-                ypos = (sizeof(T) == 4 ? (T)ca.dyf[iy] : (T)ca.dy[iy]) * Rand<T>::u(rs) * dsT;
-                if constexpr (sizeof(T) == 4) ang = two_pi_u24(rs.next() >> 8);
-                else ang = (T)(2.0 * pd * (double)Rand<T>::u(rs));
-                st = dtT * Rand<T>::u(rs);
+                q = lo;
+                next = q + 1 < nslots ? off(q + 1) : n_new;
+                b = birth_slot<St>(ca, q);
             }
-            T ux, uy;
-            if (sizeof(T) == 4) { float s_, c_; sincosf((float)ang, &s_, &c_); ux = (T)c_; uy = (T)s_; }
-            else { double s_, c_; sincos((double)ang, &s_, &c_); ux = (T)c_; uy = (T)s_; }
-            store_birth<St>(ca, pb, pid, st, xpos, ypos, ux, uy, E0, ix + iy * ca.nx, k, (float)dtT);
+            const long long pid = n_census + j;
+            BirthDraws<T> d(ca, step, (uint32_t)pid);
+            if (G == 1) {
+                T xpos, mu;
+                if (b.kind == kBody1D) {
+                    // body / source births (src/imc_sourcing.jl:193-236)
+                    xpos = b.wx * d.u() * dsT;
+                    mu = d.cosine();
+                    for (int r1 = 1; r1 < 64 && mu == (T)0; ++r1) mu = d.cosine();
+                    if (mu == (T)0) mu = (T)1;
+                } else {
+                    // surface births (src/imc_sourcing.jl:161-189)
+                    xpos = b.x0;
+                    mu = RT<T>::sqrt_(d.u());
+                    for (int r1 = 1; r1 < 64 && mu == (T)0; ++r1) mu = RT<T>::sqrt_(d.u());
+                    if (mu == (T)0) mu = (T)1;
+                    if (b.kind == kRight1D) mu = -mu;
+                }
+                const T st = dtT * d.u();
+                store_birth<St>(1, pb, pid, st, xpos, (T)0, mu, (T)0, b, (float)dtT);
+            } else {
+                T st, xpos, ypos, ang;
+                // the angles are the reference's Float64 products rounded to T
+                // (binary32: pi_n24 or two_pi_u24 of the uniform's integer m,
+                // the same value without FP64)
+                if (b.kind == kBody2D) {
+                    // body / source births (src/imc_sourcing.jl:326-366)
+                    xpos = b.wx * d.u() * dsT;
+                    ypos = b.wy * d.u() * dsT;
+                    if constexpr (sizeof(T) == 4) ang = two_pi_u24(d.word() >> 8);
+                    else ang = (T)(2.0 * pd * (double)d.u());
+                    st = dtT * d.u();
+                } else {
+                    // surface births (src/imc_sourcing.jl:265-323)
+                    st = dtT * d.u();
+                    const bool horizontal = b.kind == kBottom2D || b.kind == kTop2D;
+                    const T along = (horizontal ? b.wx : b.wy) * d.u() * dsT;
+                    xpos = horizontal ? along : b.x0;
+                    ypos = horizontal ? b.y0 : along;
+                    if constexpr (sizeof(T) == 4) {
+                        const uint32_t m = d.word() >> 8;
+                        if (b.kind == kBottom2D) ang = (T)pd * ((T)m * 0x1p-24f);
+                        else if (b.kind == kTop2D) ang = -pi_n24((int)m);
+                        else if (b.kind == kLeft2D) ang = pi_n24((1 << 23) - (int)m);
+                        else ang = (T)(pd * (0.5 + (double)((T)m * 0x1p-24f)));
+                    } else {
+                        const T u = d.u();
+                        if (b.kind == kBottom2D) ang = (T)((T)pd * u);
+                        else if (b.kind == kTop2D) ang = (T)(-pd * (double)u);
+                        else if (b.kind == kLeft2D) ang = (T)(pd * (0.5 - (double)u));
+                        else ang = (T)(pd * (0.5 + (double)u));
+                    }
+                }
+                T ux, uy;
+                if (sizeof(T) == 4) { float s_, c_; sincosf((float)ang, &s_, &c_); ux = (T)c_; uy = (T)s_; }
+                else { double s_, c_; sincos((double)ang, &s_, &c_); ux = (T)c_; uy = (T)s_; }
+                store_birth<St>(2, pb, pid, st, xpos, ypos, ux, uy, b, (float)dtT);
+            }
         }
     }
 }
@@ -773,9 +841,10 @@ void launch_source(const CellArgs &ca, Scalars *sc, int prec, PBufPair buf, int 
     if (update) launch_slots<true>(ca, sc, st);
     else launch_slots<false>(ca, sc, st);
     k_source_counts<<<ca.nblk_count, kCountThreads, 0, st>>>(ca, sc);
-    if (prec == 0) k_source_emit<StF64><<<grid, 256, 0, st>>>(ca, sc, buf);
-    else if (prec == 1) k_source_emit<StF32><<<grid, 256, 0, st>>>(ca, sc, buf);
-    else k_source_emit<StF16><<<grid, 256, 0, st>>>(ca, sc, buf);
+    auto emit = ca.geometry == 1
+                    ? (prec == 0 ? k_source_emit<StF64, 1> : prec == 1 ? k_source_emit<StF32, 1> : k_source_emit<StF16, 1>)
+                    : (prec == 0 ? k_source_emit<StF64, 2> : prec == 1 ? k_source_emit<StF32, 2> : k_source_emit<StF16, 2>);
+    emit<<<grid, 256, 0, st>>>(ca, sc, buf);
 }
 
 // ------------------------------------------------------------- compaction
