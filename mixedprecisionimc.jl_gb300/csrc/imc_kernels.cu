@@ -99,6 +99,14 @@ __device__ __forceinline__ int biased_exp(double x) { return (int)((d2u(x) >> 52
 // digits serve for finite terms that are not all tiny
 __device__ __forceinline__ bool digits_serve(int emax) { return emax >= kDigitsExpMin && emax < 0x7FF; }
 
+// the bits of the largest of the lanes' doubles, none of them negative or NaN
+__device__ __forceinline__ unsigned long long warp_max_bits(double v) {
+    const uint64_t b = d2u(v);
+    const unsigned hi = __reduce_max_sync(0xFFFFFFFFu, (unsigned)(b >> 32));
+    const unsigned lo = __reduce_max_sync(0xFFFFFFFFu, (unsigned)(b >> 32) == hi ? (unsigned)b : 0u);
+    return ((unsigned long long)hi << 32) | lo;
+}
+
 // sum of one double-double a lane over the warp, by shuffles (any values)
 __device__ __forceinline__ DD warp_sum_tree(DD d) {
     for (int off = 16; off > 0; off >>= 1) {
@@ -431,7 +439,7 @@ __device__ __forceinline__ void source_total(const CellArgs &ca, const Scalars *
 // (the scan alone took 7 us for 4002 slots, 15 us for 11,560).
 __global__ void __launch_bounds__(kCountThreads) k_source_counts(CellArgs ca, Scalars *sc) {
     constexpr int W = kCountThreads / 32;
-    __shared__ double s_max[W];
+    __shared__ unsigned long long s_max[W];
     __shared__ long long s_tot[W], s_run;
     __shared__ int s_last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -469,7 +477,7 @@ __global__ void __launch_bounds__(kCountThreads) k_source_counts(CellArgs ca, Sc
         ca.slot_nrg[q] = nrg;
         ca.slot_nrg_f[q] = (float)nrg;
         // the largest birth energy in true units (see scale_exp)
-        if (n > 0) my = times_pow2(nrg, -scale_exp(scale));
+        if (n > 0 && nrg > 0.0) my = times_pow2(nrg, -scale_exp(scale));
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         sc->totalenergy = E;
@@ -482,15 +490,11 @@ __global__ void __launch_bounds__(kCountThreads) k_source_counts(CellArgs ca, Sc
         const long long y = __shfl_up_sync(0xFFFFFFFFu, x, off);
         if (lane >= off) x += y;
     }
-    for (int off = 16; off > 0; off >>= 1) {
-        const double o = __shfl_down_sync(0xFFFFFFFFu, my, off);
-        my = o > my ? o : my;
-    }
+    unsigned long long most = warp_max_bits(my);
     if (lane == 31) s_tot[warp] = x;
-    if (lane == 0) s_max[warp] = my;
+    if (lane == 0) s_max[warp] = most;
     __syncthreads();
     long long before = 0, total = 0;
-    double most = 0.0;
     for (int w = 0; w < W; ++w) {
         before += w < warp ? s_tot[w] : 0;
         total += s_tot[w];
@@ -499,8 +503,11 @@ __global__ void __launch_bounds__(kCountThreads) k_source_counts(CellArgs ca, Sc
     if (q < ca.nslots) ca.slot_off[q] = before + x - n;
     if (threadIdx.x == 0) {
         ca.blk_off[blockIdx.x] = total;
-        ca.part_emax[blockIdx.x] = most;
+        ca.part_emax[blockIdx.x] = m64::from_bits(most);
     }
+    const long long n_census = sc->n_census;  // live particles
+    const long long len = sc->n_particles;    // list length, holes included
+    const int ce = sc->emax_census_exp;
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) s_last = atomicAdd(&sc->tally_blocks_done, 1u) == gridDim.x - 1u;
@@ -508,12 +515,12 @@ __global__ void __launch_bounds__(kCountThreads) k_source_counts(CellArgs ca, Sc
     if (!s_last) return;
     __threadfence();
     if (threadIdx.x == 0) s_run = 0;
-    double emax = 0.0;
+    double emax = 0.0;  // (energies: not negative, ordered as their bits)
     const int nb = gridDim.x;
     for (int base = 0; base < nb; base += kCountThreads) {
         const int b = base + threadIdx.x;
         const long long v = b < nb ? ca.blk_off[b] : 0;
-        if (b < nb) emax = fmax(emax, ca.part_emax[b]);
+        if (b < nb && d2u(ca.part_emax[b]) > d2u(emax)) emax = ca.part_emax[b];
         long long y = v;
         for (int off = 1; off < 32; off <<= 1) {
             const long long o = __shfl_up_sync(0xFFFFFFFFu, y, off);
@@ -528,14 +535,13 @@ __global__ void __launch_bounds__(kCountThreads) k_source_counts(CellArgs ca, Sc
         __syncthreads();
         if (threadIdx.x == kCountThreads - 1) s_run = start + y;
     }
-    for (int off = 16; off > 0; off >>= 1) emax = fmax(emax, __shfl_down_sync(0xFFFFFFFFu, emax, off));
-    if (lane == 0) s_max[warp] = emax;
+    most = warp_max_bits(emax);
+    if (lane == 0) s_max[warp] = most;
     __syncthreads();
     if (threadIdx.x == 0) {
         sc->tally_blocks_done = 0u;
-        for (int w = 0; w < W; ++w) emax = fmax(emax, s_max[w]);
-        const long long n_census = sc->n_census;  // live particles
-        const long long len = sc->n_particles;    // list length, holes included
+        for (int w = 0; w < W; ++w) most = s_max[w] > most ? s_max[w] : most;
+        emax = m64::from_bits(most);
         long long n_new = s_run;
         unsigned fl = 0;
         if (len + n_new > ca.capacity) {
@@ -543,7 +549,6 @@ __global__ void __launch_bounds__(kCountThreads) k_source_counts(CellArgs ca, Sc
             if (n_new < 0) n_new = 0;
             fl |= 1u << 3;
         }
-        const int ce = sc->emax_census_exp;
         emax = fmax(ce == kNoExp ? 0.0 : exp_top(ce), emax);
         sc->n_census_in = n_census;
         sc->n_sourced = n_new;
