@@ -1,24 +1,28 @@
 // imc_math64.cuh -- the double precision functions of a transport segment,
-// with few FP64 operations: GB300 issues FP64 at 1/64 of the FP32 rate (one
-// warp instruction in 16 cycles per SM), so an FP64 history costs its FP64
-// instructions and little else.
+// with few FP64 operations: GB300 issues FP64 at 1/64 of the FP32 rate (a warp's
+// FP64 instruction takes 64 cycles of its scheduler's unit), so an FP64
+// history costs its FP64 instructions and little else, and a function in 64-bit
+// integers -- about a hundred instructions at one or two cycles -- is a tenth of
+// the same function in sixteen FP64 instructions.
 //
 //   neglog_k53   -log(k 2^-53) of a 53-bit uniform integer k: table-driven
-//                reduction after Tang (ACM TOMS 16, 1990): the mantissa m times
-//                a short table reciprocal c leaves r = m c - 1, |r| <= 2^-8;
-//                -log v = e ln 2 + log c - log1p(r), with ln 2 and log c split
-//                in a high part on the grid 2^-42 (their sum exact) and a low part
-//   expm1_neg    exp(-y) - 1 for y >= 0: y = n ln2/64 + r, 0 <= r < ln2/64 (Tang,
-//                ACM TOMS 15, 1989), 2^(-n/64) from a two-double table
+//                reduction after Tang (ACM TOMS 16, 1990) in fixed point: the
+//                mantissa m times a short table reciprocal c leaves r = m c - 1,
+//                |r| <= 2^-8, exactly; -log v = e ln 2 + log c - log1p(r)
+//   expm1_neg    exp(-y) - 1 for y >= 0.  Below 1, in fixed point, y = j/64 + r:
+//                1 - exp(-y) = D_j + (1 - D_j) q with D_j = 1 - exp(-j/64) and
+//                q = r g(r), g(r) = 1 - r/2 + r^2/6 - ...; for j = 0 y g(y), so
+//                that small results keep their relative accuracy.  From 1 on in
+//                FP64 (Tang, ACM TOMS 15, 1989)
 //   div_r        a / b with r = RN(1/b) at hand: one residual correction
 //                (Markstein, IBM J. Res. Dev. 34, 1990), a / b correctly rounded
 //   u53, one_minus_2u53   uniforms from their integers without a conversion
 //
 // Largest errors seen (tests/test_math64.py, against extended precision):
-// 0.503 units in the last place for neglog_k53, 1.15 for expm1_neg; div_r
+// 0.60 units in the last place for neglog_k53, 1.01 for expm1_neg; div_r
 // equals the IEEE quotient.  CUDA's log, exp and expm1 are good to 1 unit each.
-// Table entries are the correctly rounded values of the stated expressions,
-// computed with 300-bit arithmetic; the polynomials are the Taylor series.
+// Table entries are the nearest integers to the stated expressions, computed
+// with 400-bit arithmetic; the polynomials are the Taylor series.
 #pragma once
 #include <cmath>
 #include <cstdint>
@@ -31,268 +35,286 @@
 namespace imc {
 namespace m64 {
 
-// one row per 1/256 of the mantissa [1, 2): c, log(c) high and low.  Mantissas
+// one row per 1/256 of the mantissa [1, 2): log(c) 2^62 and 512 c.  Mantissas
 // from 1.5 up are halved, so the rows next to 1 on both sides have c = 1.
-struct LogRow { double c, hi, lo, pad; };
-struct ExpRow { double hi, lo; };  // 2^(-j/64)
+struct LogRow { long long l, c; };
 #define IMC_LOG_ROWS \
-    {0x1.0000000000000p+0, 0x0.0p+0, 0x0.0p+0, 0.0}, \
-    {0x1.fd00000000000p-1, -0x1.8121214580000p-8, -0x1.ad50382973f27p-46, 0.0}, \
-    {0x1.fb00000000000p-1, -0x1.41929f9680000p-7, -0x1.977c755d01368p-46, 0.0}, \
-    {0x1.f900000000000p-1, -0x1.c317384c80000p-7, 0x1.41f33fcefb9fep-44, 0.0}, \
-    {0x1.f700000000000p-1, -0x1.228fb1fea0000p-6, -0x1.713e3284991fep-45, 0.0}, \
-    {0x1.f500000000000p-1, -0x1.63d6178690000p-6, -0x1.7abf389596542p-47, 0.0}, \
-    {0x1.f300000000000p-1, -0x1.a55f548c60000p-6, 0x1.de0709f2d03c9p-45, 0.0}, \
-    {0x1.f100000000000p-1, -0x1.e72bf28140000p-6, 0x1.8d75149774d47p-45, 0.0}, \
-    {0x1.f000000000000p-1, -0x1.0415d89e78000p-5, 0x1.dddc7f461c516p-44, 0.0}, \
-    {0x1.ee00000000000p-1, -0x1.252f32f8d0000p-5, -0x1.83e9ae021b67bp-45, 0.0}, \
-    {0x1.ec00000000000p-1, -0x1.466aed42e0000p-5, 0x1.c167375bdfd28p-45, 0.0}, \
-    {0x1.ea00000000000p-1, -0x1.67c94f2d48000p-5, -0x1.dac20827cca0cp-44, 0.0}, \
-    {0x1.e800000000000p-1, -0x1.894aa149f8000p-5, -0x1.9a19a8be97661p-44, 0.0}, \
-    {0x1.e600000000000p-1, -0x1.aaef2d0fb0000p-5, -0x1.0fc1a353bb42ep-45, 0.0}, \
-    {0x1.e500000000000p-1, -0x1.bbcebfc690000p-5, 0x1.7bf868c317c2ap-46, 0.0}, \
-    {0x1.e300000000000p-1, -0x1.dda8adc680000p-5, 0x1.1b1ac64d9e42fp-45, 0.0}, \
-    {0x1.e100000000000p-1, -0x1.ffa6911ab8000p-5, -0x1.3008c98381a8fp-45, 0.0}, \
-    {0x1.df00000000000p-1, -0x1.10e45b3cb0000p-4, 0x1.7cf69284a3465p-44, 0.0}, \
-    {0x1.dd00000000000p-1, -0x1.2207b5c784000p-4, -0x1.49d8cfc10c7bfp-44, 0.0}, \
-    {0x1.dc00000000000p-1, -0x1.2aa04a4470000p-4, -0x1.7a48ba8b1cb41p-44, 0.0}, \
-    {0x1.da00000000000p-1, -0x1.3bdf5a7d20000p-4, 0x1.19bd0ad125895p-44, 0.0}, \
-    {0x1.d800000000000p-1, -0x1.4d3115d208000p-4, 0x1.53a2582f4e1efp-48, 0.0}, \
-    {0x1.d700000000000p-1, -0x1.55e10050e0000p-4, -0x1.c1d740c53c72ep-47, 0.0}, \
-    {0x1.d500000000000p-1, -0x1.674f089364000p-4, -0x1.a79994c9d3302p-44, 0.0}, \
-    {0x1.d300000000000p-1, -0x1.78d02263d8000p-4, -0x1.69b5794b69fb7p-47, 0.0}, \
-    {0x1.d200000000000p-1, -0x1.8197e2f410000p-4, 0x1.c0fe460d20041p-44, 0.0}, \
-    {0x1.d000000000000p-1, -0x1.9335e5d594000p-4, -0x1.3115c3abd47dap-45, 0.0}, \
-    {0x1.ce00000000000p-1, -0x1.a4e7640b1c000p-4, 0x1.e42b6b94407c8p-47, 0.0}, \
-    {0x1.cd00000000000p-1, -0x1.adc77ee5b0000p-4, 0x1.573b209c31904p-44, 0.0}, \
-    {0x1.cb00000000000p-1, -0x1.bf968769fc000p-4, -0x1.4218c8d824283p-45, 0.0}, \
-    {0x1.c900000000000p-1, -0x1.d179788218000p-4, -0x1.36433b5efbeedp-44, 0.0}, \
-    {0x1.c800000000000p-1, -0x1.da72763844000p-4, -0x1.a89401fa71733p-46, 0.0}, \
-    {0x1.c600000000000p-1, -0x1.ec739830a0000p-4, -0x1.11fcba80cdd10p-44, 0.0}, \
-    {0x1.c500000000000p-1, -0x1.f57bc7d900000p-4, -0x1.76a6c9ea8b04ep-46, 0.0}, \
-    {0x1.c300000000000p-1, -0x1.03cdc0a51e000p-3, -0x1.81a9cf169fc5cp-44, 0.0}, \
-    {0x1.c200000000000p-1, -0x1.08598b59e4000p-3, 0x1.7e5dd7009902cp-45, 0.0}, \
-    {0x1.c000000000000p-1, -0x1.1178e8227e000p-3, -0x1.1ef78ce2d07f2p-45, 0.0}, \
-    {0x1.bf00000000000p-1, -0x1.160c8024b2000p-3, -0x1.ec2d2a9009e3dp-45, 0.0}, \
-    {0x1.bd00000000000p-1, -0x1.1f3b925f26000p-3, 0x1.5f74e9b083633p-46, 0.0}, \
-    {0x1.bc00000000000p-1, -0x1.23d712a49c000p-3, -0x1.00d238fd3df5cp-46, 0.0}, \
-    {0x1.ba00000000000p-1, -0x1.2d1610c868000p-3, -0x1.39d6ccb81b4a1p-47, 0.0}, \
-    {0x1.b900000000000p-1, -0x1.31b994d3a4000p-3, -0x1.f098ee3a50810p-44, 0.0}, \
-    {0x1.b700000000000p-1, -0x1.3b08b67580000p-3, 0x1.aade8f29320fbp-44, 0.0}, \
-    {0x1.b600000000000p-1, -0x1.3fb45a5992000p-3, -0x1.19713c0cae559p-44, 0.0}, \
-    {0x1.b400000000000p-1, -0x1.4913d8333c000p-3, 0x1.53e43558124c4p-44, 0.0}, \
-    {0x1.b300000000000p-1, -0x1.4dc7b897bc000p-3, -0x1.c79b60ae1ff0fp-47, 0.0}, \
-    {0x1.b100000000000p-1, -0x1.5737cc9018000p-3, -0x1.9baa7a6b887f6p-44, 0.0}, \
-    {0x1.b000000000000p-1, -0x1.5bf406b544000p-3, 0x1.27023eb68981cp-46, 0.0}, \
-    {0x1.ae00000000000p-1, -0x1.6574ebe8c2000p-3, 0x1.98c1d34f0f462p-44, 0.0}, \
-    {0x1.ad00000000000p-1, -0x1.6a399dabbe000p-3, 0x1.8f934e66a15a6p-44, 0.0}, \
-    {0x1.ac00000000000p-1, -0x1.6f0128b756000p-3, -0x1.577390d31ef0fp-44, 0.0}, \
-    {0x1.aa00000000000p-1, -0x1.7898d85444000p-3, -0x1.8e67be3dbaf3fp-44, 0.0}, \
-    {0x1.a900000000000p-1, -0x1.7d6903caf6000p-3, 0x1.4c06b17c301d7p-45, 0.0}, \
-    {0x1.a700000000000p-1, -0x1.871213750e000p-3, -0x1.328eb42f9af75p-44, 0.0}, \
-    {0x1.a600000000000p-1, -0x1.8beafeb390000p-3, 0x1.73d54aae92cd1p-47, 0.0}, \
-    {0x1.a500000000000p-1, -0x1.90c6db9fcc000p-3, 0x1.935f57718d7cap-46, 0.0}, \
-    {0x1.a300000000000p-1, -0x1.9a8778deba000p-3, -0x1.470fa3efec390p-44, 0.0}, \
-    {0x1.a200000000000p-1, -0x1.9f6c40708a000p-3, 0x1.337d94bcd3f43p-44, 0.0}, \
-    {0x1.a100000000000p-1, -0x1.a454082e6a000p-3, -0x1.60a77c81f7171p-44, 0.0}, \
-    {0x1.9f00000000000p-1, -0x1.ae2ca6f672000p-3, -0x1.7a8d5ae54f550p-44, 0.0}, \
-    {0x1.9e00000000000p-1, -0x1.b31d8575bc000p-3, -0x1.c794e562a63cbp-44, 0.0}, \
-    {0x1.9d00000000000p-1, -0x1.b811730b82000p-3, -0x1.e90683b9cd768p-46, 0.0}, \
-    {0x1.9c00000000000p-1, -0x1.bd087383be000p-3, 0x1.d4bc4595412b6p-45, 0.0}, \
-    {0x1.9a00000000000p-1, -0x1.c6ffbc6f00000p-3, -0x1.ee138d3a69d43p-44, 0.0}, \
-    {0x1.9900000000000p-1, -0x1.cc000c9db4000p-3, 0x1.d6d585d57aff9p-46, 0.0}, \
-    {0x1.9800000000000p-1, -0x1.d1037f2656000p-3, 0x1.84a7e75b6f6e4p-47, 0.0}, \
-    {0x1.9600000000000p-1, -0x1.db13db0d48000p-3, -0x1.2806a847527e6p-44, 0.0}, \
-    {0x1.9500000000000p-1, -0x1.e020cc6236000p-3, 0x1.52b00adb91424p-45, 0.0}, \
-    {0x1.9400000000000p-1, -0x1.e530effe72000p-3, 0x1.fdbdbb13f7c18p-44, 0.0}, \
-    {0x1.9300000000000p-1, -0x1.ea4449f04a000p-3, -0x1.5e91663732a36p-44, 0.0}, \
-    {0x1.9100000000000p-1, -0x1.f474b134e0000p-3, 0x1.bae49f1df7b5ep-44, 0.0}, \
-    {0x1.9000000000000p-1, -0x1.f991c6cb3c000p-3, 0x1.90d04cd7cc834p-44, 0.0}, \
-    {0x1.8f00000000000p-1, -0x1.feb2233ea0000p-3, -0x1.f3418de00938bp-45, 0.0}, \
-    {0x1.8e00000000000p-1, -0x1.01eae5626c000p-2, -0x1.a43dcfade85aep-44, 0.0}, \
-    {0x1.8d00000000000p-1, -0x1.047e60cde8000p-2, -0x1.dbdf10d397f3cp-45, 0.0}, \
-    {0x1.8b00000000000p-1, -0x1.09aa572e6c000p-2, -0x1.b50a1e1734342p-44, 0.0}, \
-    {0x1.8a00000000000p-1, -0x1.0c42d67616000p-2, -0x1.7188b163ceae9p-45, 0.0}, \
-    {0x1.8900000000000p-1, -0x1.0edd060b78000p-2, -0x1.019b52d8435f5p-47, 0.0}, \
-    {0x1.8800000000000p-1, -0x1.1178e8227e000p-2, -0x1.1ef78ce2d07f2p-44, 0.0}, \
-    {0x1.8700000000000p-1, -0x1.14167ef367000p-2, -0x1.e0c07824daaf5p-44, 0.0}, \
-    {0x1.8600000000000p-1, -0x1.16b5ccbad0000p-2, 0x1.23299042d74bfp-44, 0.0}, \
-    {0x1.8400000000000p-1, -0x1.1bf99635a7000p-2, 0x1.1ac89575c2125p-44, 0.0}, \
-    {0x1.8300000000000p-1, -0x1.1e9e16788a000p-2, 0x1.82eaed3c8b65ep-44, 0.0}, \
-    {0x1.8200000000000p-1, -0x1.214456d0ec000p-2, 0x1.caf0428b728a3p-44, 0.0}, \
-    {0x1.8100000000000p-1, -0x1.23ec5991ec000p-2, 0x1.6dbe448a2e522p-44, 0.0}, \
-    {0x1.8000000000000p-1, -0x1.269621134e000p-2, 0x1.1b61f10522625p-44, 0.0}, \
-    {0x1.7f00000000000p-1, -0x1.2941afb187000p-2, 0x1.210c2b730e28bp-44, 0.0}, \
-    {0x1.7e00000000000p-1, -0x1.2bef07cdc9000p-2, -0x1.a9cfa4a5004f4p-45, 0.0}, \
-    {0x1.7c00000000000p-1, -0x1.314f1e1d36000p-2, 0x1.8e27ad3213cb8p-45, 0.0}, \
-    {0x1.7b00000000000p-1, -0x1.3401e12aed000p-2, 0x1.17c73556e291dp-44, 0.0}, \
-    {0x1.7a00000000000p-1, -0x1.36b6776be1000p-2, -0x1.16ecdb0f177c8p-46, 0.0}, \
-    {0x1.7900000000000p-1, -0x1.396ce359bc000p-2, 0x1.5839c5663663dp-47, 0.0}, \
-    {0x1.7800000000000p-1, -0x1.3c25277333000p-2, -0x1.83b54b606bd5cp-46, 0.0}, \
-    {0x1.7700000000000p-1, -0x1.3edf463c17000p-2, 0x1.f067c297f2c3fp-44, 0.0}, \
-    {0x1.7600000000000p-1, -0x1.419b423d5f000p-2, 0x1.ce379226de3ecp-44, 0.0}, \
-    {0x1.7500000000000p-1, -0x1.44591e053a000p-2, 0x1.6e95892923d88p-47, 0.0}, \
-    {0x1.7400000000000p-1, -0x1.4718dc271c000p-2, -0x1.06c18fb4c14c5p-44, 0.0}, \
-    {0x1.7300000000000p-1, -0x1.49da7f3bcc000p-2, -0x1.07b334daf4b9ap-44, 0.0}, \
-    {0x1.7200000000000p-1, -0x1.4c9e09e173000p-2, 0x1.e20891b0ad8a4p-45, 0.0}, \
-    {0x1.7100000000000p-1, -0x1.4f637ebbaa000p-2, 0x1.fc158cb3124b9p-44, 0.0}, \
-    {0x1.7000000000000p-1, -0x1.522ae0738a000p-2, -0x1.ebe708164c759p-45, 0.0}, \
-    {0x1.6f00000000000p-1, -0x1.54f431b7be000p-2, -0x1.a8954c0910952p-46, 0.0}, \
-    {0x1.6e00000000000p-1, -0x1.57bf753c8d000p-2, -0x1.fadedee5d40efp-46, 0.0}, \
-    {0x1.6d00000000000p-1, -0x1.5a8cadbbee000p-2, 0x1.7c79b0af7ecf8p-48, 0.0}, \
-    {0x1.6c00000000000p-1, -0x1.5d5bddf596000p-2, 0x1.a0b2a08a465dcp-47, 0.0}, \
-    {0x1.6b00000000000p-1, -0x1.602d08af09000p-2, -0x1.ebe9176df3f65p-46, 0.0}, \
-    {0x1.6a00000000000p-1, -0x1.630030b3ab000p-2, 0x1.db623e731ae00p-45, 0.0}, \
-    {0x1.6900000000000p-1, -0x1.65d558d4ce000p-2, -0x1.544fd2dc5bdc0p-51, 0.0}, \
-    {0x1.6800000000000p-1, -0x1.68ac83e9c7000p-2, 0x1.7af966c548a30p-44, 0.0}, \
-    {0x1.6700000000000p-1, -0x1.6b85b4cffa000p-2, -0x1.fe6750d372503p-45, 0.0}, \
-    {0x1.6600000000000p-1, -0x1.6e60ee6af2000p-2, 0x1.a37a6a0f7749ep-44, 0.0}, \
-    {0x1.6500000000000p-1, -0x1.713e33a46a000p-2, -0x1.7b9b2617e9472p-46, 0.0}, \
-    {0x1.6400000000000p-1, -0x1.741d876c68000p-2, 0x1.13a7b5b11cfa7p-44, 0.0}, \
-    {0x1.6300000000000p-1, -0x1.76feecb947000p-2, -0x1.74bb9c9852c57p-46, 0.0}, \
-    {0x1.6200000000000p-1, -0x1.79e26687d0000p-2, 0x1.309c168817444p-44, 0.0}, \
-    {0x1.6100000000000p-1, -0x1.7cc7f7db47000p-2, 0x1.7c98438023cdcp-44, 0.0}, \
-    {0x1.6000000000000p-1, -0x1.7fafa3bd81000p-2, -0x1.46fb79bf6d4cbp-44, 0.0}, \
-    {0x1.5f00000000000p-1, -0x1.82996d3ef9000p-2, 0x1.0d52aa30536bbp-44, 0.0}, \
-    {0x1.5e00000000000p-1, -0x1.85855776dd000p-2, 0x1.015486666443bp-44, 0.0}, \
-    {0x1.5d00000000000p-1, -0x1.8873658328000p-2, 0x1.988e21f7fc497p-45, 0.0}, \
-    {0x1.5c00000000000p-1, -0x1.8b639a88b3000p-2, 0x1.05ae1e5e70470p-45, 0.0}, \
-    {0x1.5b00000000000p-1, -0x1.8e55f9b34a000p-2, 0x1.1f21d89c89c45p-44, 0.0}, \
-    {0x1.5a00000000000p-1, -0x1.914a8635bf000p-2, -0x1.a2652b44673e1p-44, 0.0}, \
-    {0x1.5900000000000p-1, -0x1.9441434a03000p-2, -0x1.2cb81c95fff43p-45, 0.0}, \
-    {0x1.5800000000000p-1, -0x1.973a343135000p-2, -0x1.ab73b16bf4984p-44, 0.0}, \
-    {0x1.5800000000000p-1, -0x1.973a343135000p-2, -0x1.ab73b16bf4984p-44, 0.0}, \
-    {0x1.5700000000000p-1, -0x1.9a355c33bd000p-2, -0x1.ae73535438bebp-44, 0.0}, \
-    {0x1.5600000000000p-1, -0x1.9d32bea15f000p-2, 0x1.6279e10d0c0b0p-45, 0.0}, \
-    {0x1.5500000000000p+0, 0x1.2596010df7000p-2, 0x1.8e7bc224ea3e3p-44, 0.0}, \
-    {0x1.5400000000000p+0, 0x1.22941fbcf8000p-2, -0x1.a6976f5eb0963p-44, 0.0}, \
-    {0x1.5300000000000p+0, 0x1.1f8ff9e48a000p-2, 0x1.7946c040cbe77p-45, 0.0}, \
-    {0x1.5280000000000p+0, 0x1.1e0d0c3371000p-2, 0x1.af8f2a9b0d4a0p-44, 0.0}, \
-    {0x1.5180000000000p+0, 0x1.1b05791f08000p-2, -0x1.2dd466dc55e2dp-44, 0.0}, \
-    {0x1.5080000000000p+0, 0x1.17fb98e151000p-2, -0x1.a8a8ba74a2684p-44, 0.0}, \
-    {0x1.4f80000000000p+0, 0x1.14ef67f887000p-2, -0x1.e97a65dfc9794p-44, 0.0}, \
-    {0x1.4f00000000000p+0, 0x1.136870293b000p-2, -0x1.d3e8499d67123p-44, 0.0}, \
-    {0x1.4e00000000000p+0, 0x1.1058bf9ae5000p-2, -0x1.4ab9d817d52cdp-44, 0.0}, \
-    {0x1.4d00000000000p+0, 0x1.0d46b579ab000p-2, 0x1.d2c81f640e1e6p-44, 0.0}, \
-    {0x1.4c00000000000p+0, 0x1.0a324e2739000p-2, 0x1.c6bee7ef4030ep-47, 0.0}, \
-    {0x1.4b80000000000p+0, 0x1.08a73667c5000p-2, 0x1.ebc1d40c5a329p-44, 0.0}, \
-    {0x1.4a80000000000p+0, 0x1.058f3c703f000p-2, -0x1.0e866bcd236adp-44, 0.0}, \
-    {0x1.4980000000000p+0, 0x1.0274dc16c2000p-2, 0x1.979e89cf835c2p-45, 0.0}, \
-    {0x1.4900000000000p+0, 0x1.00e6c45ad5000p-2, 0x1.cc68d52e01203p-50, 0.0}, \
-    {0x1.4800000000000p+0, 0x1.fb9186d5e4000p-3, -0x1.d572aab993c87p-47, 0.0}, \
-    {0x1.4780000000000p+0, 0x1.f871b28956000p-3, -0x1.f75fd6a526efep-44, 0.0}, \
-    {0x1.4680000000000p+0, 0x1.f22e5e72f2000p-3, -0x1.f454f1417e41fp-44, 0.0}, \
-    {0x1.4580000000000p+0, 0x1.ebe61f4dd8000p-3, -0x1.3d45330fdca4dp-45, 0.0}, \
-    {0x1.4500000000000p+0, 0x1.e8c0252aa6000p-3, -0x1.6805b80e8e6ffp-45, 0.0}, \
-    {0x1.4400000000000p+0, 0x1.e27076e2b0000p-3, -0x1.a342c2af0003cp-44, 0.0}, \
-    {0x1.4300000000000p+0, 0x1.dc1bca0abe000p-3, 0x1.8fac1a628ccc6p-44, 0.0}, \
-    {0x1.4280000000000p+0, 0x1.d8ef91af32000p-3, -0x1.5105fc364c784p-46, 0.0}, \
-    {0x1.4180000000000p+0, 0x1.d293581b6c000p-3, -0x1.83270128aaa5fp-44, 0.0}, \
-    {0x1.4100000000000p+0, 0x1.cf6354e09c000p-3, 0x1.771239a07d55bp-45, 0.0}, \
-    {0x1.4000000000000p+0, 0x1.c8ff7c79aa000p-3, -0x1.7794f689f8434p-45, 0.0}, \
-    {0x1.3f80000000000p+0, 0x1.c5cba543ae000p-3, 0x1.0929decb454fcp-45, 0.0}, \
-    {0x1.3e80000000000p+0, 0x1.bf601bb0e4000p-3, 0x1.386a947c378b5p-45, 0.0}, \
-    {0x1.3e00000000000p+0, 0x1.bc286742d8000p-3, 0x1.9ac53f39d121cp-44, 0.0}, \
-    {0x1.3d00000000000p+0, 0x1.b5b519e8fc000p-3, -0x1.4b722ec011f31p-44, 0.0}, \
-    {0x1.3c00000000000p+0, 0x1.af3c94e80c000p-3, -0x1.a4e633fcd9066p-52, 0.0}, \
-    {0x1.3b80000000000p+0, 0x1.abfe5ae462000p-3, -0x1.b68f5395f139dp-44, 0.0}, \
-    {0x1.3a80000000000p+0, 0x1.a57df28244000p-3, 0x1.b99c8ca1d9abbp-44, 0.0}, \
-    {0x1.3a00000000000p+0, 0x1.a23bc1fe2c000p-3, -0x1.539cd91dc9f0bp-44, 0.0}, \
-    {0x1.3900000000000p+0, 0x1.9bb362e7e0000p-3, -0x1.1f2a8a1ce0ffcp-45, 0.0}, \
-    {0x1.3880000000000p+0, 0x1.986d322818000p-3, 0x1.93b564dd44000p-48, 0.0}, \
-    {0x1.3780000000000p+0, 0x1.91dcc8c340000p-3, 0x1.7bc6abddeff46p-44, 0.0}, \
-    {0x1.3700000000000p+0, 0x1.8e928de886000p-3, 0x1.a8154b13d72d5p-44, 0.0}, \
-    {0x1.3600000000000p+0, 0x1.87fa06520c000p-3, 0x1.22120401202fcp-44, 0.0}, \
-    {0x1.3580000000000p+0, 0x1.84abb75866000p-3, -0x1.d8daadf4e2bd2p-44, 0.0}, \
-    {0x1.3500000000000p+0, 0x1.815c0a1436000p-3, -0x1.02a52f9201ce8p-44, 0.0}, \
-    {0x1.3400000000000p+0, 0x1.7ab890210e000p-3, -0x1.bdb9072534a58p-45, 0.0}, \
-    {0x1.3380000000000p+0, 0x1.7764c128f2000p-3, 0x1.274903479e3d1p-47, 0.0}, \
-    {0x1.3280000000000p+0, 0x1.70b8f97a1a000p-3, 0x1.4ea64f6a95befp-44, 0.0}, \
-    {0x1.3200000000000p+0, 0x1.6d60fe719e000p-3, -0x1.bc6e557134767p-44, 0.0}, \
-    {0x1.3100000000000p+0, 0x1.66acd4272a000p-3, 0x1.aa1bdbfc6c785p-44, 0.0}, \
-    {0x1.3080000000000p+0, 0x1.6350a28aaa000p-3, 0x1.d5ec0ab8163afp-45, 0.0}, \
-    {0x1.3000000000000p+0, 0x1.5ff3070a7a000p-3, -0x1.8586f183bebf2p-44, 0.0}, \
-    {0x1.2f00000000000p+0, 0x1.59338d9982000p-3, 0x1.0ba68b7555d4ap-48, 0.0}, \
-    {0x1.2e80000000000p+0, 0x1.55d1ad4232000p-3, 0x1.add94dda647e8p-44, 0.0}, \
-    {0x1.2d80000000000p+0, 0x1.4f099f4a24000p-3, -0x1.e9bf2fafeaf27p-44, 0.0}, \
-    {0x1.2d00000000000p+0, 0x1.4ba36f39a6000p-3, -0x1.4354bb3f219e5p-44, 0.0}, \
-    {0x1.2c80000000000p+0, 0x1.483bccce6e000p-3, 0x1.eea52723f6369p-46, 0.0}, \
-    {0x1.2b80000000000p+0, 0x1.41682bf728000p-3, -0x1.10047081f849dp-45, 0.0}, \
-    {0x1.2b00000000000p+0, 0x1.3dfc2b0ecc000p-3, 0x1.8a72a62b8c13fp-45, 0.0}, \
-    {0x1.2a00000000000p+0, 0x1.371fc201e8000p-3, 0x1.ee8779b2d8abcp-44, 0.0}, \
-    {0x1.2980000000000p+0, 0x1.33af575770000p-3, 0x1.c9ecca2fe72a5p-44, 0.0}, \
-    {0x1.2900000000000p+0, 0x1.303d718e48000p-3, -0x1.680b5ce3ecb05p-50, 0.0}, \
-    {0x1.2800000000000p+0, 0x1.29552f8200000p-3, -0x1.5b967f4471dfcp-44, 0.0}, \
-    {0x1.2780000000000p+0, 0x1.25ded0abc6000p-3, 0x1.5a3854f176449p-44, 0.0}, \
-    {0x1.2700000000000p+0, 0x1.2266f190a6000p-3, -0x1.4d20ab840e7f6p-45, 0.0}, \
-    {0x1.2600000000000p+0, 0x1.1b72ad52f6000p-3, 0x1.e80a41811a396p-45, 0.0}, \
-    {0x1.2580000000000p+0, 0x1.17f6458fca000p-3, 0x1.843fad093c8dcp-45, 0.0}, \
-    {0x1.2500000000000p+0, 0x1.1478584674000p-3, 0x1.563451027c750p-46, 0.0}, \
-    {0x1.2400000000000p+0, 0x1.0d77e7cd08000p-3, 0x1.cb2cd2ee2f482p-44, 0.0}, \
-    {0x1.2380000000000p+0, 0x1.09f561ee72000p-3, -0x1.8f3057157d1a8p-45, 0.0}, \
-    {0x1.2300000000000p+0, 0x1.0671512ca6000p-3, -0x1.a47579cdc0a3dp-45, 0.0}, \
-    {0x1.2280000000000p+0, 0x1.02ebb42bf4000p-3, -0x1.5a8fa5ce00e5dp-46, 0.0}, \
-    {0x1.2180000000000p+0, 0x1.f7b79fec38000p-4, -0x1.10987e897ed01p-47, 0.0}, \
-    {0x1.2100000000000p+0, 0x1.f0a30c0118000p-4, -0x1.d599e83368e91p-44, 0.0}, \
-    {0x1.2080000000000p+0, 0x1.e98b549670000p-4, 0x1.4677489c50e97p-44, 0.0}, \
-    {0x1.2000000000000p+0, 0x1.e27076e2b0000p-4, -0x1.a342c2af0003cp-45, 0.0}, \
-    {0x1.1f00000000000p+0, 0x1.d4313d66cc000p-4, -0x1.9454379135713p-45, 0.0}, \
-    {0x1.1e80000000000p+0, 0x1.cd0cdbf8c0000p-4, 0x1.3e14db50dd743p-44, 0.0}, \
-    {0x1.1e00000000000p+0, 0x1.c5e548f5bc000p-4, 0x1.d0c57585fbe06p-46, 0.0}, \
-    {0x1.1d00000000000p+0, 0x1.b78c82bb10000p-4, -0x1.25ef7bc3987e7p-44, 0.0}, \
-    {0x1.1c80000000000p+0, 0x1.b05b49bee4000p-4, 0x1.ff22c18f84a5ep-47, 0.0}, \
-    {0x1.1c00000000000p+0, 0x1.a926d3a4ac000p-4, 0x1.563650bd22a9cp-44, 0.0}, \
-    {0x1.1b80000000000p+0, 0x1.a1ef1d8060000p-4, 0x1.cd4176df97bcbp-44, 0.0}, \
-    {0x1.1b00000000000p+0, 0x1.9ab4246204000p-4, -0x1.8a64826787061p-45, 0.0}, \
-    {0x1.1a00000000000p+0, 0x1.8c345d6318000p-4, 0x1.b20f5acb42a66p-44, 0.0}, \
-    {0x1.1980000000000p+0, 0x1.84ef898e84000p-4, -0x1.7d5cd246977c9p-44, 0.0}, \
-    {0x1.1900000000000p+0, 0x1.7da766d7b0000p-4, 0x1.2cc844480c89bp-44, 0.0}, \
-    {0x1.1880000000000p+0, 0x1.765bf23a6c000p-4, -0x1.ecbc035c4256ap-48, 0.0}, \
-    {0x1.1800000000000p+0, 0x1.6f0d28ae58000p-4, -0x1.4b4641b664613p-44, 0.0}, \
-    {0x1.1700000000000p+0, 0x1.60658a9374000p-4, 0x1.0c3b1dee9c4f8p-44, 0.0}, \
-    {0x1.1680000000000p+0, 0x1.590cafdf00000p-4, 0x1.c284f5722abaap-44, 0.0}, \
-    {0x1.1600000000000p+0, 0x1.51b073f060000p-4, 0x1.83f69278e686ap-44, 0.0}, \
-    {0x1.1580000000000p+0, 0x1.4a50d3aa1c000p-4, -0x1.f7fe1308973e2p-45, 0.0}, \
-    {0x1.1500000000000p+0, 0x1.42edcbea64000p-4, 0x1.bc0eeea7c9acdp-46, 0.0}, \
-    {0x1.1400000000000p+0, 0x1.341d7961bc000p-4, 0x1.1d09299837610p-44, 0.0}, \
-    {0x1.1380000000000p+0, 0x1.2cb0283f5c000p-4, 0x1.e1ee2ca657021p-44, 0.0}, \
-    {0x1.1300000000000p+0, 0x1.253f62f0a0000p-4, 0x1.416f8fb69a701p-44, 0.0}, \
-    {0x1.1280000000000p+0, 0x1.1dcb263db0000p-4, 0x1.9444f5e9e8981p-44, 0.0}, \
-    {0x1.1200000000000p+0, 0x1.16536eea38000p-4, -0x1.47c5e768fa309p-46, 0.0}, \
-    {0x1.1180000000000p+0, 0x1.0ed839b554000p-4, -0x1.901f46d48abb4p-44, 0.0}, \
-    {0x1.1100000000000p+0, 0x1.0759835990000p-4, -0x1.b8ecfe4b59987p-44, 0.0}, \
-    {0x1.1000000000000p+0, 0x1.f0a30c0118000p-5, -0x1.d599e83368e91p-45, 0.0}, \
-    {0x1.0f80000000000p+0, 0x1.e19070c278000p-5, -0x1.fea4664629e86p-45, 0.0}, \
-    {0x1.0f00000000000p+0, 0x1.d276b8adb0000p-5, 0x1.6a423c78a64b0p-46, 0.0}, \
-    {0x1.0e80000000000p+0, 0x1.c355dd0920000p-5, 0x1.f2ccc9abf8388p-45, 0.0}, \
-    {0x1.0e00000000000p+0, 0x1.b42dd71198000p-5, -0x1.c827ae5d6704cp-46, 0.0}, \
-    {0x1.0d80000000000p+0, 0x1.a4fe9ffa40000p-5, -0x1.6e584a0402925p-44, 0.0}, \
-    {0x1.0d00000000000p+0, 0x1.95c830ec90000p-5, -0x1.c148297c5feb8p-45, 0.0}, \
-    {0x1.0c80000000000p+0, 0x1.868a830840000p-5, -0x1.2623a134ac693p-46, 0.0}, \
-    {0x1.0c00000000000p+0, 0x1.77458f6330000p-5, -0x1.181dce586af09p-44, 0.0}, \
-    {0x1.0b00000000000p+0, 0x1.58a5bafc90000p-5, -0x1.b2b739570ad39p-45, 0.0}, \
-    {0x1.0a80000000000p+0, 0x1.494acc34d8000p-5, 0x1.11c78a56fd247p-45, 0.0}, \
-    {0x1.0a00000000000p+0, 0x1.39e87b9fe8000p-5, 0x1.eafd480ad9015p-44, 0.0}, \
-    {0x1.0980000000000p+0, 0x1.2a7ec22150000p-5, -0x1.78ce77a9163fep-45, 0.0}, \
-    {0x1.0900000000000p+0, 0x1.1b0d989240000p-5, -0x1.3401e9ae889bbp-44, 0.0}, \
-    {0x1.0880000000000p+0, 0x1.0b94f7c198000p-5, -0x1.e89896f022783p-45, 0.0}, \
-    {0x1.0800000000000p+0, 0x1.f829b0e780000p-6, 0x1.980267c7e09e4p-45, 0.0}, \
-    {0x1.0780000000000p+0, 0x1.d91a66c540000p-6, 0x1.e61f1658cfb9ap-45, 0.0}, \
-    {0x1.0700000000000p+0, 0x1.b9fc027b00000p-6, -0x1.b9a010ae6922ap-44, 0.0}, \
-    {0x1.0680000000000p+0, 0x1.9ace7551d0000p-6, -0x1.d75d97ec7c410p-45, 0.0}, \
-    {0x1.0600000000000p+0, 0x1.7b91b07d60000p-6, -0x1.3b955b602ace4p-44, 0.0}, \
-    {0x1.0580000000000p+0, 0x1.5c45a51b90000p-6, -0x1.63bb6216d87d8p-45, 0.0}, \
-    {0x1.0500000000000p+0, 0x1.3cea443470000p-6, -0x1.6a2c432d6a40bp-44, 0.0}, \
-    {0x1.0480000000000p+0, 0x1.1d7f7eb9f0000p-6, -0x1.4193a83fcc7a6p-46, 0.0}, \
-    {0x1.0400000000000p+0, 0x1.fc0a8b0fc0000p-7, 0x1.f1e7cf6d3a69cp-50, 0.0}, \
-    {0x1.0380000000000p+0, 0x1.bcf712c740000p-7, 0x1.c25e097bd9771p-46, 0.0}, \
-    {0x1.0300000000000p+0, 0x1.7dc475f820000p-7, -0x1.eb1245b5da1f5p-44, 0.0}, \
-    {0x1.0280000000000p+0, 0x1.3e7295d260000p-7, -0x1.609c1ff29a114p-45, 0.0}, \
-    {0x1.0200000000000p+0, 0x1.fe02a6b100000p-8, 0x1.9e23f0dda40e4p-46, 0.0}, \
-    {0x1.0180000000000p+0, 0x1.7ee11ebd80000p-8, 0x1.749d3c2d23a07p-47, 0.0}, \
-    {0x1.0100000000000p+0, 0x1.ff00aa2b00000p-9, 0x1.0bc04a086b56ap-45, 0.0}, \
-    {0x1.0000000000000p+0, 0x0.0p+0, 0x0.0p+0, 0.0}
-#define IMC_EXP_ROWS \
+    {0ll, 512ll}, \
+    {-27101073204424016ll, 509ll}, \
+    {-45257340823377788ll, 507ll}, \
+    {-63485372532455475ll, 505ll}, \
+    {-81785737890161276ll, 503ll}, \
+    {-100159013262507360ll, 501ll}, \
+    {-118605781931934706ll, 499ll}, \
+    {-137126634208421142ll, 497ll}, \
+    {-146415028120619150ll, 496ll}, \
+    {-165048128291145683ll, 494ll}, \
+    {-183756819338657074ll, 492ll}, \
+    {-202541717077322504ll, 490ll}, \
+    {-221403444877355111ll, 488ll}, \
+    {-240342633789136771ll, 486ll}, \
+    {-249841475496346632ll, 485ll}, \
+    {-268898056407992778ll, 483ll}, \
+    {-288033710495916050ll, 481ll}, \
+    {-307249096706100262ll, 479ll}, \
+    {-326544882255865699ll, 477ll}, \
+    {-336223135584348451ll, 476ll}, \
+    {-355640789612337420ll, 474ll}, \
+    {-375140548129827607ll, 472ll}, \
+    {-384921434125820140ll, 471ll}, \
+    {-404545659561483878ll, 469ll}, \
+    {-424253749463135451ll, 467ll}, \
+    {-434139468186319879ll, 466ll}, \
+    {-453974707445850668ll, 464ll}, \
+    {-473895628350361066ll, 462ll}, \
+    {-483888451368428307ll, 461ll}, \
+    {-503939291730314290ll, 459ll}, \
+    {-524077690624727309ll, 457ll}, \
+    {-534179964146264212ll, 456ll}, \
+    {-554451144118913011ll, 454ll}, \
+    {-564620246405707431ll, 453ll}, \
+    {-585025970045847207ll, 451ll}, \
+    {-595262791160234820ll, 450ll}, \
+    {-615804856387649007ll, 448ll}, \
+    {-626110304292690010ll, 447ll}, \
+    {-646790545308295307ll, 445ll}, \
+    {-657165546351034578ll, 444ll}, \
+    {-677985834619673835ll, 442ll}, \
+    {-688431334030819940ll, 441ll}, \
+    {-709393579297559686ll, 439ll}, \
+    {-719910541708256709ll, 438ll}, \
+    {-741016693049569391ll, 436ll}, \
+    {-751606103025968078ll, 435ll}, \
+    {-772858149937245866ll, 433ll}, \
+    {-783521012533614846ll, 432ll}, \
+    {-804920986054532345ll, 430ll}, \
+    {-815658327385686451ll, 429ll}, \
+    {-826420726712327630ll, 428ll}, \
+    {-848021169098865055ll, 426ll}, \
+    {-858859449101412339ll, 425ll}, \
+    {-880612725371488827ll, 423ll}, \
+    {-891527963646838293ll, 422ll}, \
+    {-902469098122669217ll, 421ll}, \
+    {-924429549231742015ll, 419ll}, \
+    {-935449114853454346ll, 418ll}, \
+    {-946495074669527710ll, 417ll}, \
+    {-968666684771920437ll, 415ll}, \
+    {-979792591298436692ll, 414ll}, \
+    {-990945404517476615ll, 413ll}, \
+    {-1002125254885922439ll, 412ll}, \
+    {-1024566593663252558ll, 410ll}, \
+    {-1035828347778509098ll, 409ll}, \
+    {-1047117670474792364ll, 408ll}, \
+    {-1069779563833499675ll, 406ll}, \
+    {-1081152408113732256ll, 405ll}, \
+    {-1092553368230430985ll, 404ll}, \
+    {-1103982583543593542ll, 403ll}, \
+    {-1126926342403200110ll, 401ll}, \
+    {-1138441169904712895ll, 400ll}, \
+    {-1149984820533913219ll, 399ll}, \
+    {-1161557438949134583ll, 398ll}, \
+    {-1173159170900473790ll, 397ll}, \
+    {-1196450563936932904ll, 395ll}, \
+    {-1208140522080887569ll, 394ll}, \
+    {-1219860187901362382ll, 393ll}, \
+    {-1231609712775298014ll, 392ll}, \
+    {-1243389249239614210ll, 391ll}, \
+    {-1255198951003091802ll, 390ll}, \
+    {-1278909471194322142ll, 388ll}, \
+    {-1290810603008029780ll, 387ll}, \
+    {-1302742526917661759ll, 386ll}, \
+    {-1314705402674956551ll, 385ll}, \
+    {-1326699391278092920ll, 384ll}, \
+    {-1338724654984690639ll, 383ll}, \
+    {-1350781357324981151ll, 382ll}, \
+    {-1374989738470859697ll, 380ll}, \
+    {-1387141750820937955ll, 379ll}, \
+    {-1399325868921263853ll, 378ll}, \
+    {-1411542262868825059ll, 377ll}, \
+    {-1423791104115966901ll, 376ll}, \
+    {-1436072565484830305ll, 375ll}, \
+    {-1448386821181982498ll, 374ll}, \
+    {-1460734046813243573ll, 373ll}, \
+    {-1473114419398712070ll, 372ll}, \
+    {-1485528117387992781ll, 371ll}, \
+    {-1497975320675630063ll, 370ll}, \
+    {-1510456210616749994ll, 369ll}, \
+    {-1522970970042914766ll, 368ll}, \
+    {-1535519783278192789ll, 367ll}, \
+    {-1548102836155448031ll, 366ll}, \
+    {-1560720316032852194ll, 365ll}, \
+    {-1573372411810623399ll, 364ll}, \
+    {-1586059313947995113ll, 363ll}, \
+    {-1598781214480419132ll, 362ll}, \
+    {-1611538307037006498ll, 361ll}, \
+    {-1624330786858210330ll, 360ll}, \
+    {-1637158850813754575ll, 359ll}, \
+    {-1650022697420812822ll, 358ll}, \
+    {-1662922526862441371ll, 357ll}, \
+    {-1675858541006270817ll, 356ll}, \
+    {-1688830943423460540ll, 355ll}, \
+    {-1701839939407920528ll, 354ll}, \
+    {-1714885735995805087ll, 353ll}, \
+    {-1727968541985283054ll, 352ll}, \
+    {-1741088567956589237ll, 351ll}, \
+    {-1754246026292361902ll, 350ll}, \
+    {-1767441131198271204ll, 349ll}, \
+    {-1780674098723943588ll, 348ll}, \
+    {-1793945146784187257ll, 347ll}, \
+    {-1807254495180523925ll, 346ll}, \
+    {-1820602365623032176ll, 345ll}, \
+    {-1833988981752507855ll, 344ll}, \
+    {-1833988981752507855ll, 344ll}, \
+    {-1847414569162947021ll, 343ll}, \
+    {-1860879355424357132ll, 342ll}, \
+    {1322193591194761711ll, 682ll}, \
+    {1308649716501276066ll, 680ll}, \
+    {1295065948157571726ll, 678ll}, \
+    {1288259030289399357ll, 677ll}, \
+    {1274614978862336174ll, 675ll}, \
+    {1260930440576458077ll, 673ll}, \
+    {1247205174438025750ll, 671ll}, \
+    {1240327192524140639ll, 670ll}, \
+    {1226540378015585561ll, 668ll}, \
+    {1212712223671536416ll, 666ll}, \
+    {1198842480830767967ll, 664ll}, \
+    {1191891935402897159ll, 663ll}, \
+    {1177959338647209446ll, 661ll}, \
+    {1163984521836834621ll, 659ll}, \
+    {1156981200797048007ll, 658ll}, \
+    {1142942571939435847ll, 656ll}, \
+    {1135907199074706049ll, 655ll}, \
+    {1121804172736868012ll, 653ll}, \
+    {1107657885514302838ll, 651ll}, \
+    {1100568435972976629ll, 650ll}, \
+    {1086356757488956149ll, 648ll}, \
+    {1072101147935129264ll, 646ll}, \
+    {1064956783968038650ll, 645ll}, \
+    {1050634766188671844ll, 643ll}, \
+    {1043457043310243364ll, 642ll}, \
+    {1029067995697975510ll, 640ll}, \
+    {1021856600923705940ll, 639ll}, \
+    {1007399893102391509ll, 637ll}, \
+    {1000154509022227221ll, 636ll}, \
+    {985629501681226295ll, 634ll}, \
+    {971058601665755500ll, 632ll}, \
+    {963755851100267971ll, 631ll}, \
+    {949115565730358898ll, 629ll}, \
+    {941777957152272781ll, 628ll}, \
+    {927067622451560875ll, 626ll}, \
+    {919694821491238125ll, 625ll}, \
+    {904913763906744091ll, 623ll}, \
+    {897505431360282709ll, 622ll}, \
+    {882652967577356360ll, 620ll}, \
+    {875208759312948373ll, 619ll}, \
+    {867752515136648555ll, 618ll}, \
+    {852803762927731854ll, 616ll}, \
+    {845311176359318437ll, 615ll}, \
+    {830289384515648153ll, 613ll}, \
+    {822760099547778631ll, 612ll}, \
+    {807664550820620399ll, 610ll}, \
+    {800098206189071320ll, 609ll}, \
+    {792519427131828708ll, 608ll}, \
+    {777324401792140010ll, 606ll}, \
+    {769708073028073317ll, 605ll}, \
+    {754437575570643203ll, 603ll}, \
+    {746783323160507053ll, 602ll}, \
+    {739116345470348965ll, 601ll}, \
+    {723744044508635127ll, 599ll}, \
+    {716038635834774757ll, 598ll}, \
+    {700589086985402910ll, 596ll}, \
+    {692844860113627059ll, 595ll}, \
+    {685087606781766015ll, 594ll}, \
+    {669533844927058342ll, 592ll}, \
+    {661737247941683425ll, 591ll}, \
+    {653927447568147903ll, 590ll}, \
+    {638268057247272981ll, 588ll}, \
+    {630418377022834815ll, 587ll}, \
+    {622555312852915764ll, 586ll}, \
+    {606788849569836211ll, 584ll}, \
+    {598885358315037087ll, 583ll}, \
+    {590968298828248853ll, 582ll}, \
+    {583037624443118960ll, 581ll}, \
+    {567135243104909236ll, 579ll}, \
+    {559163441606601112ll, 578ll}, \
+    {551177836116122077ll, 577ll}, \
+    {543178378744478074ll, 576ll}, \
+    {527137715551786840ll, 574ll}, \
+    {519096412697589843ll, 573ll}, \
+    {511041063892406469ll, 572ll}, \
+    {494888031551711298ll, 570ll}, \
+    {486790248929492881ll, 569ll}, \
+    {478678222179227865ll, 568ll}, \
+    {470551901101307142ll, 567ll}, \
+    {462411235230280503ll, 566ll}, \
+    {446086665906604093ll, 564ll}, \
+    {437902660176841357ll, 563ll}, \
+    {429704105095901985ll, 562ll}, \
+    {421490948840588497ll, 561ll}, \
+    {413263139310326503ll, 560ll}, \
+    {396763350623858924ll, 558ll}, \
+    {388491265861683732ll, 557ll}, \
+    {380204316608565210ll, 556ll}, \
+    {371902449346940932ll, 555ll}, \
+    {363585610269703183ll, 554ll}, \
+    {346906799979656229ll, 552ll}, \
+    {338544719685978041ll, 551ll}, \
+    {330167449410667966ll, 550ll}, \
+    {321774933867122964ll, 549ll}, \
+    {313367117466351674ll, 548ll}, \
+    {304943944314765187ll, 547ll}, \
+    {296505358211947596ll, 546ll}, \
+    {279581720803300556ll, 544ll}, \
+    {271096555542151863ll, 543ll}, \
+    {262595749414529602ll, 542ll}, \
+    {254079244651718042ll, 541ll}, \
+    {245546983164360664ll, 540ll}, \
+    {236998906540082847ll, 539ll}, \
+    {228434956041092464ll, 538ll}, \
+    {219855072601758172ll, 537ll}, \
+    {211259196826165129ll, 536ll}, \
+    {194019229016300178ll, 534ll}, \
+    {185375016516461455ll, 533ll}, \
+    {176714570744179701ll, 532ll}, \
+    {168037830614650467ll, 531ll}, \
+    {159344734697631736ll, 530ll}, \
+    {150635221214834383ll, 529ll}, \
+    {141909228037287941ll, 528ll}, \
+    {133166692682681406ll, 527ll}, \
+    {124407552312678784ll, 526ll}, \
+    {115631743730209093ll, 525ll}, \
+    {106839203376730539ll, 524ll}, \
+    {98029867329468553ll, 523ll}, \
+    {89203671298627407ll, 522ll}, \
+    {80360550624575084ll, 521ll}, \
+    {71500440275001118ll, 520ll}, \
+    {62623274842047070ll, 519ll}, \
+    {53728988539409335ll, 518ll}, \
+    {44817515199413960ll, 517ll}, \
+    {35888788270063140ll, 516ll}, \
+    {26942740812053071ll, 515ll}, \
+    {17979305495762817ll, 514ll}, \
+    {0ll, 512ll}
+// D_j = 1 - exp(-j/64), times 2^64
+#define IMC_EXPM_ROWS \
+    0ull, 285990258791865196ull, 567546649590711158ull, 844737913148277362ull, \
+    1117631724489728397ull, 1386294709436213052ull, 1650792460871264869ull, 1911189554755015531ull, \
+    2167549565890130884ull, 2419935083443318773ull, 2668407726226198211ull, 2913028157739260623ull, \
+    3153856100982596093ull, 3390950353037000583ull, 3624368799419024035ull, 3854168428213464087ull, \
+    4080405343986755773ull, 4303134781484654118ull, 4522411119117553846ull, 4738287892236738577ull, \
+    4950817806204800870ull, 5160052749263424177ull, 5366043805201668333ull, 5568841265827851480ull, \
+    5768494643248073388ull, 5965052681954377915ull, 6158563370725505876ull, 6349073954343143847ull, \
+    6536630945126529359ull, 6721280134288228618ull, 6903066603113859213ull, 7082034733968487284ull, \
+    7258228221132386316ull, 7431690081468803075ull, 7602462664926335147ull, 7770587664878484220ull, \
+    7936106128302909442ull, 8099058465802866082ull, 8259484461473276195ull, 8417423282613840026ull, \
+    8572913489291559591ull, 8725993043755009064ull, 8876699319702650433ull, 9025069111407457241ull, \
+    9171138642700074143ull, 9314943575812705491ull, 9456519020085892127ull, 9595899540540302124ull, \
+    9733119166315628212ull, 9868211398978652248ull, 10001209220702505067ull, 10132145102319118672ull, \
+    10261051011246836720ull, 10387958419295118804ull, 10512898310348244006ull, 10635901187929889672ull, \
+    10756997082650432255ull, 10876215559538788475ull, 10993585725260586803ull, 11109136235224431575ull, \
+    11222895300577994696ull, 11334890695095642989ull, 11445149761959282784ull, 11553699420434077252ull
+struct ExpRow { double hi, lo; };  // 2^(-j/64)
+#define IMC_EXP2_ROWS \
     {0x1.0000000000000p+0, 0x0.0p+0}, \
     {0x1.fa7c1819e90d8p-1, 0x1.74853f3a5931ep-56}, \
     {0x1.f50765b6e4540p-1, 0x1.9d3e12dd8a18bp-55}, \
@@ -358,16 +380,19 @@ struct ExpRow { double hi, lo; };  // 2^(-j/64)
     {0x1.059b0d3158574p-1, 0x1.d73e2a475b465p-56}, \
     {0x1.02c9a3e778061p-1, -0x1.19083535b085dp-57}
 
+
 static const LogRow h_log_rows[256] = {IMC_LOG_ROWS};
-static const ExpRow h_exp_rows[64] = {IMC_EXP_ROWS};
+static const uint64_t h_expm_rows[64] = {IMC_EXPM_ROWS};
+static const ExpRow h_exp2_rows[64] = {IMC_EXP2_ROWS};
 #ifdef __CUDACC__
 static __device__ const LogRow d_log_rows[256] = {IMC_LOG_ROWS};
-static __device__ const ExpRow d_exp_rows[64] = {IMC_EXP_ROWS};
+static __device__ const uint64_t d_expm_rows[64] = {IMC_EXPM_ROWS};
+static __device__ const ExpRow d_exp2_rows[64] = {IMC_EXP2_ROWS};
 #endif
 #undef IMC_LOG_ROWS
-#undef IMC_EXP_ROWS
+#undef IMC_EXPM_ROWS
+#undef IMC_EXP2_ROWS
 
-constexpr double kLn2Hi = 0x1.62e42fefa3800p-1, kLn2Lo = 0x1.ef35793c76730p-45;          // ln 2: grid 2^-42, rest
 constexpr double kStepInv = 0x1.71547652b82fep+6;  // 64 / ln 2
 constexpr double kStepHi = 0x1.62e42fefa3800p-7, kStepLo = 0x1.ef35793c76730p-51;  // ln 2 / 64: grid 2^-48, rest
 IMC_HD uint64_t bits(double v) {
@@ -398,44 +423,94 @@ IMC_HD double one_minus_2u53(uint64_t k) {
     return ((k >> 52) ? 1.0 : 2.0) - w;
 }
 
-// -log(k 2^-53), 0 < k < 2^53
-IMC_HD double neglog_k53(uint64_t k) {
+IMC_HD uint64_t mulhi_u(uint64_t a, uint64_t b) {
 #ifdef __CUDA_ARCH__
-    const int z = __clzll((long long)k);  // 11..63
+    return __umul64hi(a, b);
 #else
-    const int z = __builtin_clzll(k);
+    return (uint64_t)(((unsigned __int128)a * b) >> 64);
 #endif
-    const uint64_t f = (k << (z - 11)) & 0xFFFFFFFFFFFFFull;  // fraction of the mantissa in [1, 2)
-    const int row = (int)(f >> 44);
-    const int up = row >> 7;  // mantissa at or above 1.5: halved
-    const double m = from_bits(((uint64_t)(0x3FF - up) << 52) | f);
+}
+IMC_HD long long mulhi_s(long long a, long long b) {
 #ifdef __CUDA_ARCH__
-    const LogRow &t = d_log_rows[row];
-    const double2 t0 = __ldg(reinterpret_cast<const double2 *>(&t));
-    const double tc = t0.x, thi = t0.y, tlo = __ldg(&t.lo);
-    const double e = __hiloint2double(0x43300000, z - 10 - up) - 0x1p52;
+    return __mul64hi(a, b);
 #else
-    const LogRow &t = h_log_rows[row];
-    const double tc = t.c, thi = t.hi, tlo = t.lo;
-    const double e = (double)(z - 10 - up);  // k 2^-53 = m 2^-e
+    return (long long)(((__int128)a * b) >> 64);
 #endif
-    const double r = fma(m, tc, -1.0);
-    const double hi = fma(e, kLn2Hi, thi);  // exact
-    const double lo = fma(e, kLn2Lo, tlo);
-    const double r2 = r * r;
-    double p = fma(r, 1.0 / 7.0, -1.0 / 6.0);
-    p = fma(r, p, 1.0 / 5.0);
-    p = fma(r, p, -1.0 / 4.0);
-    p = fma(r, p, 1.0 / 3.0);
-    p = fma(r, p, -1.0 / 2.0);
-    // hi + lo - (r + r2 p), with the rounding of hi - r kept
-    const double s = hi - r;
-    const double err = (hi - s) - r;
-    return s + (fma(-r2, p, lo) + err);
+}
+IMC_HD int mulhi_s32(int a, int b) {
+#ifdef __CUDA_ARCH__
+    return __mulhi(a, b);
+#else
+    return (int)(((long long)a * b) >> 32);
+#endif
+}
+IMC_HD uint32_t mulhi_u32(uint32_t a, uint32_t b) {
+#ifdef __CUDA_ARCH__
+    return __umulhi(a, b);
+#else
+    return (uint32_t)(((uint64_t)a * b) >> 32);
+#endif
+}
+IMC_HD int clz64(uint64_t v) {
+#ifdef __CUDA_ARCH__
+    return __clzll((long long)v);
+#else
+    return __builtin_clzll(v);
+#endif
+}
+// v 2^-scale rounded to the nearest double, v > 0
+IMC_HD double fixed_to_double(uint64_t v, int scale) {
+    const int z = clz64(v);
+    const uint64_t n = v << z;  // the leading bit at 63
+    const uint64_t m = (n >> 11) + ((n >> 10) & 1u);  // 53 bits, or 2^53
+    // the leading bit and a carry add to the exponent
+    return from_bits(((uint64_t)(1023 + 63 - scale - z - 1) << 52) + m);
 }
 
-// exp(-y) - 1, y >= 0 (NaN gives NaN)
-IMC_HD double expm1_neg(double y) {
+// -log(k 2^-53), 0 < k < 2^53
+IMC_HD double neglog_k53(uint64_t k) {
+    const int z = clz64(k);  // 11..63
+    const uint64_t f = k << (z - 11);  // mantissa in [1, 2), times 2^52
+    const int row = (int)(f >> 44) & 255;
+    const int up = row >> 7;  // mantissa at or above 1.5: halved
+    const int e = z - 10 - up;  // k 2^-53 = m 2^-e
+    if (e == 0 && row >= 254) {
+        // within 2^-8 of 1, where the result is small and wants its relative
+        // accuracy: the series in FP64
+        const double r = -u53((1ull << 53) - k);
+        const double r2 = r * r;
+        double p = fma(r, 1.0 / 7.0, -1.0 / 6.0);
+        p = fma(r, p, 1.0 / 5.0);
+        p = fma(r, p, -1.0 / 4.0);
+        p = fma(r, p, 1.0 / 3.0);
+        p = fma(r, p, -1.0 / 2.0);
+        return fma(-r2, p, -r);
+    }
+#ifdef __CUDA_ARCH__
+    const longlong2 t = __ldg(reinterpret_cast<const longlong2 *>(&d_log_rows[row]));
+    const long long tl = t.x, tc = t.y;
+#else
+    const long long tl = h_log_rows[row].l, tc = h_log_rows[row].c;
+#endif
+    // r 2^62, exact
+    const long long R = (long long)(f * (uint64_t)tc - (1ull << (61 + up))) << (1 - up);
+    // log1p(r) = r - r^2 P, P = 1/2 - r Q, Q = 1/3 - r (1/4 - r/5 + r^2/6 - r^3/7)
+    const int rh = (int)(R >> 24);  // r 2^38
+    int w = 715827883 - (mulhi_s32(rh, 613566757) >> 6);  // times 2^32 from here
+    w = 858993459 - (mulhi_s32(rh, w) >> 6);
+    w = 1073741824 - (mulhi_s32(rh, w) >> 6);
+    const long long Q = 1537228672809129301ll - (((long long)rh * w) >> 8);  // times 2^62
+    const long long P = (1ll << 61) - mulhi_s(R << 1, Q << 1);
+    const uint64_t a = (uint64_t)(R < 0 ? -R : R);
+    const uint64_t S = mulhi_u(a << 5, a << 5);  // r^2 2^70
+    const long long l = R - (long long)(mulhi_u(S << 1, (uint64_t)P << 1) >> 8);
+    const long long B = tl - l;  // log c - log1p(r), times 2^62
+    const uint64_t v = e ? (uint64_t)(e * 199786072581291495ll + ((B + 8) >> 4)) : (uint64_t)B;  // ln 2 times 2^58
+    return fixed_to_double(v, e ? 58 : 62);
+}
+
+// exp(-y) - 1, y >= 0 (NaN gives NaN), in FP64
+IMC_HD double expm1_neg_fp64(double y) {
     // 64 and beyond is -1 to the last bit; a NaN passes
     const uint32_t yh = hi32(y);
     if (yh - 0x40500000u <= 0x7FF00000u - 0x40500000u) y = 64.0;
@@ -459,15 +534,44 @@ IMC_HD double expm1_neg(double y) {
     const double p = fma(r2, q, -r);  // exp(-r) - 1
     const uint32_t j = ni & 63u;
 #ifdef __CUDA_ARCH__
-    const double2 t = __ldg(reinterpret_cast<const double2 *>(&d_exp_rows[j]));
+    const double2 t = __ldg(reinterpret_cast<const double2 *>(&d_exp2_rows[j]));
     const double th0 = t.x, tl0 = t.y;
 #else
-    const double th0 = h_exp_rows[j].hi, tl0 = h_exp_rows[j].lo;
+    const double th0 = h_exp2_rows[j].hi, tl0 = h_exp2_rows[j].lo;
 #endif
     // times 2^-(n / 64), by the exponents; the low part of row 0 is 0
     const uint64_t sh = (uint64_t)((ni >> 6) & 0x7Fu) << 52;
     const double th = from_bits(bits(th0) - sh), tl = j ? from_bits(bits(tl0) - sh) : 0.0;
     return (th - 1.0) + fma(th, p, tl);
+}
+
+// exp(-y) - 1, y >= 0 (NaN gives NaN)
+IMC_HD double expm1_neg(double y) {
+    const uint64_t yb = bits(y);
+    const int ex = (int)(yb >> 52);
+    if (ex >= 1023) return expm1_neg_fp64(y);
+    const int s = 1022 - ex;
+    uint64_t Y = ((yb & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull) << 11;  // y 2^64 once shifted
+    Y = s < 64 ? Y >> s : 0ull;
+    const int j = (int)(Y >> 58);
+    const uint64_t r = Y & 0x3FFFFFFFFFFFFFFull;  // (y - j/64) 2^64
+    // g = 1 - r (1/2 - r (1/6 - r (1/24 - r K))), K = 1/120 - r (1/720 - r (1/5040 - r/40320))
+    const uint32_t rh = (uint32_t)(r >> 26);  // r 2^38
+    uint32_t K = 54539267u - (mulhi_u32(rh, 6817408u) >> 6);  // times 2^38
+    K = 381774871u - (mulhi_u32(rh, K) >> 6);
+    K = 2290649225u - (mulhi_u32(rh, K) >> 6);
+    const uint64_t J = 192153584101141163ull - (((uint64_t)rh * K) >> 14);  // times 2^62 from here
+    const uint64_t I = 768614336404564651ull - mulhi_u(r, J);
+    const uint64_t H = (1ull << 61) - mulhi_u(r, I);
+    const uint64_t g = (1ull << 62) - mulhi_u(r, H);
+    if (j == 0) return -(y * fixed_to_double(g, 62));
+#ifdef __CUDA_ARCH__
+    const uint64_t D = __ldg(reinterpret_cast<const unsigned long long *>(&d_expm_rows[j]));
+#else
+    const uint64_t D = h_expm_rows[j];
+#endif
+    const uint64_t q = mulhi_u(r, g << 2);  // (r g) 2^64; g = 1 only where r < 2^-60
+    return -fixed_to_double(D + q - mulhi_u(D, q), 64);
 }
 
 // a / b, rb = RN(1 / b): correctly rounded while nothing under- or overflows

@@ -305,13 +305,14 @@ __device__ __forceinline__ Tab1<T> make_tab1(double sa, double f, double ss, dou
 // expm1(-sigma_a f d) -- one transcendental for both the attenuation and the
 // deposit, so the two add up to E up to one rounding -- and reciprocals
 // instead of divisions.  FP64 evaluates the same quantities from the functions
-// of imc_math64.cuh.  The FP64 pipe bounds it (16 cycles per warp instruction
-// and SM), so a segment holds as few FP64 instructions as its accuracy
-// allows: the deposits of a cell are summed as energies and divided by the
-// cell's volume once, when the tally is finalised, and comparisons run on the
-// bits.  Against CUDA's exp, expm1 and log, five divisions and FP64 compares:
-// 2000-cell slab at 2e6 histories 1.24 -> 0.65 ms per launch, 98 x 28 channel
-// 0.58 -> 0.21 ms.
+// of imc_math64.cuh.  The FP64 pipe bounds it (a warp's FP64 instruction takes
+// 64 cycles of its scheduler's unit), so a segment holds as few of them as its
+// accuracy allows: logarithm and exponential in 64-bit integers, the deposits
+// of a cell summed as energies and divided by the cell's volume once, when the
+// tally is finalised, and comparisons on the bits.  2000-cell slab at 2e6
+// histories: 1.24 ms per launch with CUDA's exp, expm1 and log, five divisions
+// and FP64 compares; 0.55 with table-driven FP64 functions and corrected
+// products; 0.35 with the functions in integers.
 template <class T> struct SegMath;
 template <> struct SegMath<double> {
     // inf for a zero opacity (rseff inf), as el / 0 is
