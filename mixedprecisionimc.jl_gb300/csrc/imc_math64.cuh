@@ -16,6 +16,7 @@
 //                FP64 (Tang, ACM TOMS 15, 1989)
 //   div_r        a / b with r = RN(1/b) at hand: one residual correction
 //                (Markstein, IBM J. Res. Dev. 34, 1990), a / b correctly rounded
+//   rcp64, Sum128   a reciprocal and the sum of a cell's deposits, in integers
 //   u53, one_minus_2u53   uniforms from their integers without a conversion
 //
 // Largest errors seen (tests/test_math64.py, against extended precision):
@@ -573,6 +574,81 @@ IMC_HD double expm1_neg(double y) {
     const uint64_t q = mulhi_u(r, g << 2);  // (r g) 2^64; g = 1 only where r < 2^-60
     return -fixed_to_double(D + q - mulhi_u(D, q), 64);
 }
+
+// 1 / b: binary32's reciprocal and two Newton steps in 64-bit integers, then
+// rounded (off by at most 0.52 units in the last place).  Beyond 2^+-1020, and
+// for zeros, infinities and NaN, the division.
+IMC_HD double rcp64(double b) {
+    const uint64_t u = bits(b);
+    const int ex = (int)(u >> 52) & 0x7FF;
+    if ((unsigned)(ex - 3) > 2040u) return 1.0 / b;
+    const uint64_t M = ((u & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull) << 11;  // |b| 2^(1022 - ex), times 2^64
+    const float f = (float)(uint32_t)(M >> 40);  // 24 bits of it
+    float r0;
+#ifdef __CUDA_ARCH__
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(f));
+#else
+    r0 = 1.0f / f;
+#endif
+    // the reciprocal, in (1, 2], times 2^61
+    long long R = (long long)(uint64_t)(uint32_t)(r0 * 0x1p53f) << 32;
+    for (int i = 0; i < 2; ++i) {
+        const long long e = (1ll << 61) - (long long)mulhi_u(M, (uint64_t)R);
+        R += mulhi_s(R, e << 3);
+    }
+    const double r = fixed_to_double((uint64_t)R, 61);
+    return from_bits((bits(r) + ((uint64_t)(int64_t)(1022 - ex) << 52)) | (u & 0x8000000000000000ull));
+}
+
+// The deposits of one cell of a history as an exact 128-bit sum in units of the
+// tally's 2^b, in place of a compensated pair: an addition in integers costs
+// less than the pair's four in FP64, and the flush has nothing left to convert.
+struct Sum128 {
+    uint64_t lo;
+    long long hi;
+    IMC_HD void clear() { lo = 0; hi = 0; }
+    IMC_HD void add128(uint64_t l, uint64_t h, bool neg) {
+        if (neg) {
+            h = ~h + (l == 0 ? 1u : 0u);
+            l = ~l + 1u;
+        }
+        const uint64_t t = lo + l;
+        hi += (long long)(h + (t < lo ? 1u : 0u));
+        lo = t;
+    }
+    // man 2^sh, rounded half up; false where it does not fit below 2^94
+    IMC_HD bool add(uint64_t man, int sh, bool neg) {
+        if (man == 0) return true;
+        if (sh >= 0) {
+            if (64 - clz64(man) + sh > 94) return false;
+            const uint64_t l = sh < 64 ? man << sh : 0ull;
+            const uint64_t h = sh == 0 ? 0ull : sh < 64 ? man >> (64 - sh) : man << (sh - 64);
+            add128(l, h, neg);
+        } else if (sh >= -64) {
+            const uint64_t half = (man >> (-sh - 1)) & 1u;
+            add128((sh == -64 ? 0ull : man >> -sh) + half, 0ull, neg);
+        }
+        return true;
+    }
+    // v in units of 2^b; false for infinities, NaN and values out of range
+    IMC_HD bool add(double v, int b) {
+        const uint64_t u = bits(v);
+        const int ex = (int)(u >> 52) & 0x7FF;
+        if (ex == 0x7FF) return false;
+        uint64_t man = u & 0xFFFFFFFFFFFFFull;
+        if (ex) man |= 0x10000000000000ull;
+        return add(man, (ex ? ex : 1) - 1075 - b, (u >> 63) != 0);
+    }
+    // x y to 64 bits (both finite), negated
+    IMC_HD bool add_minus_product(double x, double y, int b) {
+        const uint64_t u = bits(x), v = bits(y);
+        const int ex = (int)(u >> 52) & 0x7FF, ey = (int)(v >> 52) & 0x7FF;
+        if (ex == 0 || ey == 0 || ex == 0x7FF || ey == 0x7FF) return add(-(x * y), b);
+        const uint64_t m = (u & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull, n = (v & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
+        // (m 2^11)(n 2^11) = p 2^64
+        return add(mulhi_u(m << 11, n << 11), ex - 1075 + ey - 1075 + 42 - b, ((u ^ v) >> 63) == 0);
+    }
+};
 
 // a / b, rb = RN(1 / b): correctly rounded while nothing under- or overflows
 IMC_HD double div_r(double a, double b, double rb) {

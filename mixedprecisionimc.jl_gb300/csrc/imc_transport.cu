@@ -94,14 +94,15 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
     unsigned flags = 0;
     int emax_e = kNoExp;
     // Lane state of the history in flight (cs: as stored in the list; the
-    // current cell and scale are cell, k).  Deposits go to the compensated
-    // pair (acc_s, acc_c) of the current cell, flushed when it is left.
+    // current cell and scale are cell, k).  Deposits go to the sum of the
+    // current cell, flushed when it is left.
     long long i = 0;
     int cs = 0, cell = 0, k = 0, se = 0;  // se: scale k's exponent
     // shared tallies: scale k's deposition slots, and from there to its census slots
     const unsigned dep_shared = SMT ? (unsigned)__cvta_generic_to_shared(dep_acc) : 0u;
     unsigned slots_k = 0;
-    T t = (T)0, x = (T)0, mu = (T)0, E = (T)0, E0 = (T)0, minenergy = (T)0, acc_s = (T)0, acc_c = (T)0, rmu = (T)0;
+    T t = (T)0, x = (T)0, mu = (T)0, E = (T)0, E0 = (T)0, minenergy = (T)0, rmu = (T)0;
+    CellSum<T> dep_sum;
     unsigned seg = 0;
     Stream rs;  // FP64
     Words<LONG ? 7 : 5> ws;  // FP32
@@ -115,8 +116,7 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
         else if constexpr (LONG) ws.init((uint32_t)i);
         else ws.init_full((uint32_t)i, round_keys(ca), step, stage);
         minenergy = cutoff_energy(E0);  // (T)(0.01 * (double)E0), without FP64 in binary32
-        acc_s = (T)0;
-        acc_c = (T)0;
+        dep_sum.clear();
         seg = 0;
         rmu = rcp_any(mu);  // the face distance as a product (reset at each new direction)
     };
@@ -146,10 +146,14 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
     };
     // the deposits of the cell the history leaves, or ends in
     auto flush_cell = [&]() {
-        const T v = acc_s + acc_c;
-        if constexpr (SMT && sizeof(T) == 4)
-            if (add_f32_smem(slots_k + 24u * (unsigned)cell, v, b_dep + se)) return;
-        flush_rest<T, SMT>(dep_acc, k * nc + cell, v, b_dep + se, flags);
+        if constexpr (sizeof(T) == 4) {
+            const T v = dep_sum.s + dep_sum.c;
+            if constexpr (SMT)
+                if (add_f32_smem(slots_k + 24u * (unsigned)cell, v, b_dep + se)) return;
+            flush_rest<T, SMT>(dep_acc, k * nc + cell, v, b_dep + se, flags);
+        } else {
+            dep_sum.template flush<SMT>(dep_acc, k * nc + cell);
+        }
     };
     // one pass of the reference's while loop; 0 = go on, 1 = killed, 2 =
     // census, 3 = set aside for a query (kPause), 4 = escaped through a
@@ -160,7 +164,7 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
             Query q;
             const int kind = surr_decide<T>(tab[cell], x, mu, t, E, minenergy, c, ds, endsteptime, q);
             if (kind == kCertainKill) {
-                nadd(acc_s, acc_c, M::all_in(E, tab[cell]));
+                if constexpr (sizeof(T) == 4) dep_sum.add(M::all_in(E, tab[cell]));
                 ++seg;
                 ++calls;
                 return 1;
@@ -190,7 +194,7 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
             T dep;
             const T newenergy = M::attenuate(E, ce, dist, &dep);
             const bool dead = newenergy <= minenergy;
-            nadd(acc_s, acc_c, dead ? M::all_in(E, ce) : dep);
+            dep_sum.add(dead ? M::all_in(E, ce) : dep);
             x += mu * dist;
             t += dist * rdsc;
             E = newenergy;
@@ -200,8 +204,7 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
             const bool inside = (unsigned)next < (unsigned)N;
             if (at_b && inside) {
                 flush_cell();
-                acc_s = (T)0;
-                acc_c = (T)0;
+                dep_sum.clear();
                 cell = next;
                 x = right ? (T)0 : tab[next].dxs;
             }
@@ -244,7 +247,7 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
             end = dead ? 1 : escaped ? 4 : dist == dist_cen ? 2 : 0;
         } else {
             // FP64: every FP64 instruction costs more than a branch
-            T dist_b, dist_cen, dist, dep;
+            T dist_b, dist_cen, dist, em1;
             bool at_b, at_col, at_cen;
             const T dist_col = M::flight(rs, ce);
             const bool fwd = pos64(mu);
@@ -271,9 +274,9 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
                     return 1;
                 }
             }
-            const T newenergy = M::attenuate(E, ce.saf, dist, odd, &dep);
+            const T newenergy = M::attenuate(E, ce.saf, dist, odd, &em1);
             const bool dead = le64(newenergy, minenergy);
-            nadd(acc_s, acc_c, dead ? E : dep);
+            dep_sum.add(E, em1, dead, b_dep + se, flags);
             if (dead) return 1;
             x = fma(mu, dist, x);
             T dt_seg = ds_one ? dist : m64::div_r(dist, ds, rds);
@@ -285,8 +288,7 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
                 const int next = cell + (right ? 1 : -1);
                 if ((unsigned)next < (unsigned)N) {
                     flush_cell();
-                    acc_s = (T)0;
-                    acc_c = (T)0;
+                    dep_sum.clear();
                     cell = next;
                     x = right ? (T)0 : tab[next].dxs;
                 } else if (right ? reflect_r : reflect_l) {
@@ -301,7 +303,7 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
                 mu = (T)0;
                 for (int r = 0; r < 64 && mu == (T)0; ++r) mu = Rand<T>::cosine(rs);
                 if (mu == (T)0) mu = (T)1;
-                rmu = (T)1 / mu;
+                rmu = rcp_any(mu);
             }
             if (at_cen) end = 2;
         }
@@ -582,7 +584,7 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
     const unsigned rNX = NX > 1 ? 0xFFFFFFFFu / (unsigned)NX + 1u : 0u;
     auto row_of = [&](int c) { return NX > 1 ? (int)__umulhi((unsigned)c, rNX) : c; };
     T t = (T)0, xp = (T)0, yp = (T)0, vx = (T)0, vy = (T)0, E = (T)0, E0 = (T)0, minenergy = (T)0;
-    T acc_s = (T)0, acc_c = (T)0;
+    CellSum<T> dep_sum;
     T rvx = (T)0, rvy = (T)0;  // 1/vx, 1/vy (FP32: inf where div_mid is to divide)
     unsigned seg = 0;
     Stream rs;     // FP64
@@ -598,8 +600,7 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
         else if constexpr (SCHED == kLongSchedule) ws.init((uint32_t)i);
         else ws.init_full((uint32_t)i, round_keys(ca), step, kStageTransport);
         minenergy = cutoff_energy(E0);  // (T)(0.01 * (double)E0), without FP64 in binary32
-        acc_s = (T)0;
-        acc_c = (T)0;
+        dep_sum.clear();
         seg = 0;
         rvx = face_rcp(vx);
         rvy = face_rcp(vy);
@@ -626,10 +627,14 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
     // the deposits of the cell the history leaves, or ends in
     auto flush_cell = [&]() {
         const int cell = xi + yi * NX;
-        const T v = acc_s + acc_c;
-        if constexpr (SMT && sizeof(T) == 4)
-            if (add_f32_smem(slots_k + 24u * (unsigned)cell, v, b_dep + se)) return;
-        flush_rest<T, SMT>(dep_acc, k * nc + cell, v, b_dep + se, flags);
+        if constexpr (sizeof(T) == 4) {
+            const T v = dep_sum.s + dep_sum.c;
+            if constexpr (SMT)
+                if (add_f32_smem(slots_k + 24u * (unsigned)cell, v, b_dep + se)) return;
+            flush_rest<T, SMT>(dep_acc, k * nc + cell, v, b_dep + se, flags);
+        } else {
+            dep_sum.template flush<SMT>(dep_acc, k * nc + cell);
+        }
     };
     // one pass of the reference's while loop (src/imc_transport.jl:533-717);
     // 0 = go on, 1 = killed, 2 = census, 4 = escaped through a vacuum face.
@@ -640,7 +645,7 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
         if (++seg > cap) { flags |= (1u << 2); return 1; }
         const int cell = xi + yi * NX;
         const Tab2<T> ce = tab[cell];
-        T dist_bx, dist_by, dist_col, dist_cen, dist, Edens, newenergy, dep;
+        T dist_bx, dist_by, dist_col, dist_cen, dist, newenergy;
         bool at_b, at_col, at_cen, dead;
         const bool right = vx > (T)0, up = vy > (T)0;
         if constexpr (sizeof(T) == 4) {
@@ -657,9 +662,9 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
             at_cen = dist == dist_cen;
             const float em1 = expm1_seg(-ce.saf * dist);
             newenergy = E + E * em1;
-            Edens = E * ce.rarea;
-            dep = -Edens * em1;
+            const float Edens = E * ce.rarea;
             dead = newenergy <= minenergy;
+            dep_sum.add(dead ? Edens : -Edens * em1);
         } else {
             // FP64: SegMath<double>'s formulation; the deposits are energies
             dist_col = SegMath<double>::flight(rs, ce.seff, ca.tab_rs[cell]);
@@ -689,11 +694,11 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
                 at_cen = dist == dist_cen;
                 if (dist != dist) { flags |= 1u; return 1; }
             }
-            Edens = E;
-            newenergy = SegMath<double>::attenuate(E, ce.saf, dist, odd, &dep);
+            double em1;
+            newenergy = SegMath<double>::attenuate(E, ce.saf, dist, odd, &em1);
             dead = le64(newenergy, minenergy);
+            dep_sum.add(E, em1, dead, b_dep + se, flags);
         }
-        nadd(acc_s, acc_c, dead ? Edens : dep);
         if (dead) return 1;
         if constexpr (sizeof(T) == 4) {
             xp += dist * vx;
@@ -713,8 +718,7 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
             const int next = (ax ? xi : yi) + (fwd ? 1 : -1);
             if ((unsigned)next < (unsigned)(ax ? NX : NY)) {
                 flush_cell();
-                acc_s = (T)0;
-                acc_c = (T)0;
+                dep_sum.clear();
                 const T at = fwd ? (T)0 : (ax ? fx : fy)[next].ws;
                 if (ax) { xi = next; xp = at; }
                 else { yi = next; yp = at; }

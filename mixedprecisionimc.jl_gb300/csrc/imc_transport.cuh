@@ -50,16 +50,6 @@ template <> __device__ __forceinline__ void nadd<float>(float &s, float &c, floa
     c += (fmaxf(s, x) - t) + fminf(s, x);
     s = t;
 }
-// the same sums with the order chosen by the bits: four FP64 instructions
-// where the branches of the generic form issue up to eight
-template <> __device__ __forceinline__ void nadd<double>(double &s, double &c, double x) {
-    const bool ge = (long long)m64::bits(s) >= (long long)m64::bits(x);
-    const double big = ge ? s : x, small = ge ? x : s;
-    const double t = s + x;
-    c += (big - t) + small;
-    s = t;
-}
-
 // Limb adds into global memory (64-bit integer reductions in L2) or into the
 // block's private copy of the tally in shared memory.
 //
@@ -210,6 +200,36 @@ __device__ __forceinline__ void flush_rest(long long *acc, int slot, T v, int b,
     add_limbs<SMT>(acc + 3 * (size_t)slot, A);
 }
 
+// The deposits of the cell a history is in: a compensated pair of binary32
+// densities, or an exact sum of energies (FP64).
+template <class T> struct CellSum;
+template <> struct CellSum<float> {
+    float s, c;
+    __device__ __forceinline__ void clear() { s = 0.0f; c = 0.0f; }
+    __device__ __forceinline__ void add(float x) { nadd(s, c, x); }
+};
+template <> struct CellSum<double> {
+    m64::Sum128 v;
+    __device__ __forceinline__ void clear() { v.clear(); }
+    // dead: all of E, else E's share -em1; b: the tally's exponent
+    __device__ __forceinline__ void add(double E, double em1, bool dead, int b, unsigned &flags) {
+        const bool ok = dead ? v.add(E, b) : v.add_minus_product(E, em1, b);
+        if (!ok) flags |= (E != E || em1 != em1) ? 1u /*NAN*/ : (1u << 5) /*FIXPOINT_RANGE*/;
+    }
+    template <bool SMT> __device__ __forceinline__ void flush(long long *acc, int slot) const {
+        if ((v.lo | (uint64_t)v.hi) == 0) return;
+        const bool neg = v.hi < 0;
+        const uint64_t l = neg ? ~v.lo + 1u : v.lo;
+        const uint64_t h = neg ? ~(uint64_t)v.hi + (v.lo == 0 ? 1u : 0u) : (uint64_t)v.hi;
+        Limbs A;
+        A.l2 = (long long)(l & 0xFFFFFFFFull);
+        A.l1 = (long long)(l >> 32);
+        A.l0 = (long long)h;
+        if (neg) { A.l0 = -A.l0; A.l1 = -A.l1; A.l2 = -A.l2; }
+        add_limbs<SMT>(acc + 3 * (size_t)slot, A);
+    }
+};
+
 template <class T, bool SMT>
 __device__ __forceinline__ void flush_one(long long *acc, int slot, T v, int b, unsigned &flags) {
     if constexpr (SMT && sizeof(T) == 4)
@@ -324,14 +344,12 @@ template <> struct SegMath<double> {
     static __device__ __forceinline__ double flight(Stream &rs, const Tab1<double> &ce) {
         return flight(rs, ce.seff, ce.rseff);
     }
-    // new weight; *dep = the energy deposited (d < 0, a history past its
-    // census time by a rounding, takes the general expm1)
-    static __device__ __forceinline__ double attenuate(double E, double saf, double d, bool odd, double *dep) {
-        const double em1 = odd ? expm1(-saf * d) : m64::expm1_neg(saf * d);
-        *dep = -(E * em1);
-        return fma(E, em1, E);
+    // new weight; *em1 = minus the share of it deposited (d < 0, a history past
+    // its census time by a rounding, takes the general expm1)
+    static __device__ __forceinline__ double attenuate(double E, double saf, double d, bool odd, double *em1) {
+        *em1 = odd ? expm1(-saf * d) : m64::expm1_neg(saf * d);
+        return fma(E, *em1, E);
     }
-    static __device__ __forceinline__ double all_in(double E, const Tab1<double> &) { return E; }
 };
 // the least of three, NaN if one is NaN (jmin of jmin; one instruction)
 __device__ __forceinline__ float min3_nan(float a, float b, float c) {
