@@ -80,7 +80,8 @@ struct ImcHandle {
     // totals over every step run since imc_create
     int64_t tot_segments = 0, tot_histories = 0, tot_calls = 0;
     int stage = Stage::Fresh;
-    long long n_census_host = 0;
+    long long n_known = -1;   // the list's length, while no call has changed it since it was read
+    StepMirror *mirror = nullptr;  // pinned; from the first imc_step on
     ImcStepStats last{};
     std::string err;
     int err_code = IMC_OK;
@@ -396,6 +397,24 @@ int collect_events(ImcHandle *h, size_t pairs) {
         h->transport_launches += 1;
     }
     return IMC_OK;
+}
+
+// the pinned block of a handle that is stepped (without one, the copies serve)
+void ensure_mirror(ImcHandle *h) {
+    if (h->mirror) return;
+    void *p = nullptr, *d = nullptr;
+    if (cudaHostAlloc(&p, sizeof(StepMirror), cudaHostAllocMapped) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return;
+    }
+    if (cudaHostGetDevicePointer(&d, p, 0) != cudaSuccess) {
+        (void)cudaGetLastError();
+        cudaFreeHost(p);
+        return;
+    }
+    h->mirror = static_cast<StepMirror *>(p);
+    h->ca.mirror = static_cast<StepMirror *>(d);
+    drop_graphs(h);
 }
 
 int ensure_stats(ImcHandle *h, long long n) {
@@ -845,6 +864,7 @@ int imc_destroy(ImcHandle *h) {
     for (auto e : h->ev_pool) cudaEventDestroy(e);
     for (int i = 0; i < 2; ++i) if (h->ev[i]) cudaEventDestroy(h->ev[i]);
     if (h->d_stats) cudaFree(h->d_stats);
+    if (h->mirror) cudaFreeHost(h->mirror);
     if (h->d_surr_image) cudaFree(h->d_surr_image);
     free_list(h->qallocs);
     free_list(h->pallocs);
@@ -868,6 +888,7 @@ int imc_sourcing(ImcHandle *h) {
     Scalars sc;
     int rc = read_scalars(h, &sc);
     if (rc) return rc;
+    h->n_known = -1;
     if ((rc = grow(h, sc.n_particles + births_bound(h, sc.n_particles)))) return rc;
     launch_source(h->ca, h->d_sc, h->prec, pair(h), h->grid_emit, false, h->stream);
     CKL(h);
@@ -904,6 +925,7 @@ int imc_transport(ImcHandle *h) {
 int imc_clean(ImcHandle *h) {
     if (!h) return IMC_ERR_INVALID_ARG;
     // Clean.clean removes every killed particle (forced compaction)
+    h->n_known = -1;
     launch_compact(h->ca, h->d_sc, h->prec, pair(h), h->tile_cnt, h->tile_off, h->ntiles_cap, true, h->stream);
     CKL(h);
     CK(h, cudaStreamSynchronize(h->stream));
@@ -954,9 +976,14 @@ int imc_step(ImcHandle *h, ImcStepStats *stats, int *done) {
     if (!h) return IMC_ERR_INVALID_ARG;
     if (h->finished) { if (done) *done = 1; return IMC_OK; }
     Scalars sc;
-    int rc = read_scalars(h, &sc);
-    if (rc) return rc;
-    if ((rc = grow(h, sc.n_particles + births_bound(h, sc.n_particles)))) return rc;
+    int rc;
+    if (h->n_known < 0) {
+        if ((rc = read_scalars(h, &sc))) return rc;
+        h->n_known = sc.n_particles;
+    }
+    if ((rc = grow(h, h->n_known + births_bound(h, h->n_known)))) return rc;
+    ensure_mirror(h);
+    h->n_known = -1;
     if (h->timing) {
         if ((rc = ensure_events(h, 1))) return rc;
         if ((rc = enqueue_step(h, true, 0))) return rc;
@@ -964,11 +991,18 @@ int imc_step(ImcHandle *h, ImcStepStats *stats, int *done) {
         if ((rc = capture(h))) return rc;
         CK(h, cudaGraphLaunch(h->graph, h->stream));
     }
-    if ((rc = read_scalars(h, &sc))) return rc;
-    if (h->timing && (rc = collect_events(h, 1))) return rc;
     DevStats ds;
-    CK(h, hcopy(h, &ds, h->d_stats + ((sc.step - 1u) % (unsigned long long)h->stats_cap), sizeof(DevStats),
-                     cudaMemcpyDeviceToHost));
+    if (h->mirror) {
+        CK(h, cudaStreamSynchronize(h->stream));
+        ds = h->mirror->last;
+        h->n_known = h->mirror->n_particles;
+    } else {
+        if ((rc = read_scalars(h, &sc))) return rc;
+        CK(h, hcopy(h, &ds, h->d_stats + ((sc.step - 1u) % (unsigned long long)h->stats_cap), sizeof(DevStats),
+                         cudaMemcpyDeviceToHost));
+        h->n_known = sc.n_particles;
+    }
+    if (h->timing && (rc = collect_events(h, 1))) return rc;
     to_stats(ds, &h->last);
     h->tot_segments += ds.segments;
     h->tot_histories += ds.n_census_in + ds.n_sourced;
@@ -1002,6 +1036,7 @@ static int run_steps(ImcHandle *h, int64_t max_steps, ImcStepStats *stats, int64
     if ((rc = ensure_stats(h, N))) return rc;
     Scalars sc;
     if ((rc = read_scalars(h, &sc))) return rc;
+    h->n_known = -1;
     // first stats slot of this run
     const unsigned long long slot0 = sc.step;
     CK(h, cudaEventRecord(h->ev[0], h->stream));
@@ -1045,6 +1080,7 @@ static int run_steps(ImcHandle *h, int64_t max_steps, ImcStepStats *stats, int64
     unsigned allflags = 0;
     if ((rc = absorb_steps(h, slot0, done_steps, stats, &allflags))) return rc;
     if (n_steps) *n_steps = done_steps;
+    h->n_known = n_census;
     return flags_status(h, allflags);
 }
 
@@ -1134,6 +1170,7 @@ int imc_run_batch_fused(ImcHandle *const *hs, int32_t n, int64_t max_steps, int6
             host_timestep(h->deck, t, dt, fin);
         }
         Scalars sc;
+        h->n_known = -1;
         if (N[i] > 0 && ((rc = ensure_stats(h, N[i])) || (rc = read_scalars(h, &sc)))) { bad = i; break; }
         if (N[i] > 0) { slot0[i] = sc.step; ncen[i] = sc.n_particles; }
     }
@@ -1282,8 +1319,13 @@ int imc_get_field(const ImcHandle *h, int field, double *out, int64_t count) {
     double *p = field_ptr(h, field, &n);
     if (!p) return fail(hh, IMC_ERR_INVALID_ARG, "unknown field");
     if (n != count) return fail(hh, IMC_ERR_INVALID_ARG, "field size mismatch");
-    CK(hh, cudaStreamSynchronize(h->stream));
-    CK(hh, hcopy(hh, out, p, sizeof(double) * n, cudaMemcpyDeviceToHost));
+    const size_t bytes = sizeof(double) * (size_t)n;
+    if (h->mirror && bytes <= sizeof(h->mirror->stage)) {
+        CK(hh, hcopy(hh, h->mirror->stage, p, bytes, cudaMemcpyDeviceToHost));
+        std::memcpy(out, h->mirror->stage, bytes);
+        return IMC_OK;
+    }
+    CK(hh, hcopy(hh, out, p, bytes, cudaMemcpyDeviceToHost));
     return IMC_OK;
 }
 
@@ -1378,6 +1420,7 @@ int imc_load_state(ImcHandle *h, const void *buf, size_t len) {
     Scalars sc;
     std::memcpy(&sc, in, sizeof sc); in += sizeof sc;
     const long long n = hd.n_particles;
+    h->n_known = -1;
     int rc = grow(h, n);
     if (rc) return rc;
     auto cells = cell_pieces(h);
@@ -1465,6 +1508,7 @@ int imc_set_particles(ImcHandle *h, const ImcParticles *p) {
     if (!h || !p || p->n < 0 || !p->E || !p->E0 || !p->cell) return IMC_ERR_INVALID_ARG;
     const long long n = p->n;
     int rc;
+    h->n_known = -1;
     if ((rc = grow(h, n + births_bound(h, n)))) return rc;
     CK(h, cudaStreamSynchronize(h->stream));
     const int prec = h->prec;

@@ -111,6 +111,7 @@ struct CellArgs {
     // (imc_surrogate.cuh), or null for analog transport everywhere
     const uint4 *surr_image;
     long long surr_min_calls;          // queries a step needs to keep the network on (surr_gate)
+    struct StepMirror *mirror;         // device address of the handle's mirror, or null
 };
 
 // type-erased particle buffer
@@ -131,6 +132,15 @@ struct DevStats {
     double t, dt, total_energy, energy_dep, rad_energy, rad_energy_old, lost_energy, energy_error;
     long long n_census_in, n_sourced, n_census_out, segments, surrogate_calls;
     unsigned int error_flags, step_index;
+};
+
+// What a program that steps reads after every step, in pinned host memory that
+// the step's last kernel writes: no copy to wait for.  The rest of the block
+// stages the reads of small fields.
+struct StepMirror {
+    DevStats last;
+    long long n_particles;
+    unsigned char stage[1 << 16];
 };
 
 // launchers (imc_kernels.cu / imc_transport.cu); all asynchronous on `st`

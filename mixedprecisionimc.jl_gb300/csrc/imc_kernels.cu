@@ -1193,7 +1193,7 @@ __device__ void energycheck_done(const CellArgs &ca, Scalars *sc, DevStats *stat
     sc->totalenergydep = totdep;
     double err = (sc->totalenergy - totdep - (radenergy - sc->radenergyold) - sc->lostenergy) / sc->totalenergy;
     if (stats && stats_cap > 0) {
-        DevStats &d = stats[sc->step % (unsigned long long)stats_cap];
+        DevStats d;
         d.t = sc->t; d.dt = sc->dt;
         d.total_energy = sc->totalenergy;
         d.energy_dep = totdep;
@@ -1208,6 +1208,11 @@ __device__ void energycheck_done(const CellArgs &ca, Scalars *sc, DevStats *stat
         d.surrogate_calls = (long long)sc->surrogate_calls;
         d.error_flags = sc->flags;
         d.step_index = sc->step;
+        stats[sc->step % (unsigned long long)stats_cap] = d;
+        if (step && ca.mirror) {
+            ca.mirror->last = d;
+            ca.mirror->n_particles = sc->n_particles;
+        }
     }
     sc->energy_err = err;
     sc->radenergy = radenergy;
