@@ -975,6 +975,7 @@ int imc_timestep(ImcHandle *h, int *done) {
 int imc_step(ImcHandle *h, ImcStepStats *stats, int *done) {
     if (!h) return IMC_ERR_INVALID_ARG;
     if (h->finished) { if (done) *done = 1; return IMC_OK; }
+    set_side_by_side(h, false);
     Scalars sc;
     int rc;
     if (h->n_known < 0) {
