@@ -10,10 +10,11 @@
 //   k_tally            <- Tally.tally                    src/imc_tally.jl:22-142
 //   k_energycheck      <- EnergyCheck.energychecker      src/imc_energycheck.jl:19-38
 //   k_timestep         <- timestep                       src/MixedPrecisionIMC.jl:181-222
+//   k_tally_check      the step sequence: finalize, tally, energy check, clock
 //
-// Sums over cells are double-double: a fixed-order tree inside each 64-thread
-// block, then the block partials in block order -- deterministic, and within
-// a rounding of the exact sum.  Every launch has a fixed grid and reads its sizes from
+// Sums over cells are exact to 93 bits below the largest term inside a warp's
+// unit of 32, then over the units' partials in the last block to finish --
+// deterministic, and within a rounding of the exact sum.  Every launch has a fixed grid and reads its sizes from
 // device scalars, so a whole step can be captured once as a CUDA graph.
 #include <cstdint>
 #include "imc_device.cuh"
@@ -23,10 +24,10 @@
 
 namespace imc {
 
-// GB300 executes FP64 at 1/64 of the FP32 rate, so every per-cell FP64 stage
-// runs as many one-warp blocks (kCellThreads) spread over the SMs; sums are
-// double-double per block over a fixed partition of the cells, combined in
-// block order.
+// GB300 executes FP64 at 1/64 of the FP32 rate, so a per-cell FP64 stage runs as
+// one warp, or one warp for each of an SM's four FP64 units, a block, spread over
+// the SMs, and keeps what it can in integers; sums run over a fixed partition of
+// the cells (units of kCellThreads).
 
 // x / s for an energy scale s: the scales in use are 1 and powers of two, whose
 // quotients need no division
@@ -51,8 +52,8 @@ __device__ __forceinline__ double times_pow2(double v, int e) {
 // the largest exponent present: four signed 24-bit digits.  32 or more such
 // digits add up in 32 bits with the warp's integer reduction, so a sum costs a
 // handful of FP64 instructions (the digits back to two doubles) where a tree
-// of double-double adds took 40 (64 cycles each for a warp: half of the step's
-// tail).  What lies 93 bits below the largest term is rounded away, as a
+// of double-double adds took 40 (each as long as 64 FP32 instructions: half of
+// the step's tail).  What lies 93 bits below the largest term is rounded away, as a
 // double-double sum's is.
 struct Digits {
     int d[4];
@@ -698,9 +699,9 @@ template <> struct BirthDraws<double> {
 };
 
 // One thread per newborn particle; its stream is keyed by its list index.
-// (Instruction issue bounds it: 33 B are stored for 250 instructions a warp's
-// birth with the slot looked up and decoded for each, 49 us for the channel's
-// 4e6 births.)
+// (33 B are stored for 190 instructions a warp's birth, 20 us each for the
+// channel's 4e6 births; with the latency of the slot searches it takes 46.  With
+// the slot looked up and decoded for each birth, 250 instructions: 49.)
 template <class St, int G>
 __global__ void __launch_bounds__(256) k_source_emit(CellArgs ca, Scalars *sc, PBufPair bufs) {
     typedef typename St::T T;
@@ -1261,9 +1262,9 @@ __global__ void __launch_bounds__(544) k_energycheck(CellArgs ca, Scalars *sc, D
 // nothing that the compaction between them in the reference's order changes.
 // Blocks of four warps, one for each of an SM's FP64 units; each publishes its
 // partial sums before taking a ticket, and the last block's warps sum a group
-// each over every unit of cells.  (FP64 latency bounds it, a warp's FP64
-// instruction taking 64 cycles: 2000 cells 24 us with double-double trees,
-// pow and divisions by the scales, one warp a block.)
+// each over every unit of cells.  (FP64 latency bounds it, an FP64
+// instruction taking as long as 64 in FP32: 2000 cells 24 us with double-double
+// trees, pow and divisions by the scales, one warp a block, against 12.)
 constexpr int kTailThreads = 128;
 __global__ void __launch_bounds__(kTailThreads) k_tally_check(CellArgs ca, Scalars *sc, DevStats *stats,
                                                              long long stats_cap) {

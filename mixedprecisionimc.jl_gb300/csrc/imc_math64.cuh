@@ -1,9 +1,9 @@
 // imc_math64.cuh -- the double precision functions of a transport segment,
-// with few FP64 operations: GB300 issues FP64 at 1/64 of the FP32 rate (a warp's
-// FP64 instruction takes 64 cycles of its scheduler's unit), so an FP64
-// history costs its FP64 instructions and little else, and a function in 64-bit
-// integers -- about a hundred instructions at one or two cycles -- is a tenth of
-// the same function in sixteen FP64 instructions.
+// with few FP64 operations: GB300 issues FP64 at 1/64 of the FP32 rate (an FP64
+// instruction takes as long as 64 in FP32), so an FP64 history costs its FP64
+// instructions and little else, and a function in 64-bit integers -- about a
+// hundred instructions of the FP32 kind -- is a tenth of the same function in
+// sixteen FP64 instructions.
 //
 //   neglog_k53   -log(k 2^-53) of a 53-bit uniform integer k: table-driven
 //                reduction after Tang (ACM TOMS 16, 1990) in fixed point: the

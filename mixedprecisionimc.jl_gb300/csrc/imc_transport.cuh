@@ -1,8 +1,8 @@
 // imc_transport.cuh -- device helpers shared by the transport kernels
 // (imc_transport.cu, imc_transport_surr.cu): math overloads of the particle
-// type, Neumaier accumulation, exact fixed-point tally flushes into global or
-// block-shared accumulators, the per-cell table and the end-of-kernel
-// counter reduction.
+// type, the segment arithmetic, the sums of a cell's deposits, exact fixed-point
+// tally flushes into global or block-shared accumulators, the work split, the
+// per-cell table and the end-of-kernel counter reduction.
 #pragma once
 #include <cstdint>
 #include "imc_device.cuh"
@@ -12,13 +12,8 @@
 
 namespace imc {
 
-__device__ __forceinline__ float m_exp(float x) { return expf(x); }
-__device__ __forceinline__ double m_exp(double x) { return exp(x); }
-__device__ __forceinline__ float m_expm1(float x) { return expm1f(x); }
-__device__ __forceinline__ double m_expm1(double x) { return expm1(x); }
 __device__ __forceinline__ float m_abs(float x) { return fabsf(x); }
 __device__ __forceinline__ double m_abs(double x) { return fabs(x); }
-__device__ __forceinline__ void m_sincos(float a, float *s, float *c) { sincosf(a, s, c); }
 __device__ __forceinline__ void m_sincos(double a, double *s, double *c) { sincos(a, s, c); }
 
 // e^x - 1 in the FP32 segment arithmetic: for |x| <= 1/16 the Taylor series
@@ -325,8 +320,8 @@ __device__ __forceinline__ Tab1<T> make_tab1(double sa, double f, double ss, dou
 // expm1(-sigma_a f d) -- one transcendental for both the attenuation and the
 // deposit, so the two add up to E up to one rounding -- and reciprocals
 // instead of divisions.  FP64 evaluates the same quantities from the functions
-// of imc_math64.cuh.  The FP64 pipe bounds it (a warp's FP64 instruction takes
-// 64 cycles of its scheduler's unit), so a segment holds as few of them as its
+// of imc_math64.cuh.  The FP64 pipe bounds it (an FP64 instruction takes as
+// long as 64 in FP32), so a segment holds as few of them as its
 // accuracy allows: logarithm and exponential in 64-bit integers, the deposits
 // of a cell summed as energies and divided by the cell's volume once, when the
 // tally is finalised, and comparisons on the bits.  2000-cell slab at 2e6

@@ -1,6 +1,6 @@
 """In-tree build of libimc.so (the C-ABI CUDA library) for sm_103a.
 
-The three translation units compile in parallel with one ``-gencode`` and are
+The translation units compile in parallel with one ``-gencode`` and are
 linked into ``mixedprecisionimc.jl_gb300/_build/libimc.so``.  Kernels are built
 with ``--fmad=false`` so the restated reference arithmetic rounds exactly as
 written (no fused multiply-add contraction), which keeps per-history parity
