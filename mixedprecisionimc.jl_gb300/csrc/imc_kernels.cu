@@ -700,10 +700,12 @@ template <> struct BirthDraws<double> {
 
 // One thread per newborn particle; its stream is keyed by its list index.
 // (33 B are stored for 190 instructions a warp's birth, 20 us each for the
-// channel's 4e6 births; with the latency of the slot searches it takes 46.  With
-// the slot looked up and decoded for each birth, 250 instructions: 49.)
+// channel's 4e6 births; with the latency of the slot searches and the nine
+// streams of stores it takes 37.  With the slot looked up and decoded for each
+// birth, 250 instructions: 49.)
+constexpr int kEmitThreads = 256;
 template <class St, int G>
-__global__ void __launch_bounds__(256) k_source_emit(CellArgs ca, Scalars *sc, PBufPair bufs) {
+__global__ void __launch_bounds__(kEmitThreads) k_source_emit(CellArgs ca, Scalars *sc, PBufPair bufs) {
     typedef typename St::T T;
     PBuf<St> pb(bufs.b[sc->cur]);
     const long long n_new = sc->n_sourced, n_census = sc->birth_base;
@@ -711,124 +713,118 @@ __global__ void __launch_bounds__(256) k_source_emit(CellArgs ca, Scalars *sc, P
     const T dtT = (T)sc->dt, dsT = Consts<T>::ds(ca);
     const int nslots = ca.nslots;
     const double pd = 3.141592653589793;
-    // Each warp takes `run` consecutive births at a time, lane l the births
-    // base + l + 32 i (every store coalesced).  A lane finds the slot of its
+    // Each block takes an equal run of consecutive births, thread l the births
+    // base + l + 256 i: the block writes one stretch of every array, where runs
+    // of each warp wrote eight times as many at once (2D: 45 us for 4e6 births
+    // against 37, 121 for 1e7 against 93; blocks of 1024: 41 and 91).  A lane finds the slot of its
     // first birth by binary search over the slot offsets (slot = last q whose
     // first birth is at or below j) and the later ones by galloping forward
     // from there (q + 1, q + 2, q + 4, ... then bisection) once the slot's
-    // last birth is behind it.  The run is the births per warp of the grid,
-    // rounded up to a multiple of 32 in [32, 1024], so a small step's births
-    // still spread over every warp.
+    // last birth is behind it.
     auto off = [&](int s) { return ca.slot_off[s] + ca.blk_off[s / kCountThreads]; };
-    const int lane = threadIdx.x & 31;
-    const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-    const long long per_warp = (n_new + nw - 1) / nw;
-    const int run = per_warp >= 1024 ? 1024 : per_warp <= 32 ? 32 : (int)((per_warp + 31) & ~31ll);
-    for (long long base = wid * run; base < n_new; base += nw * run) {
-        int q = -1;
-        long long next = -1;  // the first birth beyond slot q
-        BirthSlot<T> b{};
-        for (int r = 0; r < run; r += 32) {
-            const long long j = base + r + lane;
-            if (j >= n_new) break;
-            if (next <= j) {
-                int lo, hi;
-                if (q < 0) {
-                    // the last block that starts at or below j, then its last such slot
-                    lo = 0;
-                    hi = ca.nblk_count;
-                    while (hi - lo > 1) {
-                        const int mid = (lo + hi) >> 1;
-                        if (ca.blk_off[mid] <= j) lo = mid;
-                        else hi = mid;
-                    }
-                    const long long rest = j - ca.blk_off[lo];
-                    lo *= kCountThreads;
-                    hi = min(lo + kCountThreads, nslots);
-                    while (hi - lo > 1) {
-                        const int mid = (lo + hi) >> 1;
-                        if (ca.slot_off[mid] <= rest) lo = mid;
-                        else hi = mid;
-                    }
-                } else {
-                    int stride = 2;
-                    lo = q + 1;  // off(lo) <= j
-                    hi = q + 2;
-                    while (hi < nslots && off(hi) <= j) {
-                        lo = hi;
-                        stride <<= 1;
-                        hi = q + stride;
-                    }
-                    if (hi > nslots) hi = nslots;  // off(hi) > j, or hi == nslots
-                    while (hi - lo > 1) {
-                        const int mid = (lo + hi) >> 1;
-                        if (off(mid) <= j) lo = mid;
-                        else hi = mid;
-                    }
+    const long long per_block = (n_new + gridDim.x - 1) / gridDim.x;
+    const long long run = (per_block + kEmitThreads - 1) & ~(long long)(kEmitThreads - 1);
+    const long long end = min((blockIdx.x + 1) * run, n_new);
+    int q = -1;
+    long long next = -1;  // the first birth beyond slot q
+    BirthSlot<T> b{};
+    for (long long j = blockIdx.x * run + threadIdx.x; j < end; j += kEmitThreads) {
+        if (next <= j) {
+            int lo, hi;
+            if (q < 0) {
+                // the last block that starts at or below j, then its last such slot
+                lo = 0;
+                hi = ca.nblk_count;
+                while (hi - lo > 1) {
+                    const int mid = (lo + hi) >> 1;
+                    if (ca.blk_off[mid] <= j) lo = mid;
+                    else hi = mid;
                 }
-                q = lo;
-                next = q + 1 < nslots ? off(q + 1) : n_new;
-                b = birth_slot<St>(ca, q);
-            }
-            const long long pid = n_census + j;
-            BirthDraws<T> d(ca, step, (uint32_t)pid);
-            if (G == 1) {
-                T xpos, mu;
-                if (b.kind == kBody1D) {
-                    // body / source births (src/imc_sourcing.jl:193-236)
-                    xpos = b.wx * d.u() * dsT;
-                    mu = d.cosine();
-                    for (int r1 = 1; r1 < 64 && mu == (T)0; ++r1) mu = d.cosine();
-                    if (mu == (T)0) mu = (T)1;
-                } else {
-                    // surface births (src/imc_sourcing.jl:161-189)
-                    xpos = b.x0;
-                    mu = RT<T>::sqrt_(d.u());
-                    for (int r1 = 1; r1 < 64 && mu == (T)0; ++r1) mu = RT<T>::sqrt_(d.u());
-                    if (mu == (T)0) mu = (T)1;
-                    if (b.kind == kRight1D) mu = -mu;
+                const long long rest = j - ca.blk_off[lo];
+                lo *= kCountThreads;
+                hi = min(lo + kCountThreads, nslots);
+                while (hi - lo > 1) {
+                    const int mid = (lo + hi) >> 1;
+                    if (ca.slot_off[mid] <= rest) lo = mid;
+                    else hi = mid;
                 }
-                const T st = dtT * d.u();
-                store_birth<St>(1, pb, pid, st, xpos, (T)0, mu, (T)0, b, (float)dtT);
             } else {
-                T st, xpos, ypos, ang;
-                // the angles are the reference's Float64 products rounded to T
-                // (binary32: pi_n24 or two_pi_u24 of the uniform's integer m,
-                // the same value without FP64)
-                if (b.kind == kBody2D) {
-                    // body / source births (src/imc_sourcing.jl:326-366)
-                    xpos = b.wx * d.u() * dsT;
-                    ypos = b.wy * d.u() * dsT;
-                    if constexpr (sizeof(T) == 4) ang = two_pi_u24(d.word() >> 8);
-                    else ang = (T)(2.0 * pd * (double)d.u());
-                    st = dtT * d.u();
-                } else {
-                    // surface births (src/imc_sourcing.jl:265-323)
-                    st = dtT * d.u();
-                    const bool horizontal = b.kind == kBottom2D || b.kind == kTop2D;
-                    const T along = (horizontal ? b.wx : b.wy) * d.u() * dsT;
-                    xpos = horizontal ? along : b.x0;
-                    ypos = horizontal ? b.y0 : along;
-                    if constexpr (sizeof(T) == 4) {
-                        const uint32_t m = d.word() >> 8;
-                        if (b.kind == kBottom2D) ang = (T)pd * ((T)m * 0x1p-24f);
-                        else if (b.kind == kTop2D) ang = -pi_n24((int)m);
-                        else if (b.kind == kLeft2D) ang = pi_n24((1 << 23) - (int)m);
-                        else ang = (T)(pd * (0.5 + (double)((T)m * 0x1p-24f)));
-                    } else {
-                        const T u = d.u();
-                        if (b.kind == kBottom2D) ang = (T)((T)pd * u);
-                        else if (b.kind == kTop2D) ang = (T)(-pd * (double)u);
-                        else if (b.kind == kLeft2D) ang = (T)(pd * (0.5 - (double)u));
-                        else ang = (T)(pd * (0.5 + (double)u));
-                    }
+                int stride = 2;
+                lo = q + 1;  // off(lo) <= j
+                hi = q + 2;
+                while (hi < nslots && off(hi) <= j) {
+                    lo = hi;
+                    stride <<= 1;
+                    hi = q + stride;
                 }
-                T ux, uy;
-                if (sizeof(T) == 4) { float s_, c_; sincosf((float)ang, &s_, &c_); ux = (T)c_; uy = (T)s_; }
-                else { double s_, c_; sincos((double)ang, &s_, &c_); ux = (T)c_; uy = (T)s_; }
-                store_birth<St>(2, pb, pid, st, xpos, ypos, ux, uy, b, (float)dtT);
+                if (hi > nslots) hi = nslots;  // off(hi) > j, or hi == nslots
+                while (hi - lo > 1) {
+                    const int mid = (lo + hi) >> 1;
+                    if (off(mid) <= j) lo = mid;
+                    else hi = mid;
+                }
             }
+            q = lo;
+            next = q + 1 < nslots ? off(q + 1) : n_new;
+            b = birth_slot<St>(ca, q);
+        }
+        const long long pid = n_census + j;
+        BirthDraws<T> d(ca, step, (uint32_t)pid);
+        if (G == 1) {
+            T xpos, mu;
+            if (b.kind == kBody1D) {
+                // body / source births (src/imc_sourcing.jl:193-236)
+                xpos = b.wx * d.u() * dsT;
+                mu = d.cosine();
+                for (int r1 = 1; r1 < 64 && mu == (T)0; ++r1) mu = d.cosine();
+                if (mu == (T)0) mu = (T)1;
+            } else {
+                // surface births (src/imc_sourcing.jl:161-189)
+                xpos = b.x0;
+                mu = RT<T>::sqrt_(d.u());
+                for (int r1 = 1; r1 < 64 && mu == (T)0; ++r1) mu = RT<T>::sqrt_(d.u());
+                if (mu == (T)0) mu = (T)1;
+                if (b.kind == kRight1D) mu = -mu;
+            }
+            const T st = dtT * d.u();
+            store_birth<St>(1, pb, pid, st, xpos, (T)0, mu, (T)0, b, (float)dtT);
+        } else {
+            T st, xpos, ypos, ang;
+            // the angles are the reference's Float64 products rounded to T
+            // (binary32: pi_n24 or two_pi_u24 of the uniform's integer m,
+            // the same value without FP64)
+            if (b.kind == kBody2D) {
+                // body / source births (src/imc_sourcing.jl:326-366)
+                xpos = b.wx * d.u() * dsT;
+                ypos = b.wy * d.u() * dsT;
+                if constexpr (sizeof(T) == 4) ang = two_pi_u24(d.word() >> 8);
+                else ang = (T)(2.0 * pd * (double)d.u());
+                st = dtT * d.u();
+            } else {
+                // surface births (src/imc_sourcing.jl:265-323)
+                st = dtT * d.u();
+                const bool horizontal = b.kind == kBottom2D || b.kind == kTop2D;
+                const T along = (horizontal ? b.wx : b.wy) * d.u() * dsT;
+                xpos = horizontal ? along : b.x0;
+                ypos = horizontal ? b.y0 : along;
+                if constexpr (sizeof(T) == 4) {
+                    const uint32_t m = d.word() >> 8;
+                    if (b.kind == kBottom2D) ang = (T)pd * ((T)m * 0x1p-24f);
+                    else if (b.kind == kTop2D) ang = -pi_n24((int)m);
+                    else if (b.kind == kLeft2D) ang = pi_n24((1 << 23) - (int)m);
+                    else ang = (T)(pd * (0.5 + (double)((T)m * 0x1p-24f)));
+                } else {
+                    const T u = d.u();
+                    if (b.kind == kBottom2D) ang = (T)((T)pd * u);
+                    else if (b.kind == kTop2D) ang = (T)(-pd * (double)u);
+                    else if (b.kind == kLeft2D) ang = (T)(pd * (0.5 - (double)u));
+                    else ang = (T)(pd * (0.5 + (double)u));
+                }
+            }
+            T ux, uy;
+            if (sizeof(T) == 4) { float s_, c_; sincosf((float)ang, &s_, &c_); ux = (T)c_; uy = (T)s_; }
+            else { double s_, c_; sincos((double)ang, &s_, &c_); ux = (T)c_; uy = (T)s_; }
+            store_birth<St>(2, pb, pid, st, xpos, ypos, ux, uy, b, (float)dtT);
         }
     }
 }
@@ -850,7 +846,7 @@ void launch_source(const CellArgs &ca, Scalars *sc, int prec, PBufPair buf, int 
     auto emit = ca.geometry == 1
                     ? (prec == 0 ? k_source_emit<StF64, 1> : prec == 1 ? k_source_emit<StF32, 1> : k_source_emit<StF16, 1>)
                     : (prec == 0 ? k_source_emit<StF64, 2> : prec == 1 ? k_source_emit<StF32, 2> : k_source_emit<StF16, 2>);
-    emit<<<grid, 256, 0, st>>>(ca, sc, buf);
+    emit<<<grid, kEmitThreads, 0, st>>>(ca, sc, buf);
 }
 
 // ------------------------------------------------------------- compaction
