@@ -511,10 +511,10 @@ __global__ void __launch_bounds__(BLOCK) k_transport1d(CellArgs ca, Scalars *sc,
 
 // One transport launch over the lists of many 1D decks (the fused batch,
 // imc_run_batch_fused), whose arguments sit in constant memory.  Blocks go
-// through the decks in order; a block sets up a deck (its cell table and
-// private tallies) only while the deck's work counter still has chunks, takes
-// chunks from that counter like the single-deck kernel, and flushes the
-// deck's tallies and counters before it moves on.  Every history runs the
+// through the decks in turn, each from its own; a block sets up a deck (its cell
+// table and private tallies) only while the deck's work counter still has
+// chunks, takes chunks from that counter like the single-deck kernel, and
+// flushes the deck's tallies and counters before it moves on.  Every history runs the
 // single-deck code with the deck's own streams and exact tallies, so each
 // deck's result is bit-identical to its own launch's.
 __constant__ Deck1DArgs c_multi_ca[kFusedMaxDecks];
@@ -524,22 +524,65 @@ __constant__ Scalars *c_multi_sc[kFusedMaxDecks];
 template <class St, int BLOCK, bool LONG>
 __global__ void __launch_bounds__(BLOCK) k_transport1d_multi(int ndecks) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int s_go;
-    for (int d = 0; d < ndecks; ++d) {
-        Scalars *sc = c_multi_sc[d];
-        if (threadIdx.x == 0) {
-            // chunks left: 128-entry chunks for short histories, 32-entry in
-            // the refill schedule (a stale, low counter only costs a setup)
-            const long long n = *(volatile long long *)&sc->n_particles;
-            const unsigned long long used = *(volatile unsigned long long *)&sc->work_next;
-            const long long per = LONG ? 32 : kListChunk1D;
-            s_go = long_histories(sc) == LONG && (long long)used * per < n;
+    static_assert(kFusedMaxDecks == 256 && BLOCK >= kFusedMaxDecks, "eight decks a lane, one a thread");
+    __shared__ float s_work[kFusedMaxDecks];
+    __shared__ int s_at;
+    // Each block starts at the deck that lies at its share of the step's
+    // segments (as many of them a history as the last step had), so that a
+    // deck's histories are walked by full blocks; with every block starting at
+    // the first deck, a small deck left each a warp or two and the wait for
+    // their longest history (24 small decks 246 ms against 231, 256 decks 18.4 s
+    // against 16.1; giving a block only the decks that its share meets, and others
+    // while they have four entries a thread: 234 ms, 16.5 s).
+    if (threadIdx.x < kFusedMaxDecks) {
+        float work = 0.0f;
+        if ((int)threadIdx.x < ndecks) {
+            const Scalars *sc = c_multi_sc[threadIdx.x];
+            if (long_histories(sc) == LONG) work = (float)sc->n_particles * fmaxf(sc->seg_per_hist, 1.0f);
+        }
+        s_work[threadIdx.x] = work;
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        float mine = 0.0f;
+        for (int i = 0; i < 8; ++i) mine += s_work[8 * lane + i];
+        float incl = mine;
+        for (int off = 1; off < 32; off <<= 1) {
+            const float o = __shfl_up_sync(0xFFFFFFFFu, incl, off);
+            if (lane >= off) incl += o;
+        }
+        const float share = __shfl_sync(0xFFFFFFFFu, incl, 31) * ((float)blockIdx.x + 0.5f) / (float)gridDim.x;
+        const unsigned before = __ballot_sync(0xFFFFFFFFu, incl <= share);  // lanes that end below it
+        if (lane == min(__popc(before), 31)) {
+            float acc = incl - mine;
+            int d = 8 * lane;
+            while (d < 8 * lane + 7 && acc + s_work[d] <= share) acc += s_work[d++];
+            s_at = min(d, ndecks - 1);
+        }
+    }
+    __syncthreads();
+    int at = s_at;
+    // then each deck once, in turn, that has chunks left
+    for (int visit = 0; visit < ndecks; ++visit) {
+        __syncthreads();
+        if (threadIdx.x == 0) s_at = ndecks;
+        __syncthreads();
+        if ((int)threadIdx.x < ndecks) {
+            const int d = at + (int)threadIdx.x < ndecks ? at + (int)threadIdx.x : at + (int)threadIdx.x - ndecks;
+            if (s_work[d] > 0.0f) {
+                // a stale, low counter only costs a setup
+                const Scalars *sc = c_multi_sc[d];
+                const unsigned long long used = *(volatile const unsigned long long *)&sc->work_next;
+                const long long per = LONG ? 32 : kListChunk1D;
+                if ((long long)used * per < sc->n_particles) atomicMin(&s_at, (int)threadIdx.x);
+            }
         }
         __syncthreads();
-        if (s_go)
-            transport1d_block<St, BLOCK, kTallyShared, kModePlain, LONG>(c_multi_ca[d], sc, c_multi_bufs[d], SurrWave{}, 0,
-                                                                    smem_raw, kListChunk1D);
-        __syncthreads();
+        if (s_at == ndecks) return;
+        at = at + s_at < ndecks ? at + s_at : at + s_at - ndecks;
+        transport1d_block<St, BLOCK, kTallyShared, kModePlain, LONG>(c_multi_ca[at], c_multi_sc[at], c_multi_bufs[at],
+                                                                SurrWave{}, 0, smem_raw, kListChunk1D);
     }
 }
 
