@@ -14,13 +14,15 @@
 //                q = r g(r), g(r) = 1 - r/2 + r^2/6 - ...; for j = 0 y g(y), so
 //                that small results keep their relative accuracy.  From 1 on in
 //                FP64 (Tang, ACM TOMS 15, 1989)
+//   attenuate    E exp(-y), a history's weight after a segment
 //   div_r        a / b with r = RN(1/b) at hand: one residual correction
 //                (Markstein, IBM J. Res. Dev. 34, 1990), a / b correctly rounded
 //   rcp64, Sum128   a reciprocal and the sum of a cell's deposits, in integers
 //   u53, one_minus_2u53   uniforms from their integers without a conversion
 //
 // Largest errors seen (tests/test_math64.py, against extended precision):
-// 0.60 units in the last place for neglog_k53, 1.01 for expm1_neg; div_r
+// 0.60 units in the last place for neglog_k53, 1.01 for expm1_neg; 1.94 units
+// of 2^-53 for attenuate (tests/test_attenuate64.py); div_r
 // equals the IEEE quotient.  CUDA's log, exp and expm1 are good to 1 unit each.
 // Table entries are the nearest integers to the stated expressions, computed
 // with 400-bit arithmetic; the polynomials are the Taylor series.
@@ -510,8 +512,8 @@ IMC_HD double neglog_k53(uint64_t k) {
     return fixed_to_double(v, e ? 58 : 62);
 }
 
-// exp(-y) - 1, y >= 0 (NaN gives NaN), in FP64
-IMC_HD double expm1_neg_fp64(double y) {
+// exp(-y) - 1, y >= 0 (NaN gives NaN), in FP64; *ex: exp(-y) for y <= 64
+IMC_HD double expm1_neg_fp64(double y, double *ex) {
     // 64 and beyond is -1 to the last bit; a NaN passes
     const uint32_t yh = hi32(y);
     if (yh - 0x40500000u <= 0x7FF00000u - 0x40500000u) y = 64.0;
@@ -543,15 +545,18 @@ IMC_HD double expm1_neg_fp64(double y) {
     // times 2^-(n / 64), by the exponents; the low part of row 0 is 0
     const uint64_t sh = (uint64_t)((ni >> 6) & 0x7Fu) << 52;
     const double th = from_bits(bits(th0) - sh), tl = j ? from_bits(bits(tl0) - sh) : 0.0;
-    return (th - 1.0) + fma(th, p, tl);
+    const double low = fma(th, p, tl);
+    *ex = th + low;
+    return (th - 1.0) + low;
 }
 
-// exp(-y) - 1, y >= 0 (NaN gives NaN)
-IMC_HD double expm1_neg(double y) {
+// exp(-y) - 1, y >= 0 (NaN gives NaN); where it is -1/2 or below and y at most
+// 64, *ex is left with exp(-y), to 0.51 units in its last place
+IMC_HD double expm1_neg(double y, double *ex) {
     const uint64_t yb = bits(y);
-    const int ex = (int)(yb >> 52);
-    if (ex >= 1023) return expm1_neg_fp64(y);
-    const int s = 1022 - ex;
+    const int e = (int)(yb >> 52);
+    if (e >= 1023) return expm1_neg_fp64(y, ex);
+    const int s = 1022 - e;
     uint64_t Y = ((yb & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull) << 11;  // y 2^64 once shifted
     Y = s < 64 ? Y >> s : 0ull;
     const int j = (int)(Y >> 58);
@@ -572,7 +577,30 @@ IMC_HD double expm1_neg(double y) {
     const uint64_t D = h_expm_rows[j];
 #endif
     const uint64_t q = mulhi_u(r, g << 2);  // (r g) 2^64; g = 1 only where r < 2^-60
-    return -fixed_to_double(D + q - mulhi_u(D, q), 64);
+    const uint64_t v = D + q - mulhi_u(D, q);
+    if (v >> 63) *ex = fixed_to_double(0ull - v, 64);  // 1 - v 2^-64
+    return -fixed_to_double(v, 64);
+}
+IMC_HD double expm1_neg(double y) {
+    double ex;
+    return expm1_neg(y, &ex);
+}
+
+// E exp(-y), the weight E after a path of y mean free paths of absorption, and
+// *em1 = exp(-y) - 1.  Up to ln 2 the weight is E + E em1.  Beyond, that sum
+// would cancel, an error of em1 growing e^y times in the weight (50 units in
+// the last place at the 1 % cut-off), and the weight is E exp(-y): one
+// fused multiply-add either way.
+IMC_HD double attenuate(double E, double y, double *em1) {
+    if (hi32(y) - 0x40500000u <= 0x7FF00000u - 0x40500000u) {  // 64 to infinity
+        *em1 = -1.0;
+        return E * exp(-y);
+    }
+    double ex = 0.0;
+    const double m = expm1_neg(y, &ex);
+    *em1 = m;
+    const bool thick = bits(ex) != 0;  // left by expm1_neg: never 0 up to 64
+    return fma(E, thick ? ex : m, thick ? 0.0 : E);
 }
 
 // 1 / b: binary32's reciprocal and two Newton steps in 64-bit integers, then

@@ -327,7 +327,9 @@ __device__ __forceinline__ Tab1<T> make_tab1(double sa, double f, double ss, dou
 // tally is finalised, and comparisons on the bits.  2000-cell slab at 2e6
 // histories: 1.24 ms per launch with CUDA's exp, expm1 and log, five divisions
 // and FP64 compares; 0.55 with table-driven FP64 functions and corrected
-// products; 0.35 with the functions in integers.
+// products; 0.35 with the functions in integers.  The weight after the segment
+// is E + E (exp(-y) - 1) while that cancels nothing and E exp(-y) from y = ln 2
+// on (m64::attenuate).
 template <class T> struct SegMath;
 template <> struct SegMath<double> {
     // inf for a zero opacity (rseff inf), as el / 0 is
@@ -342,8 +344,9 @@ template <> struct SegMath<double> {
     // new weight; *em1 = minus the share of it deposited (d < 0, a history past
     // its census time by a rounding, takes the general expm1)
     static __device__ __forceinline__ double attenuate(double E, double saf, double d, bool odd, double *em1) {
-        *em1 = odd ? expm1(-saf * d) : m64::expm1_neg(saf * d);
-        return fma(E, *em1, E);
+        if (!odd) return m64::attenuate(E, saf * d, em1);
+        *em1 = expm1(-saf * d);
+        return E * exp(-saf * d);
     }
 };
 // the least of three, NaN if one is NaN (jmin of jmin; one instruction)
