@@ -590,10 +590,11 @@ IMC_HD double expm1_neg(double y) {
 // *em1 = exp(-y) - 1.  Up to ln 2 the weight is E + E em1.  Beyond, that sum
 // would cancel, an error of em1 growing e^y times in the weight (50 units in
 // the last place at the 1 % cut-off), and the weight is E exp(-y): one
-// fused multiply-add either way.
+// fused multiply-add either way.  A negative y (a path past the census time by a
+// rounding, a negative opacity), 64 and beyond, and NaN take the general functions.
 IMC_HD double attenuate(double E, double y, double *em1) {
-    if (hi32(y) - 0x40500000u <= 0x7FF00000u - 0x40500000u) {  // 64 to infinity
-        *em1 = -1.0;
+    if (hi32(y) >= 0x40500000u) {
+        *em1 = expm1(-y);
         return E * exp(-y);
     }
     double ex = 0.0;

@@ -283,7 +283,7 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
                     return 1;
                 }
             }
-            const T newenergy = M::attenuate(E, ce.saf, dist, odd, &em1);
+            const T newenergy = M::attenuate(E, ce.saf, dist, &em1);
             const bool dead = le64(newenergy, minenergy);
             dep_sum.add(E, em1, dead, b_dep + se, flags);
             if (dead) return 1;
@@ -752,7 +752,7 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
                 if (dist != dist) { flags |= 1u; return 1; }
             }
             double em1;
-            newenergy = SegMath<double>::attenuate(E, ce.saf, dist, odd, &em1);
+            newenergy = SegMath<double>::attenuate(E, ce.saf, dist, &em1);
             dead = le64(newenergy, minenergy);
             dep_sum.add(E, em1, dead, b_dep + se, flags);
         }

@@ -341,12 +341,9 @@ template <> struct SegMath<double> {
     static __device__ __forceinline__ double flight(Stream &rs, const Tab1<double> &ce) {
         return flight(rs, ce.seff, ce.rseff);
     }
-    // new weight; *em1 = minus the share of it deposited (d < 0, a history past
-    // its census time by a rounding, takes the general expm1)
-    static __device__ __forceinline__ double attenuate(double E, double saf, double d, bool odd, double *em1) {
-        if (!odd) return m64::attenuate(E, saf * d, em1);
-        *em1 = expm1(-saf * d);
-        return E * exp(-saf * d);
+    // new weight; *em1 = minus the share of it deposited
+    static __device__ __forceinline__ double attenuate(double E, double saf, double d, double *em1) {
+        return m64::attenuate(E, saf * d, em1);
     }
 };
 // the least of three, NaN if one is NaN (jmin of jmin; one instruction)

@@ -16,7 +16,8 @@ using namespace imc;
 // name, range of y
 struct Range { const char *name; double lo, hi; };
 static const Range kRanges[] = {{"tiny", 1e-12, 1e-3}, {"thin", 1e-3, 0.5}, {"near_half", 0.5, 0.9}, {"near_one", 0.9, 1.1},
-                                {"to_two", 1.0, 2.0}, {"cutoff", 2.0, 4.6051702}, {"deep", 4.6, 64.0}, {"far", 64.0, 700.0}};
+                                {"to_two", 1.0, 2.0}, {"cutoff", 2.0, 4.6051702}, {"deep", 4.6, 64.0}, {"far", 64.0, 700.0},
+                                {"past_census", -1e-6, -1e-16}, {"negative", -4.0, -1e-6}};
 
 __global__ void k_attenuate(int n, const double *E, const double *y, double *w, double *em1) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -46,8 +47,8 @@ int main(int argc, char **argv) {
         cudaMemcpy(gw.data(), d[2], 8 * (size_t)n, cudaMemcpyDeviceToHost);
         cudaMemcpy(ge.data(), d[3], 8 * (size_t)n, cudaMemcpyDeviceToHost);
         long differ = 0;
-        // up to 64 the same integers and FP64 operations on both sides
-        for (int i = 0; i < n; ++i) differ += y[i] < 64.0 && (gw[i] != w[i] || ge[i] != em1[i]);
+        // from 0 up to 64 the same integers and FP64 operations on both sides
+        for (int i = 0; i < n; ++i) differ += y[i] >= 0.0 && y[i] < 64.0 && (gw[i] != w[i] || ge[i] != em1[i]);
         printf("differ %ld\n", differ);
         w = gw;
     }

@@ -6,7 +6,7 @@ weight is below it): where exp(-y) - 1 is above -1/2, its
 error (1.01 units in the last place of at most 1/2) is at most 1.01 of the
 weight, and the sum E + E (exp(-y) - 1) rounds once (1).  Beyond, exp(-y) itself
 is off by 0.51 units in its last place (1.02), and the product rounds once (1).
-From 64 on, CUDA's exp: one unit in the last place (2) and the product (1)."""
+From 64 on and below 0, CUDA's exp: one unit in the last place (2) and the product (1)."""
 import os
 import subprocess
 
@@ -16,11 +16,11 @@ from conftest import REPO
 
 SRC = os.path.join(REPO, "tests", "native", "attenuate_check.cu")
 BIN = os.path.join(REPO, "tests", "native", "_build", "attenuate_check")
-RANGES = ["tiny", "thin", "near_half", "near_one", "to_two", "cutoff", "deep", "far"]
+RANGES = ["tiny", "thin", "near_half", "near_one", "to_two", "cutoff", "deep", "far", "past_census", "negative"]
 
 
 def bound(name):
-    return 3.0 if name == "far" else 2.1
+    return 3.0 if name in ("far", "past_census", "negative") else 2.1
 
 
 @pytest.fixture(scope="module")
