@@ -376,9 +376,13 @@ __device__ __forceinline__ double min64(double a, double b) {
     const uint64_t x = m64::bits(a), y = m64::bits(b);
     return m64::from_bits(x < y ? x : y);
 }
-// v > 0, a <= b and a >= b without the FP64 pipe (a and b not both negative)
+// v > 0 for v not NaN, without the FP64 pipe
 __device__ __forceinline__ bool pos64(double v) { return (long long)m64::bits(v) > 0; }
-__device__ __forceinline__ bool le64(double a, double b) { return (long long)m64::bits(a) <= (long long)m64::bits(b); }
+// a <= b: the bits ordered for two numbers of [+0, inf], else (energies below 0,
+// born where a cell emits them, and NaN) the comparison itself
+__device__ __forceinline__ bool le64(double a, double b) {
+    return plain64(a) && plain64(b) ? m64::bits(a) <= m64::bits(b) : a <= b;
+}
 template <> struct SegMath<float> {
     static __device__ __forceinline__ float flight(uint32_t w, float rseff) {
         const float v = (float)((w >> 8) | 1u) * 0x1p-24f;

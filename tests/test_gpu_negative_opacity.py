@@ -8,8 +8,6 @@ from conftest import load_deck
 
 pytestmark = pytest.mark.gpu
 
-LINE = {"PRECISION": "FLOAT64", "SIGMA_S_VALS": ["1e-12"]}
-
 
 @pytest.mark.parametrize("deck", ["tiny_1d", "tiny_2d"])
 @pytest.mark.parametrize("y", [-1e-6, -0.05, -0.4])
@@ -18,7 +16,7 @@ def test_a_history_gains_energy(deck, y, gpu_lib):
     absorption, no collision on the way: every weight is E exp(-y) to 3 units of
     2^-53 for exp and the product, and the deposits are what the list gained."""
     import mpimc
-    inputs, mesh = load_deck(deck, **LINE)
+    inputs, mesh = load_deck(deck)
     e = mpimc.Engine(inputs, mesh)
     e.update()
     c, dt = float(inputs["PHYS_C"]), e.time()[1]
@@ -46,4 +44,26 @@ def test_a_history_gains_energy(deck, y, gpu_lib):
     width = np.asarray(mesh.dx) if deck == "tiny_1d" else np.outer(mesh.dy, mesh.dx).ravel()
     dep = (e.field("energydep").reshape(-1, nc)[0] * width).sum()
     np.testing.assert_allclose(dep, before - p["E"].sum(), rtol=1e-9)
+    e.close()
+
+
+@pytest.mark.parametrize("deck", ["tiny_1d", "tiny_2d"])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_births_of_negative_energy_end_at_the_cutoff(deck, precision, gpu_lib):
+    """The cells of such a deck emit negative energy.  A negative weight is below
+    its cut-off, 1 % of itself, from the first segment on: those histories end
+    there, as the reference's comparison has it, and none reaches census."""
+    import mpimc
+    inputs, _ = load_deck(deck)
+    n = len(inputs["SIGMA_A_VALS"])
+    inputs, mesh = load_deck(deck, SIGMA_A_VALS=["-1e-3"] * n, SIGMA_A_POWERS=["0.0"] * n, SIGMA_S_VALS=["20.0"])
+    e = mpimc.Engine(inputs, mesh, {"precision": precision})
+    e.update()
+    e.sourcing()
+    born = e.particles()["E"]
+    assert (born < 0).sum() >= 20 and (born > 0).sum() >= 100
+    e.transport()
+    e.clean()
+    left = e.particles()["E"]
+    assert 0 < len(left) < len(born) and (left > 0).all()
     e.close()
