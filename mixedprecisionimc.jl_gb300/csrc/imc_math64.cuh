@@ -668,6 +668,13 @@ struct Sum128 {
         if (ex) man |= 0x10000000000000ull;
         return add(man, (ex ? ex : 1) - 1075 - b, (u >> 63) != 0);
     }
+    // the sum's sign and magnitude; false from 2^94 on, beyond a tally's words
+    IMC_HD bool magnitude(bool &neg, uint64_t &l, uint64_t &h) const {
+        neg = hi < 0;
+        l = neg ? ~lo + 1u : lo;
+        h = neg ? ~(uint64_t)hi + (lo == 0 ? 1u : 0u) : (uint64_t)hi;
+        return (h >> 30) == 0;
+    }
     // x y to 64 bits (both finite), negated
     IMC_HD bool add_minus_product(double x, double y, int b) {
         const uint64_t u = bits(x), v = bits(y);

@@ -161,7 +161,7 @@ __device__ __forceinline__ void transport1d_block(const CA &ca, Scalars *sc, con
                 if (add_f32_smem(slots_k + 24u * (unsigned)cell, v, b_dep + se)) return;
             flush_rest<T, SMT>(dep_acc, k * nc + cell, v, b_dep + se, flags);
         } else {
-            dep_sum.template flush<SMT>(dep_acc, k * nc + cell);
+            dep_sum.template flush<SMT>(dep_acc, k * nc + cell, flags);
         }
     };
     // one pass of the reference's while loop; 0 = go on, 1 = killed, 2 =
@@ -690,7 +690,7 @@ __global__ void __launch_bounds__(BLOCK) k_transport2d(CellArgs ca, Scalars *sc,
                 if (add_f32_smem(slots_k + 24u * (unsigned)cell, v, b_dep + se)) return;
             flush_rest<T, SMT>(dep_acc, k * nc + cell, v, b_dep + se, flags);
         } else {
-            dep_sum.template flush<SMT>(dep_acc, k * nc + cell);
+            dep_sum.template flush<SMT>(dep_acc, k * nc + cell, flags);
         }
     };
     // one pass of the reference's while loop (src/imc_transport.jl:533-717);

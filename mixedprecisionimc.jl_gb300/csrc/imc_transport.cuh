@@ -211,11 +211,14 @@ template <> struct CellSum<double> {
         const bool ok = dead ? v.add(E, b) : v.add_minus_product(E, em1, b);
         if (!ok) flags |= (E != E || em1 != em1) ? 1u /*NAN*/ : (1u << 5) /*FIXPOINT_RANGE*/;
     }
-    template <bool SMT> __device__ __forceinline__ void flush(long long *acc, int slot) const {
+    template <bool SMT> __device__ __forceinline__ void flush(long long *acc, int slot, unsigned &flags) const {
         if ((v.lo | (uint64_t)v.hi) == 0) return;
-        const bool neg = v.hi < 0;
-        const uint64_t l = neg ? ~v.lo + 1u : v.lo;
-        const uint64_t h = neg ? ~(uint64_t)v.hi + (v.lo == 0 ? 1u : 0u) : (uint64_t)v.hi;
+        bool neg;
+        uint64_t l, h;
+        if (!v.magnitude(neg, l, h)) {
+            flags |= 1u << 5;  // FIXPOINT_RANGE
+            return;
+        }
         Limbs A;
         A.l2 = (long long)(l & 0xFFFFFFFFull);
         A.l1 = (long long)(l >> 32);
