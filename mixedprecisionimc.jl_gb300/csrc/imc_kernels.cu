@@ -188,20 +188,6 @@ __device__ __forceinline__ double warp_sum_partials(const double *part, int nb, 
 }
 
 // ------------------------------------------------------------------ update
-// x^p; the small whole powers of opacity laws by products, rounded no more than
-// three times (pow is good to two units), without pow's hundred instructions.
-// pow(x, 0) is 1 for every x, NaN included.
-__device__ __forceinline__ double pow_law(double x, double p) {
-    if (p == 0.0) return 1.0;
-    if (p == 1.0) return x;
-    if (p == 2.0) return x * x;
-    if (p == 3.0) return x * x * x;
-    if (p == -1.0) return 1.0 / x;
-    if (p == -2.0) return 1.0 / (x * x);
-    if (p == -3.0) return 1.0 / (x * x * x);
-    return pow(x, p);
-}
-
 struct CellLaws { double T, f, sa; };
 // Update.update for cell i (src/imc_update.jl:12-56); WRITE: also leaves the
 // fields and the transport's table row
@@ -220,7 +206,7 @@ __device__ __forceinline__ CellLaws update_cell(const CellArgs &ca, double dt, i
         beta = ((4.0 * a) * T3) / ca.bee[i];
     }
     const double Tc = (ca.temp_floor > 0.0 && T < ca.temp_floor) ? ca.temp_floor : T;
-    double sa = ca.sa_val[i] * pow_law(Tc, ca.sa_pow[i]);
+    double sa = ca.sa_val[i] * m64::pow_law(Tc, ca.sa_pow[i]);
     if (ca.marshak) sa = ca.sa_val[i] / Tc / Tc / Tc;
     double v[6] = {ca.ds, ca.alpha, beta, c, dt, sa};
     int j;
@@ -229,7 +215,7 @@ __device__ __forceinline__ CellLaws update_cell(const CellArgs &ca, double dt, i
     u.sa = sa;
     u.f = 1.0 / (1.0 + prod);
     if (WRITE) {
-        const double ss = ca.ss_val[i] * pow_law(Tc, ca.ss_pow[i]);
+        const double ss = ca.ss_val[i] * m64::pow_law(Tc, ca.ss_pow[i]);
         ca.beta[i] = beta;
         ca.sa[i] = sa;
         ca.ss[i] = ss;
