@@ -430,7 +430,15 @@ __global__ void __launch_bounds__(kTrainThreads) k_surr_grad(const float *P, con
     __shared__ float sloss[kSlice];
     const long long s0 = off + (long long)blockIdx.x * kSlice;
     float *g = gpart + (size_t)blockIdx.x * kParams;
-    if (threadIdx.x < kTileThreads) {
+    // the two roles; every barrier is the whole block's
+    const bool tiles = threadIdx.x < kTileThreads;
+    const int j = threadIdx.x - kTileThreads;  // the serial sums' sample and output
+    // this thread's sample of the output gradient
+    const int smp = tiles ? threadIdx.x >> 2 : j;
+    const bool valid = s0 + smp < n;
+    int c = 0;
+    float y0 = 0.0f, y1 = 0.0f, l = 0.0f;
+    if (tiles) {
         static_assert(kHid * kIn == kTileThreads && kSlice * kIn == kTileThreads, "one element a thread");
         const long long i = s0 + threadIdx.x / kIn;
         const float w1 = P[kW1 + threadIdx.x], x1 = i < n ? x[i * kIn + threadIdx.x % kIn] : 0.0f;
@@ -447,43 +455,38 @@ __global__ void __launch_bounds__(kTrainThreads) k_surr_grad(const float *P, con
         fetch(W4, P + kW4);
         W1[threadIdx.x] = w1;
         X[threadIdx.x] = x1;
-        // this thread's sample of the output gradient
-        const int smp = threadIdx.x >> 2;
-        const bool valid = s0 + smp < n;
-        const int c = valid ? cls[s0 + smp] : 0;
-        const float y0 = valid ? tgt[2 * (s0 + smp)] : 0.0f, y1 = valid ? tgt[2 * (s0 + smp) + 1] : 0.0f;
-        __syncthreads();
+        if (valid) { c = cls[s0 + smp]; y0 = tgt[2 * (s0 + smp)]; y1 = tgt[2 * (s0 + smp) + 1]; }
+    } else {
+        if (valid) c = cls[s0 + smp];
+        B[j] = P[kB1 + j]; B[kHid + j] = P[kB2 + j]; B[2 * kHid + j] = P[kB3 + j]; B[3 * kHid + j] = P[kB4 + j];
+    }
+    __syncthreads();
+    if (tiles) {
         dense_fwd<kIn>(W1, kIn, B, X, kIn, A1, true);
         copies_arrived<2>();
-        __syncthreads();
+    }
+    __syncthreads();
+    if (tiles) {
         dense_fwd<kHid>(W2, kLd, B + kHid, A1, kLd, A2, true);
         copies_arrived<1>();
-        __syncthreads();
+    }
+    __syncthreads();
+    if (tiles) {
         dense_fwd<kHid>(W3, kLd, B + 2 * kHid, A2, kLd, A3, true);
         copies_arrived<0>();
-        __syncthreads();
-        dense_fwd<kHid>(W4, kLd, B + 3 * kHid, A3, kLd, O, false);
-        __syncthreads();
+    }
+    __syncthreads();
+    if (tiles) dense_fwd<kHid>(W4, kLd, B + 3 * kHid, A3, kLd, O, false);
+    __syncthreads();
+    if (tiles)
         heads_grad(O + smp * kLd, threadIdx.x & 3, valid, c, y0, y1, SP + smp * kQMax, SG + smp * kQMax, TM + smp * kQMax);
-        __syncthreads();
+    else
+        l = outcome_grad(O + j * kLd, valid, c);
+    __syncthreads();
+    if (tiles) {
         dense_wgrad(O, A3, g + kW4);
         dense_bwd(W4, O, A3, D);  // delta at layer 3 output
-        __syncthreads();
-        dense_wgrad(D, A2, g + kW3);
-        dense_bwd(W3, D, A2, O);  // delta at layer 2 output (reuses O)
-        __syncthreads();
-        dense_wgrad(O, A1, g + kW2);
-        dense_bwd(W2, O, A1, D);  // delta at layer 1 output
-        __syncthreads();
-        input_wgrad(D, X, g + kW1);
     } else {
-        const int j = threadIdx.x - kTileThreads;
-        const bool valid = s0 + j < n;
-        const int c = valid ? cls[s0 + j] : 0;
-        B[j] = P[kB1 + j]; B[kHid + j] = P[kB2 + j]; B[2 * kHid + j] = P[kB3 + j]; B[3 * kHid + j] = P[kB4 + j];
-        for (int i = 0; i < 5; ++i) __syncthreads();  // the four layers
-        float l = outcome_grad(O + j * kLd, valid, c);
-        __syncthreads();
         bias_grad(O, j, g + kB4);
         if (valid) {
             int h0, k0, h1, k1;
@@ -491,7 +494,12 @@ __global__ void __launch_bounds__(kTrainThreads) k_surr_grad(const float *P, con
             for (int k = 0; k < k0 + k1; ++k) l += TM[j * kQMax + k];
         }
         sloss[j] = l;
-        __syncthreads();
+    }
+    __syncthreads();
+    if (tiles) {
+        dense_wgrad(D, A2, g + kW3);
+        dense_bwd(W3, D, A2, O);  // delta at layer 2 output (reuses O)
+    } else {
         bias_grad(D, j, g + kB3);
         if (j == 0) {
             float sum = 0.0f;
@@ -499,11 +507,17 @@ __global__ void __launch_bounds__(kTrainThreads) k_surr_grad(const float *P, con
             for (int s = 0; s < kSlice; ++s) sum += sloss[s];
             lpart[blockIdx.x] = sum;
         }
-        __syncthreads();
-        bias_grad(O, j, g + kB2);
-        __syncthreads();
-        bias_grad(D, j, g + kB1);
     }
+    __syncthreads();
+    if (tiles) {
+        dense_wgrad(O, A1, g + kW2);
+        dense_bwd(W2, O, A1, D);  // delta at layer 1 output
+    } else {
+        bias_grad(O, j, g + kB2);
+    }
+    __syncthreads();
+    if (tiles) input_wgrad(D, X, g + kW1);
+    else bias_grad(D, j, g + kB1);
 }
 
 // scale * sum_b gpart[b][p], in block order (the loads of 64 blocks in flight:
