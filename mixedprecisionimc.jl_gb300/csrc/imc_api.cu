@@ -4,7 +4,7 @@
 // One handle owns one CUDA stream and all device memory of one simulation.
 // Sizes that change from step to step (census length, births) live in device
 // scalars, so the host never needs them to launch: a step is a fixed sequence
-// of launches, captured once per ping-pong parity as a CUDA graph.  The host
+// of launches, captured once as a CUDA graph.  The host
 // keeps an exact mirror of the simulation clock (the timestep arithmetic is
 // deterministic FP64), so it knows how many steps a run has without reading
 // the device.
@@ -58,8 +58,8 @@ struct ImcHandle {
     DevStats *d_stats = nullptr;
     long long stats_cap = 0;
     int block_transport = 256, block_transport_long = 256, grid_emit = 0;
-    TransportGrid grid_full{}, grid_transport{};  // resident blocks on the whole GPU; those of this handle's launches
-    bool side_by_side = false;  // one of several handles running at once (imc_run_batch): smaller grids
+    TransportGrid grid_full{};  // resident transport blocks on the whole GPU
+    bool side_by_side = false;  // one of several handles running at once, for the time of imc_run_batch: smaller grids
     // learned surrogate: device image of the network (ca.surr_image points
     // into it while the surrogate is on) and its kernel's persistent grid
     void *d_surr_image = nullptr;
@@ -67,7 +67,7 @@ struct ImcHandle {
     std::vector<void *> qallocs;
     long long qcap = 0;
     SurrShapes sshape{};
-    cudaGraphExec_t graph = nullptr;  // one step, captured once
+    cudaGraphExec_t graph[2] = {nullptr, nullptr};  // one step, captured once: alone, side by side
     bool timing = false;
     cudaEvent_t ev[2] = {nullptr, nullptr};
     std::vector<cudaEvent_t> ev_pool;
@@ -170,7 +170,8 @@ void free_list(std::vector<void *> &list) {
 }
 
 void drop_graphs(ImcHandle *h) {
-    if (h->graph) { cudaGraphExecDestroy(h->graph); h->graph = nullptr; }
+    for (cudaGraphExec_t &g : h->graph)
+        if (g) { cudaGraphExecDestroy(g); g = nullptr; }
 }
 
 // Transport blocks for this handle: the resident grid of the whole GPU, or
@@ -182,11 +183,6 @@ int sized_grid(const ImcHandle *h, int full, int block) {
     const long long per = h->side_by_side ? 16 : 1;
     const long long want = (h->capacity + per * block - 1) / (per * block);
     return (int)std::max<long long>(1, std::min<long long>(full, want));
-}
-
-void size_grids(ImcHandle *h) {
-    h->grid_transport.grid = sized_grid(h, h->grid_full.grid, h->block_transport);
-    h->grid_transport.grid_long = sized_grid(h, h->grid_full.grid_long, h->block_transport_long);
 }
 
 PBufPair pair(const ImcHandle *h) {
@@ -279,19 +275,10 @@ int grow(ImcHandle *h, long long need) {
     sc.cur = 0;
     CK(h, hcopy(h, h->d_sc, &sc, sizeof(Scalars), cudaMemcpyHostToDevice));
     h->ca.capacity = ncap;
-    size_grids(h);
     if ((rc = tile_alloc(h))) return rc;
     if (h->ca.surr_image && (rc = surr_queue_alloc(h))) return rc;
     drop_graphs(h);
     return IMC_OK;
-}
-
-// the handle's launch shapes for a run of its own or one among others
-void set_side_by_side(ImcHandle *h, bool on) {
-    if (h->side_by_side == on) return;
-    h->side_by_side = on;
-    size_grids(h);
-    drop_graphs(h);
 }
 
 int read_scalars(ImcHandle *h, Scalars *sc) {
@@ -352,8 +339,12 @@ void run_transport(ImcHandle *h, PBufPair bufs, cudaStream_t st) {
         sh.analog_grid.grid_long = sized_grid(h, sh.analog_grid.grid_long, sh.analog_block_long);
         sh.query_grid = sized_grid(h, sh.query_grid, sh.query_block);
         launch_transport_surr(h->ca, h->d_sc, h->prec, bufs, h->wave, sh, st);
+    } else {
+        TransportGrid g;
+        g.grid = sized_grid(h, h->grid_full.grid, h->block_transport);
+        g.grid_long = sized_grid(h, h->grid_full.grid_long, h->block_transport_long);
+        launch_transport(h->ca, h->d_sc, h->prec, bufs, g, st);
     }
-    else launch_transport(h->ca, h->d_sc, h->prec, bufs, h->grid_transport, st);
 }
 
 // The kernel sequence of one step, asynchronous on `st`; the list's buffer is
@@ -445,7 +436,8 @@ cudaError_t raise_smem_limit(const void *kp, int smem) {
 }
 
 int capture(ImcHandle *h) {
-    if (h->graph) return IMC_OK;
+    cudaGraphExec_t &exec = h->graph[h->side_by_side];
+    if (exec) return IMC_OK;
     std::lock_guard<std::mutex> lock(g_capture_mutex);
     cudaGraph_t g;
     CK(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
@@ -453,7 +445,7 @@ int capture(ImcHandle *h) {
     cudaError_t e = cudaStreamEndCapture(h->stream, &g);
     if (rc) return rc;
     if (e != cudaSuccess) return fail(h, IMC_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
-    e = cudaGraphInstantiate(&h->graph, g, 0);
+    e = cudaGraphInstantiate(&exec, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return fail(h, IMC_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
     return IMC_OK;
@@ -849,7 +841,6 @@ int imc_create(const ImcDeck *d, ImcHandle **out) {
         (v ? h->grid_full.grid_long : h->grid_full.grid) = h->sm_count * per_sm;
     }
     ca.surr_min_calls = 2ll * h->sm_count * 1024;  // two queries per thread of the GPU
-    size_grids(h);
     h->grid_emit = h->sm_count * 8;
     if (cudaEventCreate(&h->ev[0]) != cudaSuccess || cudaEventCreate(&h->ev[1]) != cudaSuccess)
         return bail(fail(h, IMC_ERR_CUDA, "cudaEventCreate"));
@@ -975,7 +966,6 @@ int imc_timestep(ImcHandle *h, int *done) {
 int imc_step(ImcHandle *h, ImcStepStats *stats, int *done) {
     if (!h) return IMC_ERR_INVALID_ARG;
     if (h->finished) { if (done) *done = 1; return IMC_OK; }
-    set_side_by_side(h, false);
     Scalars sc;
     int rc;
     if (h->n_known < 0) {
@@ -990,7 +980,7 @@ int imc_step(ImcHandle *h, ImcStepStats *stats, int *done) {
         if ((rc = enqueue_step(h, true, 0))) return rc;
     } else {
         if ((rc = capture(h))) return rc;
-        CK(h, cudaGraphLaunch(h->graph, h->stream));
+        CK(h, cudaGraphLaunch(h->graph[h->side_by_side], h->stream));
     }
     DevStats ds;
     if (h->mirror) {
@@ -1064,7 +1054,7 @@ static int run_steps(ImcHandle *h, int64_t max_steps, ImcStepStats *stats, int64
                 if ((rc = enqueue_step(h, true, (int)s))) return rc;
         } else {
             if ((rc = capture(h))) return rc;
-            for (int64_t s = 0; s < m; ++s) CK(h, cudaGraphLaunch(h->graph, h->stream));
+            for (int64_t s = 0; s < m; ++s) CK(h, cudaGraphLaunch(h->graph[h->side_by_side], h->stream));
         }
         done_steps += m;
         if ((rc = read_scalars(h, &sc))) return rc;
@@ -1087,7 +1077,6 @@ static int run_steps(ImcHandle *h, int64_t max_steps, ImcStepStats *stats, int64
 
 int imc_run(ImcHandle *h, int64_t max_steps, ImcStepStats *stats, int64_t *n_steps, double *device_ms) {
     if (!h) return IMC_ERR_INVALID_ARG;
-    set_side_by_side(h, false);
     return run_steps(h, max_steps, stats, n_steps, device_ms);
 }
 
@@ -1110,9 +1099,10 @@ int imc_run_batch(ImcHandle *const *hs, int32_t n, int64_t max_steps, int32_t n_
             if (i >= n) return;
             ImcHandle *h = hs[i];
             int64_t st = 0;
-            set_side_by_side(h, nt > 1);
+            h->side_by_side = nt > 1;
             int rc = cudaSetDevice(h->device) == cudaSuccess ? run_steps(h, max_steps, nullptr, &st, nullptr)
                                                              : fail(h, IMC_ERR_CUDA, "cudaSetDevice");
+            h->side_by_side = false;
             if (steps) steps[i] = st;
             if (rc != IMC_OK) {
                 int expect = IMC_OK;
