@@ -12,6 +12,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <memory>
 #include <mutex>
 #include <thread>
 #include <chrono>
@@ -81,7 +82,7 @@ struct ImcHandle {
     int64_t tot_segments = 0, tot_histories = 0, tot_calls = 0;
     int stage = Stage::Fresh;
     long long n_known = -1;   // the list's length, while no call has changed it since it was read
-    StepMirror *mirror = nullptr;  // pinned; from the first imc_step on
+    std::unique_ptr<StepMirror> mirror;  // null where the GPU cannot write to the host's memory
     ImcStepStats last{};
     std::string err;
     int err_code = IMC_OK;
@@ -388,24 +389,6 @@ int collect_events(ImcHandle *h, size_t pairs) {
         h->transport_launches += 1;
     }
     return IMC_OK;
-}
-
-// the pinned block of a handle that is stepped (without one, the copies serve)
-void ensure_mirror(ImcHandle *h) {
-    if (h->mirror) return;
-    void *p = nullptr, *d = nullptr;
-    if (cudaHostAlloc(&p, sizeof(StepMirror), cudaHostAllocMapped) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return;
-    }
-    if (cudaHostGetDevicePointer(&d, p, 0) != cudaSuccess) {
-        (void)cudaGetLastError();
-        cudaFreeHost(p);
-        return;
-    }
-    h->mirror = static_cast<StepMirror *>(p);
-    h->ca.mirror = static_cast<StepMirror *>(d);
-    drop_graphs(h);
 }
 
 int ensure_stats(ImcHandle *h, long long n) {
@@ -797,6 +780,19 @@ int imc_create(const ImcDeck *d, ImcHandle **out) {
     ca.seg_cap = d->segment_cap > 0 ? d->segment_cap : 10000000;
     ca.seed = d->seed;
     ca.rk.set(d->seed);
+    {
+        // memory of the host's own, coherent over NVLink-C2C: nothing to allocate
+        // or register with the driver, and no step graph to capture again
+        int coherent = 0;
+        if (cudaDeviceGetAttribute(&coherent, cudaDevAttrPageableMemoryAccessUsesHostPageTables, h->device) != cudaSuccess) {
+            (void)cudaGetLastError();
+            coherent = 0;
+        }
+        if (coherent) {
+            h->mirror.reset(new StepMirror());
+            ca.mirror = h->mirror.get();
+        }
+    }
     double dxmin = *std::min_element(d->dx, d->dx + h->nx);
     double dymin = d->geometry == IMC_GEOM_2D ? *std::min_element(d->dy, d->dy + h->ny) : 1.0;
     ca.vol_min = h->prec == IMC_FP64 ? 1.0 : dxmin * dymin;  // least divisor of a deposit (FP64: energies)
@@ -855,7 +851,6 @@ int imc_destroy(ImcHandle *h) {
     for (auto e : h->ev_pool) cudaEventDestroy(e);
     for (int i = 0; i < 2; ++i) if (h->ev[i]) cudaEventDestroy(h->ev[i]);
     if (h->d_stats) cudaFree(h->d_stats);
-    if (h->mirror) cudaFreeHost(h->mirror);
     if (h->d_surr_image) cudaFree(h->d_surr_image);
     free_list(h->qallocs);
     free_list(h->pallocs);
@@ -973,7 +968,6 @@ int imc_step(ImcHandle *h, ImcStepStats *stats, int *done) {
         h->n_known = sc.n_particles;
     }
     if ((rc = grow(h, h->n_known + births_bound(h, h->n_known)))) return rc;
-    ensure_mirror(h);
     h->n_known = -1;
     if (h->timing) {
         if ((rc = ensure_events(h, 1))) return rc;
@@ -1310,13 +1304,7 @@ int imc_get_field(const ImcHandle *h, int field, double *out, int64_t count) {
     double *p = field_ptr(h, field, &n);
     if (!p) return fail(hh, IMC_ERR_INVALID_ARG, "unknown field");
     if (n != count) return fail(hh, IMC_ERR_INVALID_ARG, "field size mismatch");
-    const size_t bytes = sizeof(double) * (size_t)n;
-    if (h->mirror && bytes <= sizeof(h->mirror->stage)) {
-        CK(hh, hcopy(hh, h->mirror->stage, p, bytes, cudaMemcpyDeviceToHost));
-        std::memcpy(out, h->mirror->stage, bytes);
-        return IMC_OK;
-    }
-    CK(hh, hcopy(hh, out, p, bytes, cudaMemcpyDeviceToHost));
+    CK(hh, hcopy(hh, out, p, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost));
     return IMC_OK;
 }
 

@@ -111,7 +111,7 @@ struct CellArgs {
     // (imc_surrogate.cuh), or null for analog transport everywhere
     const uint4 *surr_image;
     long long surr_min_calls;          // queries a step needs to keep the network on (surr_gate)
-    struct StepMirror *mirror;         // device address of the handle's mirror, or null
+    struct StepMirror *mirror;         // the handle's mirror in host memory, or null
 };
 
 // type-erased particle buffer
@@ -134,13 +134,12 @@ struct DevStats {
     unsigned int error_flags, step_index;
 };
 
-// What a program that steps reads after every step, in pinned host memory that
-// the step's last kernel writes: no copy to wait for.  The rest of the block
-// stages the reads of small fields.
+// What a program that steps reads after every step, in host memory that the
+// step's last kernel writes: no copy to wait for (a step of the Su-Olson deck
+// 64 us, 80 with the copies).
 struct StepMirror {
     DevStats last;
     long long n_particles;
-    unsigned char stage[1 << 16];
 };
 
 // launchers (imc_kernels.cu / imc_transport.cu); all asynchronous on `st`
