@@ -339,7 +339,8 @@ template <> struct SegMath<double> {
     static __device__ __forceinline__ double flight(Stream &rs, double seff, double rseff) {
         const double el = Rand<double>::exp1(rs), q = el * rseff;
         const double d = fma(fma(-q, seff, el), rseff, q);
-        return m64::hi32(rseff) < 0x7FE00000u ? d : el / seff;
+        // opacities of zero, infinity, beyond 2^1022 or below 0: the division
+        return m64::hi32(rseff) - 0x00100000u < 0x7FE00000u - 0x00100000u ? d : el / seff;
     }
     static __device__ __forceinline__ double flight(Stream &rs, const Tab1<double> &ce) {
         return flight(rs, ce.seff, ce.rseff);
