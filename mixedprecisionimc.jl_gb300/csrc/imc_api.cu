@@ -357,7 +357,7 @@ void enqueue_before_transport(ImcHandle *h, cudaStream_t st) {
     launch_source(h->ca, h->d_sc, h->prec, pair(h), h->grid_emit, true, st);
 }
 void enqueue_after_transport(ImcHandle *h, cudaStream_t st) {
-    launch_compact(h->ca, h->d_sc, h->prec, pair(h), h->tile_cnt, h->tile_off, h->ntiles_cap, false, st);
+    launch_compact(h->ca, h->d_sc, h->prec, pair(h), h->tile_cnt, h->tile_off, h->ntiles_cap, h->sm_count, false, st);
     launch_tally_check_timestep(h->ca, h->d_sc, h->d_stats, h->stats_cap, st);
 }
 
@@ -912,7 +912,7 @@ int imc_clean(ImcHandle *h) {
     if (!h) return IMC_ERR_INVALID_ARG;
     // Clean.clean removes every killed particle (forced compaction)
     h->n_known = -1;
-    launch_compact(h->ca, h->d_sc, h->prec, pair(h), h->tile_cnt, h->tile_off, h->ntiles_cap, true, h->stream);
+    launch_compact(h->ca, h->d_sc, h->prec, pair(h), h->tile_cnt, h->tile_off, h->ntiles_cap, h->sm_count, true, h->stream);
     CKL(h);
     CK(h, cudaStreamSynchronize(h->stream));
     h->stage = Stage::Cleaned;

@@ -23,9 +23,11 @@
 
 namespace imc {
 
-// query rounds per step of the surrogate transport (launch_transport_surr)
-constexpr unsigned kSurrProbe = 32;  // steps between re-openings of the surrogate gate (k_energycheck)
-constexpr int kSurrRounds = 1;  // measured best on GB300 (thick slab: 1 round 84 ms, 3 rounds 104 ms, 6 rounds 134 ms)
+constexpr unsigned kSurrProbe = 32;  // steps between re-openings of the surrogate gate (energycheck_done)
+// query rounds per step of the surrogate transport (launch_transport_surr):
+// one is fastest (200,000 histories a step of the heated thick cells, 21 steps: 41
+// ms, with three rounds 57, with six 76)
+constexpr int kSurrRounds = 1;
 
 // scalars that live in device memory so a whole step can replay as a graph
 struct Scalars {
@@ -57,7 +59,9 @@ struct Scalars {
     int compact_now;                   // this step compacts the list
     int surr_gate;                     // learned surrogate: this step may set histories aside
     long long surr_closed_h;           // histories of the step that last closed the gate
-    unsigned int tally_blocks_done;    // fused tally + energy check: blocks finished (the last one checks)
+    unsigned int tally_blocks_done;    // blocks finished, of whichever kernel is running whose last block
+                                       // goes on alone (source slots, birth counts, compaction counts,
+                                       // tally); 0 between launches
 };
 
 struct CellArgs {
@@ -103,7 +107,9 @@ struct CellArgs {
     double vol_min, scale_min;
     double t_end, dtmax, kfac;
     // the transport's per-cell table (imc_transport.cuh: Tab1 rows, or Tab2
-    // rows and, FP64 in 2D, 1/seff), written by k_update
+    // rows and, FP64 in 2D, 1/seff), written with the update of the cells: in
+    // a step by k_source_slots, by stages by k_update and, before a transport
+    // of fields that the caller may have set, k_table
     int prec;
     void *tab;
     double *tab_rs;
@@ -163,7 +169,8 @@ struct TransportGrid {
 TransportShape transport_shape(const CellArgs &ca, int prec);
 void launch_transport(const CellArgs &ca, Scalars *sc, int prec, PBufPair bufs, TransportGrid grid, cudaStream_t st);
 // 1D transport with the learned surrogate in thick cells (ca.surr_image set;
-// FP32 or FP16 state), as 1 + 2 kSurrRounds kernels per step: an analog pass
+// FP32 or FP16 state), as 2 + 3 kSurrRounds kernels per step (an analog pass is
+// a short- and a long-history kernel): an analog pass
 // over the list that sets aside the histories that want a network query,
 // then rounds of (query pass, analog pass over the continuing histories).
 // histories set aside between passes (FP32 state)
@@ -201,11 +208,12 @@ void launch_surr_image(const float *params, void *dst, cudaStream_t st);
 // compacted only when the holes exceed 1/16 of its length (kDeferHoles);
 // otherwise the holes stay and only the live count is updated.
 constexpr long long kDeferHoles = 16;
+// sms: the device's SMs
 void launch_compact(const CellArgs &ca, Scalars *sc, int prec, PBufPair bufs, long long *tile_cnt,
-                    long long *tile_off, long long ntiles_cap, bool force, cudaStream_t st);
+                    long long *tile_off, long long ntiles_cap, int sms, bool force, cudaStream_t st);
 // forced compaction of `src` into `dst` (the list must be in src: Scalars::cur == 0)
 void launch_compact(const CellArgs &ca, Scalars *sc, int prec, PBufRaw src, PBufRaw dst, long long *tile_cnt,
-                    long long *tile_off, long long ntiles_cap, cudaStream_t st);
+                    long long *tile_off, long long ntiles_cap, int sms, cudaStream_t st);
 void launch_finalize(const CellArgs &ca, Scalars *sc, cudaStream_t st);
 void launch_tally(const CellArgs &ca, Scalars *sc, cudaStream_t st);
 void launch_energycheck(const CellArgs &ca, Scalars *sc, DevStats *stats, long long stats_cap, cudaStream_t st);

@@ -844,7 +844,7 @@ void launch_source(const CellArgs &ca, Scalars *sc, int prec, PBufPair buf, int 
 // block decides alike; a step that does not compact leaves at once.  The blocks
 // stride over the tiles: one per tile of the buffer's capacity, the launches
 // cost 5 us each on the 2000-cell slab's 5900 tiles with nothing to do.
-constexpr int kCompactGrid = 152 * 8;
+constexpr int kCompactBlocksPerSM = 8;
 __global__ void __launch_bounds__(kCompactThreads) k_compact_count(Scalars *sc, PBufPair bufs, long long *tile_cnt,
                                                                    long long *tile_off, long long *n_before, int force) {
     constexpr int W = kCompactThreads / 32;
@@ -1002,10 +1002,11 @@ __global__ void __launch_bounds__(kCompactThreads) k_compact_scatter(int geometr
 }
 
 void launch_compact(const CellArgs &ca, Scalars *sc, int prec, PBufPair bufs, long long *tile_cnt,
-                    long long *tile_off, long long ntiles_cap, bool force, cudaStream_t st) {
+                    long long *tile_off, long long ntiles_cap, int sms, bool force, cudaStream_t st) {
     // tile_off has ntiles_cap + 1 entries; the last holds the pre-compaction length
     long long *n_before = tile_off + ntiles_cap;
-    const unsigned grid = (unsigned)(ntiles_cap < kCompactGrid ? ntiles_cap : kCompactGrid);
+    const long long most = (long long)sms * kCompactBlocksPerSM;
+    const unsigned grid = (unsigned)(ntiles_cap < most ? ntiles_cap : most);
     k_compact_count<<<grid, kCompactThreads, 0, st>>>(sc, bufs, tile_cnt, tile_off, n_before, force ? 1 : 0);
     if (prec == 0)
         k_compact_scatter<StF64><<<grid, kCompactThreads, 0, st>>>(ca.geometry, sc, tile_off, bufs, n_before);
@@ -1016,11 +1017,11 @@ void launch_compact(const CellArgs &ca, Scalars *sc, int prec, PBufPair bufs, lo
 }
 
 void launch_compact(const CellArgs &ca, Scalars *sc, int prec, PBufRaw src, PBufRaw dst, long long *tile_cnt,
-                    long long *tile_off, long long ntiles_cap, cudaStream_t st) {
+                    long long *tile_off, long long ntiles_cap, int sms, cudaStream_t st) {
     PBufPair p;
     p.b[0] = src;
     p.b[1] = dst;
-    launch_compact(ca, sc, prec, p, tile_cnt, tile_off, ntiles_cap, true, st);
+    launch_compact(ca, sc, prec, p, tile_cnt, tile_off, ntiles_cap, sms, true, st);
 }
 
 // ------------------------------------------------------------------- tally
@@ -1226,7 +1227,6 @@ __device__ void energycheck_done(const CellArgs &ca, Scalars *sc, DevStats *stat
 
 // EnergyCheck.energychecker as its own launch: one warp per partial-sum
 // group (K deposition scales, then the radiation energy).
-template <bool STEP>
 __global__ void __launch_bounds__(544) k_energycheck(CellArgs ca, Scalars *sc, DevStats *stats, long long stats_cap) {
     __shared__ double g[17];
     const int warp = threadIdx.x >> 5, np = ca.K + 1;
@@ -1235,7 +1235,7 @@ __global__ void __launch_bounds__(544) k_energycheck(CellArgs ca, Scalars *sc, D
         if ((threadIdx.x & 31) == 0) g[warp] = v;
     }
     __syncthreads();
-    if (threadIdx.x == 0) energycheck_done(ca, sc, stats, stats_cap, g, STEP);
+    if (threadIdx.x == 0) energycheck_done(ca, sc, stats, stats_cap, g, false);
 }
 
 // Finalize + tally per cell, then, in the block that finishes last, the
@@ -1246,7 +1246,7 @@ __global__ void __launch_bounds__(544) k_energycheck(CellArgs ca, Scalars *sc, D
 // partial sums before taking a ticket, and the last block's warps sum a group
 // each over every unit of cells.  (FP64 latency bounds it, an FP64
 // instruction taking as long as 64 in FP32: 2000 cells 24 us with double-double
-// trees, pow and divisions by the scales, one warp a block, against 12.)
+// trees, pow and divisions by the scales, one warp a block, against 14 to 15.)
 constexpr int kTailThreads = 128;
 __global__ void __launch_bounds__(kTailThreads) k_tally_check(CellArgs ca, Scalars *sc, DevStats *stats,
                                                              long long stats_cap) {
@@ -1282,7 +1282,7 @@ __global__ void k_timestep(CellArgs ca, Scalars *sc) { advance_clock(ca, sc); }
 void launch_timestep(const CellArgs &ca, Scalars *sc, cudaStream_t st) { k_timestep<<<1, 1, 0, st>>>(ca, sc); }
 
 void launch_energycheck(const CellArgs &ca, Scalars *sc, DevStats *stats, long long stats_cap, cudaStream_t st) {
-    k_energycheck<false><<<1, 32 * (ca.K + 1), 0, st>>>(ca, sc, stats, stats_cap);
+    k_energycheck<<<1, 32 * (ca.K + 1), 0, st>>>(ca, sc, stats, stats_cap);
 }
 
 void launch_tally_check_timestep(const CellArgs &ca, Scalars *sc, DevStats *stats, long long stats_cap,

@@ -15,8 +15,8 @@
 //                that small results keep their relative accuracy.  From 1 on in
 //                FP64 (Tang, ACM TOMS 15, 1989)
 //   attenuate    E exp(-y), a history's weight after a segment
-//   div_r        a / b with r = RN(1/b) at hand: one residual correction
-//                (Markstein, IBM J. Res. Dev. 34, 1990), a / b correctly rounded
+//   div_r        a / b with r = 1/b at hand: one residual correction
+//                (Markstein, IBM J. Res. Dev. 34, 1990)
 //   pow_law      x^p of the opacity laws
 //   rcp64, Sum128   a reciprocal and the sum of a cell's deposits, in integers
 //   u53, one_minus_2u53   uniforms from their integers without a conversion
@@ -24,7 +24,7 @@
 // Largest errors seen (tests/test_math64.py, against extended precision):
 // 0.60 units in the last place for neglog_k53, 1.01 for expm1_neg; 1.94 units
 // of 2^-53 for attenuate (tests/test_attenuate64.py); div_r
-// equals the IEEE quotient.  CUDA's log, exp and expm1 are good to 1 unit each.
+// equals the IEEE quotient wherever it was compared.  CUDA's log, exp and expm1 are good to 1 unit each.
 // Table entries are the nearest integers to the stated expressions, computed
 // with 400-bit arithmetic; the polynomials are the Taylor series.
 #pragma once
@@ -527,7 +527,7 @@ IMC_HD double expm1_neg_fp64(double y, double *ex) {
 #endif
     const double n = big - 0x1.8p52;
     const uint32_t ni = (uint32_t)bits(big);
-    double r = fma(-n, kStepHi, y);  // n kStepHi is exact (n < 2^13)
+    double r = fma(-n, kStepHi, y);  // exact: y >= 1 and kStepHi are multiples of 2^-52, r is below 2^-6
     r = fma(-n, kStepLo, r);
     const double r2 = r * r;
     double q = fma(r, -1.0 / 5040.0, 1.0 / 720.0);
@@ -717,7 +717,12 @@ IMC_HD double pow_law(double x, double p) {
     return pow(x, p);
 }
 
-// a / b, rb = RN(1 / b): correctly rounded while nothing under- or overflows
+// a / b while nothing under- or overflows.  For rb = RN(1 / b) it is correctly
+// rounded (Markstein).  rcp64's rb may be RN(1 / b)'s neighbour where 1 / b lies
+// within 1/32 of a unit of a tie; the sum that is rounded here is then off by
+// less than 2^-52 units in the last place, and the quotient its neighbour only
+// where a / b is that close to a tie itself (none found in 4e6 draws, most of them
+// next to one: tests/test_div64.py).
 IMC_HD double div_r(double a, double b, double rb) {
     const double q = a * rb;
     return fma(fma(-q, b, a), rb, q);

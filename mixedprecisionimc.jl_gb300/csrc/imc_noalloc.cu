@@ -111,8 +111,9 @@ extern "C" int imc_clean_noalloc(int precision, int geometry, const ImcDevicePar
     for (int i = 0; i < ns; ++i)
         for (int j = 0; j < nd; ++j)
             if (overlap(fs[i], fd[j], n)) return IMC_ERR_INVALID_ARG;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices)
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return IMC_ERR_NO_DEVICE;
     unsigned char *base;
     {
@@ -138,7 +139,7 @@ extern "C" int imc_clean_noalloc(int precision, int geometry, const ImcDevicePar
     PBufRaw d{dst->t, dst->x, dst->y, dst->ux, dst->uy, dst->E, dst->E0, dst->cs, dst->alive};
     CellArgs ca{};
     ca.geometry = geometry;
-    launch_compact(ca, sc, precision, s, d, tile_cnt, tile_off, ntiles, st);
+    launch_compact(ca, sc, precision, s, d, tile_cnt, tile_off, ntiles, sms, st);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return IMC_ERR_CUDA;
     long long kept = 0;

@@ -137,9 +137,9 @@ __device__ void draw_state(Stream &rs, float *d_n, float *d_f, float *mu, float 
 // their warp: 2^18 walks 12.3 ms).  Every sample has its own stream, so who walks it
 // changes nothing.
 constexpr int kDatagenThreads = 256;
-// samples a lane walks before the grid grows past one block an SM: fewer leave
-// the lanes idle behind the longest walks (3: 9.2 ms for 2^18 walks), more leave
-// SMs short of warps (12: 11.2 ms); 8.4 ms
+// samples a lane walks on average until the grid has its four blocks an SM (2^18
+// walks: 171 blocks): fewer leave the lanes idle behind the longest walks (3: 9.2
+// ms for 2^18 walks), more leave SMs short of warps (12: 11.2 ms); 8.4 ms
 constexpr int kDatagenPerLane = 6;
 __global__ void __launch_bounds__(kDatagenThreads, 4) k_surr_datagen(unsigned long long seed, long long n,
                                                                      const float *state_in, float *x, int *cls,
@@ -297,10 +297,12 @@ __device__ __forceinline__ float outcome_grad(float *O, bool valid, int c) {
 // The three products of a layer, each thread a 4 x 4 tile of the result in
 // registers: two shared float4 loads feed 32 multiplies and adds, where one
 // result per thread and step loaded two floats for one of each.  Every sum runs
-// over its index in order, one product at a time.  (FP32 issue bounds them:
-// 256 threads x 16 sums x 64 products x 2 instructions are 4096 cycles a
-// product on an SM; they take 5200 to 5800
-// whatever the mapping, prefetch or layout tried.)
+// over its index in order, one product at a time, a multiply and an add each, as
+// the library is built without contraction.  (FP32 issue bounds them: 256 threads x
+// 16 sums x 64 products x 2 instructions are 4096 cycles a product on an SM; they
+// take 5200 to 5800 whatever the mapping, prefetch or layout tried.  The
+// histories need the separate roundings, these sums do not: fused they would be
+// 2048 cycles, with parameters that differ in rounding; not tried.)
 __device__ __forceinline__ float lane4(const float4 &v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
 
 // z[s][j] = b[j] + sum_k W[j][k] a[s][k], the 64 x 64 outputs of a layer:

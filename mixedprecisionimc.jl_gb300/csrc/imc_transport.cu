@@ -13,9 +13,10 @@
 // A persistent grid, no larger than the list has warps' worth of entries,
 // walks the particle list in chunks of consecutive entries that warps take from
 // a counter, so every warp loads 32 consecutive particles (coalesced
-// structure-of-arrays loads) and the blocks run out of work together; a history stays in registers: each particle's state is read
-// once and written once per step.  The per-cell transport table (sigma_a*f,
-// effective scatter, face widths) is built in shared memory by every block.
+// structure-of-arrays loads) and the blocks run out of work together; a history
+// stays in registers: each particle's state is read once and written once per
+// step.  Every block copies the step's per-cell transport table (sigma_a f,
+// effective scatter opacity, its reciprocal, widths) to shared memory.
 //
 // Tallies: a history accumulates its deposits for the cell it is in as a
 // Neumaier-compensated pair (FP32) or a 128-bit fixed-point sum (FP64), and

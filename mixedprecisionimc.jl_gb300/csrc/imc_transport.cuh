@@ -296,7 +296,7 @@ template <> struct Tab1<double> { double saf, seff, rseff, dxs; };
 template <> struct Tab1<float> { float saf, seff, dxs, dxT, rseff, rdxT, pad0, pad1; };
 static_assert(sizeof(Tab1<double>) == 32 && sizeof(Tab1<float>) == 32, "32-byte table rows");
 
-// The rows are written once per step by k_update (store_tab) and copied to
+// The rows are written once per step with the cells' update (store_tab) and copied to
 // shared memory by every transport block (load_tab): built by each block,
 // they cost every SM the FP64 conversions and divisions of all cells.
 template <class T>
