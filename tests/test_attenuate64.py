@@ -6,7 +6,7 @@ weight is below it): where exp(-y) - 1 is above -1/2, its
 error (1.01 units in the last place of at most 1/2) is at most 1.01 of the
 weight, and the sum E + E (exp(-y) - 1) rounds once (1).  Beyond, exp(-y) itself
 is off by 0.51 units in its last place (1.02), and the product rounds once (1).
-From 64 on and below 0, CUDA's exp: one unit in the last place (2) and the product (1)."""
+From 600 on and below 0, CUDA's exp: one unit in the last place (2) and the product (1)."""
 import os
 import subprocess
 
