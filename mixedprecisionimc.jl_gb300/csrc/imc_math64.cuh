@@ -22,7 +22,7 @@
 //   u53, one_minus_2u53   uniforms from their integers without a conversion
 //
 // Largest errors seen (tests/test_math64.py, against extended precision):
-// 0.60 units in the last place for neglog_k53, 1.01 for expm1_neg; 1.94 units
+// 0.60 units in the last place for neglog_k53, 0.99 for expm1_neg; 1.94 units
 // of 2^-53 for attenuate (tests/test_attenuate64.py); div_r
 // equals the IEEE quotient wherever it was compared.  CUDA's log, exp and expm1 are good to 1 unit each.
 // Table entries are the nearest integers to the stated expressions, computed
@@ -513,7 +513,7 @@ IMC_HD double neglog_k53(uint64_t k) {
     return fixed_to_double(v, e ? 58 : 62);
 }
 
-// exp(-y) - 1 and *ex = exp(-y) for 1 <= y <= 600 (NaN gives NaN), in FP64
+// exp(-y) - 1 and *ex = exp(-y), 1 <= y <= 760, in FP64
 IMC_HD double expm1_neg_fp64(double y, double *ex) {
     // n = floor(64 y / ln 2): the remainder r >= 0 keeps 2^(-n/64) - 1 and
     // exp(-r) - 1 of one sign, so their sum cancels nothing
@@ -540,12 +540,15 @@ IMC_HD double expm1_neg_fp64(double y, double *ex) {
 #else
     const double th0 = h_exp2_rows[j].hi, tl0 = h_exp2_rows[j].lo;
 #endif
-    // times 2^-(n / 64), by the exponents; the low part of row 0 is 0
-    const uint64_t sh = (uint64_t)((ni >> 6) & 0x3FFu) << 52;
+    // times 2^-(n / 64), by the exponents, what is beyond 2^-512 at the end; the
+    // low part of row 0 is 0
+    const uint32_t k = ni >> 6, k1 = k < 512u ? k : 512u;
+    const uint64_t sh = (uint64_t)k1 << 52;
     const double th = from_bits(bits(th0) - sh), tl = j ? from_bits(bits(tl0) - sh) : 0.0;
-    const double low = fma(th, p, tl);
-    *ex = th + low;
-    return (th - 1.0) + low;
+    double e = th + fma(th, p, tl);
+    if (k > 512u) e *= from_bits((uint64_t)(1023u - (k - 512u)) << 52);
+    *ex = e;
+    return e - 1.0;
 }
 
 // exp(-y) - 1, 0 <= y < 1, in fixed point; where it is -1/2 or below, *ex is
@@ -579,11 +582,11 @@ IMC_HD double expm1_neg_fixed(double y, double *ex) {
     return -fixed_to_double(v, 64);
 }
 
-// exp(-y) - 1, y >= 0 (NaN gives NaN); beyond 600 it is -1 to the last bit
+// exp(-y) - 1, y >= 0 (NaN gives NaN); from 760 on exp(-y) rounds to 0
 IMC_HD double expm1_neg(double y) {
     double ex;
     if (hi32(y) < 0x3FF00000u) return expm1_neg_fixed(y, &ex);
-    return expm1_neg_fp64(y > 600.0 ? 600.0 : y, &ex);
+    return y == y ? expm1_neg_fp64(y > 760.0 ? 760.0 : y, &ex) : y;
 }
 
 // E exp(-y), the weight E after a path of y mean free paths of absorption, and
@@ -591,23 +594,19 @@ IMC_HD double expm1_neg(double y) {
 // would cancel, an error of em1 growing e^y times in the weight (50 units in
 // the last place at the 1 % cut-off), and the weight is E exp(-y): one
 // fused multiply-add either way.  A negative y (a path past the census time by a
-// rounding, a negative opacity), 600 and beyond, and NaN take the general functions.
-// (The ranges are told apart once, here: with the general functions from 64 on
-// and the tests inside each function, the FP64 channel's walls cost 10.76 ms
-// against 10.57, the FP64 heat wave 46.5 against 44.6.)
+// rounding, a negative opacity) and NaN take CUDA's expm1, whose sum with 1
+// cancels nothing.  (FP64 heat waves of 60,000 and 200,000 histories 45.0 and 46.7
+// ms, the 98 x 28 channel 10.36 ms; with E + E em1 throughout 46.1, 45.3 and
+// 10.26; with CUDA's exp in the kernel for what lies beyond the table's range
+// 48.4, 46.2 and 10.45.)
 IMC_HD double attenuate(double E, double y, double *em1) {
     const uint32_t yh = hi32(y);
     double ex = 0.0, m;
-    if (yh < 0x3FF00000u) {
-        m = expm1_neg_fixed(y, &ex);
-    } else if (yh < 0x4082C000u) {
-        m = expm1_neg_fp64(y, &ex);
-    } else {
-        m = expm1(-y);
-        ex = exp(-y);
-    }
+    if (yh < 0x3FF00000u) m = expm1_neg_fixed(y, &ex);
+    else if (yh <= 0x7FF00000u) m = expm1_neg_fp64(yh < 0x4087C000u ? y : 760.0, &ex);
+    else m = expm1(-y);
     *em1 = m;
-    const bool thick = yh >= 0x3FF00000u || bits(ex) != 0;
+    const bool thick = (yh >= 0x3FF00000u && yh <= 0x7FF00000u) || bits(ex) != 0;
     return fma(E, thick ? ex : m, thick ? 0.0 : E);
 }
 
