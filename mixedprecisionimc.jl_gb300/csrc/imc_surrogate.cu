@@ -421,7 +421,8 @@ template <int LEFT> __device__ __forceinline__ void copies_arrived() { asm volat
 // output each, the serial sums beside them: cross entropy, bias gradients, loss.
 // The weights of a layer arrive while the layer before it runs.  (With the sums
 // after the products on the same threads, the first layer's gradients on 16
-// threads and the weights waited for at the start: 33.5 us against 30.6.)
+// threads and the weights waited for at the start: 33.5 us against 30.6; the
+// barriers at block scope, which both roles share, add 0.4.)
 __global__ void __launch_bounds__(kTrainThreads) k_surr_grad(const float *P, const float *x, const int *cls,
                                                              const float *tgt, long long n, long long off,
                                                              float *gpart, float *lpart) {
